@@ -107,8 +107,9 @@ _SIGNATURES = {
                             _c_int, _c_void_p, _c_void_p, _c_void_p],
     "bg_attention_tc_sink": [_c_void_p, _c_int, _c_void_p, _c_int, _c_int, _c_void_p, _c_int, _c_void_p, _c_void_p, _c_int,
                              _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_float, _c_int, _c_void_p, _c_void_p],
+    "bg_gemm_f32_scratch": [_c_int, _c_int, _c_int, _c_int],
     "bg_gemm_f32_nt": [_c_void_p, _c_int, _c_void_p, _c_int, _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int,
-                       _c_int, _c_void_p],
+                       _c_int, _c_void_p, _c_void_p],
     "bg_gemm_bf16_tn": [_c_void_p, _c_int, _c_int, _c_int, _c_void_p, _c_int, _c_int, _c_void_p, _c_void_p, _c_int,
                         _c_int, _c_int, _c_void_p, _c_void_p],
     "bg_gemm_pair": [_c_void_p, _c_int, _c_int, _c_int, _c_void_p, _c_int, _c_int, _c_void_p, _c_void_p, _c_int, _c_int,
@@ -158,11 +159,13 @@ _SIGNATURES = {
     "bg_gated_group_rmsnorm": [_c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_void_p, _c_int, _c_float, _c_void_p, _c_int,
                                _c_int, _c_int, _c_int, _c_int, _c_void_p],
     "bg_gemm_f32_nt_batched": [_c_void_p, _c_int, _c_ll, _c_void_p, _c_int, _c_ll, _c_void_p, _c_int, _c_ll, _c_int, _c_int,
-                               _c_int, _c_int, _c_void_p],
+                               _c_int, _c_int, _c_void_p, _c_void_p],
     "bg_sample": [_c_void_p, _c_int, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p],
     "bg_sample_feed": [_c_void_p, _c_int, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p,
                        _c_void_p],
 }
+
+_RESULTS = {"bg_gemm_f32_scratch": _c_ll}         # what does not return a code
 
 _lib = None
 
@@ -181,7 +184,7 @@ def lib():
             except AttributeError as e:
                 raise KernelError(f"the kernel library lacks '{name}'") from e
             fn.argtypes = argtypes
-            fn.restype = _c_int
+            fn.restype = _RESULTS.get(name, _c_int)
         _lib = handle
     return _lib
 
@@ -818,8 +821,15 @@ def gemm_f32_nt(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], 
         raise KernelError(f"gemm_f32_nt: shapes a{tuple(a.shape)} w{tuple(w.shape)} out{tuple(out.shape)} do not fit")
     if bias is not None and (bias.numel() != N or not bias.is_contiguous()):
         raise KernelError("gemm_f32_nt: bias must have one value per output feature")
+    scratch = _gemm_f32_scratch(M, N, K, 1, out.device)
     _check(lib().bg_gemm_f32_nt(_p(a), a.stride(0), _p(w), w.stride(0), _p(bias), _p(out), out.stride(0), M, N, K,
-                                1 if accumulate else 0, _stream()), "gemm_f32_nt")
+                                1 if accumulate else 0, _p(scratch), _stream()), "gemm_f32_nt")
+
+
+def _gemm_f32_scratch(M: int, N: int, K: int, batch: int, device) -> Optional[torch.Tensor]:
+    """Room for the sums of the ranges of K, where the float32 product cuts it."""
+    n = lib().bg_gemm_f32_scratch(M, N, K, batch)
+    return torch.empty((n,), dtype=torch.float32, device=device) if n > 0 else None
 
 
 def gemm_bf16_tn(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], out: torch.Tensor,
@@ -1157,8 +1167,9 @@ def gemm_f32_nt_batched(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> 
     N = w.shape[1]
     if w.shape[0] != B or w.shape[2] != K or tuple(out.shape) != (B, M, N):
         raise KernelError(f"gemm_f32_nt_batched: shapes a{tuple(a.shape)} w{tuple(w.shape)} out{tuple(out.shape)} do not fit")
+    scratch = _gemm_f32_scratch(M, N, K, B, out.device)
     _check(lib().bg_gemm_f32_nt_batched(_p(a), a.stride(1), a.stride(0), _p(w), w.stride(1), w.stride(0), _p(out),
-                                        out.stride(1), out.stride(0), B, M, N, K, _stream()), "gemm_f32_nt_batched")
+                                        out.stride(1), out.stride(0), B, M, N, K, _p(scratch), _stream()), "gemm_f32_nt_batched")
 
 
 # ------------------------------------------------------------------------------------------------

@@ -161,6 +161,36 @@ def test_gemm_f32_is_true_float_and_row_invariant(ops):
     assert (acc.double() - (2 * want - b.double())).abs().max() < 1e-4
 
 
+@pytest.mark.parametrize("K", [4, 60, 301, 1020, 1024, 1028, 6200])       # one range of k and several, whole and not, odd
+@pytest.mark.parametrize("N", [1, 15, 130, 700])
+def test_gemm_f32_kernels_agree_bit_for_bit(ops, N, K):
+    """The kernels of few and of many rows, with ranges of k in one CTA and in CTAs of their own: every row the same bits."""
+    a, w, b = rnd(400, K, seed=6), rnd(N, K, seed=7), rnd(N, seed=8)
+    want = a.double() @ w.double().t() + b.double()
+    bound = (K + 8) * 2.0 ** -24 * (a.abs().double() @ w.abs().double().t() + b.abs().double())    # a chain of K rounded sums
+    rows = None
+    for M in (400, 129, 65, 64, 17, 16, 9, 8, 3, 1):
+        out = torch.empty((M, N), device=DEV)
+        ops.gemm_f32_nt(a[:M], w, b, out)
+        assert bool(((out.double() - want[:M]).abs() <= bound[:M]).all())
+        rows = out if rows is None else rows
+        assert torch.equal(out, rows[:M]), M
+    acc = rows[:40].clone()
+    ops.gemm_f32_nt(a[:40], w, b, acc, accumulate=True)
+    assert torch.equal(acc, rows[:40] + rows[:40])
+    # a batch of products, through views whose rows lie apart
+    wide = torch.zeros((3, 20, K + 4), device=DEV)
+    wide[:, :, :K] = a[:60].view(3, 20, K)
+    ws = torch.stack([w, 2 * w, -w])
+    for M in (20, 5):
+        out = torch.empty((3, M, N), device=DEV)
+        ops.gemm_f32_nt_batched(wide[:, :M, :K], ws, out)
+        for e, f in enumerate((1.0, 2.0, -1.0)):
+            plain = torch.empty((M, N), device=DEV)
+            ops.gemm_f32_nt(wide[e, :M, :K], w, None, plain)
+            assert torch.equal(out[e], f * plain)
+
+
 @pytest.mark.parametrize("interleaved", [False, True])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("hd,rot", [(48, 32), (64, 64), (128, 128)])      # partial rotary; whole heads (16-byte path)
