@@ -24,6 +24,7 @@
 // query.  With `keep` k > 0 a window never loses the sequence's first k positions: a query at `pos` sees t <= pos with
 // t >= first_visible(pos, window) or t < k, the tiles and splits between the two ranges being passed over.
 #include "common.cuh"
+#include "attention_f32.cuh"
 
 namespace bg {
 
@@ -317,11 +318,18 @@ static size_t attention_smem_bytes(int bq, int group, int hd, int vd, int tile) 
     return floats * sizeof(float) + (size_t)2 * tile * sizeof(long long) + 16;
 }
 
+// Whether attention_f32_kernel takes blocks of `rows` rows of these sizes: whole 16-byte pieces of queries, keys and values, and tiles
+// that fit a CTA.
+static bool attention_f32_takes(int rows, int hd, int vd, int maps) {
+    return rows <= AF_ROWS && hd % (4 * maps) == 0 && vd % 4 == 0 && vd <= 256 && af_smem(hd / maps, hd, vd) <= 226 * 1024;
+}
+
 // Rows per query block and keys per tile that fit the shared memory of one CTA for these sizes.
 // Returns 0 and fills bq and tile, or BG_ERR_UNSUPPORTED.
-// (`hd` counts a whole key row; with two maps in it, it may be twice as wide)
-extern "C" int bg_attention_plan(int group, int hd, int vd, int maps, int* bq_out, int* tile_out) {
+// (`hd` counts a whole key row; with two maps in it, it may be twice as wide; `f32`: float queries over a float cache)
+extern "C" int bg_attention_plan(int group, int hd, int vd, int maps, int f32, int* bq_out, int* tile_out) {
     if (maps < 1 || hd <= 0 || hd > 32 * ATT_MAX_DPL * maps || vd <= 0 || vd > 32 * ATT_MAX_DPL || group <= 0) return BG_ERR_UNSUPPORTED;
+    if (f32 && attention_f32_takes(group, hd, vd, maps)) { *bq_out = AF_ROWS / group; *tile_out = AF_KEYS; return BG_OK; }
     const size_t limit = 200 * 1024;
     for (int tile = 64; tile >= 32; tile >>= 1) {
         for (int bq = 16; bq >= 1; bq >>= 1) {
@@ -347,9 +355,27 @@ extern "C" int bg_attention_partial(const void* q, int q_dtype, int q_stride, co
     p.part_o = part_o; p.part_ml = part_ml; p.max_splits = max_splits; p.nh = nh; p.nkv = nkv; p.hd = hd; p.vd = vd;
     p.group = nh / nkv; p.window = window; p.split = split; p.tile = tile; p.bq = bq; p.scale = scale; p.softcap = softcap; p.status = status;
     p.keep = keep; p.slopes = slopes; p.maps = maps;
+    dim3 grid(n_qblk, nkv, n_splits_launch);
+    if (q_dtype == BG_DTYPE_F32 && cache_dtype == BG_DTYPE_F32 && bq * p.group <= AF_ROWS && attention_f32_takes(p.group, hd, vd, maps) &&
+        split % AF_KEYS == 0 && q_stride % 4 == 0 && (uintptr_t)q % 16 == 0 && (uintptr_t)kv_pool % 16 == 0 && (uintptr_t)part_o % 16 == 0) {
+        const size_t need = af_smem(hd / maps, hd, vd);
+#define BG_AF_LAUNCH(NC)                                                                                                    \
+        do {                                                                                                                \
+            auto kern = attention_f32_kernel<AttnParams, NC>;                                                               \
+            cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)need);             \
+            if (e != cudaSuccess) return (int)e;                                                                            \
+            launch(kern, grid, dim3(AF_THREADS), need, stream, p);                                                          \
+        } while (0)
+        if (vd <= 64) BG_AF_LAUNCH(1);
+        else if (vd <= 128) BG_AF_LAUNCH(2);
+        else if (vd <= 192) BG_AF_LAUNCH(3);
+        else BG_AF_LAUNCH(4);
+#undef BG_AF_LAUNCH
+        BG_LAUNCH_CHECK();
+        return BG_OK;
+    }
     size_t smem = attention_smem_bytes(bq, p.group, hd, vd, tile);
     if (smem > 227 * 1024) return BG_ERR_UNSUPPORTED;
-    dim3 grid(n_qblk, nkv, n_splits_launch);
 #define BG_ATT_LAUNCH(TQ, TC)                                                                              \
     do {                                                                                                   \
         auto kern = attention_partial_kernel<TQ, TC>;                                                      \

@@ -33,7 +33,7 @@ _SIGNATURES = {
     "bg_rope_kv_append": [_c_void_p, _c_int, _c_int, _c_int, _c_ll, _c_void_p, _c_int, _c_int, _c_void_p, _c_void_p,
                           _c_void_p, _c_void_p, _c_int, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int,
                           _c_int, _c_int, _c_int, _c_void_p, _c_void_p],
-    "bg_attention_plan": [_c_int, _c_int, _c_int, _c_int, ctypes.POINTER(_c_int), ctypes.POINTER(_c_int)],
+    "bg_attention_plan": [_c_int, _c_int, _c_int, _c_int, _c_int, ctypes.POINTER(_c_int), ctypes.POINTER(_c_int)],
     "bg_attention_partial": [_c_void_p, _c_int, _c_int, _c_void_p, _c_int, _c_int, _c_int, _c_void_p, _c_int,
                              _c_void_p, _c_void_p, _c_int, _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int,
                              _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_float, _c_float, _c_int, _c_void_p, _c_int,
@@ -566,7 +566,7 @@ def attention_plan(group: int, hd: int, dtype: torch.dtype = torch.float32, deco
             raise KernelError(f"the tensor-core attention kernel does not take head_dim {hd} with {group} query "
                               "heads per kv head (head_dim 64 or 128; at most 64 heads per kv head)")
     bq, tile = _c_int(0), _c_int(0)
-    rc = L.bg_attention_plan(group, hd, vd, 1, ctypes.byref(bq), ctypes.byref(tile))
+    rc = L.bg_attention_plan(group, hd, vd, 1, 1 if dtype == torch.float32 else 0, ctypes.byref(bq), ctypes.byref(tile))
     if rc != 0:
         raise KernelError(f"attention: head_dim {hd} (values of {vd}) with {group} query heads per kv head is not "
                           "supported (both sizes must be at most 256)")
@@ -741,7 +741,7 @@ def difference_plan(group: int, kw: int, vw: int, dtype: torch.dtype, decode_onl
                 return "mma_keys", bq.value, 64
         elif prefer in TC_ROWS_FOR and L.bg_attention_tc_plan(group, vw, page_size, ctypes.byref(bq)) == 0:
             return "tc_rows", bq.value, 64
-    if L.bg_attention_plan(2 * group, 2 * kw, vw, 2, ctypes.byref(bq), ctypes.byref(tile)) != 0:
+    if L.bg_attention_plan(2 * group, 2 * kw, vw, 2, 1 if dtype == torch.float32 else 0, ctypes.byref(bq), ctypes.byref(tile)) != 0:
         raise KernelError(f"differential attention: maps of {kw} features (values of {vw}) with {group} query heads per kv head are not "
                           "supported (both sizes must be at most 256)")
     return "generic", bq.value, tile.value

@@ -379,6 +379,49 @@ def test_attention_float32(ops, nh, nkv, hd, page):
     assert (got - want).abs().max() < 1e-5 * max(1.0, float(want.abs().max()))
 
 
+@pytest.mark.parametrize("nh,nkv,hd,vd,options", [(6, 1, 128, 128, {}), (1, 1, 4, 12, {}), (32, 1, 64, 64, {"window": 50}), (10, 2, 36, 132, {}),
+                                                  (64, 1, 32, 64, {}), (65, 1, 32, 32, {}), (3, 3, 256, 256, {"softcap": 5.0}), (4, 2, 30, 30, {}),
+                                                  (8, 4, 64, 192, {"window": 40, "keep": 3, "slopes": True})])
+def test_attention_float32_in_blocks_of_any_rows(ops, nh, nkv, hd, vd, options):
+    """Float attention for sizes on both sides of what the kernel in blocks of registers takes: the blocks that the plan asks for, single
+    rows and blocks in between give the same bits, and the values of a plain softmax in 64 bits."""
+    page, held, n = 16, 131, 70
+    total, group = held + n, nh // nkv
+    window, keep, cap = options.get("window", 0), options.get("keep", 0), options.get("softcap", 0.0)
+    q, k, v = rnd(n, nh, hd, seed=1), rnd(total, nkv, hd, seed=2), rnd(total, nkv, vd, seed=3)
+    slopes = torch.linspace(0.01, 0.2, nh, device=DEV) if options.get("slopes") else None
+    pages = -(-total // page)
+    pool = torch.full((pages + 1, nkv * page * (hd + vd)), float("nan"), device=DEV)
+    pad = lambda t: torch.cat([t, torch.full((pages * page - total,) + t.shape[1:], float("nan"), device=DEV)]).view(pages, page, nkv, -1)
+    table = torch.arange(pages - 1, -1, -1, dtype=torch.int32, device=DEV).view(1, -1)
+    pool[table[0].long()] = torch.cat([pad(k).transpose(1, 2).reshape(pages, -1), pad(v).transpose(1, 2).reshape(pages, -1)], dim=1)
+    if vd == hd:
+        pool = pool.view(pages + 1, 2, nkv, page, hd)
+    positions = torch.arange(held, total, dtype=torch.int32, device=DEV)
+    status = ops.new_status(DEV)
+    _, bq, tile = ops.attention_plan(group, hd, torch.float32, False, "generic", page, vd=vd)
+    outs = []
+    for cut in sorted({bq, 1, max(1, bq // 3)}):
+        qblk = torch.tensor([(0, b, min(cut, n - b)) for b in range(0, n, cut)], dtype=torch.int32, device=DEV)
+        out = torch.full((n, nh * vd), float("nan"), device=DEV)
+        ops.attention(q.view(n, -1), nh * hd, pool, table, positions, qblk, qblk.shape[0], total - 1, n, nh, nkv, hd, window, 64, tile, bq,
+                      hd ** -0.5, out, status, "generic", vd=vd, softcap=cap, keep=keep, slopes=slopes)
+        outs.append(out)
+    ops.raise_on_status(status)
+    assert all(torch.equal(outs[0], o) for o in outs[1:])
+    at, key = positions.long()[:, None], torch.arange(total, device=DEV)[None, :]
+    seen = (key <= at) & ((key > at - window) | (key < keep) if window else key >= 0)
+    s = torch.einsum("thd,shd->hts", q.double(), k.double().repeat_interleave(group, 1)) * hd ** -0.5
+    if cap:
+        s = cap * torch.tanh(s / cap)
+    if slopes is not None:
+        s = s - slopes.double()[:, None, None] * (at - key)
+    want = torch.einsum("hts,shd->thd", torch.softmax(s.masked_fill(~seen, -math.inf), -1), v.double().repeat_interleave(group, 1)).reshape(n, -1)
+    # a score's rounding (a chain of hd products, |q||k| at most, and the exponent's) moves a weight by as much, relatively
+    bound = (hd + 16) * 2.0 ** -24 * float((q.abs().sum(-1).max() * k.abs().max() * hd ** -0.5).double() + 4) * float(v.abs().max())
+    assert float((outs[0].double() - want).abs().max()) < bound
+
+
 @pytest.mark.parametrize("nh,nkv,hd,page,window", [(4, 2, 16, 8, 10), (12, 2, 128, 16, 64), (5, 5, 48, 16, 1),
                                                    (3, 1, 32, 16, 100)])
 def test_attention_window(ops, nh, nkv, hd, page, window):
