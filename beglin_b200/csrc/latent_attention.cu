@@ -15,6 +15,7 @@
 // Everything is float, and a row shares no accumulator with another row, so a row's result does not
 // depend on how the step was cut or on what else is in the batch.
 #include "common.cuh"
+#include "latent_range.cuh"
 
 namespace bg {
 
@@ -362,8 +363,9 @@ latent_attention_merge_kernel(const float* __restrict__ part_o, const float* __r
     pdl_wait();
     const int w = blockIdx.x;
     const int t = w / H, h = w - t * H;
-    const int s_hi = positions[t] / split;
-    const int s_lo = first_visible(positions[t], window) / split;
+    const int pos = positions[t], lo = first_visible(pos, window);
+    // splits at absolute positions, or (split 0) ranges that follow the row's own keys
+    const int s_lo = split > 0 ? lo / split : 0, s_hi = split > 0 ? pos / split : latent_range(pos, lo, max_splits).count - 1;
     const size_t prow = (size_t)w * max_splits;
     const int lane = threadIdx.x & 31;
     if (threadIdx.x < 32) {

@@ -144,6 +144,10 @@ _SIGNATURES = {
                                         _c_int, _c_void_p, _c_int, _c_void_p, _c_void_p, _c_int, _c_void_p, _c_void_p, _c_int,
                                         _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_float,
                                         _c_void_p, _c_void_p],
+    "bg_latent_attention_tc_plan": [_c_int, _c_int, _c_int, _c_int],
+    "bg_latent_attention_tc_partial": [_c_void_p, _c_ll, _c_int, _c_void_p, _c_int, _c_int, _c_int, _c_void_p, _c_void_p, _c_int, _c_int,
+                                       _c_void_p, _c_int, _c_void_p, _c_void_p, _c_int, _c_void_p, _c_void_p, _c_int, _c_int, _c_int,
+                                       _c_int, _c_int, _c_int, _c_float, _c_void_p, _c_void_p],
     "bg_latent_gather": [_c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void_p, _c_void_p,
                          _c_void_p],
     "bg_latent_expand": [_c_void_p, _c_int, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_void_p, _c_void_p],
@@ -1228,6 +1232,24 @@ def latent_append(src: torch.Tensor, col0: int, rank: int, rot: int, rot_dims: i
                "latent_append")
 
 
+LATENT_TC_KEYS = 128          # keys of a tile of the tcgen05 kernel
+
+
+def latent_splits(rows: int, keys: int, sms: Optional[int] = None) -> int:
+    """How many CTAs share a row's keys in the tcgen05 kernel, for `rows` rows (times chunks of heads) of up to `keys` keys: the
+    number that makes the waves of one CTA an SM shortest, a CTA's start, queries and results counted as three tiles of keys.  (64 rows of
+    4,000 keys, in 1, 2, 3, 4, 6 and 9 ranges: 169, 103, 140, 120, 141, 157 us; the rule takes 2.)"""
+    sms = sm_count() if sms is None else sms
+    tiles = -(-keys // LATENT_TC_KEYS)
+    best, best_cost = 1, None
+    for s in range(1, min(tiles, 64) + 1):
+        per = -(-tiles // s)
+        cost = -(-rows * -(-tiles // per) // sms) * (per + 3)
+        if best_cost is None or cost < best_cost:
+            best, best_cost = s, cost
+    return best
+
+
 def latent_attention(q_lat: torch.Tensor, q_raw: torch.Tensor, dim: int, rot: int, rot_dims: int,
                      cos_sin: Optional[torch.Tensor], pool: torch.Tensor, block_table: torch.Tensor,
                      positions: torch.Tensor, qblk: torch.Tensor, n_qblk: int, max_position: int, bq: int, hc: int,
@@ -1238,7 +1260,8 @@ def latent_attention(q_lat: torch.Tensor, q_raw: torch.Tensor, dim: int, rot: in
     [pages, page_size, rank + rot]; out [H, T, rank] receives, per head, the softmax-weighted sum of the cached
     latents.  `qblk` is cut for `bq` rows; a CTA takes `hc` heads; keys are cut into splits of `split` positions.
     With `mma_stages` 1 or 2 the products run on the tensor cores (bfloat16 q_raw and pool, bq * hc at most 64, sizes as
-    `latent_attention_mma_plan` says); else on the CUDA cores in float, for every size and type.  `window` w > 0: a row
+    `latent_attention_mma_plan` says; blocks of one row on tcgen05, which spreads a row's own keys over the SMs, where rank is a
+    multiple of 64, rot of 8 up to 64 and a page of 64 positions); else on the CUDA cores in float, for every size and type.  `window` w > 0: a row
     sees itself and the w - 1 positions before it.  `sink_weight` (float32 [H]): the softmax's denominator also holds exp of the
     head's number."""
     if sink_weight is not None and (sink_weight.dtype != torch.float32 or sink_weight.numel() != q_lat.shape[0] or not sink_weight.is_contiguous()):
@@ -1255,12 +1278,26 @@ def latent_attention(q_lat: torch.Tensor, q_raw: torch.Tensor, dim: int, rot: in
     if rot_dims > 0 and (cos_sin is None or cos_sin.dtype != torch.float32 or cos_sin.shape[0] < T
                          or cos_sin.shape[1] != rot_dims // 2 or not cos_sin.is_contiguous()):
         raise KernelError("latent_attention: cos_sin must be float32 [T, rot_dims/2, 2]")
-    n_splits = max_position // split + 1
+    L = lib()
+    # one row per block (decoding) on tcgen05 where it takes the sizes: a row's own keys spread over the SMs
+    tc = bool(mma_stages) and bq == 1 and q_raw.dtype == pool.dtype == torch.bfloat16 \
+        and q_lat.stride(0) % 4 == 0 and q_lat.stride(1) % 4 == 0 and q_lat.data_ptr() % 16 == 0 and pool.data_ptr() % 16 == 0 \
+        and L.bg_latent_attention_tc_plan(H, rank, rot, pool.shape[1]) == 0
+    if tc:
+        keys = min(max_position + 1, window + LATENT_TC_KEYS) if window > 0 else max_position + 1
+        split, n_splits = 0, latent_splits(n_qblk * -(-H // 32), keys)
+    else:
+        n_splits = max_position // split + 1
     part_o = torch.empty((T * H * n_splits, rank), dtype=torch.float32, device=q_lat.device)
     part_ml = torch.empty((T * H * n_splits, 2), dtype=torch.float32, device=q_lat.device)
-    L = lib()
     with phase("attn"):
-        if mma_stages:
+        if tc:
+            _check(L.bg_latent_attention_tc_partial(_p(q_lat), q_lat.stride(0), q_lat.stride(1), _p(q_raw), q_raw.stride(0), dim + rot, dim,
+                                                    _p(cos_sin), _p(pool), pool.shape[0], pool.shape[1], _p(block_table),
+                                                    block_table.shape[1], _p(positions), _p(qblk), n_qblk, _p(part_o), _p(part_ml), n_splits,
+                                                    H, rank, rot, rot_dims, int(window), float(scale), _p(status), _stream()),
+                   "latent_attention_tc_partial")
+        elif mma_stages:
             if q_raw.dtype != torch.bfloat16 or pool.dtype != torch.bfloat16:
                 raise KernelError("latent_attention: the tensor-core kernel takes bfloat16 query rows and caches")
             _check(L.bg_latent_attention_mma_partial(_p(q_lat), q_lat.stride(0), q_lat.stride(1), _p(q_raw), q_raw.stride(0),

@@ -452,6 +452,61 @@ def test_latent_attention_over_many_tiles(case, kernel, sinks):
     assert rel_err(out, want) < (2e-5 if kernel == "float" else 2e-2)
 
 
+LATENT_DECODING = [  # heads, latent, rotated part, turning features, page, window, positions of the requests' tokens
+    (32, 512, 64, 64, 64, 0, [0, 1, 63, 64, 127, 128, 129, 2300]), (16, 64, 8, 0, 64, 0, [700, 5]), (1, 320, 0, 0, 128, 0, [1023, 1024]),
+    (17, 448, 64, 32, 64, 200, [199, 200, 201, 1500]), (40, 256, 32, 32, 192, 0, [600] * 9), (12, 384, 64, 64, 64, 64, [5000, 63, 64]),
+    (20, 128, 0, 0, 64, 0, [3] * 200),
+]
+
+
+@pytest.mark.parametrize("case", LATENT_DECODING, ids=["-".join(map(str, c[:6])) for c in LATENT_DECODING])
+def test_latent_attention_decoding_on_tcgen05(case):
+    """Single tokens of requests of unequal lengths, from one key to many tiles and ranges of them: heads that fill the kernel's sixteen
+    or thirty-two or do not, latents of an odd number of blocks, windows that begin in the middle of a tile; NaN in all that may not be
+    read.  A key that stands out in every 50 positions shows a tile that is taken twice or left out."""
+    H, rank, rot, dims, page, window, at = case
+    o = ops()
+    assert o.lib().bg_latent_attention_tc_plan(H, rank, rot, page) == 0
+    g = torch.Generator().manual_seed(sum(at) + H)
+    width, T = rank + rot, len(at)
+    q_lat = torch.randn(H, T, rank, generator=g)
+    q_raw = torch.randn(T, H * (8 + rot), generator=g).to(torch.bfloat16)
+    angle = torch.rand(T, max(dims, 2) // 2, generator=g) * 6.0
+    cos_sin = torch.stack([angle.cos(), angle.sin()], -1)
+    turned = q_raw.view(T, H, 8 + rot)[:, :, 8:].float().clone()
+    if dims:
+        a, b = turned[..., 0:dims:2].clone(), turned[..., 1:dims:2].clone()
+        turned[..., 0:dims:2] = a * cos_sin[:, None, :, 0] - b * cos_sin[:, None, :, 1]
+        turned[..., 1:dims:2] = b * cos_sin[:, None, :, 0] + a * cos_sin[:, None, :, 1]
+    full = torch.cat([q_lat.transpose(0, 1), turned], -1)                                     # [T, H, width]
+    per = [-(-(p + 1) // page) for p in at]
+    pool = torch.full((sum(per) + 1, page, width), NAN).to(torch.bfloat16)
+    table = torch.full((T, max(per) + 1), -1, dtype=torch.int32)
+    order = iter(torch.randperm(sum(per) + 1, generator=g).tolist())
+    sink = 2.0 * torch.randn(H, generator=g)
+    scale = 2.0 / math.sqrt(width)
+    want = torch.zeros(H, T, rank, dtype=torch.float64)
+    for r, p in enumerate(at):
+        rows = torch.randn(p + 1, width, generator=g).to(torch.bfloat16)
+        for j in range(7, p + 1, 50):
+            rows[j] = (1.5 * full[r, j % H] * math.sqrt(width) / full[r, j % H].norm()).to(torch.bfloat16)
+        lo = max(0, p - window + 1) if window else 0
+        for i in range(per[r]):
+            if (i + 1) * page > lo:
+                table[r, i] = next(order)
+                n = min(page, p + 1 - i * page)
+                pool[table[r, i], :n] = rows[i * page:i * page + n]
+        s = torch.cat([(rows[lo:].double() @ full[r].double().T) * scale, sink.double()[None]])
+        want[:, r] = (torch.softmax(s, 0)[:-1].T @ rows[lo:, :rank].double())
+    status = o.new_status(DEV)
+    out = torch.full((H, T, rank), NAN, dtype=torch.bfloat16, device=DEV)
+    qblk = i32([[r, r, 1] for r in range(T)])
+    o.latent_attention(dev(q_lat), dev(q_raw), 8, rot, dims, dev(cos_sin) if dims else None, dev(pool), dev(table), i32(at), qblk, T, max(at),
+                       1, min(H, 32), 64, 256, scale, out, status, mma_stages=1, window=window, sink_weight=dev(sink))
+    o.raise_on_status(status)
+    assert rel_err(out, want) < 2e-2
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 @pytest.mark.parametrize("dim,rank", [(64, 64), (24, 40)])
 def test_a_key_inside_and_outside_the_window_and_the_sink(tmp_path, dtype, dim, rank):
