@@ -11,8 +11,10 @@ the cache manager's slab, float32, zero when the request starts): a step continu
 slot, however the request's tokens are cut into steps and whatever else the step holds.  Everything that
 enters the recurrence is float in both number formats.
 
-With the spec's `chunked`, a request that brings `LONG_FROM` rows or more runs in chunks (the chunks' own sums and outputs side
-by side, a short pass over their states between), where the sizes allow it; fewer rows, and single tokens, are walked one by one.
+A request that brings `LONG_FROM` rows or more runs in chunks (the chunks' own sums and outputs side by side, a short pass over their
+states between), where the sizes allow it, in bfloat16 and with the spec's `chunked`; fewer rows, and single tokens, are walked one by
+one.  In float32 without `chunked` all rows are walked: ways of cutting a prompt then agree bit for bit, which chunks cannot keep and
+bfloat16 steps, whose products change with the number of rows, do not promise.
 """
 from __future__ import annotations
 
@@ -76,9 +78,14 @@ class Mamba2:
         self.dt_bias, self.A_log, self.D = same(tensors["dt_bias"]), same(tensors["A_log"]), same(tensors["D"])
         self.norm_w = ctx.vector(tensors["norm.weight"])
         self.conv_off = spec.n_heads * spec.state * spec.vdim
-        self.chunk = ops.ssm_chunk(spec.n_heads, spec.vdim, spec.state, spec.groups) if spec.chunked and ctx.device.type == "cuda" else 0
+        chunked = spec.chunked or ctx.compute_dtype == torch.bfloat16
+        self.chunk = ops.ssm_chunk(spec.n_heads, spec.vdim, spec.state, spec.groups) if chunked and ctx.device.type == "cuda" else 0
+        # rows whose chunks' states still fit CHUNK_BYTES; a longer step of a spec that does not ask for chunks is walked
+        self.most_rows = None if spec.chunked or not self.chunk else self.CHUNK_BYTES // (4 * self.conv_off) * self.chunk
 
-    LONG_FROM = 64             # rows of a request in a step from which its tokens run in chunks
+    LONG_FROM = 64             # rows of a request in a step from which its tokens run in chunks (2,048 rows of 24 heads of 128 x 128:
+    #                            989 us for the whole mixer walked row by row, 308 in chunks)
+    CHUNK_BYTES = 1 << 28
     takes_stream = True        # forward takes a NormedInput and may add its result to the stream itself
 
     def forward(self, h, batch, cache: FixedStateView, stream: Optional[ResidualStream] = None) -> Optional[torch.Tensor]:
@@ -95,7 +102,7 @@ class Mamba2:
                       batch.row_req, reqs, n_req, xbc)
         y = torch.empty((T, self.inner), dtype=torch.float32, device=h.device)
         chunks, n_chunks, longs, n_long = None, 0, None, 0
-        if self.chunk and not batch.decode_only and hasattr(batch, "long_blocks"):
+        if self.chunk and not batch.decode_only and hasattr(batch, "long_blocks") and (self.most_rows is None or T <= self.most_rows):
             reqs, n_req, chunks, n_chunks, longs, n_long = batch.long_blocks(self.chunk, self.LONG_FROM)
         ops.ssm_scan(xbc, proj, self.inner + self.channels, self.dt_bias, self.A_log, self.D, cache.state, cache.slots,
                      reqs, n_req, y, s.n_heads, s.vdim, s.state, s.groups, chunks, n_chunks, longs, n_long)
