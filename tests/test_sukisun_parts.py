@@ -270,6 +270,29 @@ def test_mamba2_long_portions_in_bfloat16(heads, vdim, state, groups):
             assert rel_err(torch.cat(outs[r]), plain.mamba2(hs[r].double(), plain_names(t, "l."), "l.", m, 1e-5)) < 3e-2, (r, most_rows)
 
 
+@pytest.mark.parametrize("taps", [2, 3, 4])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_convolution_in_runs_of_rows(taps, dtype):
+    """Runs of eight rows that begin, end and lie inside requests (one row, fewer than the taps, many), 16-byte rows against the same rows
+    an odd number of floats apart: the same bits, and the same state behind them."""
+    from beglin_b200.csrc import ops
+    lens, channels, col, off = [1, 2, 30, 3, 1, 8, 9, 64], 516, 8, 4
+    T, first = sum(lens), [sum(lens[:i]) for i in range(len(lens))]
+    i32 = lambda a: torch.tensor(a, dtype=torch.int32, device=DEV)
+    row_req, reqs = i32([r for r, n in enumerate(lens) for _ in range(n)]), i32([[r, f, n] for r, (f, n) in enumerate(zip(first, lens))])
+    x, w, b = rnd(T, channels, seed=1).to(DEV), rnd(channels, taps, seed=2).to(DEV, dtype), rnd(channels, seed=3).to(DEV, dtype)
+    state0, slots = rnd(len(lens) + 2, off + (taps - 1) * channels, seed=4).to(DEV), i32([9, 3, 0, 5, 1, 8, 2, 7])
+    for activation, src_bias in (("silu", None), ("none", rnd(channels, seed=5).to(DEV))):
+        got = []
+        for stride in (channels + 12, channels + 13):
+            src = torch.full((T, stride), float("nan"), device=DEV)
+            src[:, col:col + channels] = x
+            state, out = state0.clone(), torch.full((T, channels), float("nan"), device=DEV)
+            ops.conv_silu(src, col, channels, w, b, state, off, slots, row_req, reqs, len(lens), out, activation, src_bias)
+            got.append((out, state))
+        assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1]) and not got[0][0].isnan().any()
+
+
 def test_mamba2_state_is_kept_in_32_bit():
     """In bfloat16 the slot that carries the recurrence is float32 all the same."""
     from beglin_b200.parts import Mamba2Spec
