@@ -11,7 +11,7 @@ the cache manager's slab, float32, zero when the request starts): a step continu
 slot, however the request's tokens are cut into steps and whatever else the step holds.  Everything that
 enters the recurrence is float in both number formats.
 
-A request that brings `LONG_FROM` rows or more runs in chunks (the chunks' own sums and outputs side by side, a short pass over their
+A request that brings many rows (`LONG_FROM`, `LONG_FROM_BF16`) runs in chunks (the chunks' own sums and outputs side by side, a short pass over their
 states between), where the sizes allow it, in bfloat16 and with the spec's `chunked`; fewer rows, and single tokens, are walked one by
 one.  In float32 without `chunked` all rows are walked: ways of cutting a prompt then agree bit for bit, which chunks cannot keep and
 bfloat16 steps, whose products change with the number of rows, do not promise.
@@ -81,10 +81,14 @@ class Mamba2:
         chunked = spec.chunked or ctx.compute_dtype == torch.bfloat16
         self.chunk = ops.ssm_chunk(spec.n_heads, spec.vdim, spec.state, spec.groups) if chunked and ctx.device.type == "cuda" else 0
         # rows whose chunks' states still fit CHUNK_BYTES; a longer step of a spec that does not ask for chunks is walked
+        self.long_from = self.LONG_FROM if spec.chunked else self.LONG_FROM_BF16
         self.most_rows = None if spec.chunked or not self.chunk else self.CHUNK_BYTES // (4 * self.conv_off) * self.chunk
 
-    LONG_FROM = 64             # rows of a request in a step from which its tokens run in chunks (2,048 rows of 24 heads of 128 x 128:
-    #                            989 us for the whole mixer walked row by row, 308 in chunks)
+    # Rows of a request in a step from which its tokens run in chunks: with the spec's `chunked`, and in bfloat16 without it, where the
+    # five kernels of the chunks are a later choice than the walk's one (the whole mixer of 24 heads of 128 x 128, walked and in chunks:
+    # 128 rows 86 and 99 us, 160 rows 101 and 96, 192 rows 115 and 97; nine heads 75 and 97, 83 and 97, 94 and 96; 2,048 rows of 24 heads
+    # 989 and 308)
+    LONG_FROM, LONG_FROM_BF16 = 64, 192
     CHUNK_BYTES = 1 << 28
     takes_stream = True        # forward takes a NormedInput and may add its result to the stream itself
 
@@ -103,7 +107,7 @@ class Mamba2:
         y = torch.empty((T, self.inner), dtype=torch.float32, device=h.device)
         chunks, n_chunks, longs, n_long = None, 0, None, 0
         if self.chunk and not batch.decode_only and hasattr(batch, "long_blocks") and (self.most_rows is None or T <= self.most_rows):
-            reqs, n_req, chunks, n_chunks, longs, n_long = batch.long_blocks(self.chunk, self.LONG_FROM)
+            reqs, n_req, chunks, n_chunks, longs, n_long = batch.long_blocks(self.chunk, self.long_from)
         ops.ssm_scan(xbc, proj, self.inner + self.channels, self.dt_bias, self.A_log, self.D, cache.state, cache.slots,
                      reqs, n_req, y, s.n_heads, s.vdim, s.state, s.groups, chunks, n_chunks, longs, n_long)
         out = torch.empty((T, self.inner), dtype=ctx.compute_dtype, device=h.device)

@@ -239,8 +239,8 @@ def test_mamba2_portions_and_two_requests(dtype, tol, heads, vdim, state, groups
 
 @pytest.mark.parametrize("heads,vdim,state,groups", [(4, 16, 32, 2), (3, 64, 128, 1), (2, 128, 48, 2)])
 def test_mamba2_long_portions_in_bfloat16(heads, vdim, state, groups):
-    """Portions around the length from which a request's rows run in chunks (63, 64, 65, 130, then 70 behind them), the same ones walked
-    row by row where the chunks' states would be too many, both against the plain recurrence."""
+    """Portions around the length from which a request's rows run in chunks, and others behind them, the same ones walked row by row where
+    the chunks' states would be too many, both against the plain recurrence."""
     from beglin_b200.parts import Mamba2Spec
     from beglin_b200.parts.mamba2 import Mamba2
     d = 48
@@ -251,13 +251,14 @@ def test_mamba2_long_portions_in_bfloat16(heads, vdim, state, groups):
         t[role.name] = ((role.name in ("D", "norm.weight")) - 0.5 * (role.name in ("A_log", "dt_bias"))
                         + rnd(*role.shape, seed=300 + k, scale=scale)).to(torch.bfloat16)
     part = Mamba2(spec, t, ctx_for(torch.bfloat16))
-    assert part.chunk and part.most_rows > 4096
-    lens = {"a": (63, 70), "b": (64, 1), "c": (65, 63), "d": (130, 64)}
+    at = part.long_from
+    assert part.chunk and part.most_rows > 4096 and at > 64
+    lens = {"a": (at - 1, at + 7), "b": (at, 1), "c": (at + 1, at - 1), "d": (3, at + 64)}
     hs = {r: rnd(sum(n), d, seed=i).to(torch.bfloat16) for i, (r, n) in enumerate(lens.items())}
     m = {"heads": heads, "vdim": vdim, "state": state, "groups": groups, "conv": 4, "norm_groups": 1}
     for most_rows in (part.most_rows, 0):
         part.most_rows = most_rows
-        reqs, outs, at = Requests([Mamba2.cache_need(spec)], 8, torch.bfloat16, slots=4), {r: [] for r in lens}, dict.fromkeys(lens, 0)
+        reqs, outs, at = Requests([Mamba2.cache_need(spec)], 8, torch.bfloat16, pages=400, slots=4), {r: [] for r in lens}, dict.fromkeys(lens, 0)
         for step in range(2):
             b = reqs.batch([(r, n[step]) for r, n in lens.items()])
             o = part.forward(torch.cat([hs[r][at[r]:at[r] + n[step]] for r, n in lens.items()]).to(DEV), b, reqs.cache.view(0, b))
