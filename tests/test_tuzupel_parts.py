@@ -114,6 +114,31 @@ def test_recurrence_row_by_row_in_chunks_over_steps_and_slots(W, blocks):
     assert torch.isnan(state[[1, 3]]).all() and torch.isnan(state[:, W:]).all()
 
 
+@pytest.mark.parametrize("W,blocks", [(2, 1), (24, 3), (258, 1), (512, 2)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_recurrence_in_chunks_two_channels_a_thread(W, blocks, dtype):
+    """Rows on 8-byte boundaries against the same rows an odd number of floats apart: the same bits out and in the state, for chunks that
+    fill their batches of rows and chunks that do not."""
+    from beglin_b200.engine.batch import cut_long_requests
+    o, g, lens = ops(), torch.Generator().manual_seed(W), [200, 65, 129, 34]
+    T, starts = sum(lens), [sum(lens[:i]) for i in range(4)]
+    rnd = lambda *n: torch.randn(*n, generator=g).to(DEV)
+    gates, u, y, br, bi, by = rnd(blocks, T, 2 * W // blocks), rnd(T, W), rnd(T, W), rnd(W), rnd(W), rnd(W)
+    decay, state0 = torch.rand(W, generator=g).to(DEV), rnd(4, W)
+    slots = torch.tensor([2, 0, 3, 1], dtype=torch.int32, device=DEV)
+    _, chunks, longs = cut_long_requests(starts, lens, 32, 1)
+    chunked = (torch.from_numpy(chunks).to(DEV), chunks.shape[0], torch.from_numpy(longs).to(DEV), longs.shape[0], 32)
+    for bias in (None, by):
+        got = []
+        for col in (4, 3):
+            src = torch.full((T, W + col), float("nan"), device=DEV)
+            src[:, col:] = y
+            state, out = state0.clone(), torch.full((T, W), float("nan"), dtype=dtype, device=DEV)
+            o.rglru_scan(gates, u, src, col, br, bi, decay, state, slots, None, 0, out, chunked=chunked, y_bias=bias)
+            got.append((out, state))
+        assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1]) and not got[0][0].isnan().any()
+
+
 def test_recurrence_keeps_a_far_token():
     """One token 900 rows back whose input gate is open while all others are shut: a decay of e^(-8 r softplus(lam)) per
     row with lam = -12 keeps it, lam = -4 fades it."""
