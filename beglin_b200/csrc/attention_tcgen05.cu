@@ -74,11 +74,6 @@ struct AttnTcDiffParams : AttnTcParams {
 template <bool DIFF> struct AtParams { using type = AttnTcParams; };
 template <> struct AtParams<true> { using type = AttnTcDiffParams; };
 
-__device__ __forceinline__ bool at_elect() {
-    unsigned one;
-    asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(one));
-    return one != 0;
-}
 __device__ __forceinline__ float at_ex2(float x) {
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;\n" : "=f"(y) : "f"(x));
@@ -232,7 +227,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_kv, typename At
                 if (!ok) break;
                 tc_fence_after();
                 const unsigned k_addr = smem_u32(k_s + st * KV_BYTES);
-                if (at_elect()) {
+                if (elect_one()) {
                     if constexpr (DIFF) {                // the map's half of the features
                         constexpr int HALF_STEPS = HD / 32;
 #pragma unroll
@@ -268,7 +263,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_kv, typename At
                     if (ok) ok = wait_all(&p_full[b], (i / NSB) & 1);
                     if (!ok) break;
                     tc_fence_after();
-                    if (at_elect()) {
+                    if (elect_one()) {
 #pragma unroll
                         for (int ks = 0; ks < AT_BK / 16; ++ks)
                             tc_mma_ts(tmem + O_COL + 128u * (unsigned)g, tmem + (unsigned)b * AT_BK + (unsigned)ks * 8,
@@ -282,7 +277,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_kv, typename At
                     ok = wait_all(&p_full[2 * b + g], (i / NSB) & 1);
                     if (!ok) break;
                     tc_fence_after();
-                    if (at_elect()) {
+                    if (elect_one()) {
 #pragma unroll
                         for (int ks = 0; ks < AT_HALF / 16; ++ks)
                             tc_mma_ts(tmem + O_COL + 128u * (unsigned)g, tmem + (unsigned)b * AT_BK + (unsigned)g * AT_HALF + (unsigned)ks * 8,
@@ -294,7 +289,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_kv, typename At
                 }
                 }
             }
-            if (ok) { if (at_elect()) tc_commit(&o_ready); }
+            if (ok) { if (elect_one()) tc_commit(&o_ready); }
             __syncwarp();
         }
         if (!ok && lane == 0) atomicExch(&failed, 1);

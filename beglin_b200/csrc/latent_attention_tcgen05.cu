@@ -16,10 +16,12 @@
 // The ring is cut finer than a tile: slots of 128 features x 128 keys, given back one by one as the value products have read them, and
 // one slot for the rotated part, given back by the score products.  A tile of 576 features is 147 KB, so that two of them do not fit
 // an SM; with the finer slots the next tile sets out while the last one is used.  One CTA an SM; bound by the bytes of the cache.
-// Measured (kernel and merge, 512 + 64 features, 32 heads): 64 requests of 4,000 keys 258.7 us with latent_attention_mma.cu -> 102.5 us
-// (2.9 TB/s of cache), 8 requests 49.2 -> 37.8, 32 requests of 300 keys 39.2 -> 27.2; 12 heads of 384 + 64, 64 requests of 4,096
-// keys 128.0 -> 67.8, one request 30.7 -> 31.4.  What is left beside the bytes is a range's start and end (queries, the first rows, the
-// results) and the chain of a tile's softmax, of which only two tiles are under way at a time.
+// Measured (kernel and merge, 512 + 64 features, 32 heads): 64 requests of 4,000 keys 258.7 us with latent_attention_mma.cu -> 92.6 us
+// (3.2 TB/s of cache; 102.5 with MMAs issued under a test of the lane's number), 8 requests 49.2 -> 36.2, 32 requests of 300 keys 39.2 ->
+// 25.9; 12 heads of 384 + 64, 64 requests of 4,096 keys 128.0 -> 62.7, one request 30.7 -> 30.2.  What is left beside the bytes is a
+// range's start and end (queries, the first rows, the results) and the chain of a tile, whose rows are held until its last value
+// product while only a part of the next tile's fit.  Tiles of 64 keys, of which 2.5 fit, took 100 us: half of every score product's
+// rows are then not keys, and the chain is walked twice as often.
 // Keys behind the range's last lie in pages that this request may never have written: their rows are zeroed in shared memory before
 // the value products read them (0 x NaN would reach every head).
 #include "tc_common.cuh"
@@ -216,12 +218,16 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_attention_tc_kernel(cons
                     ok = wait_all(&slot_full[slot], (it / p.slots) & 1);
                     if (!ok) break;
                     tc_fence_after();
-                    if (lane == 0) {
-                        const unsigned k_a = ring_a + (unsigned)slot * LT_SLOT;
-                        const int n = 2 * i + 1 < blocks ? 8 : 4;
-                        for (int ks = 0; ks < n; ++ks)
-                            tc_mma(tmem + (unsigned)b * NH, smem_desc_sw128(k_a + (ks >> 2) * LT_BLOCK + (ks & 3) * 32),
-                                   smem_desc_sw128(q_a + (unsigned)(2 * i + (ks >> 2)) * (NH * 128) + (ks & 3) * 32), idesc_s, (i > 0 || ks > 0) ? 1u : 0u);
+                    if (elect_one()) {
+                        const unsigned k_a = ring_a + (unsigned)slot * LT_SLOT, q_i = q_a + (unsigned)(2 * i) * (NH * 128), d = tmem + (unsigned)b * NH;
+#pragma unroll
+                        for (int ks = 0; ks < 4; ++ks)
+                            tc_mma(d, smem_desc_sw128(k_a + ks * 32), smem_desc_sw128(q_i + ks * 32), idesc_s, (i > 0 || ks > 0) ? 1u : 0u);
+                        if (2 * i + 1 < blocks) {
+#pragma unroll
+                            for (int ks = 0; ks < 4; ++ks)
+                                tc_mma(d, smem_desc_sw128(k_a + LT_BLOCK + ks * 32), smem_desc_sw128(q_i + NH * 128 + ks * 32), idesc_s, 1u);
+                        }
                         if (i == pairs - 1 && p.rot == 0) tc_commit(&s_full[b]);
                     }
                     __syncwarp();
@@ -230,7 +236,7 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_attention_tc_kernel(cons
                     ok = wait_all(&rot_full, ti & 1);
                     if (!ok) break;
                     tc_fence_after();
-                    if (lane == 0) {
+                    if (elect_one()) {
                         for (int ks = 0; ks * 16 < p.rot; ++ks)
                             tc_mma(tmem + (unsigned)b * NH, smem_desc_sw128(rot_a + ks * 32), smem_desc_sw128(q_a + (unsigned)blocks * (NH * 128) + ks * 32),
                                    idesc_s, 1u);
@@ -247,7 +253,7 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_attention_tc_kernel(cons
                 if (!ok) break;
                 tc_fence_after();
                 for (int i = 0; i < pairs; ++i, ++it) {
-                    if (lane == 0) {
+                    if (elect_one()) {
                         const int slot = it % p.slots;
                         const unsigned v_a = ring_a + (unsigned)slot * LT_SLOT;
 #pragma unroll

@@ -79,6 +79,13 @@ __device__ __forceinline__ void tma_prefetch_map(const CUtensorMap* map) {
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory"); }
 
 // ------------------------------------------------------------------------------------------------ tcgen05
+// One lane of a warp that is here as a whole.  Where the whole warp runs a loop and the elected lane issues, addresses and descriptors stay
+// in uniform registers and an MMA costs a few cycles to issue; under a test of the lane's number it costs some two hundred.
+__device__ __forceinline__ bool elect_one() {
+    unsigned one;
+    asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(one));
+    return one != 0;
+}
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory"); }
 __device__ __forceinline__ void tc_commit(unsigned long long* bar) {
