@@ -14,6 +14,7 @@
 //                                 starts, then every chunk's outputs in parallel (the earlier chunks through the state,
 //                                 the chunk's own tokens through their decayed scores).
 #include "common.cuh"
+#include "chunk_tc.cuh"
 
 namespace bg {
 
@@ -163,7 +164,7 @@ __global__ void __launch_bounds__(256) decay_attention_reg_kernel(DecayAttnParam
 //                           the chunk's start, the request's slot gets the state behind its last chunk
 // decay_chunk_out_kernel    o of every chunk (a block per head and chunk): scores of the chunk's own tokens times their
 //                           powers of d, then both sums
-// Powers of d come from one table made by repeated multiplication, so d = 0 and d = 1 need no logarithm.  Threads own
+// Powers of d come from squarings in double precision, so d = 0 and d = 1 need no logarithm.  Threads own
 // 4 x 4 tiles of outputs; rows of shared memory are padded to multiples of four floats and read as float4.
 constexpr int DC = 64;                    // tokens of a chunk
 constexpr int DCP = DC + 4;               // row stride of the transposed tiles [feature][token]
@@ -180,11 +181,15 @@ struct DecayChunkParams {
     int H, n, nv, np, nvp;                // np, nvp: n, nv rounded up to multiples of 4
 };
 
+// d^k, rounded once: a chain of float products would be off by the rounding of each, again and again over the chunks of a long request
+__device__ __forceinline__ float decay_power(float d, int k) {
+    double v = 1.0;
+    for (double b = d; k > 0; k >>= 1, b *= b)
+        if (k & 1) v *= b;
+    return (float)v;
+}
 __device__ __forceinline__ void decay_powers(float* pw, float d) {      // pw[k] = d^k, k = 0 .. DC
-    if (threadIdx.x == 0) {
-        float v = 1.0f;
-        for (int k = 0; k <= DC; ++k) { pw[k] = v; v *= d; }
-    }
+    for (int k = threadIdx.x; k <= DC; k += blockDim.x) pw[k] = decay_power(d, k);
 }
 
 #define DA_FMA44(acc, a, b)                                                                                      \
@@ -277,8 +282,7 @@ __global__ void __launch_bounds__(256) decay_chunk_scan_kernel(DecayChunkParams 
     const int req = p.longs[l * 4 + 0], rows = p.longs[l * 4 + 2], c0 = p.longs[l * 4 + 3];
     const int n_chunks = (rows + DC - 1) / DC, last_rows = rows - (n_chunks - 1) * DC;
     const float d = p.decay[h];
-    float dfull = 1.0f, dlast = 1.0f;
-    for (int k = 0; k < DC; ++k) { dfull *= d; if (k + 1 == last_rows) dlast = dfull; }
+    const float dfull = decay_power(d, DC), dlast = decay_power(d, last_rows);
     float* st = p.state + (size_t)p.slots[req] * p.slot_stride + (size_t)h * sz + e;
     float* a0 = p.work + ((size_t)c0 * p.H + h) * sz + e;
     const size_t step = (size_t)p.H * sz;
@@ -414,6 +418,54 @@ __global__ void __launch_bounds__(DC_THREADS) decay_chunk_out_kernel(DecayChunkP
 static size_t decay_chunk_out_smem(int np, int nvp) {
     return ((size_t)2 * np * DCP + (size_t)DC * nvp + (size_t)np * nvp + (size_t)DC * DCP + DC + 4) * sizeof(float);
 }
+
+// The same products on the tensor cores, from operands in three bfloat16 parts (chunk_tc.cuh), for float rows of whole 16-byte pieces.
+struct DecayTc {
+    static constexpr bool SCORES = true;
+    struct Shared { float pw[DC + 1]; };
+    DecayChunkParams p;
+    int n, nv, nv_ld;
+    unsigned* status;
+    __device__ float* sum_out(int h, int ch) const { return p.work + ((size_t)ch * p.H + h) * n * nv; }
+    __device__ const float* state(int h, int ch) const { return sum_out(h, ch); }
+    struct Chunk {
+        const DecayTc& r;
+        const float* src;
+        const float* pw;
+        int h, row0, rows;
+        __device__ Chunk(const DecayTc& r_, int h_, int ch, Shared& s) : r(r_), pw(s.pw), h(h_) {
+            row0 = r.p.chunks[ch * 4 + 1]; rows = r.p.chunks[ch * 4 + 2];
+            src = (const float*)r.p.src + (size_t)row0 * r.p.src_stride;
+            decay_powers(s.pw, r.p.decay[h]);
+            __syncthreads();
+        }
+        __device__ void sum_begin() {}
+        __device__ void out_begin() {}
+        __device__ float4 raw(int col, int t, int c) const {
+            return t < rows ? *reinterpret_cast<const float4*>(src + (size_t)t * r.p.src_stride + col + c) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        }
+        __device__ static float4 silu(const float4& x, float f) { return make_float4(da_silu(x.x) * f, da_silu(x.y) * f, da_silu(x.z) * f, da_silu(x.w) * f); }
+        __device__ float4 key_raw(int j, int i) const { return raw(r.p.k_col + h * r.n, j, i); }
+        __device__ float4 key(const float4& x, int j, int) const { return silu(x, j < rows ? pw[rows - 1 - j] : 0.0f); }
+        __device__ float4 value_raw(int j, int v) const { return raw(r.p.v_col + h * r.nv, j, v); }
+        __device__ float4 value(const float4& x, int, int) const { return silu(x, 1.0f); }
+        __device__ float4 out_value(const float4& x, int, int) const { return silu(x, 1.0f); }
+        __device__ float4 query_raw(int t, int i) const { return raw(r.p.q_col + h * r.n, t, i); }
+        __device__ float4 query(const float4& x, int, int) const { return silu(x, 1.0f); }
+        __device__ float4 score_key_raw(int j, int i) const { return key_raw(j, i); }
+        __device__ float4 score_key(const float4& x, int, int) const { return silu(x, 1.0f); }
+        __device__ float weight(float score, int t, int j) const { return score * pw[t - j]; }
+        __device__ float factor(int t) const { return pw[t + 1]; }
+        template <typename W> __device__ void weights(W) const {}
+        __device__ void finish(const float* o) const {
+            const int w4 = r.nv >> 2;
+            for (int idx = threadIdx.x; idx < rows * w4; idx += blockDim.x) {
+                const int t = idx / w4, v = (idx - t * w4) * 4;
+                *reinterpret_cast<float4*>(r.p.y + (size_t)(row0 + t) * r.p.H * r.nv + (size_t)h * r.nv + v) = *reinterpret_cast<const float4*>(o + t * CT_OUT_LD + v);
+            }
+        }
+    };
+};
 
 // ---------------------------------------------------------------------------------------------------------------
 // x[t] (= or +=) sum_i scale_i * term_i[t], term_i a [T, d] tensor of either type or the float partial sums of a
@@ -671,13 +723,27 @@ extern "C" int bg_decay_attention_chunk_plan(int n, int nv, int* chunk) {
 extern "C" int bg_decay_attention_chunked(const void* src, int src_dtype, int src_stride, int parts, long long part_stride,
                                           int q_col, int k_col, int v_col, const float* decay, float* state, long long slot_stride,
                                           const int* slots, const int* chunks, int n_chunks, const int* longs, int n_long,
-                                          float* work, float* y, int H, int n, int nv, cudaStream_t stream) {
+                                          float* work, float* y, int H, int n, int nv, int tensor_cores, unsigned* status,
+                                          cudaStream_t stream) {
     if (n_chunks <= 0 || n_long <= 0) return BG_OK;
     if (H <= 0 || n <= 0 || nv <= 0 || parts < 1 || n_chunks > 65535 || n_long > 65535 || H > 65535) return BG_ERR_SHAPE;
     DecayChunkParams p;
     p.src = src; p.src_stride = src_stride; p.parts = parts; p.part_stride = (size_t)part_stride; p.q_col = q_col; p.k_col = k_col;
     p.v_col = v_col; p.decay = decay; p.state = state; p.slot_stride = (size_t)slot_stride; p.slots = slots; p.chunks = chunks;
     p.longs = longs; p.work = work; p.y = y; p.H = H; p.n = n; p.nv = nv; p.np = (n + 3) / 4 * 4; p.nvp = (nv + 3) / 4 * 4;
+    if (tensor_cores && ct_takes(n, nv) && src_dtype == BG_DTYPE_F32 && parts == 1 && src_stride % 4 == 0 && q_col % 4 == 0 && k_col % 4 == 0 &&
+        v_col % 4 == 0 && (uintptr_t)src % 16 == 0 && (uintptr_t)work % 16 == 0 && (uintptr_t)y % 16 == 0) {
+        DecayTc r;
+        r.p = p; r.n = n; r.nv = r.nv_ld = nv; r.status = status;
+        int rc = ct_sum(r, H, n_chunks, stream);
+        if (rc != BG_OK) return rc;
+        launch(decay_chunk_scan_kernel, dim3((n * nv + 255) / 256, H, n_long), dim3(256), 0, stream, p);
+        BG_LAUNCH_CHECK();
+        rc = ct_out(r, H, n_chunks, stream);
+        if (rc != BG_OK) return rc;
+        BG_LAUNCH_CHECK();
+        return BG_OK;
+    }
     const size_t smem_sum = ((size_t)DC * p.np + (size_t)DC * p.nvp + DC + 4) * sizeof(float);
     const size_t smem_out = decay_chunk_out_smem(p.np, p.nvp);
     if (smem_out > 200 * 1024 || smem_sum > 200 * 1024) return BG_ERR_UNSUPPORTED;

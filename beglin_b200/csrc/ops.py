@@ -85,7 +85,7 @@ _SIGNATURES = {
     "bg_decay_attention_chunk_plan": [_c_int, _c_int, ctypes.POINTER(_c_int)],
     "bg_decay_attention_chunked": [_c_void_p, _c_int, _c_int, _c_int, _c_ll, _c_int, _c_int, _c_int, _c_void_p, _c_void_p, _c_ll,
                                    _c_void_p, _c_void_p, _c_int, _c_void_p, _c_int, _c_void_p, _c_void_p, _c_int, _c_int, _c_int,
-                                   _c_void_p],
+                                   _c_int, _c_void_p, _c_void_p],
     "bg_add_terms_norm": [_c_void_p, _c_int, _c_int, _c_int, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p,
                           _c_void_p, _c_void_p, _c_int, _c_float, _c_void_p, _c_void_p, _c_int, _c_void_p, _c_void_p, _c_int,
                           _c_void_p, _c_void_p, _c_void_p],
@@ -1621,7 +1621,7 @@ def decay_attention_chunk(n: int, nv: int) -> int:
 def decay_attention(src: torch.Tensor, q_col: int, k_col: int, v_col: int, decay: torch.Tensor, state: torch.Tensor,
                     slots: torch.Tensor, reqs: torch.Tensor, n_req: int, y: torch.Tensor, H: int, n: int, nv: int,
                     chunks: Optional[torch.Tensor] = None, n_chunks: int = 0, longs: Optional[torch.Tensor] = None,
-                    n_long: int = 0) -> None:
+                    n_long: int = 0, tensor_cores: bool = False, status: Optional[torch.Tensor] = None) -> None:
     """Linear attention with a constant decay per head.  `src` [T, W] (or float partial sums [parts, T, W]) holds, from the
     columns given, the products for q, k ([H, n] each) and v ([H, nv]); q, k, v = silu of them.  Per request (`reqs`
     [n_req, 3] = request, first row, rows) and head, for its rows in turn: S <- decay[h] S + k v^T, y = S^T q, with S
@@ -1630,8 +1630,10 @@ def decay_attention(src: torch.Tensor, q_col: int, k_col: int, v_col: int, decay
     Requests of many rows may be given apart, cut into chunks of `decay_attention_chunk(n, nv)` rows: `chunks`
     [n_chunks, 4] = (request, first row, rows, -) and `longs` [n_long, 4] = (request, first row, rows, index of the first
     chunk).  Their chunks run in parallel (sums of a chunk's own k v^T, a pass over the chunks' states, the outputs); the
-    results are those of the walk token by token up to rounding.  A request stands in `reqs` or in `longs`, not both."""
-    _cuda(src, decay, state, slots, reqs, y, chunks, longs)
+    results are those of the walk token by token up to rounding.  A request stands in `reqs` or in `longs`, not both.
+    `tensor_cores`: the chunks' products may run on the tensor cores, from float operands in three bfloat16 parts (`status`: the
+    word in which their bounded waits leave a mark)."""
+    _cuda(src, decay, state, slots, reqs, y, chunks, longs, status)
     _i32(slots, "slots")
     if n_req:
         _i32(reqs, "reqs")
@@ -1657,7 +1659,8 @@ def decay_attention(src: torch.Tensor, q_col: int, k_col: int, v_col: int, decay
             work = torch.empty((n_chunks, H, n * nv), dtype=torch.float32, device=y.device)
             _check(lib().bg_decay_attention_chunked(_p(src), _dt(src), src.stride(-2), parts, stride, q_col, k_col, v_col, _p(decay),
                                                     _p(state), state.stride(0), _p(slots), _p(chunks), n_chunks, _p(longs), n_long,
-                                                    _p(work), _p(y), H, n, nv, _stream()), "decay_attention_chunked")
+                                                    _p(work), _p(y), H, n, nv, 1 if tensor_cores else 0, _p(status), _stream()),
+                   "decay_attention_chunked")
 
 
 def add_terms_norm(x: torch.Tensor, terms, assign: bool = False, weight1: Optional[torch.Tensor] = None,

@@ -81,7 +81,8 @@ class DecayAttention:
             reqs, n_req = batch.query_blocks(1 << 30)                   # one (request, first row, rows) per request
             chunks, n_chunks, longs, n_long = None, 0, None, 0
         ops.decay_attention(proj, 0, self.qd, 2 * self.qd, self.decay, cache.state, cache.slots, reqs, n_req, y,
-                            s.n_heads, s.dim, s.vdim, chunks, n_chunks, longs, n_long)
+                            s.n_heads, s.dim, s.vdim, chunks, n_chunks, longs, n_long,
+                            tensor_cores=self.ctx.compute_dtype == torch.bfloat16, status=self.ctx.status)
         out = torch.empty((T, self.vd), dtype=self.ctx.compute_dtype, device=h.device)
         ops.gated_group_rmsnorm(y, proj, self.g_col, self.norm_w, s.eps, 1, out, gate_after=True)
         if stream is None:

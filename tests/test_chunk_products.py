@@ -1,0 +1,82 @@
+"""The recurrences' chunks on the tensor cores: float products from operands in three bfloat16 parts are held to the same bounds as the
+float units' kernels, against the recurrence walked token by token in 64 bits."""
+import math
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+@pytest.fixture(scope="module")
+def ops():
+    from beglin_b200.csrc import ops as o
+    o.lib()
+    return o
+
+
+def lists(lens, chunk):
+    from beglin_b200.engine.batch import cut_long_requests
+    starts = [sum(lens[:i]) for i in range(len(lens))]
+    _, blocks, longs = cut_long_requests(starts, lens, chunk, 1)
+    dev = lambda a: torch.tensor(a, dtype=torch.int32, device=DEV)
+    return dev(blocks), len(blocks), dev(longs), len(longs)
+
+
+def walk(a, k, v, q, S):
+    """S <- diag(a_t) S + k_t v_t^T, o_t = S^T q_t over rows [n, heads, features]."""
+    out = []
+    for t in range(k.shape[0]):
+        S = S * a[t][:, :, None] + k[t][:, :, None] * v[t][:, None, :]
+        out.append((q[t][:, None, :] @ S)[:, 0])
+    return torch.stack(out), S
+
+
+def rnd(*shape, seed):
+    g = torch.Generator().manual_seed(seed)
+    return torch.randn(*shape, generator=g).to(DEV)
+
+
+def close(got, want, terms):
+    """Within `terms` roundings of 2^-24 of the largest value: a chunk's sums of some 200 products and the chunks' states."""
+    assert float((got.double() - want).abs().max()) <= terms * 2.0 ** -24 * float(want.abs().max())
+
+
+def walked_requests(make, lens, state0):
+    """(outputs [T, ...], states) of every request by `walk`; `make(first row, rows)` gives (a, k, v, q)."""
+    outs, states, row = [], [], 0
+    for i, n in enumerate(lens):
+        o, S = walk(*make(row, n), state0[i])
+        outs.append(o.reshape(n, -1))
+        states.append(S)
+        row += n
+    return torch.cat(outs), torch.stack(states)
+
+
+SIZES = [(2, 128, 128, [64]), (3, 64, 48, [1, 65, 200]), (2, 96, 64, [130, 63]), (1, 64, 112, [700]), (2, 48, 128, [129]), (2, 48, 48, [64, 7]), (2, 32, 64, [70]),
+         (1, 128, 144, [70])]
+
+
+@pytest.mark.parametrize("H,n,nv,lens", SIZES)          # (the last two: sizes that stay with the float units)
+def test_constant_decay(ops, H, n, nv, lens):
+    T = sum(lens)
+    src, decay = rnd(T, H * (2 * n + 2 * nv), seed=1), torch.tensor([0.0, 1.0 - 2.0 ** -8, 0.875][:H], device=DEV)
+    state0 = rnd(len(lens), H, n, nv, seed=2)
+    silu = lambda x: x * torch.sigmoid(x)
+
+    def make(row, rows):
+        x = silu(src[row:row + rows].double())
+        q, k, v = x[:, :H * n].view(rows, H, n), x[:, H * n:2 * H * n].view(rows, H, n), x[:, 2 * H * n:2 * H * n + H * nv].view(rows, H, nv)
+        return decay.double()[None, :, None].expand(rows, H, 1), k, v, q
+
+    want, states = walked_requests(make, lens, state0.double())
+    slots = torch.arange(len(lens) - 1, -1, -1, dtype=torch.int32, device=DEV)
+    state = state0.flip(0).reshape(len(lens), -1).contiguous()
+    y, status = torch.full((T, H * nv), float("nan"), device=DEV), ops.new_status(DEV)
+    chunks, n_chunks, longs, n_long = lists(lens, ops.decay_attention_chunk(n, nv))
+    ops.decay_attention(src, 0, H * n, 2 * H * n, decay, state, slots, None, 0, y, H, n, nv, chunks, n_chunks, longs, n_long, tensor_cores=True,
+                        status=status)
+    ops.raise_on_status(status)
+    close(y, want, 64)
+    close(state.flip(0).view_as(states), states, 64)
