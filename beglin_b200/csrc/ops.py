@@ -91,7 +91,8 @@ _SIGNATURES = {
                           _c_void_p, _c_void_p, _c_void_p],
     "bg_gla_walk": [_c_void_p, _c_void_p, _c_int, _c_void_p],
     "bg_gla_chunk_plan": [_c_int, _c_int, ctypes.POINTER(_c_int)],
-    "bg_gla_chunked": [_c_void_p, _c_void_p, _c_int, _c_void_p, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p],
+    "bg_gla_chunked": [_c_void_p, _c_void_p, _c_int, _c_void_p, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p,
+                       _c_void_p],
     "bg_attention_mma_plan": [_c_int, _c_int, _c_int, ctypes.POINTER(_c_int)],
     "bg_attention_mma_partial": [_c_void_p, _c_int, _c_void_p, _c_int, _c_int, _c_void_p, _c_int, _c_void_p, _c_void_p,
                                  _c_int, _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int,
@@ -1729,7 +1730,7 @@ def gated_linear_attention(src: torch.Tensor, q_col: int, k_col: int, v_col: int
                            n: int, nv: int, *, lower: Optional[torch.Tensor] = None, decay_matrix: Optional[torch.Tensor] = None,
                            r_col: int = 0, power: float = 1.0, q_silu: bool = False, q_scale: float = 1.0, g_col: int = -1,
                            chunks: Optional[torch.Tensor] = None, n_chunks: int = 0, longs: Optional[torch.Tensor] = None,
-                           n_long: int = 0) -> None:
+                           n_long: int = 0, status: Optional[torch.Tensor] = None) -> None:
     """Linear attention with a decay per key channel, its head norm and its gate.  `src` float32 [T, W] holds the products of
     the mixer's input: from `q_col` the queries' [H, n] (q = q_scale times the product, or times its silu with `q_silu`), from
     `k_col` either the forget gate's [H, n] (with `lower`, float32 [H n]: a = l + (1 - l) sigmoid(f + bias), k = 1 - a) or the
@@ -1737,8 +1738,9 @@ def gated_linear_attention(src: torch.Tensor, q_col: int, k_col: int, v_col: int
     a = sigmoid(decay_matrix r + bias)^power), from `v_col` the values [H, nv], and from `g_col` (if not negative) the
     gate's [H, nv].  Per request and head, for its rows in turn: S <- diag(a) S + k v^T, o = S^T q, with S [n, nv] float32 at
     state[slots[request], h * n * nv ...]; out[t] = o / rms(o) * norm_weight (float32 [nv]) (* silu(gate)), [T, H nv] in either
-    type.  `reqs` [n_req, 3], or `chunks` and `longs` for requests of many rows, as in `decay_attention`."""
-    _cuda(src, bias, norm_weight, state, slots, reqs, out, lower, decay_matrix, chunks, longs)
+    type.  `reqs` [n_req, 3], or `chunks` and `longs` for requests of many rows, as in `decay_attention`; with a bfloat16 `out` the
+    chunks' products run on the tensor cores as there."""
+    _cuda(src, bias, norm_weight, state, slots, reqs, out, lower, decay_matrix, chunks, longs, status)
     _i32(slots, "slots")
     T, W = src.shape
     if src.dtype != torch.float32 or src.stride(1) != 1:
@@ -1772,7 +1774,7 @@ def gated_linear_attention(src: torch.Tensor, q_col: int, k_col: int, v_col: int
             scores, work = torch.empty((n_chunks, H, size * size), **f32), torch.empty((n_chunks, H, np_ * nvp), **f32)
             decay = torch.empty((n_chunks, H, n), **f32)
             _check(lib().bg_gla_chunked(ctypes.byref(a), _p(chunks), n_chunks, _p(longs), n_long, _p(qkd[0]), _p(qkd[1]), _p(scores),
-                                        _p(work), _p(decay), _stream()), "gla_chunked")
+                                        _p(work), _p(decay), _p(status), _stream()), "gla_chunked")
             count_launches(3)
 
 

@@ -97,7 +97,7 @@ class GatedLinearAttention:
         ops.gated_linear_attention(proj, 0, self.qd, 2 * self.qd, self.bias, self.norm_w, s.eps, cache.state, cache.slots, reqs, n_req,
                                    out, s.n_heads, s.dim, s.vdim, lower=self.lower, decay_matrix=self.decay_w, r_col=self.r_col,
                                    power=s.decay_power, q_silu=s.query_silu, q_scale=s.query_scale, g_col=self.g_col,
-                                   chunks=chunks, n_chunks=n_chunks, longs=longs, n_long=n_long)
+                                   chunks=chunks, n_chunks=n_chunks, longs=longs, n_long=n_long, status=self.ctx.status)
         if stream is None:
             return self.o_proj.partial(out)
         self.o_proj.into(out, stream)

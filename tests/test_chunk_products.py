@@ -80,3 +80,39 @@ def test_constant_decay(ops, H, n, nv, lens):
     ops.raise_on_status(status)
     close(y, want, 64)
     close(state.flip(0).view_as(states), states, 64)
+
+
+@pytest.mark.parametrize("H,n,nv,lens", SIZES)
+@pytest.mark.parametrize("forget", [True, False])
+def test_decay_per_channel(ops, H, n, nv, lens, forget):
+    T, rank, qd, vd = sum(lens), 5, H * n, H * nv
+    src = rnd(T, 2 * qd + 2 * vd + 8, seed=1)
+    bias, lower, wa, norm_w = rnd(qd, seed=2), torch.rand(qd, generator=torch.Generator().manual_seed(3)).to(DEV), rnd(qd, rank, seed=4), rnd(nv, seed=5)
+    state0 = rnd(len(lens), H, n, nv, seed=6)
+
+    def make(row, rows):
+        x = src[row:row + rows].double()
+        q, f, v = x[:, :qd], x[:, qd:2 * qd], x[:, 2 * qd:2 * qd + vd].view(rows, H, nv)
+        if forget:
+            a = lower.double() + (1 - lower.double()) * torch.sigmoid(f + bias.double())
+            k = 1 - a
+        else:
+            a, k = torch.sigmoid(x[:, 2 * qd + 2 * vd:2 * qd + 2 * vd + rank] @ wa.double().T + bias.double()) ** (1 / 16), f
+        return a.view(rows, H, n), k.reshape(rows, H, n), v, q.reshape(rows, H, n) * 0.5
+
+    want, states = walked_requests(make, lens, state0.double())
+    want = want.view(T, H, nv)
+    want = (want / ((want * want).mean(-1, keepdim=True) + 1e-6).sqrt() * norm_w.double()).reshape(T, -1)
+    gate = src[:, 2 * qd + vd:2 * qd + 2 * vd].double()
+    want = want * gate * torch.sigmoid(gate)
+    slots = torch.arange(len(lens), dtype=torch.int32, device=DEV)
+    state, status = state0.reshape(len(lens), -1).clone(), ops.new_status(DEV)
+    out = torch.full((T, vd), float("nan"), dtype=torch.bfloat16, device=DEV)
+    chunks, n_chunks, longs, n_long = lists(lens, ops.gla_chunk(n, nv))
+    how = dict(lower=lower) if forget else dict(decay_matrix=wa, r_col=2 * qd + 2 * vd, power=1 / 16)
+    ops.gated_linear_attention(src, 0, qd, 2 * qd, bias, norm_w, 1e-6, state, slots, None, 0, out, H, n, nv, q_scale=0.5, g_col=2 * qd + vd,
+                               chunks=chunks, n_chunks=n_chunks, longs=longs, n_long=n_long, status=status, **how)
+    ops.raise_on_status(status)
+    close(state.view_as(states), states, 128)
+    # (bfloat16 rounds a value to 2^-9 of it; the norm magnifies a head's own rounding where its values nearly cancel)
+    assert float((out.double() - want).abs().max()) <= (2.0 ** -8 + 1e-4) * float(want.abs().max())
