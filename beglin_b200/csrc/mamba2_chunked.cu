@@ -11,6 +11,7 @@
 // the chunk), never a quotient or a difference of sums, so that nothing cancels after a token with a large step.
 // Everything is float.  N and P are multiples of 4.  The slot's layout is that of ssm_scan_kernel: [H][P][N].
 #include "common.cuh"
+#include "chunk_tc.cuh"
 
 namespace bg {
 
@@ -296,6 +297,83 @@ __global__ void __launch_bounds__(128) ssm_chunk_out_kernel(SsmChunkParams p) {
     }
 }
 
+// The chunks' sums and outputs on the tensor cores, from operands in three bfloat16 parts (chunk_tc.cuh).
+template <typename TI, typename TW>
+struct SsmTc {
+    static constexpr bool SCORES = false;
+    struct Shared { float dt[MC], a[MC], pre[MC], suf[MC]; };
+    SsmChunkParams p;
+    int n, nv, nv_ld;
+    unsigned* status;
+    __device__ float* sum_out(int h, int ch) const { return p.work + ((size_t)ch * p.H + h) * n * nv; }
+    __device__ const float* state(int h, int ch) const { return sum_out(h, ch); }
+    struct Chunk {
+        const SsmTc& r;
+        Shared& s;
+        int h, ch, g, row0, rows;
+        const float* row;
+        __device__ Chunk(const SsmTc& r_, int h_, int ch_, Shared& s_) : r(r_), s(s_), h(h_), ch(ch_) {
+            row0 = r.p.chunks[ch * 4 + 1]; rows = r.p.chunks[ch * 4 + 2];
+            g = h / (r.p.H / r.p.G);
+            row = r.p.xbc + (size_t)row0 * r.p.channels;
+            sc_steps<TI, TW>(r.p, h, row0, rows, s.dt, s.a, s.pre, s.suf);
+            __syncthreads();
+        }
+        __device__ void sum_begin() {
+            if (threadIdx.x == 0) r.p.decay[(size_t)ch * r.p.H + h] = s.pre[MC / 2 - 1] * s.pre[MC - 1];
+        }
+        __device__ void out_begin() {}
+        __device__ float4 at(int t, int c) const {
+            return t < rows ? *reinterpret_cast<const float4*>(row + (size_t)t * r.p.channels + c) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        }
+        __device__ float4 key_raw(int j, int i) const { return at(j, r.p.H * r.nv + g * r.n + i); }
+        __device__ float4 key(const float4& x, int, int) const { return x; }
+        __device__ float4 value_raw(int j, int v) const { return at(j, h * r.nv + v); }
+        __device__ float4 value(const float4& x, int j, int) const {       // times the step and the decay behind the token
+            const float w = s.dt[j] * (j < MC / 2 ? s.suf[j] * s.pre[MC - 1] : s.suf[j]);
+            return make_float4(x.x * w, x.y * w, x.z * w, x.w * w);
+        }
+        __device__ float4 out_value(const float4& x, int, int) const { return x; }
+        __device__ float4 query_raw(int t, int i) const { return at(t, r.p.H * r.nv + (r.p.G + g) * r.n + i); }
+        __device__ float4 query(const float4& x, int, int) const { return x; }
+        __device__ float4 score_key_raw(int, int) const { return make_float4(0.0f, 0.0f, 0.0f, 0.0f); }
+        __device__ float4 score_key(const float4& x, int, int) const { return x; }
+        __device__ float weight(float score, int, int) const { return score; }
+        __device__ float factor(int t) const { return (t >= MC / 2 ? s.pre[MC / 2 - 1] : 1.0f) * s.pre[t]; }
+        // the weight of key j at query t: score x (product of the decays behind j up to t) x step.  Threads 0 .. 63: the queries of the
+        // key's own half of the chunk, one decay after the other; 64 .. 127: those of the second half for keys of the first; 128 ..
+        // 191: noughts at the queries of the first half for keys of the second
+        template <typename W> __device__ void weights(W put) const {
+            const int j = threadIdx.x & (MC - 1), part = threadIdx.x / MC, half = j / (MC / 2);
+            const float* sc = r.p.scores + ((size_t)ch * r.p.G + g) * MC * MC + j;
+            if (part > 2 || (part == 1 && half == 1) || (part == 2 && half == 0)) return;
+            const int t_begin = part == 0 ? half * (MC / 2) : part == 1 ? MC / 2 : 0;
+            float l = part == 0 ? s.dt[j] : s.suf[j] * s.dt[j];
+            for (int t0 = t_begin; t0 < t_begin + MC / 2; t0 += 8) {
+                float x[8];
+#pragma unroll
+                for (int u = 0; u < 8; ++u) x[u] = part != 2 && t0 + u >= j ? sc[(size_t)(t0 + u) * MC] : 0.0f;
+#pragma unroll
+                for (int u = 0; u < 8; ++u) {
+                    const int t = t0 + u;
+                    if (part == 0 && t > j) l *= s.a[t];
+                    put(t, j, part == 1 ? x[u] * (l * s.pre[t]) : x[u] * l);
+                }
+            }
+        }
+        __device__ void finish(const float* o) const {
+            const int w4 = r.nv >> 2;
+            const float D = to_float(((const TW*)r.p.D)[h]);
+            for (int idx = threadIdx.x; idx < rows * w4; idx += blockDim.x) {
+                const int t = idx / w4, v = (idx - t * w4) * 4;
+                const float4 x = at(t, h * r.nv + v), y = *reinterpret_cast<const float4*>(o + t * CT_OUT_LD + v);
+                *reinterpret_cast<float4*>(r.p.y + (size_t)(row0 + t) * r.p.H * r.nv + (size_t)h * r.nv + v) =
+                    make_float4(fmaf(D, x.x, y.x), fmaf(D, x.y, y.y), fmaf(D, x.z, y.z), fmaf(D, x.w, y.w));
+            }
+        }
+    };
+};
+
 static size_t sc_smem_scores(int N) { return (size_t)2 * MC * (N + 4) * sizeof(float); }
 static size_t sc_smem_sum(int N) { return ((size_t)MC * N + (size_t)MC * MPT) * sizeof(float); }
 static size_t sc_smem_out(int N) { return ((size_t)MC * (N + 4) + (size_t)N * MPT + (size_t)MC * MPT + (size_t)MC * MCP) * sizeof(float); }
@@ -317,7 +395,7 @@ extern "C" int bg_ssm_chunk_plan(int H, int P, int N, int G, int* chunk) {
 extern "C" int bg_ssm_chunked(const float* xbc, int channels, const void* src, int src_dtype, int src_stride, int dt_col,
                               const void* dt_bias, const void* A_log, const void* D, int w_dtype, float* state, long long slot_stride,
                               const int* slots, const int* chunks, int n_chunks, const int* longs, int n_long, float* scores, float* work,
-                              float* decay, float* y, int H, int P, int N, int G, cudaStream_t stream) {
+                              float* decay, float* y, int H, int P, int N, int G, int tensor_cores, unsigned* status, cudaStream_t stream) {
     if (n_chunks <= 0 || n_long <= 0) return BG_OK;
     const int rc = bg_ssm_chunk_plan(H, P, N, G, nullptr);
     if (rc != BG_OK) return rc;
@@ -336,6 +414,24 @@ extern "C" int bg_ssm_chunked(const float* xbc, int channels, const void* src, i
     }
     launch(ssm_chunk_scores_kernel, dim3(G, n_chunks), dim3(256), s_scores, stream, p);
     BG_LAUNCH_CHECK();
+    // from 80 features on both sides: 24 heads of 128 x 128, 2,048 tokens, 180 -> 121 us; with 64 on one side the conversions cost what the
+    // float units need for the products (12 heads of 64 x 128, 2,174 tokens: 70 us there, 78 here)
+    if (tensor_cores && ct_takes(N, P) && N > 64 && P > 64 && channels % 4 == 0 && (uintptr_t)xbc % 16 == 0 && (uintptr_t)work % 16 == 0 &&
+        (uintptr_t)y % 16 == 0) {
+        int trc = BG_OK;
+        BG_DISPATCH_DTYPE(src_dtype, TI, BG_DISPATCH_DTYPE(w_dtype, TW, {
+            SsmTc<TI, TW> r;
+            r.p = p; r.n = N; r.nv = r.nv_ld = P; r.status = status;
+            trc = ct_launch(chunk_sum_tc_kernel<SsmTc<TI, TW>, 5, 5>, r, H, n_chunks, stream);
+            if (trc == BG_OK) {
+                launch(ssm_chunk_scan_kernel, dim3((N * P + 255) / 256, H, n_long), dim3(256), 0, stream, p);
+                trc = ct_launch(chunk_out_tc_kernel<SsmTc<TI, TW>, 5, 5>, r, H, n_chunks, stream);
+            }
+        }));
+        if (trc != BG_OK) return trc;
+        BG_LAUNCH_CHECK();
+        return BG_OK;
+    }
     BG_DISPATCH_DTYPE(src_dtype, TI, BG_DISPATCH_DTYPE(w_dtype, TW, {
         auto ksum = ssm_chunk_sum_kernel<TI, TW>;
         auto kout = ssm_chunk_out_kernel<TI, TW>;

@@ -160,7 +160,7 @@ _SIGNATURES = {
     "bg_ssm_chunk_plan": [_c_int, _c_int, _c_int, _c_int, ctypes.POINTER(_c_int)],
     "bg_ssm_chunked": [_c_void_p, _c_int, _c_void_p, _c_int, _c_int, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_void_p, _c_ll,
                        _c_void_p, _c_void_p, _c_int, _c_void_p, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_int,
-                       _c_int, _c_int, _c_void_p],
+                       _c_int, _c_int, _c_int, _c_void_p, _c_void_p],
     "bg_gated_group_rmsnorm": [_c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_void_p, _c_int, _c_float, _c_void_p, _c_int,
                                _c_int, _c_int, _c_int, _c_int, _c_void_p],
     "bg_gemm_f32_nt_batched": [_c_void_p, _c_int, _c_ll, _c_void_p, _c_int, _c_ll, _c_void_p, _c_int, _c_ll, _c_int, _c_int,
@@ -1411,12 +1411,12 @@ def ssm_chunk(H: int, P: int, N: int, G: int) -> int:
 def ssm_scan(xbc: torch.Tensor, src: torch.Tensor, dt_col: int, dt_bias: torch.Tensor, A_log: torch.Tensor, D: torch.Tensor,
              state: torch.Tensor, slots: torch.Tensor, reqs: Optional[torch.Tensor], n_req: int, y: torch.Tensor, H: int, P: int,
              N: int, G: int, chunks: Optional[torch.Tensor] = None, n_chunks: int = 0, longs: Optional[torch.Tensor] = None,
-             n_long: int = 0) -> None:
+             n_long: int = 0, tensor_cores: bool = False, status: Optional[torch.Tensor] = None) -> None:
     """The recurrence over each request's rows, from and into the slots' state S [H, P, N] (float32, at the start of
     a slot): dt = softplus(src[t, dt_col + h] + dt_bias[h]); S = exp(-exp(A_log[h]) dt) S + dt B_t x_t^T;
     y_t = S^T C_t + D[h] x_t.  xbc float32 [T, H P + 2 G N] = [x | B | C]; y float32 [T, H P].  Requests of many rows may be
-    given apart, in chunks of `ssm_chunk(...)` rows (`chunks`, `longs` as in `decay_attention`)."""
-    _cuda(xbc, src, dt_bias, A_log, D, state, slots, reqs, y, chunks, longs)
+    apart, in chunks of `ssm_chunk(...)` rows (`chunks`, `longs`, `tensor_cores`, `status` as in `decay_attention`)."""
+    _cuda(xbc, src, dt_bias, A_log, D, state, slots, reqs, y, chunks, longs, status)
     _i32(slots, "slots")
     if n_req:
         _i32(reqs, "reqs")
@@ -1445,7 +1445,8 @@ def ssm_scan(xbc: torch.Tensor, src: torch.Tensor, dt_col: int, dt_bias: torch.T
             decay = torch.empty((n_chunks, H), **f32)
             _check(lib().bg_ssm_chunked(_p(xbc), xbc.shape[1], _p(src), _dt(src), src.stride(0), dt_col, _p(dt_bias), _p(A_log), _p(D),
                                         _dt(D), _p(state), state.stride(0), _p(slots), _p(chunks), n_chunks, _p(longs), n_long,
-                                        _p(scores), _p(work), _p(decay), _p(y), H, P, N, G, _stream()), "ssm_chunked")
+                                        _p(scores), _p(work), _p(decay), _p(y), H, P, N, G, 1 if tensor_cores else 0, _p(status),
+                                        _stream()), "ssm_chunked")
             count_launches(3)
 
 

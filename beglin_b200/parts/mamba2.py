@@ -109,7 +109,8 @@ class Mamba2:
         if self.chunk and not batch.decode_only and hasattr(batch, "long_blocks") and (self.most_rows is None or T <= self.most_rows):
             reqs, n_req, chunks, n_chunks, longs, n_long = batch.long_blocks(self.chunk, self.long_from)
         ops.ssm_scan(xbc, proj, self.inner + self.channels, self.dt_bias, self.A_log, self.D, cache.state, cache.slots,
-                     reqs, n_req, y, s.n_heads, s.vdim, s.state, s.groups, chunks, n_chunks, longs, n_long)
+                     reqs, n_req, y, s.n_heads, s.vdim, s.state, s.groups, chunks, n_chunks, longs, n_long,
+                     tensor_cores=ctx.compute_dtype == torch.bfloat16, status=ctx.status)
         out = torch.empty((T, self.inner), dtype=ctx.compute_dtype, device=h.device)
         ops.gated_group_rmsnorm(y, proj, 0, self.norm_w, s.eps, s.norm_groups, out)
         if stream is None:

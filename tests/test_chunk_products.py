@@ -116,3 +116,30 @@ def test_decay_per_channel(ops, H, n, nv, lens, forget):
     close(state.view_as(states), states, 128)
     # (bfloat16 rounds a value to 2^-9 of it; the norm magnifies a head's own rounding where its values nearly cancel)
     assert float((out.double() - want).abs().max()) <= (2.0 ** -8 + 1e-4) * float(want.abs().max())
+
+
+@pytest.mark.parametrize("H,P,N,G,lens", [(2, 128, 128, 1, [64]), (4, 80, 96, 2, [1, 65, 200]), (3, 96, 128, 1, [130, 63]), (2, 128, 112, 2, [700]), (2, 64, 128, 1, [70])])
+def test_mamba2(ops, H, P, N, G, lens):
+    T = sum(lens)
+    xbc, raw = rnd(T, H * P + 2 * G * N, seed=1), rnd(T, H + 1, seed=2)
+    bias, A_log, D = rnd(H, seed=3) - 1.0, rnd(H, seed=4), rnd(H, seed=5)
+    raw[::9] += 6.0                                     # large steps that forget everything between small ones
+    state0 = rnd(len(lens), H, N, P, seed=6)
+
+    def make(row, rows):
+        x = xbc[row:row + rows].double()
+        B = x[:, H * P:H * P + G * N].view(rows, G, N).repeat_interleave(H // G, 1)
+        C = x[:, H * P + G * N:].view(rows, G, N).repeat_interleave(H // G, 1)
+        dt = torch.nn.functional.softplus(raw[row:row + rows, 1:].double() + bias.double())
+        return torch.exp(-torch.exp(A_log.double()) * dt)[:, :, None], B, x[:, :H * P].view(rows, H, P) * dt[:, :, None], C
+
+    want, states = walked_requests(make, lens, state0.double())
+    want = want + (D.double()[:, None] * xbc[:, :H * P].double().view(T, H, P)).reshape(T, -1)
+    slots = torch.arange(len(lens), dtype=torch.int32, device=DEV)
+    state = state0.transpose(2, 3).reshape(len(lens), -1).contiguous()                      # a slot holds [H, P, N]
+    y, status = torch.full((T, H * P), float("nan"), device=DEV), ops.new_status(DEV)
+    chunks, n_chunks, longs, n_long = lists(lens, ops.ssm_chunk(H, P, N, G))
+    ops.ssm_scan(xbc, raw, 1, bias, A_log, D, state, slots, None, 0, y, H, P, N, G, chunks, n_chunks, longs, n_long, tensor_cores=True, status=status)
+    ops.raise_on_status(status)
+    close(y, want, 64)
+    close(state.view(len(lens), H, P, N).transpose(2, 3), states, 64)
