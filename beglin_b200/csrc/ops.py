@@ -78,6 +78,8 @@ _SIGNATURES = {
                         _c_int, _c_int, _c_int, _c_void_p],
     "bg_gemm_grouped_tc": [_c_void_p, _c_int, _c_int, _c_int, _c_int, _c_void_p, _c_int, _c_int, _c_void_p, _c_int, _c_int,
                            _c_void_p, _c_int, _c_void_p, _c_void_p],
+    "bg_gemm_grouped_pair": [_c_void_p, _c_int, _c_int, _c_int, _c_int, _c_void_p, _c_int, _c_int, _c_void_p, _c_int, _c_int,
+                           _c_void_p, _c_int, _c_void_p, _c_void_p],
     "bg_sigmoid_gate": [_c_void_p, _c_int, _c_int, _c_void_p, _c_int, _c_int, _c_int, _c_void_p, _c_int, _c_int, _c_int, _c_ll,
                         _c_int, _c_int, _c_int, _c_int, _c_void_p],
     "bg_decay_attention": [_c_void_p, _c_int, _c_int, _c_int, _c_ll, _c_int, _c_int, _c_int, _c_void_p, _c_void_p, _c_ll, _c_void_p,
@@ -2032,6 +2034,13 @@ def rglru_scan(gates: torch.Tensor, u: torch.Tensor, src: torch.Tensor, y_col: i
             count_launches(2)
 
 
+def grouped_pairs(rows: int, experts: int) -> bool:
+    """Whether the experts' products run on pairs of CTAs: from more than 128 rows an expert on (on average: the routing is known on the
+    device only).  With 300 rows an expert 16.1 against 18.0 us on single CTAs, with 512 42.1 against 57.4; with 75 a tile of 256
+    features on a pair would be three parts empty."""
+    return rows > 128 * experts and experts <= 512
+
+
 def gemm_grouped(x: torch.Tensor, w: torch.Tensor, offsets: torch.Tensor, out: torch.Tensor, activation: str = "none",
                  status: Optional[torch.Tensor] = None, tensor_cores: bool = True) -> None:
     """out[row] = act(x[row] w[e]^T) for the rows offsets[e] .. offsets[e + 1] of every expert e: x [A, K], w [E, N, K],
@@ -2047,8 +2056,8 @@ def gemm_grouped(x: torch.Tensor, w: torch.Tensor, offsets: torch.Tensor, out: t
     act = EXPERT_ACTIVATIONS[activation]
     with phase("experts"):
         if tensor_cores and x.dtype == torch.bfloat16 and K % 8 == 0:
-            _check(lib().bg_gemm_grouped_tc(_p(w), E, N, K, K, _p(x), A, K, _p(out), _dt(out), N, _p(offsets), act, _p(status),
-                                            _stream()), "gemm_grouped_tc")
+            f = lib().bg_gemm_grouped_pair if grouped_pairs(A, E) else lib().bg_gemm_grouped_tc
+            _check(f(_p(w), E, N, K, K, _p(x), A, K, _p(out), _dt(out), N, _p(offsets), act, _p(status), _stream()), "gemm_grouped on tcgen05")
         else:
             _check(lib().bg_gemm_grouped(_p(x), _dt(x), K, _p(w), K, N * K, _p(out), _dt(out), N, _p(offsets), E, A, N, K, act,
                                          _stream()), "gemm_grouped")

@@ -1,0 +1,43 @@
+"""Routed experts in steps of many rows: the experts' products on pairs of CTAs over experts with no rows, a few and many, sizes that fill
+no tile, and the kernels around them where their 16-byte forms begin and end."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+@pytest.fixture(scope="module")
+def ops():
+    from beglin_b200.csrc import ops as o
+    o.lib()
+    return o
+
+
+CASES = [  # rows of the experts, rows behind them that no expert has, features in, features out
+    ([129], 0, 64, 256), ([700, 0, 1], 0, 72, 264), ([0, 257, 256, 255, 128, 64], 5, 1000, 8), ([191, 192, 193, 385, 0, 600], 0, 512, 520),
+    ([2048, 3], 0, 136, 1024), ([0, 0, 0, 900], 40, 328, 392), ([150] * 40, 0, 128, 128), ([1024] * 4, 0, 1536, 3072),
+]
+
+
+@pytest.mark.parametrize("rows,behind,K,N", CASES)
+@pytest.mark.parametrize("out_dtype", [torch.float32, torch.bfloat16])
+def test_products_of_many_rows(ops, rows, behind, K, N, out_dtype):
+    E, A = len(rows), sum(rows) + behind
+    assert ops.grouped_pairs(A, E)
+    g = torch.Generator().manual_seed(A + K)
+    x = torch.randn(A, K, generator=g).to(DEV, torch.bfloat16)
+    w = torch.randn(E, N, K, generator=g).to(DEV, torch.bfloat16)
+    x[sum(rows):] = float("nan")
+    starts = [sum(rows[:e]) for e in range(E + 1)]
+    out, status = torch.full((A, N), 7.0, dtype=out_dtype, device=DEV), ops.new_status(DEV)
+    ops.gemm_grouped(x, w, torch.tensor(starts, dtype=torch.int32, device=DEV), out, "relu2", status)
+    ops.raise_on_status(status)
+    for e in range(E):
+        a, b = starts[e], starts[e + 1]
+        z, size = x[a:b].double() @ w[e].double().T, x[a:b].double().abs() @ w[e].double().abs().T
+        off = K * 2.0 ** -24 * size                           # sums of K float products
+        want = z.clamp(min=0) ** 2
+        bound = 2.0 * want.sqrt() * off + off * off + (2.0 ** -8 if out_dtype == torch.bfloat16 else 2.0 ** -23) * want
+        assert ((out[a:b].double() - want).abs() <= bound).all(), (e, a, b)
+    assert (out[sum(rows):] == 7.0).all()
