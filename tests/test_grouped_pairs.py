@@ -41,3 +41,22 @@ def test_products_of_many_rows(ops, rows, behind, K, N, out_dtype):
         bound = 2.0 * want.sqrt() * off + off * off + (2.0 ** -8 if out_dtype == torch.bfloat16 else 2.0 ** -23) * want
         assert ((out[a:b].double() - want).abs() <= bound).all(), (e, a, b)
     assert (out[sum(rows):] == 7.0).all()
+
+
+@pytest.mark.parametrize("T,d", [(1, 8), (5, 24), (9, 36), (3, 7), (130, 1032), (33, 2048)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("scale", [False, True])
+def test_rows_out_and_back(ops, T, d, dtype, scale):
+    top, A = 3, 3 * T
+    g = torch.Generator().manual_seed(T * d)
+    x, y = torch.randn(T, d, generator=g).to(DEV, dtype), torch.randn(A, d, generator=g).to(DEV)
+    weights, src_of = torch.rand(A, generator=g).to(DEV), torch.randperm(A, generator=g).to(DEV, torch.int32)
+    row_of = torch.empty_like(src_of)
+    row_of[src_of.long()] = torch.arange(A, dtype=torch.int32, device=DEV)
+    xp, out = torch.full((A, d), float("nan"), dtype=dtype, device=DEV), torch.full((T, d), float("nan"), device=DEV)
+    ops.route_gather(x, weights, src_of, xp, top, scale=scale)
+    want = x[src_of.long() // top]
+    assert torch.equal(xp, (weights[src_of.long()][:, None] * want.float()).to(dtype) if scale else want)
+    ops.route_combine(y, weights, row_of, out, top, scale=scale)
+    terms = y[row_of.long()].view(T, top, d).double() * (weights.view(T, top, 1).double() if scale else 1.0)
+    assert ((out.double() - terms.sum(1)).abs() <= top * 2.0 ** -23 * terms.abs().sum(1)).all()
