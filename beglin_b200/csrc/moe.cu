@@ -8,6 +8,7 @@
 //                  offsets[e] .. offsets[e + 1] are expert e's rows; row_of[a] is where assignment a went and
 //                  src_of[row] the assignment that row holds.  ONE CTA; the order inside an expert is whatever the
 //                  atomics give, which no result depends on (a row's product is a function of that row alone).
+//   route_rows     the three above and below for a step of few tokens in one kernel, a cluster of CTAs.
 //   route_gather   xp[row] = (weight * x[token]) rounded to the compute type (or x[token] as it is).
 //   gemm_grouped   yp[row] = act(xp[row] W[e]^T) on CUDA cores, float accumulation, every output summed over k in index
 //                  order by one thread: the float32 path, and the sizes the tensor-core product does not take.
@@ -147,29 +148,12 @@ route_kernel(const TI* __restrict__ h, int ldh, const float* __restrict__ W, int
     if (warp < n) choose_experts(logit_s + warp * E, E, top, rule, ids, weights, (size_t)(t0 + warp), lane);
 }
 
-// The same for a width that is a multiple of 8 and 16-byte aligned rows.  A block of eight warps takes TPB tokens, 8 / TPB
-// warps to a token, which share the experts in groups of G; a lane walks the token's features in chunks of eight, 32 chunks
-// apart (16-byte loads: one of the token's row, which stays in the first-level cache from expert to expert, and two of
-// each expert's row), and the warp adds up; the first warp of a token then chooses.  Steps of many tokens: a warp per token,
-// four experts at a time.  Steps of few tokens: a block per token and an expert per warp at a time, so that a decoding step
-// spreads over as many SMs as it has tokens and a warp's chain of loads is one expert long.  (The walk through the features
-// one at a time above cost 53 us for 1,536 features whatever the number of tokens.)
-template <typename TI, int TPB, int G>
-__global__ void __launch_bounds__(32 * ROUTE_TOKENS)
-route_vec8_kernel(const TI* __restrict__ h, int ldh, const float* __restrict__ W, int T, int d, int E, int top, RouteRule rule,
-                  int* __restrict__ ids, float* __restrict__ weights, float* __restrict__ logits_out) {
-    constexpr int WPT = ROUTE_TOKENS / TPB;                // warps per token
-    extern __shared__ float logit_s[];                     // [TPB][E]
-    pdl_launch();
-    pdl_wait();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int tl = warp / WPT, wq = warp % WPT;
-    const int t = blockIdx.x * TPB + tl;
-    const bool live = t < T;
-    const TI* row = h + (size_t)(live ? t : 0) * ldh;
-    float* sc = logit_s + tl * E;
-    const int d8 = d >> 3;
-    for (int e0 = wq * G; live && e0 < E; e0 += WPT * G) {
+// The logits of one token's row by `warps` warps of a block (this is the `warp`-th), each a group of G experts at a time: a lane walks the
+// features in chunks of eight, 32 chunks apart (16-byte loads), and the warp adds up.
+template <typename TI, int G>
+__device__ __forceinline__ void route_logits_of(const TI* row, const float* __restrict__ W, int d8, int d, int E, float* sc, float* logits_out,
+                                                int warp, int warps, int lane) {
+    for (int e0 = warp * G; e0 < E; e0 += warps * G) {
         float acc[G];
 #pragma unroll
         for (int u = 0; u < G; ++u) acc[u] = 0.0f;
@@ -192,12 +176,102 @@ route_vec8_kernel(const TI* __restrict__ h, int ldh, const float* __restrict__ W
             const float v = warp_sum(acc[u]);
             if (lane == 0 && e0 + u < E) {
                 sc[e0 + u] = v;
-                if (logits_out) logits_out[(size_t)t * E + e0 + u] = v;
+                if (logits_out) logits_out[e0 + u] = v;
             }
         }
     }
+}
+
+// The same for a width that is a multiple of 8 and 16-byte aligned rows.  A block of eight warps takes TPB tokens, 8 / TPB
+// warps to a token, which share the experts in groups of G; a lane walks the token's features in chunks of eight, 32 chunks
+// apart (16-byte loads: one of the token's row, which stays in the first-level cache from expert to expert, and two of
+// each expert's row), and the warp adds up; the first warp of a token then chooses.  Steps of many tokens: a warp per token,
+// four experts at a time.  Steps of few tokens: a block per token and an expert per warp at a time, so that a decoding step
+// spreads over as many SMs as it has tokens and a warp's chain of loads is one expert long.  (The walk through the features
+// one at a time above cost 53 us for 1,536 features whatever the number of tokens.)
+template <typename TI, int TPB, int G>
+__global__ void __launch_bounds__(32 * ROUTE_TOKENS)
+route_vec8_kernel(const TI* __restrict__ h, int ldh, const float* __restrict__ W, int T, int d, int E, int top, RouteRule rule,
+                  int* __restrict__ ids, float* __restrict__ weights, float* __restrict__ logits_out) {
+    constexpr int WPT = ROUTE_TOKENS / TPB;                // warps per token
+    extern __shared__ float logit_s[];                     // [TPB][E]
+    pdl_launch();
+    pdl_wait();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int tl = warp / WPT, wq = warp % WPT;
+    const int t = blockIdx.x * TPB + tl;
+    const bool live = t < T;
+    const TI* row = h + (size_t)(live ? t : 0) * ldh;
+    float* sc = logit_s + tl * E;
+    const int d8 = d >> 3;
+    if (live) route_logits_of<TI, G>(row, W, d8, d, E, sc, logits_out ? logits_out + (size_t)t * E : nullptr, wq, WPT, lane);
     __syncthreads();                                       // every warp comes here, with or without a token
     if (live && wq == 0) choose_experts(sc, E, top, rule, ids, weights, (size_t)t, lane);
+}
+
+// Routing, layout and gather of a step of few tokens as ONE kernel: three dependent launches cost more than their work, on
+// the device (eight tokens, ten router outputs: 7.9 us as three kernels, 6.8 as one) and most of all, outside a graph, on the host (a
+// gated layer with identity and shared experts: 140 -> 126 us).  A cluster of eight CTAs, a token each, routed as in the kernel above
+// (the same sums, so the same choice); with two tokens a CTA, one after the other, it lost (10.7 against 8.1 us).  The CTAs read each other's choices through the cluster, each lays out all
+// assignments for itself (an assignment's row: those of smaller experts and the earlier ones of its own, counted) and gathers its own
+// tokens' rows.  Inside an expert the rows stand in the order of the assignments.
+constexpr int RR_CTAS = 8, RR_TOKENS = 8, RR_MAX_A = 256;
+template <typename TI, int G>
+__global__ void __launch_bounds__(32 * ROUTE_TOKENS)
+route_rows_kernel(const TI* __restrict__ h, int ldh, const float* __restrict__ W, int T, int d, int E, int top, RouteRule rule,
+                  int* __restrict__ ids, float* __restrict__ weights, int* __restrict__ offsets, int* __restrict__ row_of,
+                  int* __restrict__ src_of, TI* __restrict__ xp, int scale) {
+    extern __shared__ float logit_s[];                     // [E]
+    __shared__ int all_s[RR_MAX_A], row_s[RR_MAX_A];       // every assignment's expert (own tokens' first), its row
+    pdl_launch();
+    pdl_wait();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, tid = threadIdx.x;
+    const int rank = blockIdx.z, A = T * top, d8 = d >> 3;
+    const int t = rank;                                    // this CTA's token
+    if (t < T) {
+        route_logits_of<TI, G>(h + (size_t)t * ldh, W, d8, d, E, logit_s, nullptr, warp, ROUTE_TOKENS, lane);
+        __syncthreads();
+        if (warp == 0) {
+            choose_experts(logit_s, E, top, rule, ids, weights, (size_t)t, lane);
+            if (lane < top) all_s[t * top + lane] = ids[(size_t)t * top + lane];
+        }
+    }
+    cluster_sync_all();
+    for (int a = tid; a < A; a += blockDim.x) {            // the other CTAs' tokens, from where they were routed
+        const int owner = a / top;
+        if (owner == rank) continue;
+        int v;
+        asm volatile("ld.shared::cluster.s32 %0, [%1];\n" : "=r"(v) : "r"(peer_addr((unsigned)__cvta_generic_to_shared(&all_s[a]), (unsigned)owner)) : "memory");
+        all_s[a] = v;
+    }
+    cluster_sync_all();                                    // (nobody leaves, or is read, before all have read)
+    for (int a = tid; a < A; a += blockDim.x) {
+        const int e = all_s[a];
+        int row = 0;
+        for (int b = 0; b < A; ++b) row += all_s[b] < e || (all_s[b] == e && b < a) ? 1 : 0;
+        row_s[a] = row;
+        if (rank == 0) { row_of[a] = row; src_of[row] = a; }
+    }
+    if (rank == 0) {
+        for (int e = tid; e <= E; e += blockDim.x) {
+            int n = 0;
+            for (int b = 0; b < A; ++b) n += all_s[b] < e ? 1 : 0;
+            offsets[e] = n;
+        }
+    }
+    __syncthreads();
+    for (int c = tid; t < T && c < d8; c += blockDim.x) {
+        float x[8];
+        load8(h + (size_t)t * ldh + 8 * c, x);
+        for (int j = 0; j < top; ++j) {
+            const int a = t * top + j;
+            const float w = scale ? weights[a] : 1.0f;
+            float v[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) v[i] = w * x[i];
+            store8(xp + (size_t)row_s[a] * d + 8 * c, v);
+        }
+    }
 }
 
 __global__ void __launch_bounds__(1024)
@@ -600,6 +674,28 @@ extern "C" int bg_route(const void* h, int h_dtype, int ldh, const float* W, int
 #undef BG_ROUTE_VEC
         BG_DISPATCH_DTYPE(h_dtype, TI, launch(route_kernel<TI>, grid, block, smem, stream, (const TI*)h, ldh, W, T, d, E, top, rule,
                                               ids, weights, logits_out));
+    BG_LAUNCH_CHECK();
+    return BG_OK;
+}
+
+// bg_route, bg_route_sort and bg_route_gather (xp in h's type) in one kernel, for up to 8 tokens whose width is a multiple of 8 on 16-byte
+// rows; BG_ERR_UNSUPPORTED, with nothing launched, where it does not take the sizes.
+extern "C" int bg_route_rows(const void* h, int h_dtype, int ldh, const float* W, int T, int d, int E, int top, int mode, int renorm,
+                             const float* bias, float scale, const float* logit_bias, int* ids, float* weights, int* offsets, int* row_of,
+                             int* src_of, void* xp, int scale_input, cudaStream_t stream) {
+    if (T <= 0) return BG_OK;
+    if (E <= 0 || top <= 0 || top > E || top > 32 || d <= 0 || mode < 0 || mode > 3 || (mode == 3 && bias)) return BG_ERR_SHAPE;
+    if (T > RR_TOKENS || T * top > RR_MAX_A || E > 1024 || d % 8 || ldh % 8 || (uintptr_t)h % 16 || (uintptr_t)W % 16 || (uintptr_t)xp % 16)
+        return BG_ERR_UNSUPPORTED;
+    const RouteRule rule = {mode, renorm, bias, scale, logit_bias};
+    const size_t smem = (size_t)E * sizeof(float);
+#define BG_ROUTE_ROWS(G)                                                                                                    \
+    BG_DISPATCH_DTYPE(h_dtype, TI, launch_cluster(route_rows_kernel<TI, G>, dim3(1, 1, RR_CTAS), dim3(32 * ROUTE_TOKENS), smem, stream, RR_CTAS, (const TI*)h, \
+                                                  ldh, W, T, d, E, top, rule, ids, weights, offsets, row_of, src_of, (TI*)xp, scale_input))
+    if (E <= ROUTE_TOKENS) BG_ROUTE_ROWS(1);
+    else if (E <= 2 * ROUTE_TOKENS) BG_ROUTE_ROWS(2);
+    else BG_ROUTE_ROWS(4);
+#undef BG_ROUTE_ROWS
     BG_LAUNCH_CHECK();
     return BG_OK;
 }

@@ -71,6 +71,8 @@ _SIGNATURES = {
                               _c_int, _c_int, _c_void_p],
     "bg_rglru_softplus": [_c_void_p, _c_int, _c_float, _c_void_p, _c_int, _c_void_p],
     "bg_rglru_split": [_c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_void_p],
+    "bg_route_rows": [_c_void_p, _c_int, _c_int, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void_p, _c_float, _c_void_p,
+                      _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_void_p],
     "bg_route_sort": [_c_void_p, _c_int, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_void_p],
     "bg_route_gather": [_c_void_p, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void_p],
     "bg_route_combine": [_c_void_p, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_void_p],
@@ -1847,6 +1849,38 @@ def route(h: torch.Tensor, router: torch.Tensor, top: int, ids: torch.Tensor, we
     with phase("router"):
         _check(lib().bg_route(_p(h), _dt(h), h.stride(0), _p(router), T, d, E, top, _route_rule(E, sigmoid, bias, "route", logit_bias),
                               1 if renorm else 0, _p(bias), float(scale), _p(logit_bias), _p(ids), _p(weights), _p(logits), _stream()), "route")
+
+
+_UNSUPPORTED = -4             # a size that a kernel does not take
+ROUTE_ROWS_TOKENS = 8         # tokens up to which `route_rows` may take a step
+
+
+def route_rows(h: torch.Tensor, router: torch.Tensor, top: int, ids: torch.Tensor, weights: torch.Tensor, offsets: torch.Tensor,
+               row_of: torch.Tensor, src_of: torch.Tensor, out: torch.Tensor, scale_input: bool, sigmoid=True, renorm: bool = False,
+               bias: Optional[torch.Tensor] = None, scale: float = 1.0, logit_bias: Optional[torch.Tensor] = None) -> bool:
+    """`route`, `route_sort` and `route_gather` (out of h's type) of a step of few tokens as one kernel; False, with nothing done, where
+    it does not take the sizes."""
+    T, d = h.shape
+    E, A = router.shape[0], T * top
+    if T > ROUTE_ROWS_TOKENS or out.dtype != h.dtype or h.dtype not in (torch.float32, torch.bfloat16) or not h.is_contiguous():
+        return False
+    _cuda(h, router, ids, weights, offsets, row_of, src_of, out, bias, logit_bias)
+    for t, n in ((ids, "ids"), (offsets, "offsets"), (row_of, "row_of"), (src_of, "src_of")):
+        _i32(t, n)
+    if router.dtype != torch.float32 or router.shape[1] != d or not router.is_contiguous() or tuple(ids.shape) != (T, top) \
+            or tuple(weights.shape) != (T, top) or weights.dtype != torch.float32 or not weights.is_contiguous() \
+            or not ids.is_contiguous() or offsets.numel() != E + 1 or row_of.numel() != A or src_of.numel() != A \
+            or tuple(out.shape) != (A, d) or not out.is_contiguous():
+        raise KernelError("route_rows: h [T, d], router float32 [E, d], ids and weights [T, top], offsets [E + 1], row_of and src_of [T * top], "
+                          "out [T * top, d]")
+    rule = _route_rule(E, sigmoid, bias, "route_rows", logit_bias)
+    with phase("router"):
+        rc = lib().bg_route_rows(_p(h), _dt(h), h.stride(0), _p(router), T, d, E, top, rule, 1 if renorm else 0, _p(bias), float(scale),
+                                 _p(logit_bias), _p(ids), _p(weights), _p(offsets), _p(row_of), _p(src_of), _p(out), 1 if scale_input else 0, _stream())
+        if rc == _UNSUPPORTED:
+            return False
+        _check(rc, "route_rows")
+    return True
 
 
 def route_sort(ids: torch.Tensor, E: int, offsets: torch.Tensor, row_of: torch.Tensor, src_of: torch.Tensor) -> None:

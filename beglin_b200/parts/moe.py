@@ -137,13 +137,14 @@ class RoutedExperts:
         ints = torch.empty((3 * A + outputs + 1,), dtype=torch.int32, device=dev)
         ids, row_of, src_of, offsets = ints[:A].view(T, s.top), ints[A:2 * A], ints[2 * A:3 * A], ints[3 * A:]
         weights = torch.empty((T, s.top), dtype=torch.float32, device=dev)
-        ops.route(h, self.router, s.top, ids, weights, sigmoid=s.router_activation, renorm=s.renormalize,
-                  bias=self.choice_bias, scale=s.route_scale, logit_bias=self.logit_bias)
-        ops.route_sort(ids.view(-1), outputs, offsets, row_of, src_of)
+        xp = torch.empty((A, s.hidden), dtype=ct, device=dev)
+        how = dict(sigmoid=s.router_activation, renorm=s.renormalize, bias=self.choice_bias, scale=s.route_scale, logit_bias=self.logit_bias)
+        if T > ops.ROUTE_ROWS_TOKENS or not ops.route_rows(h, self.router, s.top, ids, weights, offsets, row_of, src_of, xp, s.scale_input, **how):
+            ops.route(h, self.router, s.top, ids, weights, **how)
+            ops.route_sort(ids.view(-1), outputs, offsets, row_of, src_of)
+            ops.route_gather(h, weights.view(-1), src_of, xp, s.top, scale=s.scale_input)
         if s.identity:                                 # (rows of experts without weights: assigned, never computed)
             offsets = offsets[:s.experts + 1]
-        xp = torch.empty((A, s.hidden), dtype=ct, device=dev)
-        ops.route_gather(h, weights.view(-1), src_of, xp, s.top, scale=s.scale_input)
         hp = torch.empty((A, s.intermediate), dtype=ct, device=dev)
         if self.glu:
             gu = torch.empty((A, 2 * s.intermediate), dtype=ct, device=dev)

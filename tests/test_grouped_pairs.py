@@ -60,3 +60,28 @@ def test_rows_out_and_back(ops, T, d, dtype, scale):
     ops.route_combine(y, weights, row_of, out, top, scale=scale)
     terms = y[row_of.long()].view(T, top, d).double() * (weights.view(T, top, 1).double() if scale else 1.0)
     assert ((out.double() - terms.sum(1)).abs() <= top * 2.0 ** -23 * terms.abs().sum(1)).all()
+
+
+@pytest.mark.parametrize("T,E,top,d", [(1, 1, 1, 8), (8, 10, 2, 1536), (5, 16, 3, 264), (8, 8, 8, 64), (8, 40, 32, 512), (3, 130, 5, 2056), (7, 17, 17, 128)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_routing_of_few_tokens_in_one_kernel(ops, T, E, top, d, dtype):
+    """The three kernels of a larger step as one: the same choices and weights bit for bit, a layout in which every expert holds its
+    assignments, the same rows."""
+    g = torch.Generator().manual_seed(T * E)
+    h, W = torch.randn(T, d, generator=g).to(DEV, dtype), torch.randn(E, d, generator=g).to(DEV)
+    bias, A = torch.randn(E, generator=g).to(DEV), T * top
+    i32 = lambda *n: torch.full(n, -7, dtype=torch.int32, device=DEV)
+    for scale_input in (False, True):
+        for how in (dict(sigmoid="sigmoid", renorm=True), dict(sigmoid="softmax", bias=bias, scale=2.5), dict(sigmoid="softmax_chosen", logit_bias=bias)):
+            ids, weights, offsets, row_of, src_of = i32(T, top), torch.zeros((T, top), device=DEV), i32(E + 1), i32(A), i32(A)
+            xp = torch.full((A, d), float("nan"), dtype=dtype, device=DEV)
+            assert ops.route_rows(h, W, top, ids, weights, offsets, row_of, src_of, xp, scale_input, **how)
+            ids2, weights2, xp2 = i32(T, top), torch.zeros((T, top), device=DEV), torch.full_like(xp, float("nan"))
+            ops.route(h, W, top, ids2, weights2, **how)
+            assert torch.equal(ids, ids2) and torch.equal(weights, weights2)
+            chosen, starts = ids.view(-1).long(), offsets.long()
+            assert torch.equal(starts, torch.cat([torch.zeros(1, device=DEV), torch.bincount(chosen, minlength=E).cumsum(0)]).long())
+            assert torch.equal(row_of[src_of.long()].long(), torch.arange(A, device=DEV))
+            assert ((row_of.long() >= starts[chosen]) & (row_of.long() < starts[chosen + 1])).all()
+            ops.route_gather(h, weights.view(-1), src_of, xp2, top, scale=scale_input)
+            assert torch.equal(xp, xp2)
