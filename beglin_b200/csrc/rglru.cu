@@ -50,7 +50,7 @@ __device__ __forceinline__ float gelu_tanh32(float z) {
 __device__ __forceinline__ void lru_values(float gr, float gi, float u, float spc, float* a, float* b) {
     const float e = expm1f(-sigmoid32(gr) * spc);
     *a = 1.0f + e;
-    *b = sqrtf(-e * (2.0f + e)) * (sigmoid32(gi) * u);
+    *b = sqrtf(fmaf(-e, e, -2.0f * e)) * (sigmoid32(gi) * u);
 }
 
 // The same for row t of channel c.

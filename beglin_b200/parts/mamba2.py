@@ -11,9 +11,9 @@ the cache manager's slab, float32, zero when the request starts): a step continu
 slot, however the request's tokens are cut into steps and whatever else the step holds.  Everything that
 enters the recurrence is float in both number formats.
 
-A request that brings many rows (`LONG_FROM`, `LONG_FROM_BF16`) runs in chunks (the chunks' own sums and outputs side by side, a short pass over their
-states between), where the sizes allow it, in bfloat16 and with the spec's `chunked`; fewer rows, and single tokens, are walked one by
-one.  In float32 without `chunked` all rows are walked: ways of cutting a prompt then agree bit for bit, which chunks cannot keep and
+A request that brings many rows (`LONG_FROM`, `LONG_FROM_BF16`) runs in chunks (the chunks' own sums and outputs side by side, a
+short pass over their states between), where the sizes allow it, in bfloat16 and with the spec's `chunked`; fewer rows, and single
+tokens, are walked one by one.  In float32 without `chunked` all rows are walked: ways of cutting a prompt then agree bit for bit, which chunks cannot keep and
 bfloat16 steps, whose products change with the number of rows, do not promise.
 """
 from __future__ import annotations
