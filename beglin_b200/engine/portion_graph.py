@@ -148,7 +148,7 @@ class PortionGraphs:
 
     BOUND_STEP = 4096          # `bound` grows in steps of this many positions
 
-    def __init__(self, engine, min_rows: int = 256, max_wanted: int = 8, keep: int = 4):
+    def __init__(self, engine, min_rows: int = 256, max_wanted: int = 64, keep: int = 4):
         self.engine, self.min_rows, self.max_wanted, self.keep = engine, min_rows, max_wanted, keep
         self.graphs: Dict[tuple, PortionGraph] = {}
         self.seen: List[tuple] = []
