@@ -99,6 +99,22 @@ class TensorCoreProduct:
                                       None if norm_weight is None else norm_weight.data_ptr(), eps,
                                       None if bias is None else bias.data_ptr(), *rope, self.fused_splits(T), self._status_ptr)
 
+    def complete_splits(self, T: int) -> int:
+        """The ranges of K of a COMPLETE product of few rows (no consumer adds partial sums up), which the fused kernel's CTAs of a tile
+        add inside a cluster; 1: the plain kernel, one CTA a tile.  As `fused_splits`, but no more CTAs than run side by side: some
+        256 with up to 32 rows (two share an SM), one an SM with 64.  4,096 x 4,096: 20.8 us on 32 CTAs -> 8.7 in eight ranges (32
+        rows), 21.9 -> 11.1 in four (64 rows; in eight 20.9); 9,216 x 1,536: 10.4 -> 9.8 in two (32 rows; in four 13.3), 11.4 and
+        11.5 (64 rows)."""
+        s = self._splits.get(("complete", T))
+        if s is None:
+            s = 1
+            if self.ctx.fuse and T <= FEW_TOKENS and self.k % 8 == 0:
+                s, most = self.fused_splits(T), 256 if T <= 32 else self.sms
+                while s > 1 and (self.tiles * s > most or (s - 1) * -(-self.k_blocks // s) >= self.k_blocks):
+                    s //= 2
+            self._splits[("complete", T)] = s
+        return s
+
     # ------------------------------------------------------------------ the product of many rows on pairs of CTAs
     def pairs(self, T: int) -> bool:
         """Whether a step of T rows runs gate/up with SwiGLU as ONE kernel of CTA pairs (measured at the 1.5B and
@@ -135,6 +151,13 @@ class TensorCoreProduct:
             out = torch.empty((T, self.n_out), dtype=torch.bfloat16, device=x.device)
             ops.gemm_pair_unchecked(x, self._w_ptr, self.n_out, self.k, self._ldw, out, ops.PAIR_PLAIN, self._status_ptr,
                                     None if bias is None else bias.data_ptr())
+            return out
+        if not partial and self.complete_splits(T) > 1:
+            if x.dtype != torch.bfloat16 or x.stride(1) != 1 or x.shape[1] != self.k or x.stride(0) % 8:
+                raise ops.KernelError(f"the tcgen05 product takes contiguous bfloat16 rows of {self.k} features")
+            out = torch.empty((T, self.n_out), dtype=out_dtype, device=x.device)
+            ops.gemm_fused_unchecked(self._w_ptr, self.n_out, self.k, self._ldw, T, out, ops.FUSED_PLAIN, x, None, None, None, 0.0,
+                                     None if bias is None else bias.data_ptr(), None, self.complete_splits(T), self._status_ptr)
             return out
         s = self.splits(T) if partial else 1
         if s > 1:
