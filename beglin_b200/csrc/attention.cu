@@ -361,7 +361,7 @@ extern "C" int bg_attention_partial(const void* q, int q_dtype, int q_stride, co
         const size_t need = af_smem(hd / maps, hd, vd);
 #define BG_AF_LAUNCH(NC)                                                                                                    \
         do {                                                                                                                \
-            auto kern = attention_f32_kernel<AttnParams, NC>;                                                               \
+            auto kern = maps == 1 && hd <= AF_NARROW ? attention_f32_kernel<AttnParams, NC, true> : attention_f32_kernel<AttnParams, NC, false>; \
             cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)need);             \
             if (e != cudaSuccess) return (int)e;                                                                            \
             launch(kern, grid, dim3(AF_THREADS), need, stream, p);                                                          \

@@ -5,9 +5,9 @@
 // 16 x 16 owns rows ty + 16 i (i < RI, as many sixteens as the block has rows), of the scores keys tx + 16 j, of the output columns
 // 4 tx .. 4 tx + 3 of every 64.  Scores: rows and keys lie with the features innermost, so four features of a row are one 16-byte
 // read and two of them one operand of the packed multiply-add (fma.rn.f32x2: two float multiply-adds; the even and the odd features
-// are two chains whose sums are added).  A row's sixteen threads lie in one half of a warp: maximum and sum are shuffles, and the
-// weights pass through shared memory behind a warp's barrier only.  The keys of the next tile come (cp.async) under the value
-// product, the values under the scores.  112 KB of shared memory for heads of 128, so that two CTAs share an SM.  Bound by the float
+// are two chains whose sums are added; heads of up to AF_NARROW features are one chain, which takes no longer there: 2,048 rows of 8 heads of
+// 32, 188 and 194 us).  A row's sixteen threads lie in one half of a warp: maximum and sum are shuffles, and the weights pass through
+// shared memory behind a warp's barrier only.  The keys of the next tile come (cp.async) under the value product, the values under the scores.  112 KB of shared memory for heads of 128, so that two CTAs share an SM.  Bound by the float
 // units' issue: the mixer of 550 rows of 12 heads of 128 over 1,536 to 3,000 held positions takes 563 us with its products, 2,818 us
 // with a key a lane and two reads of shared memory for every multiply-add.
 //
@@ -19,6 +19,7 @@
 namespace bg {
 
 constexpr int AF_ROWS = 64, AF_KEYS = 64, AF_THREADS = 256;
+constexpr int AF_NARROW = 32;              // features of a head up to which a score is one chain of sums
 
 __device__ __forceinline__ unsigned long long af_fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
     unsigned long long d;
@@ -58,7 +59,7 @@ __host__ __device__ __forceinline__ size_t af_smem(int qhd, int hd, int vd) {
     return ((size_t)AF_ROWS * qhd + (size_t)AF_KEYS * (af_kld(hd) + af_vld(vd)) + (size_t)AF_ROWS * AF_KEYS + AF_KEYS) * sizeof(float);
 }
 
-template <typename P, int RI, int NC>
+template <typename P, int RI, int NC, bool NARROW>
 __device__ __forceinline__ void af_walk(const P& p, const AfShared& s, int req, int row0, int kvh, int sp, int n_rows,
                                         int k_first, int k_end, int lo_first) {
     const int tid = threadIdx.x, lane = tid & 31, ty = (tid >> 5) * 2 + (lane >> 4), tx = lane & 15;
@@ -138,7 +139,20 @@ __device__ __forceinline__ void af_walk(const P& p, const AfShared& s, int req, 
         const float* qr = s.q + ty * s.qld;
         const float* kr = s.k + tx * s.kld;
         const int sw = tx & 7;             // (rows tx + 16 j have the same low bits)
-        if (p.maps == 1) {
+        if constexpr (NARROW) {
+            for (int c = 0; c < (qhd >> 2); ++c) {
+                float4 a[RI], b[4];
+#pragma unroll
+                for (int i = 0; i < RI; ++i) a[i] = *reinterpret_cast<const float4*>(qr + i * 16 * s.qld + c * 4);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) b[j] = *reinterpret_cast<const float4*>(kr + j * 16 * s.kld + ((c & ~7) | ((c ^ sw) & 7)) * 4);
+#pragma unroll
+                for (int i = 0; i < RI; ++i)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)            // (in the low half; the high one stays nought)
+                        sc[i][j] = __float_as_uint(fmaf(a[i].w, b[j].w, fmaf(a[i].z, b[j].z, fmaf(a[i].y, b[j].y, fmaf(a[i].x, b[j].x, af_low(sc[i][j]))))));
+            }
+        } else if (p.maps == 1) {
 #pragma unroll 4
             for (int c = 0; c < (qhd >> 2); ++c) {
                 ulonglong2 a[RI], b[4];
@@ -261,7 +275,8 @@ __device__ __forceinline__ void af_walk(const P& p, const AfShared& s, int req, 
     }
 }
 
-template <typename P, int NC>
+// (NARROW: one map of heads of up to AF_NARROW features)
+template <typename P, int NC, bool NARROW>
 __global__ void __launch_bounds__(AF_THREADS, NC <= 2 ? 2 : 1) attention_f32_kernel(P p) {
     extern __shared__ __align__(16) float af_s[];
     pdl_launch();
@@ -289,9 +304,9 @@ __global__ void __launch_bounds__(AF_THREADS, NC <= 2 ? 2 : 1) attention_f32_ker
     if (s.vld > p.vd)
         for (int idx = threadIdx.x; idx < AF_KEYS * (s.vld - p.vd); idx += AF_THREADS)
             s.v[idx / (s.vld - p.vd) * s.vld + p.vd + idx % (s.vld - p.vd)] = 0.0f;
-    if (n_rows <= 16) af_walk<P, 1, NC>(p, s, req, row0, kvh, sp, n_rows, k_first, k_end, lo_first);
-    else if (n_rows <= 32) af_walk<P, 2, NC>(p, s, req, row0, kvh, sp, n_rows, k_first, k_end, lo_first);
-    else af_walk<P, 4, NC>(p, s, req, row0, kvh, sp, n_rows, k_first, k_end, lo_first);
+    if (n_rows <= 16) af_walk<P, 1, NC, NARROW>(p, s, req, row0, kvh, sp, n_rows, k_first, k_end, lo_first);
+    else if (n_rows <= 32) af_walk<P, 2, NC, NARROW>(p, s, req, row0, kvh, sp, n_rows, k_first, k_end, lo_first);
+    else af_walk<P, 4, NC, NARROW>(p, s, req, row0, kvh, sp, n_rows, k_first, k_end, lo_first);
 }
 
 }  // namespace bg

@@ -12,6 +12,10 @@
 // float units, is what an 8 x 8 block of single multiply-adds waits for: 51 TFLOP/s on 148 SMs from registers alone, 68 with packed
 // ones whose rows are walked to and fro, so that each shares an operand with the one before.
 //
+// Inner sizes of up to GF_SHORT are summed in one chain, k = 0 .. K-1 in order, whatever the rows: two chains and a pipeline over k gain
+// nothing there.
+//
+//   gemm_f32_short_kernel  inner sizes of up to 64
 //   gemm_f32_tile_kernel   tiles of 128 (or 64) rows x 128 columns, for more than 16 rows
 //   gemm_f32_few_kernel    up to 16 rows: the product is a stream of weights
 //   gemm_f32_ranges_kernel adds the sums of ranges that went to CTAs of their own
@@ -22,6 +26,7 @@ namespace bg {
 constexpr int GF_RANGE = 1024;             // a multiple of every step of k below
 constexpr int GF_BN = 128, GF_BK = 16, GF_LD = GF_BK + 4, GF_STAGES = 4, GF_THREADS = 256;
 constexpr int GF_FEW = 16;                 // rows up to which the product is treated as a stream of weights
+constexpr int GF_SHORT = 64;               // inner sizes up to which a product is one chain of sums
 
 struct GfParams {
     const float* A; const float* W; const float* bias; float* C;
@@ -61,6 +66,64 @@ __device__ __forceinline__ void gf_fetch(float* dst, const float* src, int ld, i
         const int r = threadIdx.x / PER_ROW + i * (GF_THREADS / PER_ROW), c = threadIdx.x % PER_ROW * W;
         const bool in = r < rows && k + c < K;
         gf_async<W * 4>(dst + r * GF_LD + c, src + (in ? (size_t)((unsigned)r * (unsigned)ld + (unsigned)(k + c)) : 0), in);
+    }
+}
+
+// Inner sizes of up to GF_SHORT (narrow models, small heads): both operands come whole, BM rows and 64 columns, and a thread sums
+// rows ty + 16 i and columns tx + 16 j, four k of a row at a read (rows 68 floats apart: eight neighbouring ones in different banks).
+// Bound by its reads of shared memory and by the results it writes.  2,048 x 4,096 with k of 64: 36 us, 51 in two chains by the pipelined
+// tiles; sixteen products of 2,048 x 512: 71 and 89, with k of 32 43 and 63.
+constexpr int GS_BN = 64, GS_LD = GF_SHORT + 4;
+template <int BM>
+__global__ void __launch_bounds__(GF_THREADS) gemm_f32_short_kernel(GfParams p) {
+    constexpr int RI = BM / 16, CJ = GS_BN / 16, EACH = GF_THREADS / 32;          // EACH: rows that the threads bring at a time
+    __shared__ __align__(16) float As[BM * GS_LD], Ws[GS_BN * GS_LD];
+    pdl_launch();
+    pdl_wait();
+    const int m0 = blockIdx.y * BM, n0 = blockIdx.x * GS_BN, tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const float* A = p.A + (size_t)blockIdx.z * p.batch_a;
+    const float* W = p.W + (size_t)blockIdx.z * p.batch_w;
+#pragma unroll
+    for (int h = 0; h < GF_SHORT; h += 32) {             // (zeros behind K, the rows and the columns)
+        const int k = h + lane;
+        if (h >= p.K) break;
+#pragma unroll
+        for (int r = warp; r < BM; r += EACH) As[r * GS_LD + k] = k < p.K && m0 + r < p.M ? A[(size_t)(m0 + r) * p.lda + k] : 0.0f;
+#pragma unroll
+        for (int r = warp; r < GS_BN; r += EACH) Ws[r * GS_LD + k] = k < p.K && n0 + r < p.N ? W[(size_t)(n0 + r) * p.ldw + k] : 0.0f;
+    }
+    __syncthreads();
+    float acc[RI][CJ];
+#pragma unroll
+    for (int i = 0; i < RI; ++i)
+#pragma unroll
+        for (int j = 0; j < CJ; ++j) acc[i][j] = 0.0f;
+#pragma unroll 4
+    for (int k = 0; k < p.K; k += 4) {
+        float4 a[RI], w[CJ];
+#pragma unroll
+        for (int i = 0; i < RI; ++i) a[i] = *reinterpret_cast<const float4*>(As + (ty + 16 * i) * GS_LD + k);
+#pragma unroll
+        for (int j = 0; j < CJ; ++j) w[j] = *reinterpret_cast<const float4*>(Ws + (tx + 16 * j) * GS_LD + k);
+#pragma unroll
+        for (int i = 0; i < RI; ++i)
+#pragma unroll
+            for (int j = 0; j < CJ; ++j)
+                acc[i][j] = fmaf(a[i].w, w[j].w, fmaf(a[i].z, w[j].z, fmaf(a[i].y, w[j].y, fmaf(a[i].x, w[j].x, acc[i][j]))));
+    }
+#pragma unroll
+    for (int i = 0; i < RI; ++i) {
+        const int m = m0 + ty + 16 * i;
+        if (m >= p.M) continue;
+#pragma unroll
+        for (int j = 0; j < CJ; ++j) {
+            const int n = n0 + tx + 16 * j;
+            if (n >= p.N) continue;
+            const float v = p.bias ? acc[i][j] + p.bias[n] : acc[i][j];
+            float* c = p.C + (size_t)blockIdx.z * p.batch_c + (size_t)m * p.ldc + n;
+            *c = p.accumulate ? *c + v : v;
+        }
     }
 }
 
@@ -354,6 +417,14 @@ static int gf_run(GfParams p, cudaStream_t stream) {
     const bool vec = p.K % 4 == 0 && p.lda % 4 == 0 && p.ldw % 4 == 0 && p.batch_a % 4 == 0 && p.batch_w % 4 == 0 &&
                      (uintptr_t)p.A % 16 == 0 && (uintptr_t)p.W % 16 == 0;
     p.ranges = (p.K + GF_RANGE - 1) / GF_RANGE;
+    if (p.K <= GF_SHORT) {
+        const int bm = p.M <= 16 ? 16 : 64;
+        const dim3 grid((p.N + GS_BN - 1) / GS_BN, (p.M + bm - 1) / bm, p.batch);
+        if (grid.y > 65535) return BG_ERR_SHAPE;
+        const cudaError_t e = bm == 16 ? launch(gemm_f32_short_kernel<16>, grid, dim3(GF_THREADS), 0, stream, p)
+                                       : launch(gemm_f32_short_kernel<64>, grid, dim3(GF_THREADS), 0, stream, p);
+        return e == cudaSuccess ? BG_OK : (int)e;
+    }
     if (gf_few(p.M, p.ranges, vec)) {
         if (gf_few_shares(p.N, p.ranges, p.batch) == 1) p.part = nullptr;
         cudaError_t e = p.M <= 2 ? gf_launch_few<1>(p, stream) : p.M <= 4 ? gf_launch_few<2>(p, stream)

@@ -191,6 +191,19 @@ def test_gemm_f32_kernels_agree_bit_for_bit(ops, N, K):
             assert torch.equal(out[e], f * plain)
 
 
+@pytest.mark.parametrize("K", [1, 31, 32, 33, 63, 64, 65])                # on both sides of what is summed in one chain
+def test_gemm_f32_short_inner_sizes(ops, K):
+    test_gemm_f32_kernels_agree_bit_for_bit(ops, 130, K)
+    a, w = rnd(70, K, seed=1), rnd(67, K, seed=2)
+    if K <= 64:                                                           # the chain itself: products are exact in 64 bits
+        chain = torch.zeros((70, 67), dtype=torch.float64, device=DEV)
+        for k in range(K):
+            chain = (chain + a[:, k:k + 1].double() * w[:, k].double()).float().double()
+        out = torch.empty((70, 67), device=DEV)
+        ops.gemm_f32_nt(a, w, None, out)
+        assert float((out.double() == chain).double().mean()) > 0.999     # (one sum in 2^29 is rounded twice here)
+
+
 @pytest.mark.parametrize("interleaved", [False, True])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("hd,rot", [(48, 32), (64, 64), (128, 128)])      # partial rotary; whole heads (16-byte path)
