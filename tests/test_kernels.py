@@ -435,6 +435,43 @@ def test_attention_float32_in_blocks_of_any_rows(ops, nh, nkv, hd, vd, options):
     assert float((outs[0].double() - want).abs().max()) < bound
 
 
+@pytest.mark.parametrize("nh,nkv,hd,vd,window,keep", [(6, 1, 128, 128, 0, 0), (2, 2, 64, 64, 40, 3), (3, 1, 36, 132, 70, 0), (1, 1, 256, 256, 0, 0), (4, 2, 30, 30, 50, 0)])
+@pytest.mark.parametrize("bad", [math.inf, math.nan])
+def test_attention_float32_leaves_out_what_a_row_does_not_see(ops, nh, nkv, hd, vd, window, keep, bad):
+    """A value that is infinite or not a number reaches the rows that see its position, and no other: not the rows of the same block in
+    front of it, nor those whose window has left it behind, nor one that gives it a weight of nought."""
+    page, n, group = 16, 200, nh // nkv
+    at = 130                                               # inside a tile, a block of rows and a page
+    q, k, v = rnd(n, nh, hd, seed=1), rnd(n, nkv, hd, seed=2), rnd(n, nkv, vd, seed=3)
+    q[:, :, 0] = 0.0
+    q[150] = 0.0
+    k[at, :, 0] = -1e4
+    q[150, :, 0] = 1e3                                     # a weight that underflows
+    pages = -(-n // page)
+    positions = torch.arange(n, dtype=torch.int32, device=DEV)
+    table = torch.arange(pages, dtype=torch.int32, device=DEV).view(1, -1)
+    _, bq, tile = ops.attention_plan(group, hd, torch.float32, False, "generic", page, vd=vd)
+    qblk = torch.tensor([(0, b, min(bq, n - b)) for b in range(0, n, bq)], dtype=torch.int32, device=DEV)
+    outs = []
+    for value in (0.25, bad):
+        v[at, :, 1] = value
+        pad = lambda t: torch.cat([t, torch.zeros((pages * page - n,) + t.shape[1:], device=DEV)]).view(pages, page, nkv, -1)
+        pool = torch.cat([pad(k).transpose(1, 2).reshape(pages, -1), pad(v).transpose(1, 2).reshape(pages, -1)], dim=1)
+        if vd == hd:
+            pool = pool.view(pages, 2, nkv, page, hd)
+        status = ops.new_status(DEV)
+        out = torch.full((n, nh * vd), -7.0, device=DEV)
+        ops.attention(q.view(n, -1), nh * hd, pool, table, positions, qblk, qblk.shape[0], n - 1, n, nh, nkv, hd, window, 64, tile, bq,
+                      hd ** -0.5, out, status, "generic", vd=vd, keep=keep)
+        ops.raise_on_status(status)
+        outs.append(out.view(n, nh, vd))
+    sees = (positions >= at) & ((positions < at + window) if window else (positions >= 0)) & (positions != 150)
+    assert torch.isfinite(outs[0]).all() and torch.equal(outs[1][~sees], outs[0][~sees])
+    assert not torch.isfinite(outs[1][at, :, 1]).any()
+    other = torch.arange(vd, device=DEV) != 1              # (nor any other feature)
+    assert torch.equal(outs[1][..., other], outs[0][..., other])
+
+
 @pytest.mark.parametrize("nh,nkv,hd,page,window", [(4, 2, 16, 8, 10), (12, 2, 128, 16, 64), (5, 5, 48, 16, 1),
                                                    (3, 1, 32, 16, 100)])
 def test_attention_window(ops, nh, nkv, hd, page, window):
