@@ -9,6 +9,11 @@
 // small parts are added up before any h h, so that their sums are not rounded at the size of the large ones, and the h h products go
 // half to an accumulator of their own; both are float in tensor memory and meet once, at the end.
 //
+// A number without three parts (infinite, not a number, or within a rounding of the largest float) makes whatever it is multiplied with not a
+// number.  Where floats would do the same or make an infinity of it, that is left so: the sums, the state, a row's own query and scores.
+// A value must not: the product multiplies it with the weights of nought of the queries in front of it, too.  Such values go into the
+// tile as nought and are added afterwards, by floats, to the outputs of their own token and those behind it.
+//
 // The values' features are the M side of both products (an operand stored [token][feature] or [i][feature] is read M-major), so a lane
 // of tensor memory is a feature and results leave in rows of 128 bytes.  A CTA of 256 threads converts what it fetches into swizzled
 // tiles, the first warp issues the MMAs, all wait; two CTAs share an SM (96 KB, half of tensor memory each), so that one converts while the
@@ -29,6 +34,7 @@ struct CtShared {
     unsigned long long done;
     unsigned tmem;
     int failed;
+    int odd;                                 // a value of the chunk has no three parts
 };
 
 // x = h + m + l
@@ -38,6 +44,7 @@ __device__ __forceinline__ void ct_split(float x, __nv_bfloat16& h, __nv_bfloat1
     m = __float2bfloat16_rn(r);
     l = __float2bfloat16_rn(r - __bfloat162float(m));
 }
+__device__ __forceinline__ bool ct_splits(float x) { return fabsf(x) <= 3.3895313e38f; }       // (the largest bfloat16 number)
 // the byte of element (row, col) in a part of a tile of 64 rows: blocks of 64 columns, rows of 128 bytes, 128-byte swizzle
 __device__ __forceinline__ unsigned ct_at(int row, int col) {
     return (unsigned)(col >> 6) * CT_BLOCK + (unsigned)row * 128 + ((unsigned)(((col >> 3) ^ row) & 7) << 4) + (unsigned)(col & 7) * 2;
@@ -111,7 +118,7 @@ __host__ __device__ constexpr unsigned ct_idesc(int n, bool a_m, bool b_n) { ret
 
 // Barrier and tensor memory; the kernel behind this one may come only once the columns are held.
 __device__ __forceinline__ void ct_begin(CtShared& s) {
-    if (threadIdx.x == 0) { mbar_init(&s.done, 1); s.failed = 0; mbar_init_fence(); }
+    if (threadIdx.x == 0) { mbar_init(&s.done, 1); s.failed = 0; s.odd = 0; mbar_init_fence(); }
     if (threadIdx.x < 32) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(&s.tmem)), "r"(CT_COLS) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
@@ -256,10 +263,18 @@ __global__ void __launch_bounds__(CT_THREADS, 2) chunk_out_tc_kernel(R r) {
     } else {
         c.weights([&](int t, int j, float w) { ct_put1(qt, part, t, j, w); });
     }
-    ct_put<SV>(xt, part, raw, r.nv, [&](const float4& x, int j, int v) { return c.out_value(x, j, v); });
+    ct_put<SV>(xt, part, raw, r.nv, [&](const float4& x, int j, int v) {
+        float4 y = c.out_value(x, j, v);
+        if (!(ct_splits(y.x) && ct_splits(y.y) && ct_splits(y.z) && ct_splits(y.w))) {
+            s.odd = 1;
+            y.x = ct_splits(y.x) ? y.x : 0.0f; y.y = ct_splits(y.y) ? y.y : 0.0f;
+            y.z = ct_splits(y.z) ? y.z : 0.0f; y.w = ct_splits(y.w) ? y.w : 0.0f;
+        }
+        return y;
+    });
     ct_issue(s, [&] { ct_mma<true, false>(d, d + 64, x_a, part, q_a, part, CT / 16, CT / 32, ct_idesc(CT, true, false), true); });
     ct_wait(s, phase);
-    float* out = reinterpret_cast<float*>(qt);               // [CT][CT_OUT_LD]
+    float* out = reinterpret_cast<float*>(xt);               // [CT][CT_OUT_LD] (the weights stay where they are)
     {
         const int v = (warp & 3) * 32 + lane;
         for (int t0 = (warp >> 2) * 32; t0 < (warp >> 2) * 32 + 32; t0 += 16) {
@@ -278,6 +293,21 @@ __global__ void __launch_bounds__(CT_THREADS, 2) chunk_out_tc_kernel(R r) {
     }
     tc_fence_before();
     __syncthreads();
+    if (s.odd) {                             // values that the product left out: column v by two threads, every other query each
+        const int v = threadIdx.x & 127;
+        for (int j = 0; v < r.nv && j < c.rows; ++j) {
+            const float4 x4 = c.out_value(c.value_raw(j, v & ~3), j, v & ~3);
+            const float x = (v & 2) ? ((v & 1) ? x4.w : x4.z) : ((v & 1) ? x4.y : x4.x);
+            if (ct_splits(x)) continue;
+            for (int t = j + ((threadIdx.x >> 7) ^ (j & 1)); t < c.rows; t += 2) {
+                const unsigned char* w = qt + ct_at(t, j);
+                const float P = __bfloat162float(*reinterpret_cast<const __nv_bfloat16*>(w)) + __bfloat162float(*reinterpret_cast<const __nv_bfloat16*>(w + part)) +
+                                __bfloat162float(*reinterpret_cast<const __nv_bfloat16*>(w + 2 * part));
+                out[t * CT_OUT_LD + v] = fmaf(P, x, out[t * CT_OUT_LD + v]);
+            }
+        }
+        __syncthreads();
+    }
     if (!s.failed) c.finish(out);
     ct_end(s, r.status);
 }

@@ -143,3 +143,61 @@ def test_mamba2(ops, H, P, N, G, lens):
     ops.raise_on_status(status)
     close(y, want, 64)
     close(state.view(len(lens), H, P, N).transpose(2, 3), states, 64)
+
+
+def _decay(ops, bad):
+    H, n, nv, T, at = 2, 64, 96, 150, 90
+    src = rnd(T, H * (2 * n + 2 * nv), seed=1)
+    src[at, 2 * H * n + nv + 5] = bad                    # head 1, value 5
+    state, y = rnd(1, H * n * nv, seed=2), torch.full((T, H * nv), float("nan"), device=DEV)
+    chunks, n_chunks, longs, n_long = lists([T], ops.decay_attention_chunk(n, nv))
+    status = ops.new_status(DEV)
+    ops.decay_attention(src, 0, H * n, 2 * H * n, torch.tensor([0.5, 0.875], device=DEV), state, torch.zeros(1, dtype=torch.int32, device=DEV), None, 0,
+                        y, H, n, nv, chunks, n_chunks, longs, n_long, tensor_cores=True, status=status)
+    ops.raise_on_status(status)
+    return y.view(T, H, nv), state.view(H, n, nv), at
+
+
+def _per_channel(ops, bad):
+    H, n, nv, T, at = 2, 96, 64, 150, 90
+    qd, vd = H * n, H * nv
+    src = rnd(T, 2 * qd + 2 * vd, seed=1)
+    src[at, 2 * qd + nv + 5] = bad
+    state, out = rnd(1, H * n * nv, seed=6), torch.full((T, vd), float("nan"), dtype=torch.bfloat16, device=DEV)
+    chunks, n_chunks, longs, n_long = lists([T], ops.gla_chunk(n, nv))
+    status = ops.new_status(DEV)
+    ops.gated_linear_attention(src, 0, qd, 2 * qd, rnd(qd, seed=2), rnd(nv, seed=5), 1e-6, state, torch.zeros(1, dtype=torch.int32, device=DEV), None, 0,
+                               out, H, n, nv, lower=torch.full((qd,), 0.5, device=DEV), q_scale=0.5, g_col=2 * qd + vd, chunks=chunks,
+                               n_chunks=n_chunks, longs=longs, n_long=n_long, status=status)
+    ops.raise_on_status(status)
+    return out.view(T, H, nv), state.view(H, n, nv), at
+
+
+def _mamba2(ops, bad):
+    H, P, N, T, at = 2, 80, 96, 150, 90
+    xbc = rnd(T, H * P + 2 * N, seed=1)
+    xbc[at, P + 5] = bad
+    state, y = rnd(1, H * N * P, seed=6), torch.full((T, H * P), float("nan"), device=DEV)
+    chunks, n_chunks, longs, n_long = lists([T], ops.ssm_chunk(H, P, N, 1))
+    status = ops.new_status(DEV)
+    ops.ssm_scan(xbc, rnd(T, H + 1, seed=2), 1, rnd(H, seed=3), rnd(H, seed=4), rnd(H, seed=5), state, torch.zeros(1, dtype=torch.int32, device=DEV), None, 0,
+                 y, H, P, N, 1, chunks, n_chunks, longs, n_long, tensor_cores=True, status=status)
+    ops.raise_on_status(status)
+    return y.view(T, H, P), state.view(H, P, N).transpose(1, 2), at
+
+
+@pytest.mark.parametrize("bad", [math.inf, math.nan, -3.4e38])
+@pytest.mark.parametrize("run", [_decay, _per_channel, _mamba2], ids=["constant", "per_channel", "mamba2"])
+def test_a_value_reaches_its_own_token_and_those_behind_it(ops, run, bad):
+    """A value that is infinite, not a number or at float's end: the tokens of its chunk in front of it and the other heads keep their bits, and
+    without a norm over the head the other features, too; its own column of the state holds it."""
+    clean, clean_state, at = run(ops, 0.25)
+    y, state, _ = run(ops, bad)
+    assert torch.isfinite(clean).all() and torch.equal(y[:at], clean[:at]) and torch.equal(y[:, 0], clean[:, 0])
+    assert torch.equal(state[0], clean_state[0])
+    other = torch.arange(clean.shape[2], device=DEV) != 5
+    assert torch.equal(state[1][:, other], clean_state[1][:, other])
+    if run is not _per_channel:
+        assert torch.equal(y[:, 1][:, other], clean[:, 1][:, other])
+    if bad != -3.4e38:
+        assert not torch.isfinite(y[at, 1, 5]) and not torch.isfinite(state[1][:, 5]).any()
