@@ -50,7 +50,7 @@ __global__ void conv_silu_kernel(const TI* __restrict__ src, int src_stride, int
 // keeps the last TAPS - 1 inputs in registers, so that an input is read once and not TAPS times, 16 bytes at a time; where a request
 // begins inside the run the inputs before it come from its state.  Every output is the same chain of multiply-adds.  Bound by bytes
 // (2,048 rows of 3,328 channels, four taps: 57 -> 20 us; 4,096 channels 70 -> 18).
-constexpr int CONV_ROWS = 8;
+constexpr int CONV_ROWS = 8, CONV_FROM = 96;
 template <typename TW, int TAPS>
 __global__ void __launch_bounds__(128)
 conv_silu_vec4_kernel(const float* __restrict__ src, int src_stride, int col0, int channels, const TW* __restrict__ w,
@@ -389,6 +389,12 @@ gated_group_rmsnorm_vec8_kernel(const float* __restrict__ y, const TI* __restric
 
 using namespace bg;
 
+// Rows that a thread of the convolution takes: runs where requests fill them, eight rows or more a request on average, and there are blocks for
+// the SMs.  Rows of requests of their own (a decoding step) stay a thread each: in a run every one of them is a chain of
+// loads, of its request, its slot and its state, behind the one before.  3,328 channels: 64 rows of 64 requests 6.9 us, in runs 10.0; 64 rows of
+// one request 5.1 and 6.3, 96 6.2 and 6.4, 128 7.0 and 6.5, 256 10.2 and 7.1; 256 rows of 32 requests 10.2 and 7.8.
+extern "C" int bg_conv_silu_run(int n_rows, int n_req) { return n_rows >= CONV_FROM && n_rows >= CONV_ROWS * (long long)n_req ? CONV_ROWS : 1; }
+
 extern "C" int bg_conv_silu(const void* src, int src_dtype, int src_stride, int col0, int channels, int taps, const void* w,
                             const void* b, int w_dtype, float* state, long long slot_stride, long long conv_off,
                             const int* slots, const int* row_req, const int* reqs, int n_req, float* out, int n_rows,
@@ -397,9 +403,8 @@ extern "C" int bg_conv_silu(const void* src, int src_dtype, int src_stride, int 
     if (channels <= 0 || taps < 1 || n_req > 65535) return BG_ERR_SHAPE;
     const unsigned bx = (unsigned)((channels + 127) / 128);
     if (bx > 65535) return BG_ERR_SHAPE;
-    // Runs of rows from 32 rows on (fewer would leave most SMs without a block, and a decoding step's rows are runs of one anyway),
-    // for 2 to 4 taps, where every row of inputs, state and outputs is made of whole 16-byte pieces.
-    if (src_dtype == BG_DTYPE_F32 && n_rows >= 32 && taps >= 2 && taps <= 4 && channels % 4 == 0 && col0 % 4 == 0 && src_stride % 4 == 0 &&
+    // Runs of rows for 2 to 4 taps, where every row of inputs, state and outputs is made of whole 16-byte pieces.
+    if (src_dtype == BG_DTYPE_F32 && bg_conv_silu_run(n_rows, n_req) > 1 && taps >= 2 && taps <= 4 && channels % 4 == 0 && col0 % 4 == 0 && src_stride % 4 == 0 &&
         slot_stride % 4 == 0 && conv_off % 4 == 0 && (uintptr_t)src % 16 == 0 && (uintptr_t)state % 16 == 0 && (uintptr_t)out % 16 == 0) {
         const dim3 grid((n_rows + CONV_ROWS - 1) / CONV_ROWS, (channels / 4 + 127) / 128);
 #define BG_CONV(TAPS)                                                                                                          \

@@ -59,3 +59,12 @@ def test_query_blocks_cut_rows_of_one_request_only():
 def test_ids_beyond_int32_become_a_value_the_embedding_kernel_reports():
     b = StepBatch([Entry("a", [3, 2 ** 40, -7], [])], [0], "cpu")
     assert b.token_ids.tolist() == [3, -1, -1]
+
+
+def test_convolution_keeps_decoding_steps_out_of_runs():
+    """Runs of eight rows a thread are for requests that fill them: single tokens of many requests stay a thread each."""
+    from beglin_b200.csrc import ops
+    run = ops.lib().bg_conv_silu_run
+    for n in (1, 8, 32, 64, 256, 4096):
+        assert run(n, n) == 1                                     # decoding
+    assert run(95, 1) == 1 and run(96, 1) == 8 and run(2048, 1) == 8 and run(2048 + 60, 61) == 8 and run(127, 16) == 1 and run(128, 16) == 8
