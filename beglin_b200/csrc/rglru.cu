@@ -5,8 +5,8 @@
 //   S <- a S + sqrt(1 - a^2) (i u),   out = S * gelu_tanh(y)      y: the other branch's product of the same token
 //
 // from S = 0 at a request's start (the first token is no special case).  Everything is float: the gates, the decay and
-// its logarithm, the step and the state.  a = 1 + e and 1 - a^2 = -e (2 + e) with e = expm1(log a): one exponential for both, and no
-// cancellation for a near one.
+// its logarithm, the step and the state.  1 - a^2 = -e (2 + e) with e = expm1(log a), which does not cancel for a near one, and a = 1 + e
+// down to a half; below, where 1 + e would keep fewer and fewer of a's own digits, a is an exponential of its own.
 //
 //   rglru_scan          one thread per (request, channel) walks the request's rows of the step in order from the state
 //                       in the request's slot and leaves the new state there.  Steps of single tokens and short portions.
@@ -48,8 +48,8 @@ __device__ __forceinline__ float gelu_tanh32(float z) {
 
 // (a, b) of S <- a S + b from the gates' arguments and the convolved input
 __device__ __forceinline__ void lru_values(float gr, float gi, float u, float spc, float* a, float* b) {
-    const float e = expm1f(-sigmoid32(gr) * spc);
-    *a = 1.0f + e;
+    const float log_a = -sigmoid32(gr) * spc, e = expm1f(log_a);
+    *a = e > -0.5f ? 1.0f + e : expf(log_a);
     *b = sqrtf(fmaf(-e, e, -2.0f * e)) * (sigmoid32(gi) * u);
 }
 

@@ -114,6 +114,31 @@ def test_recurrence_row_by_row_in_chunks_over_steps_and_slots(W, blocks):
     assert torch.isnan(state[[1, 3]]).all() and torch.isnan(state[:, W:]).all()
 
 
+@pytest.mark.parametrize("walk", ["row by row", "chunks", "chunks of odd rows"])
+def test_recurrence_without_input_decays_to_the_last_digit(walk):
+    """Decays from e^-0.01 to e^-60 and no input: the state is the start's times the product of the decays, each to its own digits."""
+    from beglin_b200.engine.batch import cut_long_requests
+    o, W, T = ops(), 128, 3 if walk == "row by row" else 70
+    log_a = torch.linspace(0.01, 60.0 if T == 3 else 1.2, W, dtype=torch.float64)
+    gates = torch.full((1, T, 2 * W), 40.0, device=DEV)              # a sigmoid of one
+    decay, state = log_a.float().to(DEV), torch.full((1, W), 3.0, device=DEV)
+    zero, odd = torch.zeros(W, device=DEV), 1 if walk == "chunks of odd rows" else 0
+    src, u, out = torch.ones(T, W + odd, device=DEV), torch.zeros(T, W, device=DEV), torch.full((T, W), float("nan"), device=DEV)
+    if walk == "row by row":
+        lists = dict()
+        args = (torch.tensor([[0, 0, T]], dtype=torch.int32, device=DEV), 1, out)
+    else:
+        _, chunks, longs = cut_long_requests([0], [T], 32, 1)
+        lists = dict(chunked=(torch.from_numpy(chunks).to(DEV), chunks.shape[0], torch.from_numpy(longs).to(DEV), longs.shape[0], 32))
+        args = (None, 0, out)
+    o.rglru_scan(gates, u, src, odd, zero, zero, decay, state, torch.zeros(1, dtype=torch.int32, device=DEV), *args, **lists)
+    want = 3.0 * torch.exp(-T * log_a.float().double())
+    kept = want > 2.0 ** -120                                        # (what float still holds)
+    off = (state[0].double().cpu() - want).abs() / want
+    # a row's decay: the rounding of log a moves it by log a 2^-24 of itself (the sigmoid's and the product's), expf by two more
+    assert kept.sum() > 40 and bool((off <= T * (2 * log_a + 4) * 2.0 ** -24)[kept].all())
+
+
 @pytest.mark.parametrize("W,blocks", [(2, 1), (24, 3), (258, 1), (512, 2)])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_recurrence_in_chunks_two_channels_a_thread(W, blocks, dtype):
