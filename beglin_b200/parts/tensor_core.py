@@ -108,7 +108,7 @@ class TensorCoreProduct:
         s = self._splits.get(("complete", T))
         if s is None:
             s = 1
-            if self.ctx.fuse and T <= FEW_TOKENS and self.k % 8 == 0:
+            if self.ctx.fuse and 0 < T <= FEW_TOKENS and self.k % 8 == 0:
                 s, most = self.fused_splits(T), 256 if T <= 32 else self.sms
                 while s > 1 and (self.tiles * s > most or (s - 1) * -(-self.k_blocks // s) >= self.k_blocks):
                     s //= 2

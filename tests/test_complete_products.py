@@ -28,3 +28,14 @@ def test_complete_products_of_few_rows(N, K, T):
         off = K * 2.0 ** -24 * size                           # sums of K products in float
         assert ((full.double() - exact).abs() <= off).all()
         assert ((short.double() - exact).abs() <= off + 2.0 ** -8 * (exact.abs() + off)).all()
+
+
+def test_complete_product_of_no_rows():
+    from beglin_b200.csrc import ops
+    from beglin_b200.parts import BuildContext
+    from beglin_b200.parts.linear import Linear
+    ctx = BuildContext(device=DEV, compute_dtype=torch.bfloat16)
+    ctx.status = ops.new_status(DEV)
+    lin = Linear(torch.randn(264, 72), None, ctx)
+    out = lin(torch.empty(0, 72, dtype=torch.bfloat16, device=DEV))
+    assert out.shape == (0, 264) and out.dtype == torch.bfloat16
