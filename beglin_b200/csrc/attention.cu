@@ -312,9 +312,9 @@ __global__ void attention_merge_kernel(const float* __restrict__ part_o, const f
 
 using namespace bg;
 
-static size_t attention_smem_bytes(int bq, int group, int hd, int vd, int tile) {
+static size_t attention_smem_bytes(int bq, int group, int qhd, int hd, int vd, int tile) {
     size_t rows = (size_t)bq * group;
-    size_t floats = rows * (hd + vd) + (size_t)tile * (hd + 1) + (size_t)tile * vd + rows * 2;
+    size_t floats = rows * (qhd + vd) + (size_t)tile * (hd + 1) + (size_t)tile * vd + rows * 2;
     return floats * sizeof(float) + (size_t)2 * tile * sizeof(long long) + 16;
 }
 
@@ -326,14 +326,14 @@ static bool attention_f32_takes(int rows, int hd, int vd, int maps) {
 
 // Rows per query block and keys per tile that fit the shared memory of one CTA for these sizes.
 // Returns 0 and fills bq and tile, or BG_ERR_UNSUPPORTED.
-// (`hd` counts a whole key row; with two maps in it, it may be twice as wide; `f32`: float queries over a float cache)
+// (`hd` counts a whole key row; with two maps in it, it may be twice as wide; `f32`: queries and cache are float)
 extern "C" int bg_attention_plan(int group, int hd, int vd, int maps, int f32, int* bq_out, int* tile_out) {
     if (maps < 1 || hd <= 0 || hd > 32 * ATT_MAX_DPL * maps || vd <= 0 || vd > 32 * ATT_MAX_DPL || group <= 0) return BG_ERR_UNSUPPORTED;
     if (f32 && attention_f32_takes(group, hd, vd, maps)) { *bq_out = AF_ROWS / group; *tile_out = AF_KEYS; return BG_OK; }
     const size_t limit = 200 * 1024;
     for (int tile = 64; tile >= 32; tile >>= 1) {
         for (int bq = 16; bq >= 1; bq >>= 1) {
-            if (attention_smem_bytes(bq, group, hd, vd, tile) <= limit) { *bq_out = bq; *tile_out = tile; return BG_OK; }
+            if (attention_smem_bytes(bq, group, hd, hd, vd, tile) <= limit) { *bq_out = bq; *tile_out = tile; return BG_OK; }
         }
     }
     return BG_ERR_UNSUPPORTED;
@@ -374,7 +374,9 @@ extern "C" int bg_attention_partial(const void* q, int q_dtype, int q_stride, co
         BG_LAUNCH_CHECK();
         return BG_OK;
     }
-    size_t smem = attention_smem_bytes(bq, p.group, hd, vd, tile);
+    size_t smem = attention_smem_bytes(bq, p.group, hd / maps, hd, vd, tile);
+    // blocks that were cut for attention_f32_kernel, which does not take the rows as they lie: its 64 rows fit beside tiles of half as many keys
+    if (smem > 227 * 1024 && tile == 64) smem = attention_smem_bytes(bq, p.group, hd / maps, hd, vd, p.tile = tile = 32);
     if (smem > 227 * 1024) return BG_ERR_UNSUPPORTED;
 #define BG_ATT_LAUNCH(TQ, TC)                                                                              \
     do {                                                                                                   \

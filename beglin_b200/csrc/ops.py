@@ -545,8 +545,9 @@ SINK_KERNELS = ("generic", "tc_rows", "mma_keys", "mma_rows")   # every kernel c
 
 def attention_plan(group: int, hd: int, dtype: torch.dtype = torch.float32, decode_only: bool = False,
                    prefer: str = "auto", page_size: int = 64, vd: Optional[int] = None, softcap: bool = False,
-                   learned_sink: bool = False) -> Tuple[str, int, int]:
-    """(kernel, rows per query block, keys per tile) for these sizes.  Kernels: "mma_keys" (tensor
+                   learned_sink: bool = False, query_dtype: Optional[torch.dtype] = None) -> Tuple[str, int, int]:
+    """(kernel, rows per query block, keys per tile) for these sizes, a cache of `dtype` and queries of `query_dtype` (the cache's, where not
+    given).  Kernels: "mma_keys" (tensor
     cores, one token per block, for steps of single tokens), "mma_rows" (tensor cores, up to 64 rows
     per block) and "generic" (CUDA cores, every size up to head_dim 256, float or bfloat16)."""
     L = lib()
@@ -576,7 +577,7 @@ def attention_plan(group: int, hd: int, dtype: torch.dtype = torch.float32, deco
             raise KernelError(f"the tensor-core attention kernel does not take head_dim {hd} with {group} query "
                               "heads per kv head (head_dim 64 or 128; at most 64 heads per kv head)")
     bq, tile = _c_int(0), _c_int(0)
-    rc = L.bg_attention_plan(group, hd, vd, 1, 1 if dtype == torch.float32 else 0, ctypes.byref(bq), ctypes.byref(tile))
+    rc = L.bg_attention_plan(group, hd, vd, 1, 1 if dtype == (query_dtype or dtype) == torch.float32 else 0, ctypes.byref(bq), ctypes.byref(tile))
     if rc != 0:
         raise KernelError(f"attention: head_dim {hd} (values of {vd}) with {group} query heads per kv head is not "
                           "supported (both sizes must be at most 256)")
@@ -739,7 +740,7 @@ def _attention(q: torch.Tensor, q_stride: int, kv_pool: torch.Tensor, block_tabl
 # ------------------------------------------------------------------------------------------------
 # Differential attention: heads that are pairs of maps over the same values
 def difference_plan(group: int, kw: int, vw: int, dtype: torch.dtype, decode_only: bool, prefer: str = "auto",
-                    page_size: int = 64) -> Tuple[str, int, int]:
+                    page_size: int = 64, query_dtype: Optional[torch.dtype] = None) -> Tuple[str, int, int]:
     """(kernel, rows per query block, keys per tile) for `group` query heads per kv head, maps stored `kw` features wide and values
     `vw`: "tc_rows" (portions on tcgen05, the difference inside the kernel), "mma_keys" (decoding on the tensor cores) or "generic"
     (CUDA cores, every size)."""
@@ -751,7 +752,7 @@ def difference_plan(group: int, kw: int, vw: int, dtype: torch.dtype, decode_onl
                 return "mma_keys", bq.value, 64
         elif prefer in TC_ROWS_FOR and L.bg_attention_tc_plan(group, vw, page_size, ctypes.byref(bq)) == 0:
             return "tc_rows", bq.value, 64
-    if L.bg_attention_plan(2 * group, 2 * kw, vw, 2, 1 if dtype == torch.float32 else 0, ctypes.byref(bq), ctypes.byref(tile)) != 0:
+    if L.bg_attention_plan(2 * group, 2 * kw, vw, 2, 1 if dtype == (query_dtype or dtype) == torch.float32 else 0, ctypes.byref(bq), ctypes.byref(tile)) != 0:
         raise KernelError(f"differential attention: maps of {kw} features (values of {vw}) with {group} query heads per kv head are not "
                           "supported (both sizes must be at most 256)")
     return "generic", bq.value, tile.value

@@ -140,7 +140,7 @@ class GQAAttention:
         khd, kvd_ = (self.hd, self.vd) if self.stored is None else (self.stored, self.stored)     # what the kernels see
         self.plans = {d: ops.attention_plan(self.nh // self.nkv, khd, ctx.cache_dtype, d, ctx.attention,
                                             ctx.page_size, vd=kvd_, softcap=self.score_cap > 0.0,
-                                            learned_sink=self.sink_weight is not None) for d in (False, True)}
+                                            learned_sink=self.sink_weight is not None, query_dtype=ctx.compute_dtype) for d in (False, True)}
         if spec.block is not None and (spec.window is not None or spec.block <= 0):
             raise ValueError("blocks of positions stand in place of a window and hold at least one position")
         if spec.keep_first < 0 or (spec.keep_first and spec.window is None):

@@ -85,7 +85,8 @@ class DifferentialAttention:
         self.lam, self.out_scale = float(np.float32(float(lam))), float(np.float32(1.0 - float(spec.diff)))
         self.kw, self.vw = self.stored(spec, ctx)
         self.window = int(spec.window) if spec.window else 0
-        self.plans = {d: ops.difference_plan(self.nh // self.nkv, self.kw, self.vw, ctx.cache_dtype, d, ctx.attention, ctx.page_size)
+        self.plans = {d: ops.difference_plan(self.nh // self.nkv, self.kw, self.vw, ctx.cache_dtype, d, ctx.attention, ctx.page_size,
+                                              query_dtype=ctx.compute_dtype)
                       for d in (False, True)}
 
     takes_stream = True        # forward takes a NormedInput and may add its result to the stream itself

@@ -472,6 +472,32 @@ def test_attention_float32_leaves_out_what_a_row_does_not_see(ops, nh, nkv, hd, 
     assert torch.equal(outs[1][..., other], outs[0][..., other])
 
 
+@pytest.mark.parametrize("nh,nkv,hd", [(2, 2, 256), (6, 1, 128), (1, 1, 36)])
+@pytest.mark.parametrize("queries", ["bfloat16", "off a boundary"])
+def test_attention_over_a_float_cache_of_other_queries(ops, nh, nkv, hd, queries):
+    """Queries in bfloat16, or float ones off a 16-byte boundary, over a float cache: the CUDA-core kernel, with the blocks of either plan."""
+    page, n, group = 16, 100, nh // nkv
+    q, k, v = rnd(n, nh * hd, seed=1), rnd(n, nkv, hd, seed=2), rnd(n, nkv, hd, seed=3)
+    if queries == "bfloat16":
+        q = q.to(torch.bfloat16)
+    else:
+        q = torch.cat([torch.zeros(1, device=DEV), q.flatten()])[1:].view(n, -1)
+    pages = -(-n // page)
+    pad = lambda t: torch.cat([t, torch.zeros((pages * page - n, nkv, hd), device=DEV)]).view(pages, page, nkv, hd).transpose(1, 2)
+    pool = torch.stack([pad(k), pad(v)], dim=1).contiguous()
+    table, positions = torch.arange(pages, dtype=torch.int32, device=DEV).view(1, -1), torch.arange(n, dtype=torch.int32, device=DEV)
+    s = torch.einsum("thd,shd->hts", q.double().view(n, nh, hd), k.double().repeat_interleave(group, 1)) * hd ** -0.5
+    s = s.masked_fill(positions[None, :] > positions[:, None], -math.inf)
+    want = torch.einsum("hts,shd->thd", torch.softmax(s, -1), v.double().repeat_interleave(group, 1)).reshape(n, -1)
+    for _, bq, tile in (ops.attention_plan(group, hd, torch.float32, False, "generic", page),
+                        ops.attention_plan(group, hd, torch.float32, False, "generic", page, query_dtype=q.dtype)):
+        qblk = torch.tensor([(0, b, min(bq, n - b)) for b in range(0, n, bq)], dtype=torch.int32, device=DEV)
+        out, status = torch.full((n, nh * hd), float("nan"), device=DEV), ops.new_status(DEV)
+        ops.attention(q, nh * hd, pool, table, positions, qblk, qblk.shape[0], n - 1, n, nh, nkv, hd, 0, 64, tile, bq, hd ** -0.5, out, status, "generic")
+        ops.raise_on_status(status)
+        assert float((out.double() - want).abs().max()) < 1e-5 * float(want.abs().max())
+
+
 @pytest.mark.parametrize("nh,nkv,hd,page,window", [(4, 2, 16, 8, 10), (12, 2, 128, 16, 64), (5, 5, 48, 16, 1),
                                                    (3, 1, 32, 16, 100)])
 def test_attention_window(ops, nh, nkv, hd, page, window):
