@@ -27,6 +27,7 @@ constexpr int GF_RANGE = 1024;             // a multiple of every step of k belo
 constexpr int GF_BN = 128, GF_BK = 16, GF_LD = GF_BK + 4, GF_STAGES = 4, GF_THREADS = 256;
 constexpr int GF_FEW = 16;                 // rows up to which the product is treated as a stream of weights
 constexpr int GF_SHORT = 64;               // inner sizes up to which a product is one chain of sums
+constexpr long long GF_SCRATCH = 32 << 20; // floats that the sums of ranges may take
 
 struct GfParams {
     const float* A; const float* W; const float* bias; float* C;
@@ -370,11 +371,15 @@ static int gf_few_shares(int N, int ranges, int batch) {
     return (ranges + each - 1) / each;                   // no CTA without a range
 }
 
-// Whether the ranges of K go to CTAs of their own (and through `part`): when the tiles alone leave SMs idle.
-static bool gf_cuts(int M, int N, int ranges, int batch, int bm) {
-    if (ranges < 2) return false;
+// Rows at a time whose ranges of K go to CTAs of their own (and through `part`), 0: none, a CTA walks all its ranges.  They do where the
+// tiles alone make fewer than two rounds of the SMs, the last of them partly empty (550 x 1,536 with k of 8,960: 60 tiles, 540 with their
+// ranges), in pieces of rows whose sums fit GF_SCRATCH.  Where they go changes no bit.
+static int gf_cuts(int M, int N, int ranges, int batch, int bm) {
+    if (ranges < 2) return 0;
     const long long tiles = (long long)((M + bm - 1) / bm) * ((N + GF_BN - 1) / GF_BN) * batch;
-    return tiles < 2LL * sm_count();
+    if (tiles >= 2LL * sm_count()) return 0;
+    const long long rows = GF_SCRATCH / ((long long)ranges * batch * N);
+    return rows >= M ? M : (int)(rows / bm * bm);
 }
 
 static bool gf_few(int M, int ranges, bool vec) { return vec && M <= GF_FEW && ranges <= 64; }
@@ -433,15 +438,20 @@ static int gf_run(GfParams p, cudaStream_t stream) {
         return e == cudaSuccess ? BG_OK : (int)e;
     }
     const int bm = gf_bm(p.M, p.N, p.ranges, p.batch);
-    const bool cut = gf_cuts(p.M, p.N, p.ranges, p.batch, bm);
-    if (cut && !p.part) return BG_ERR_SHAPE;
-    if (!cut) p.part = nullptr;
-    if ((p.M + bm - 1) / bm > 65535 || (long long)p.batch * p.ranges > 65535) return BG_ERR_SHAPE;
-    cudaError_t e = bm == 64 ? (vec ? gf_launch_tile<64, true>(p, stream) : gf_launch_tile<64, false>(p, stream))
-                             : (vec ? gf_launch_tile<128, true>(p, stream) : gf_launch_tile<128, false>(p, stream));
-    if (e != cudaSuccess) return (int)e;
-    if (cut) e = gf_add_ranges(p, stream);
-    return e == cudaSuccess ? BG_OK : (int)e;
+    const int cut = gf_cuts(p.M, p.N, p.ranges, p.batch, bm), rows = cut > 0 ? cut : p.M, M = p.M;
+    if (cut > 0 && !p.part) return BG_ERR_SHAPE;
+    if (cut == 0) p.part = nullptr;
+    if ((rows + bm - 1) / bm > 65535 || (long long)p.batch * (cut > 0 ? p.ranges : 1) > 65535) return BG_ERR_SHAPE;
+    for (int m0 = 0; m0 < M; m0 += rows) {
+        p.M = M - m0 < rows ? M - m0 : rows;
+        cudaError_t e = bm == 64 ? (vec ? gf_launch_tile<64, true>(p, stream) : gf_launch_tile<64, false>(p, stream))
+                                 : (vec ? gf_launch_tile<128, true>(p, stream) : gf_launch_tile<128, false>(p, stream));
+        if (e == cudaSuccess && cut > 0) e = gf_add_ranges(p, stream);
+        if (e != cudaSuccess) return (int)e;
+        p.A += (size_t)rows * p.lda;
+        p.C += (size_t)rows * p.ldc;
+    }
+    return BG_OK;
 }
 
 }  // namespace bg
@@ -452,8 +462,8 @@ extern "C" long long bg_gemm_f32_scratch(int M, int N, int K, int batch) {
     const int ranges = (K + bg::GF_RANGE - 1) / bg::GF_RANGE;
     // (asked without the operands' alignment: both kernels' wants count)
     const bool few = bg::gf_few(M, ranges, true) && bg::gf_few_shares(N, ranges, batch) > 1;
-    if (!few && !bg::gf_cuts(M, N, ranges, batch, bg::gf_bm(M, N, ranges, batch))) return 0;
-    return (long long)ranges * batch * M * N;
+    const int cut = bg::gf_cuts(M, N, ranges, batch, bg::gf_bm(M, N, ranges, batch)), rows = few ? M : cut;
+    return (long long)ranges * batch * rows * N;
 }
 
 extern "C" int bg_gemm_f32_nt(const float* A, int lda, const float* W, int ldw, const float* bias, float* C, int ldc,

@@ -948,3 +948,23 @@ def test_decoding_attention_under_a_bound_finds_every_needle(ops, dtype, page, b
             assert (got[r] - (100.0 + r)).abs().max() < 1.0, (r, t, place(t), got[r][:4])
         for pg, sl, old in changed:
             pool[pg, :, :, sl] = old
+
+
+def test_gemm_f32_takes_many_batches_and_little_scratch(ops):
+    """A batch whose ranges of k would be too many for a grid, which walks them; sums of ranges of more than 128 MB, which go piece by piece:
+    the bits of one row alone, and room for the pieces only."""
+    a, w = rnd(1, 17, 1028, seed=1).expand(40000, -1, -1), rnd(1, 4, 1028, seed=2).expand(40000, -1, -1)
+    out, one = torch.empty((40000, 17, 4), device=DEV), torch.empty((17, 4), device=DEV)
+    ops.gemm_f32_nt_batched(a, w, out)
+    ops.gemm_f32_nt(a[0], w[0], None, one)
+    assert torch.equal(out, one.expand(40000, -1, -1))
+    M, N, K = 700, 4096, 20 * 1024 + 4
+    a, w, b, part = rnd(M, K, seed=3), rnd(N, K, seed=4), rnd(N, seed=5), ops.lib().bg_gemm_f32_scratch(M, N, K, 1)
+    assert 0 < part <= 32 << 20
+    out = torch.empty((M, N), device=DEV)
+    ops.gemm_f32_nt(a, w, b, out)
+    for m in (0, 255, 256, 699):
+        one = torch.empty((1, N), device=DEV)
+        ops.gemm_f32_nt(a[m:m + 1], w, b, one)
+        assert torch.equal(one[0], out[m]), m
+    assert ops.lib().bg_gemm_f32_scratch(16, 1 << 20, 1 << 20, 1) <= 32 << 20 and ops.lib().bg_gemm_f32_scratch(600, 1 << 15, 1 << 22, 1) <= 32 << 20
