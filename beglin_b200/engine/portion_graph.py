@@ -16,7 +16,7 @@ the scratch of the attention kernels that cut the keys into ranges at fixed posi
 """
 from __future__ import annotations
 
-from typing import Dict, List, Optional, Tuple
+from typing import Dict, Optional, Tuple
 
 import numpy as np
 import torch
@@ -144,14 +144,23 @@ class PortionGraph:
 
 class PortionGraphs:
     """The portion graphs of an engine: a shape is captured when it comes for the second time, and the
-    shapes used least recently are dropped beyond `keep` graphs (each holds its step's activations)."""
+    shapes used least recently are dropped beyond `keep` graphs (each holds its step's activations).
+
+    A shape of more than FEW_WANTED wanted places takes the place of another only if that one was not used since
+    the shape came last: the exact number of places is part of a shape, so that prompts which want many places
+    bring ever new ones, and more of them in turn than graphs are kept would pay for a warm-up pass and a capture
+    with every step, where a step kernel by kernel costs 0.3 ms more than a replayed one (2,048 tokens with sixteen
+    places at the 1.5B sizes, 6.4 ms).  Beyond 64 places the logits, which a graph holds, are what its memory goes to."""
 
     BOUND_STEP = 4096          # `bound` grows in steps of this many positions
+    FEW_WANTED = 8
 
     def __init__(self, engine, min_rows: int = 256, max_wanted: int = 64, keep: int = 4):
         self.engine, self.min_rows, self.max_wanted, self.keep = engine, min_rows, max_wanted, keep
         self.graphs: Dict[tuple, PortionGraph] = {}
-        self.seen: List[tuple] = []
+        self.seen: Dict[tuple, int] = {}       # shapes that came lately: when last
+        self.used: Dict[tuple, int] = {}       # of the graphs: when last
+        self.steps = 0
         self.replays = 0
 
     def key_of(self, ents, starts) -> Optional[tuple]:
@@ -166,18 +175,25 @@ class PortionGraphs:
         return rows, wanted, bound
 
     def get(self, key) -> Optional[PortionGraph]:
+        self.steps += 1
         g = self.graphs.get(key)
         if g is None:
-            if key not in self.seen:           # first sighting: remember it, run the step kernel by kernel
-                self.seen.append(key)
-                del self.seen[:-16]
+            last = self.seen.get(key)
+            if last is None:                   # first sighting: remember it, run the step kernel by kernel
+                self.seen[key] = self.steps
+                while len(self.seen) > 16:
+                    del self.seen[next(iter(self.seen))]
                 return None
+            self.seen[key] = self.steps
             while len(self.graphs) >= self.keep:
-                del self.graphs[next(iter(self.graphs))]
+                oldest = next(iter(self.graphs))
+                if key[1] > self.FEW_WANTED and self.used[oldest] > last:
+                    return None                # every graph was used since this shape came last
+                del self.graphs[oldest], self.used[oldest]
             g = PortionGraph(self.engine, *key)
         else:
             del self.graphs[key]               # moved to the end: used most recently
-        self.graphs[key] = g
+        self.graphs[key], self.used[key] = g, self.steps
         return g
 
     def step(self, g: PortionGraph, entry, start: int) -> Optional[torch.Tensor]:

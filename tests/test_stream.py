@@ -95,6 +95,28 @@ def test_which_steps_a_portion_graph_stands_for_and_which_graphs_are_kept():
         pg.PortionGraph = pg_class
 
 
+def test_shapes_of_many_wanted_places_do_not_push_one_another_out():
+    """More shapes in turn than graphs are kept: some keep theirs, the others run kernel by kernel, and none is made twice; a
+    shape that comes again while the others no longer do gets a graph."""
+    from types import SimpleNamespace
+    from beglin_b200.engine import portion_graph as pg
+
+    graphs, made = pg.PortionGraphs(SimpleNamespace(cache=SimpleNamespace(max_context=10000)), keep=4), []
+    pg_class, pg.PortionGraph = pg.PortionGraph, lambda eng, *key: made.append(key) or ("graph", key)
+    try:
+        shapes = [(256, n, 4095) for n in (16, 17, 40, 63, 64, 30)]
+        for turn in range(5):
+            got = [graphs.get(s) for s in shapes]
+        assert made == shapes[:4] and [g is not None for g in got] == [True] * 4 + [False] * 2
+        few = (512, 1, 4095)
+        assert graphs.get(few) is None and graphs.get(few) == ("graph", few)          # a prompt's usual shape finds room
+        new = (256, 33, 4095)
+        assert graphs.get(new) is None and graphs.get(few) and graphs.get(new) == ("graph", new)
+        assert len(graphs.graphs) == len(graphs.used) == 4
+    finally:
+        pg.PortionGraph = pg_class
+
+
 def test_no_collection_collects_first_and_keeps_the_collector_off():
     """A dropped cycle (an engine and its graphs are one) is collected before the block begins, not inside it."""
     import gc
