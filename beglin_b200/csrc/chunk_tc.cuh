@@ -263,15 +263,19 @@ __global__ void __launch_bounds__(CT_THREADS, 2) chunk_out_tc_kernel(R r) {
     } else {
         c.weights([&](int t, int j, float w) { ct_put1(qt, part, t, j, w); });
     }
+    bool split = true;
     ct_put<SV>(xt, part, raw, r.nv, [&](const float4& x, int j, int v) {
-        float4 y = c.out_value(x, j, v);
-        if (!(ct_splits(y.x) && ct_splits(y.y) && ct_splits(y.z) && ct_splits(y.w))) {
-            s.odd = 1;
-            y.x = ct_splits(y.x) ? y.x : 0.0f; y.y = ct_splits(y.y) ? y.y : 0.0f;
-            y.z = ct_splits(y.z) ? y.z : 0.0f; y.w = ct_splits(y.w) ? y.w : 0.0f;
-        }
+        const float4 y = c.out_value(x, j, v);
+        split = split && ct_splits(y.x) && ct_splits(y.y) && ct_splits(y.z) && ct_splits(y.w);
         return y;
     });
+    if (!split) {                            // (out of the way of the usual tile: once more, with noughts)
+        s.odd = 1;
+        ct_put<SV>(xt, part, raw, r.nv, [&](const float4& x, int j, int v) {
+            const float4 y = c.out_value(x, j, v);
+            return make_float4(ct_splits(y.x) ? y.x : 0.0f, ct_splits(y.y) ? y.y : 0.0f, ct_splits(y.z) ? y.z : 0.0f, ct_splits(y.w) ? y.w : 0.0f);
+        });
+    }
     ct_issue(s, [&] { ct_mma<true, false>(d, d + 64, x_a, part, q_a, part, CT / 16, CT / 32, ct_idesc(CT, true, false), true); });
     ct_wait(s, phase);
     float* out = reinterpret_cast<float*>(xt);               // [CT][CT_OUT_LD] (the weights stay where they are)
