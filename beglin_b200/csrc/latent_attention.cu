@@ -357,17 +357,17 @@ __global__ void __launch_bounds__(LAT_MERGE_THREADS)
 latent_attention_merge_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml,
                               const int* __restrict__ positions, TO* __restrict__ out, long long out_head,
                               int out_row, int T, int H, int rank, int max_splits, int split, int window,
-                              const float* __restrict__ sink_w) {
+                              const float* __restrict__ sink_w, int ctas, int sms) {
     extern __shared__ float f_s[];                 // [max_splits] weights e^(m_s - m) / l
     pdl_launch();
-    pdl_wait();
     const int w = blockIdx.x;
     const int t = w / H, h = w - t * H;
-    const int pos = positions[t], lo = first_visible(pos, window);
+    const int pos = positions[t], lo = first_visible(pos, window);         // (written by no kernel of the step)
     // splits at absolute positions, or (split 0) ranges that follow the row's own keys
-    const int s_lo = split > 0 ? lo / split : 0, s_hi = split > 0 ? pos / split : latent_range(pos, lo, max_splits).count - 1;
+    const int s_lo = split > 0 ? lo / split : 0, s_hi = split > 0 ? pos / split : latent_range(pos, lo, max_splits, ctas, sms).count - 1;
     const size_t prow = (size_t)w * max_splits;
     const int lane = threadIdx.x & 31;
+    pdl_wait();
     if (threadIdx.x < 32) {
         float m = -INFINITY;
         for (int s = s_lo + lane; s <= s_hi; s += 32) m = fmaxf(m, part_ml[(prow + s) * 2]);
@@ -563,13 +563,13 @@ extern "C" int bg_latent_attention_partial(const void* q_lat, int ql_dtype, long
 
 extern "C" int bg_latent_attention_merge(const float* part_o, const float* part_ml, const int* positions, void* out,
                                          int out_dtype, long long out_head, int out_row, int T, int H, int rank,
-                                         int max_splits, int split, int window, const float* sink_w, cudaStream_t stream) {
+                                         int max_splits, int split, int window, const float* sink_w, int ctas, cudaStream_t stream) {
     const long long blocks = (long long)T * H;
     if (blocks <= 0) return BG_OK;
     if (blocks > 0x7fffffffLL || max_splits > 8192) return BG_ERR_SHAPE;
     BG_DISPATCH_DTYPE(out_dtype, TO,
         launch(latent_attention_merge_kernel<TO>, dim3((unsigned)blocks), dim3(LAT_MERGE_THREADS), (size_t)max_splits * sizeof(float),
-               stream, part_o, part_ml, positions, (TO*)out, out_head, out_row, T, H, rank, max_splits, split, window, sink_w));
+               stream, part_o, part_ml, positions, (TO*)out, out_head, out_row, T, H, rank, max_splits, split, window, sink_w, ctas, sm_count()));
     BG_LAUNCH_CHECK();
     return BG_OK;
 }

@@ -45,6 +45,7 @@ struct LtParams {
     const int* positions; const int* qblk;
     float* part_o; float* part_ml; int max_splits;
     int H, rank, rot, rot_dims, window, slots;
+    int ctas, sms;          // rows times chunks of heads, SMs: what the number of a row's ranges goes by (latent_range.cuh)
     float scale_log2;
     unsigned* status;
 };
@@ -93,10 +94,12 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_attention_tc_kernel(cons
     constexpr unsigned TMEM_COLS = NH == 32 ? 256 : 128, O_COL = 2 * NH;
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    // (the list and the positions are read in front of the wait, here as in the decoding attention: no kernel between a step's upload, or the
+    // sampling kernel that ends a replay, and its last layer writes them)
     const int qb = blockIdx.x, h0 = blockIdx.y * NH, nh = min(NH, p.H - h0), sp = blockIdx.z;
     const int req = p.qblk[qb * 3 + 0], t = p.qblk[qb * 3 + 1];
     const int pos = p.positions[t], lo = first_visible(pos, p.window);
-    const LatentRange range = latent_range(pos, lo, p.max_splits);
+    const LatentRange range = latent_range(pos, lo, p.max_splits, p.ctas, p.sms);
     if (p.qblk[qb * 3 + 2] <= 0 || sp >= range.count) return;              // (the whole CTA)
     const int k_begin = range.begin + sp * range.per, k_end = min(k_begin + range.per, pos + 1);
     const int n_tiles = (k_end - k_begin + LT_KEYS - 1) / LT_KEYS;
@@ -399,8 +402,19 @@ extern "C" int bg_latent_attention_tc_plan(int H, int rank, int rot, int page_si
     return lt_slots(nh, rank, rot) > (rank / 64 + 1) / 2 ? BG_OK : BG_ERR_UNSUPPORTED;
 }
 
+// How many ranges the longest-cut row of up to `keys` keys makes, of `ctas` rows (times chunks of heads) on `sms` SMs: what a grid and partial results are sized for.
+extern "C" int bg_latent_attention_tc_ranges(int ctas, int keys, int sms) {
+    const int tiles = (keys + LATENT_RANGE_STEP - 1) / LATENT_RANGE_STEP;
+    int most = 1;
+    for (int t = 2; t <= tiles; ++t) {
+        const int n = latent_ranges(t, LATENT_MAX_RANGES, ctas, sms);
+        if (n > most) most = n;
+    }
+    return most;
+}
+
 // The arguments of bg_latent_attention_mma_partial; query blocks of one row each; a request's keys are spread over `max_splits` ranges
-// as latent_range.cuh says.
+// as latent_range.cuh says, at most LATENT_MAX_RANGES.
 extern "C" int bg_latent_attention_tc_partial(const float* q_lat, long long ql_head, int ql_row, const void* q_raw, int qr_row, int qr_head,
                                               int qr_off, const float* cos_sin, const void* pool, int num_pages, int page_size,
                                               const int* block_table, int max_pages, const int* positions, const int* qblk, int n_qblk,
@@ -409,7 +423,7 @@ extern "C" int bg_latent_attention_tc_partial(const float* q_lat, long long ql_h
     if (n_qblk <= 0 || max_splits <= 0) return BG_OK;
     const int rc = bg_latent_attention_tc_plan(H, rank, rot, page_size);
     if (rc != BG_OK) return rc;
-    if (rot_dims > rot || (rot_dims & 1) || max_splits > 65535) return BG_ERR_SHAPE;
+    if (rot_dims > rot || (rot_dims & 1) || max_splits > LATENT_MAX_RANGES || (long long)n_qblk * ((H + 31) / 32) > (1 << 25)) return BG_ERR_SHAPE;
     if ((uintptr_t)pool % 16 || (uintptr_t)q_lat % 16 || ql_head % 4 || ql_row % 4 || (uintptr_t)cos_sin % 8) return BG_ERR_ALIGN;
     if ((long long)num_pages * page_size > 0x7fffffffLL) return BG_ERR_SHAPE;
     CUtensorMap map;
@@ -422,6 +436,7 @@ extern "C" int bg_latent_attention_tc_partial(const float* q_lat, long long ql_h
     p.H = H; p.rank = rank; p.rot = rot; p.rot_dims = rot_dims; p.window = window; p.scale_log2 = scale * LT_LOG2E; p.status = status;
     const int nh = H <= 16 ? 16 : 32;
     p.slots = lt_slots(nh, rank, rot);
+    p.ctas = n_qblk * ((H + nh - 1) / nh); p.sms = sm_count();
     const size_t smem = lt_fixed_smem(nh, rank, rot) + (size_t)p.slots * LT_SLOT;
     const dim3 grid(n_qblk, (H + nh - 1) / nh, max_splits);
 #define BG_LT_LAUNCH(NH)                                                                                                   \

@@ -7,6 +7,7 @@ loaded, or a tensor is not on a CUDA device, they raise.
 from __future__ import annotations
 
 import ctypes
+import functools
 from typing import Optional, Tuple
 
 import torch
@@ -143,13 +144,14 @@ _SIGNATURES = {
                                     _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int,
                                     _c_int, _c_int, _c_int, _c_float, _c_void_p, _c_void_p],
     "bg_latent_attention_merge": [_c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_ll, _c_int, _c_int, _c_int, _c_int,
-                                  _c_int, _c_int, _c_int, _c_void_p, _c_void_p],
+                                  _c_int, _c_int, _c_int, _c_void_p, _c_int, _c_void_p],
     "bg_latent_attention_mma_plan": [_c_int, _c_int, ctypes.POINTER(_c_int), ctypes.POINTER(_c_int)],
     "bg_latent_attention_mma_partial": [_c_void_p, _c_ll, _c_int, _c_void_p, _c_int, _c_int, _c_int, _c_void_p, _c_void_p, _c_int,
                                         _c_int, _c_void_p, _c_int, _c_void_p, _c_void_p, _c_int, _c_void_p, _c_void_p, _c_int,
                                         _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_float,
                                         _c_void_p, _c_void_p],
     "bg_latent_attention_tc_plan": [_c_int, _c_int, _c_int, _c_int],
+    "bg_latent_attention_tc_ranges": [_c_int, _c_int, _c_int],
     "bg_latent_attention_tc_partial": [_c_void_p, _c_ll, _c_int, _c_void_p, _c_int, _c_int, _c_int, _c_void_p, _c_void_p, _c_int, _c_int,
                                        _c_void_p, _c_int, _c_void_p, _c_void_p, _c_int, _c_void_p, _c_void_p, _c_int, _c_int, _c_int,
                                        _c_int, _c_int, _c_int, _c_float, _c_void_p, _c_void_p],
@@ -1242,19 +1244,12 @@ def latent_append(src: torch.Tensor, col0: int, rank: int, rot: int, rot_dims: i
 LATENT_TC_KEYS = 128          # keys of a tile of the tcgen05 kernel
 
 
+@functools.lru_cache(maxsize=1024)
 def latent_splits(rows: int, keys: int, sms: Optional[int] = None) -> int:
-    """How many CTAs share a row's keys in the tcgen05 kernel, for `rows` rows (times chunks of heads) of up to `keys` keys: the
-    number that makes the waves of one CTA an SM shortest, a CTA's start, queries and results counted as three tiles of keys.  (64 rows of
-    4,000 keys, in 1, 2, 3, 4, 6 and 9 ranges: 169, 103, 140, 120, 141, 157 us; the rule takes 2.)"""
-    sms = sm_count() if sms is None else sms
-    tiles = -(-keys // LATENT_TC_KEYS)
-    best, best_cost = 1, None
-    for s in range(1, min(tiles, 64) + 1):
-        per = -(-tiles // s)
-        cost = -(-rows * -(-tiles // per) // sms) * (per + 3)
-        if best_cost is None or cost < best_cost:
-            best, best_cost = s, cost
-    return best
+    """How many CTAs at most share a row's keys in the tcgen05 kernel, for `rows` rows (times chunks of heads) of up to `keys` keys.  Every
+    row's own number follows from its own length, by the rule of latent_range.cuh; this is the largest of them, which the grid and the
+    partial results are sized for."""
+    return lib().bg_latent_attention_tc_ranges(rows, keys, sm_count() if sms is None else sms)
 
 
 def latent_attention(q_lat: torch.Tensor, q_raw: torch.Tensor, dim: int, rot: int, rot_dims: int,
@@ -1292,9 +1287,10 @@ def latent_attention(q_lat: torch.Tensor, q_raw: torch.Tensor, dim: int, rot: in
         and L.bg_latent_attention_tc_plan(H, rank, rot, pool.shape[1]) == 0
     if tc:
         keys = min(max_position + 1, window + LATENT_TC_KEYS) if window > 0 else max_position + 1
-        split, n_splits = 0, latent_splits(n_qblk * -(-H // 32), keys)
+        split, ctas = 0, n_qblk * -(-H // 32)
+        n_splits = latent_splits(ctas, -(-keys // LATENT_TC_KEYS) * LATENT_TC_KEYS, sm_count())
     else:
-        n_splits = max_position // split + 1
+        n_splits, ctas = max_position // split + 1, 0
     part_o = torch.empty((T * H * n_splits, rank), dtype=torch.float32, device=q_lat.device)
     part_ml = torch.empty((T * H * n_splits, 2), dtype=torch.float32, device=q_lat.device)
     with phase("attn"):
@@ -1320,7 +1316,8 @@ def latent_attention(q_lat: torch.Tensor, q_raw: torch.Tensor, dim: int, rot: in
                                                  n_qblk, _p(part_o), _p(part_ml), n_splits, n_splits, H, hc, rank, rot, rot_dims,
                                                  split, tile, bq, int(window), float(scale), _p(status), _stream()), "latent_attention_partial")
         _check(L.bg_latent_attention_merge(_p(part_o), _p(part_ml), _p(positions), _p(out), _dt(out), out.stride(0),
-                                           out.stride(1), T, H, rank, n_splits, split, int(window), _p(sink_weight), _stream()), "latent_attention_merge")
+                                           out.stride(1), T, H, rank, n_splits, split, int(window), _p(sink_weight), ctas, _stream()),
+               "latent_attention_merge")
 
 
 def latent_gather(pool: torch.Tensor, block_table: torch.Tensor, req: int, rank: int, lat: torch.Tensor, kr: torch.Tensor,

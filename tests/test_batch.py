@@ -68,3 +68,13 @@ def test_convolution_keeps_decoding_steps_out_of_runs():
     for n in (1, 8, 32, 64, 256, 4096):
         assert run(n, n) == 1                                     # decoding
     assert run(95, 1) == 1 and run(96, 1) == 8 and run(2048, 1) == 8 and run(2048 + 60, 61) == 8 and run(127, 16) == 1 and run(128, 16) == 8
+
+
+def test_latent_decoding_ranges_of_the_longest_row():
+    """The grid of latent decoding is sized for the row that is cut into the most ranges; 64 rows of 4,000 keys are cut in two (measured)."""
+    from beglin_b200.csrc import ops
+    most = lambda rows, keys: ops.latent_splits(rows, keys, 148)
+    assert most(64, 4096) == 2 and most(1, 128) == 1 and most(1, 4096) == 32 and most(148, 1 << 17) >= 1
+    for rows in (1, 7, 64, 100, 148, 500):
+        sizes = [most(rows, 128 * t) for t in (1, 3, 32, 33, 256, 1024)]
+        assert sizes == sorted(sizes) and all(1 <= s <= min(t, 64) for s, t in zip(sizes, (1, 3, 32, 33, 256, 1024)))

@@ -547,3 +547,22 @@ def test_a_key_inside_and_outside_the_window_and_the_sink(tmp_path, dtype, dim, 
     for i in range(head, head + 8):
         row = eng.step([("d", [ids[i]], [0])])
         assert rel_err(row[0], want[i]) < tol * float(want.abs().max() / want[i].abs().max()), i
+
+
+@pytest.mark.parametrize("H,rank,window", [(32, 512, 0), (12, 64, 0), (32, 128, 700)])
+def test_latent_decoding_cuts_a_row_by_its_own_length(H, rank, window):
+    """A captured decoding step knows the longest context only: with that bound a row's keys are cut as with the row's own, bit for bit."""
+    o, rot, page, T = ops(), 64, 64, 40
+    g = torch.Generator().manual_seed(rank)
+    at = [(4001 if i % 2 else 300) - i for i in range(T)]
+    pages = -(-max(at) // page)
+    pool = torch.randn(pages, page, rank + rot, generator=g).to(DEV, torch.bfloat16)
+    table = torch.arange(pages, dtype=torch.int32, device=DEV).repeat(T, 1)
+    q_lat, q_raw = torch.randn(H, T, rank, generator=g).to(DEV), torch.randn(T, H * (8 + rot), generator=g).to(DEV, torch.bfloat16)
+    qblk, status, outs = i32([[r, r, 1] for r in range(T)]), o.new_status(DEV), []
+    for bound in (max(at), 32767, 100000):
+        out = torch.full((H, T, rank), NAN, dtype=torch.bfloat16, device=DEV)
+        o.latent_attention(q_lat, q_raw, 8, rot, 0, None, pool, table, i32(at), qblk, T, bound, 1, min(H, 32), 64, 256, 0.05, out, status, mma_stages=1, window=window)
+        outs.append(out)
+    o.raise_on_status(status)
+    assert torch.isfinite(outs[0].float()).all() and torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
