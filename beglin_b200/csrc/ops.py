@@ -1284,6 +1284,7 @@ def latent_attention(q_lat: torch.Tensor, q_raw: torch.Tensor, dim: int, rot: in
     # one row per block (decoding) on tcgen05 where it takes the sizes: a row's own keys spread over the SMs
     tc = bool(mma_stages) and bq == 1 and q_raw.dtype == pool.dtype == torch.bfloat16 \
         and q_lat.stride(0) % 4 == 0 and q_lat.stride(1) % 4 == 0 and q_lat.data_ptr() % 16 == 0 and pool.data_ptr() % 16 == 0 \
+        and (cos_sin is None or cos_sin.data_ptr() % 8 == 0) and pool.shape[0] * pool.shape[1] <= 0x7fffffff \
         and L.bg_latent_attention_tc_plan(H, rank, rot, pool.shape[1]) == 0
     if tc:
         keys = min(max_position + 1, window + LATENT_TC_KEYS) if window > 0 else max_position + 1

@@ -566,3 +566,20 @@ def test_latent_decoding_cuts_a_row_by_its_own_length(H, rank, window):
         outs.append(out)
     o.raise_on_status(status)
     assert torch.isfinite(outs[0].float()).all() and torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
+
+
+def test_latent_decoding_takes_rotations_off_a_boundary():
+    """Rotations on a 4-byte boundary only: decoded by the kernel that reads them a float at a time."""
+    o, H, rank, rot, T, page = ops(), 12, 64, 32, 3, 64
+    g = torch.Generator().manual_seed(5)
+    pool = torch.randn(T, page, rank + rot, generator=g).to(DEV, torch.bfloat16)
+    q_lat, q_raw = torch.randn(H, T, rank, generator=g).to(DEV), torch.randn(T, H * (8 + rot), generator=g).to(DEV, torch.bfloat16)
+    flat = torch.randn(1 + T * rot, generator=g).to(DEV)
+    status, outs = o.new_status(DEV), []
+    for cos_sin in (flat[1:].view(T, rot // 2, 2), flat[1:].clone().view(T, rot // 2, 2)):
+        out = torch.full((H, T, rank), NAN, dtype=torch.bfloat16, device=DEV)
+        o.latent_attention(q_lat, q_raw, 8, rot, rot, cos_sin, pool, i32([[0], [1], [2]]), i32([50, 3, 63]), i32([[r, r, 1] for r in range(T)]), T, 63, 1, H, 64, 256,
+                           0.1, out, status, mma_stages=1)
+        outs.append(out)
+    o.raise_on_status(status)
+    assert rel_err(outs[0], outs[1]) < 2e-2
