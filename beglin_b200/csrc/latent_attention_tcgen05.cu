@@ -6,22 +6,25 @@
 // and both products read them there as they lie.  Keys and features are the M side, heads the N side, so that 16 or 32 heads leave
 // no part of a 128-row MMA unused:
 //     S^T [128 keys, NH]         = K [128, width] Q^T            (K: a box as it is, features innermost)
-//     O^T [128 features, NH]    += V^T [128 features, 128 keys] P^T, for every 128 features of the latent
-// V is the first `rank` features of the same rows, read with the features as M (an M-major left operand).  Scores and results live in
-// tensor memory.  Warps: 0 asks for the rows, 1 issues the score products, 2 the value products, 4 to 7 are the softmax, a thread per
-// key: the maximum over the keys of a head is one redux over the warp and one exchange of the four warps through shared memory; P goes
-// to shared memory as bfloat16.  The kept maximum of a head moves only when it would grow by more than 2^8, so O^T is rescaled in
-// the first tiles at most.
+//     O^T [128 features, NH]     = V^T [128 features, 128 keys] P^T, of one tile, for every 128 features of the latent
+// V is the first `rank` features of the same rows, read with the features as M (an M-major left operand).  Scores and a tile's results
+// live in tensor memory, two of each.  Warps: 0 asks for the rows, 1 issues the score products, 2 the value products, 4 to 7 are the
+// softmax, a thread per key: the maximum over the keys of a head is one redux over the warp and one exchange of the four warps through
+// shared memory; P goes to shared memory as bfloat16, relative to the largest weight of its OWN tile, which is then one and not rounded;
+// the sums of weights are of the rounded ones.  (A maximum kept over tiles left the weights that matter most between powers of two:
+// scores with a deviation of six, 0.00081 of the result, 0.00013 so.)  A tile's results are added up by the softmax's threads, a thread
+// per feature with all its heads in registers, when the next tile's weights are on their way.
 //
 // The ring is cut finer than a tile: slots of 128 features x 128 keys, given back one by one as the value products have read them, and
 // one slot for the rotated part, given back by the score products.  A tile of 576 features is 147 KB, so that two of them do not fit
 // an SM; with the finer slots the next tile sets out while the last one is used.  One CTA an SM; bound by the bytes of the cache.
-// Measured (kernel and merge, 512 + 64 features, 32 heads): 64 requests of 4,000 keys 258.7 us with latent_attention_mma.cu -> 92.6 us
-// (3.2 TB/s of cache; 102.5 with MMAs issued under a test of the lane's number), 8 requests 49.2 -> 36.2, 32 requests of 300 keys 39.2 ->
-// 25.9; 12 heads of 384 + 64, 64 requests of 4,096 keys 128.0 -> 62.7, one request 30.7 -> 30.2.  What is left beside the bytes is a
-// range's start and end (queries, the first rows, the results) and the chain of a tile, whose rows are held until its last value
-// product while only a part of the next tile's fit.  Tiles of 64 keys, of which 2.5 fit, took 100 us: half of every score product's
-// rows are then not keys, and the chain is walked twice as often.
+// Measured (kernel and merge, 512 + 64 features, 32 heads): 64 requests of 4,000 keys 257.9 us with latent_attention_mma.cu -> 96.3 us
+// (3.1 TB/s of cache; 91.7 with a maximum kept over tiles and sums in tensor memory, 10 us more with MMAs issued under a test of the lane's
+// number), 8 requests 48.9 -> 35.4, 32 requests of 300 keys 38.7 -> 24.4; 12 heads of 384 + 64, 64 requests of 4,096 keys 127.7 -> 61.8,
+// one request 30.6 -> 23.9.  What is left beside the bytes is a range's start and end (queries, the first rows, the results: 5 us of the
+// whole when they left as 128 stores of 4 bytes a thread, whose instructions every CTA fetched for one use) and the chain of a tile, whose rows
+// are held until its last value product while only a part of the next tile's fit.  Tiles of 64 keys, of which 2.5 fit, took 100 us against
+// 92.6 then: half of every score product's rows are then not keys, and the chain is walked twice as often.
 // Keys behind the range's last lie in pages that this request may never have written: their rows are zeroed in shared memory before
 // the value products read them (0 x NaN would reach every head).
 #include "tc_common.cuh"
@@ -35,7 +38,7 @@ constexpr unsigned LT_BLOCK = LT_KEYS * 128;             // 64 features x 128 ke
 constexpr unsigned LT_SLOT = 2 * LT_BLOCK;               // 128 features
 constexpr int LT_MAX_SLOTS = 8;
 constexpr float LT_LOG2E = 1.4426950408889634f, LT_LN2 = 0.6931471805599453f;
-constexpr float LT_SLACK = 8.0f;                         // how far (in powers of two) scores may rise above the kept maximum
+constexpr float LT_FALL = 60.0f;                         // how far (in powers of two) a tile's reference may lie under the largest score
 
 struct LtParams {
     const float* q_lat; long long ql_head; int ql_row;
@@ -79,19 +82,14 @@ __device__ __forceinline__ void lt_load(unsigned taddr, float (&v)[NH]) {
     }
 }
 template <int NH>
-__device__ __forceinline__ void lt_store(unsigned taddr, const float (&v)[NH]) {
-    if constexpr (NH == 32) tc_st32(taddr, v); else tc_st16(taddr, v);
-}
-
-template <int NH>
 __global__ void __launch_bounds__(LT_THREADS, 1) latent_attention_tc_kernel(const __grid_constant__ CUtensorMap map, LtParams p) {
     extern __shared__ unsigned char lt_raw[];
     __shared__ __align__(8) unsigned long long slot_full[LT_MAX_SLOTS], slot_empty[LT_MAX_SLOTS], rot_full, rot_empty, s_full[2], s_empty[2],
         p_full, p_empty;
-    __shared__ __align__(16) float wmax[2][4][32], mrow[4][32], frow[4][32], lsum[4][32];
+    __shared__ __align__(16) float wmax[2][4][32], mrow[4][32], frow[2][4][32], lsum[4][32];      // (mrow, frow: a warp's own copies)
     __shared__ unsigned tmem_sh;
     __shared__ int failed;
-    constexpr unsigned TMEM_COLS = NH == 32 ? 256 : 128, O_COL = 2 * NH;
+    constexpr unsigned TMEM_COLS = NH == 32 ? 512 : 256, O_COL = 2 * NH, O_COLS = 4 * NH;      // (a tile's results: up to four pairs)
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     // (the list and the positions are read in front of the wait, here as in the decoding attention: no kernel between a step's upload, or the
@@ -261,8 +259,8 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_attention_tc_kernel(cons
                         const unsigned v_a = ring_a + (unsigned)slot * LT_SLOT;
 #pragma unroll
                         for (int ks = 0; ks < LT_KEYS / 16; ++ks)
-                            tc_mma(tmem + O_COL + (unsigned)i * NH, smem_desc_sw128_nmajor(v_a + ks * 2048, LT_BLOCK, 1024),
-                                   smem_desc_sw128(p_a + (ks >> 2) * (NH * 128) + (ks & 3) * 32), idesc_o, (ti > 0 || ks > 0) ? 1u : 0u);
+                            tc_mma(tmem + O_COL + (unsigned)(ti & 1) * O_COLS + (unsigned)i * NH, smem_desc_sw128_nmajor(v_a + ks * 2048, LT_BLOCK, 1024),
+                                   smem_desc_sw128(p_a + (ks >> 2) * (NH * 128) + (ks & 3) * 32), idesc_o, ks > 0 ? 1u : 0u);
                         tc_commit(&slot_empty[slot]);
                         if (i == pairs - 1) tc_commit(&p_empty);
                     }
@@ -274,105 +272,124 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_attention_tc_kernel(cons
         // ------------------------------------------------------------------ softmax: a thread per key of the tile
         const int quarter = warp & 3, kk = quarter * 32 + lane;
         const unsigned lane_addr = (unsigned)(quarter * 32) << 16;
-        float m = -INFINITY, l[NH];                      // m: of head `lane`, alike in the four warps; l: of this thread's keys
+        float m = -INFINITY, ref = -INFINITY;            // of head `lane`, alike in the four warps: the largest score, what l and acc are relative to
+        float l[NH], acc[4][NH];                         // of this thread's keys, of this thread's features
 #pragma unroll
-        for (int h = 0; h < NH; ++h) l[h] = 0.0f;
-        for (int ti = 0; ti < n_tiles && ok; ++ti) {
+        for (int h = 0; h < NH; ++h) l[h] = acc[0][h] = acc[1][h] = acc[2][h] = acc[3][h] = 0.0f;
+#pragma unroll 1
+        for (int ti = 0; ti <= n_tiles; ++ti) {          // (the last time round: the last tile's results)
             const int b = ti & 1, key = k_begin + ti * LT_KEYS + kk;
-            ok = mbar_wait(&s_full[b], (ti >> 1) & 1, &failed);
-            if (!lt_all(ok)) { ok = false; break; }
-            tc_fence_after();
-            float s[NH];
-            lt_load<NH>(tmem + lane_addr + (unsigned)b * NH, s);
-            tc_fence_before();
-            mbar_arrive(&s_empty[b]);
-            const bool seen = key >= lo && key < k_end;
-            float top = -INFINITY;
+            const bool tile = ti < n_tiles;
+            __nv_bfloat162 w2[NH / 2];                   // the key's weights
+            if (tile) {
+                float s[NH];
+                ok = mbar_wait(&s_full[b], (ti >> 1) & 1, &failed);
+                if (!lt_all(ok)) { ok = false; break; }
+                tc_fence_after();
+                lt_load<NH>(tmem + lane_addr + (unsigned)b * NH, s);
+                tc_fence_before();
+                mbar_arrive(&s_empty[b]);
+                const bool seen = key >= lo && key < k_end;
+                float top = -INFINITY;
 #pragma unroll
-            for (int h = 0; h < NH; ++h) {
-                s[h] = seen ? s[h] * p.scale_log2 : -INFINITY;
-                const float w = lt_warp_max(s[h]);
-                if (lane == h) top = w;
-            }
-            wmax[b][quarter][lane] = top;
-            lt_bar(2, 128);
-            top = fmaxf(fmaxf(wmax[b][0][lane], wmax[b][1][lane]), fmaxf(wmax[b][2][lane], wmax[b][3][lane]));
-            const bool rise = lane < NH && (top > m + LT_SLACK || m == -INFINITY);
-            const float m_new = rise ? top : m;
-            const bool any = __any_sync(0xffffffffu, rise);
-            mrow[quarter][lane] = m_new;
-            if (any) frow[quarter][lane] = rise ? (m == -INFINITY ? 0.0f : lt_exp2(m - m_new)) : 1.0f;
-            m = m_new;
-            __syncwarp();
-            if (any) {
+                for (int h = 0; h < NH; ++h) {
+                    s[h] = seen ? s[h] * p.scale_log2 : -INFINITY;
+                    const float w = lt_warp_max(s[h]);
+                    if (lane == h) top = w;
+                }
+                wmax[b][quarter][lane] = top;
+                lt_bar(2, 128);
+                top = fmaxf(fmaxf(wmax[b][0][lane], wmax[b][1][lane]), fmaxf(wmax[b][2][lane], wmax[b][3][lane]));
+                // the tile's own maximum; far below the largest so far its weights count for nothing, and the sums before must not overflow
+                m = fmaxf(m, top);
+                const float now = fmaxf(top, m - LT_FALL);
+                mrow[quarter][lane] = now;
+                frow[b][quarter][lane] = ref == -INFINITY ? 0.0f : lt_exp2(ref - now);
+                ref = now;
+                __syncwarp();
 #pragma unroll
-                for (int h = 0; h < NH; ++h) l[h] *= frow[quarter][h];
-            }
+                for (int h = 0; h < NH; h += 4) {
+                    const float4 r = *reinterpret_cast<const float4*>(&mrow[quarter][h]), f = *reinterpret_cast<const float4*>(&frow[b][quarter][h]);
+                    w2[h / 2] = __floats2bfloat162_rn(lt_exp2(s[h] - r.x), lt_exp2(s[h + 1] - r.y));
+                    w2[h / 2 + 1] = __floats2bfloat162_rn(lt_exp2(s[h + 2] - r.z), lt_exp2(s[h + 3] - r.w));
+                    const float2 u = __bfloat1622float2(w2[h / 2]), v = __bfloat1622float2(w2[h / 2 + 1]);
+                    l[h] = fmaf(l[h], f.x, u.x); l[h + 1] = fmaf(l[h + 1], f.y, u.y);
+                    l[h + 2] = fmaf(l[h + 2], f.z, v.x); l[h + 3] = fmaf(l[h + 3], f.w, v.y);
+                }
+                if (ti == n_tiles - 1 && key >= k_end) { // rows that this request has not written (the scores have read them)
+                    for (int i = 0; i < pairs; ++i) {
+                        unsigned char* row = ring + (size_t)((ti * pairs + i) % p.slots) * LT_SLOT + kk * 128;
 #pragma unroll
-            for (int h = 0; h < NH; ++h) {
-                s[h] = lt_exp2(s[h] - mrow[quarter][h]);
-                l[h] += s[h];
-            }
-            if (ti == n_tiles - 1 && key >= k_end) {     // rows that this request has not written (the scores have read them)
-                for (int i = 0; i < pairs; ++i) {
-                    unsigned char* row = ring + (size_t)((ti * pairs + i) % p.slots) * LT_SLOT + kk * 128;
-#pragma unroll
-                    for (int c = 0; c < 8; ++c) {
-                        *reinterpret_cast<uint4*>(row + c * 16) = make_uint4(0u, 0u, 0u, 0u);
-                        *reinterpret_cast<uint4*>(row + LT_BLOCK + c * 16) = make_uint4(0u, 0u, 0u, 0u);
+                        for (int c = 0; c < 8; ++c) {
+                            *reinterpret_cast<uint4*>(row + c * 16) = make_uint4(0u, 0u, 0u, 0u);
+                            *reinterpret_cast<uint4*>(row + LT_BLOCK + c * 16) = make_uint4(0u, 0u, 0u, 0u);
+                        }
                     }
                 }
             }
-            if (ti > 0) {                                // the value products of the last tile are done: P and O^T are this group's
+            if (ti > 0) {                                // the value products of the last tile are done: P and their results are this group's
                 ok = mbar_wait(&p_empty, (ti - 1) & 1, &failed);
                 if (!lt_all(ok)) { ok = false; break; }
                 tc_fence_after();
-                if (any) {
-                    for (int i = 0; i < pairs; ++i) {
-                        float o[NH];
-                        lt_load<NH>(tmem + lane_addr + O_COL + (unsigned)i * NH, o);
+            }
+            if (tile) {
+                unsigned char* pk = p_s + (kk >> 6) * (NH * 128) + (kk & 7) * 2;
 #pragma unroll
-                        for (int h = 0; h < NH; ++h) o[h] *= frow[quarter][h];
-                        lt_store<NH>(tmem + lane_addr + O_COL + (unsigned)i * NH, o);
+                for (int h = 0; h < NH; ++h)
+                    *reinterpret_cast<__nv_bfloat16*>(pk + h * 128 + (((((kk & 63) >> 3) ^ h) & 7) << 4)) = h & 1 ? w2[h / 2].y : w2[h / 2].x;
+                fence_proxy_async();
+                tc_fence_before();
+                mbar_arrive(&p_full);                    // (this tile's results go where those of the last but one were, which were added
+            }                                            // up before the last tile's weights were handed over)
+            if (ti > 0) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    if (i >= pairs) break;
+                    float o[NH];
+                    lt_load<NH>(tmem + lane_addr + O_COL + (unsigned)(b ^ 1) * O_COLS + (unsigned)i * NH, o);
+#pragma unroll
+                    for (int h = 0; h < NH; h += 4) {
+                        const float4 f = *reinterpret_cast<const float4*>(&frow[b ^ 1][quarter][h]);
+                        acc[i][h] = fmaf(acc[i][h], f.x, o[h]); acc[i][h + 1] = fmaf(acc[i][h + 1], f.y, o[h + 1]);
+                        acc[i][h + 2] = fmaf(acc[i][h + 2], f.z, o[h + 2]); acc[i][h + 3] = fmaf(acc[i][h + 3], f.w, o[h + 3]);
                     }
-                    tc_wait_st();
                 }
             }
-            unsigned char* pk = p_s + (kk >> 6) * (NH * 128) + (kk & 7) * 2;
-#pragma unroll
-            for (int h = 0; h < NH; ++h)
-                *reinterpret_cast<__nv_bfloat16*>(pk + h * 128 + (((((kk & 63) >> 3) ^ h) & 7) << 4)) = __float2bfloat16_rn(s[h]);
-            fence_proxy_async();
-            tc_fence_before();
-            mbar_arrive(&p_full);
-            __syncwarp();                                // (mrow and frow have been read)
+            __syncwarp();                                // (mrow, and the factors of the last tile, have been read)
         }
-        if (ok) ok = mbar_wait(&p_empty, (n_tiles - 1) & 1, &failed);
-        if (lt_all(ok)) {
-            tc_fence_after();
+        if (ok) {
+            // l[h] over the warp: every step halves the heads that a lane still holds
 #pragma unroll
-            for (int h = 0; h < NH; ++h) {
-                const float sum = warp_sum(l[h]);
-                if (lane == h) lsum[quarter][lane] = sum;
+            for (int w = NH / 2, o = 16; o > 0; o >>= 1, w >>= 1) {
+                if (w > 0) {
+#pragma unroll
+                    for (int h = 0; h < w; ++h) {
+                        const float mine = lane & o ? l[h + w] : l[h], other = lane & o ? l[h] : l[h + w];
+                        l[h] = mine + __shfl_xor_sync(0xffffffffu, other, o);
+                    }
+                } else l[0] += __shfl_xor_sync(0xffffffffu, l[0], o);
             }
+            if (NH == 32 || (lane & 1) == 0) lsum[quarter][NH == 32 ? lane : lane >> 1] = l[0];
+            // the results through the ring, which is free: rows of a head, 16 bytes a store (and few instructions: each is fetched once a CTA)
+            float* o_s = reinterpret_cast<float*>(ring);             // [NH][512]
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int h = 0; h < NH; ++h) o_s[h * 512 + i * 128 + kk] = acc[i][h];
             lt_bar(2, 128);
             if (quarter == 0 && lane < nh) {
                 const size_t prow = ((size_t)t * p.H + h0 + lane) * p.max_splits + sp;
-                p.part_ml[prow * 2 + 0] = m * LT_LN2;
+                p.part_ml[prow * 2 + 0] = ref * LT_LN2;
                 p.part_ml[prow * 2 + 1] = (lsum[0][lane] + lsum[1][lane]) + (lsum[2][lane] + lsum[3][lane]);
             }
-            for (int i = 0; i < pairs; ++i) {
-                float o[NH];
-                lt_load<NH>(tmem + lane_addr + O_COL + (unsigned)i * NH, o);
-                const int f = i * 128 + kk;
-                if (f < p.rank) {
-#pragma unroll
-                    for (int h = 0; h < NH; ++h)
-                        if (h < nh) p.part_o[(((size_t)t * p.H + h0 + h) * p.max_splits + sp) * p.rank + f] = o[h];
-                }
+            if (kk * 4 < p.rank) {
+                float* to = p.part_o + (((size_t)t * p.H + h0) * p.max_splits + sp) * p.rank + kk * 4;
+#pragma unroll 4
+                for (int h = 0; h < nh; ++h)
+                    *reinterpret_cast<float4*>(to + (size_t)h * p.max_splits * p.rank) = *reinterpret_cast<const float4*>(o_s + h * 512 + kk * 4);
             }
             tc_fence_before();
-        } else ok = false;
+        }
     }
     if (!ok && lane == 0) atomicExch(&failed, 1);
     __syncthreads();
@@ -402,7 +419,8 @@ extern "C" int bg_latent_attention_tc_plan(int H, int rank, int rot, int page_si
     return lt_slots(nh, rank, rot) > (rank / 64 + 1) / 2 ? BG_OK : BG_ERR_UNSUPPORTED;
 }
 
-// How many ranges the longest-cut row of up to `keys` keys makes, of `ctas` rows (times chunks of heads) on `sms` SMs: what a grid and partial results are sized for.
+// How many ranges the row that is cut into the most of them makes, of up to `keys` keys, with `ctas` rows (times chunks of heads) on `sms` SMs:
+// what a grid and partial results are sized for.
 extern "C" int bg_latent_attention_tc_ranges(int ctas, int keys, int sms) {
     const int tiles = (keys + LATENT_RANGE_STEP - 1) / LATENT_RANGE_STEP;
     int most = 1;

@@ -583,3 +583,24 @@ def test_latent_decoding_takes_rotations_off_a_boundary():
         outs.append(out)
     o.raise_on_status(status)
     assert rel_err(outs[0], outs[1]) < 2e-2
+
+
+@pytest.mark.parametrize("H,rank,spread,bound", [(32, 512, 6.0, 2e-4), (32, 512, 12.0, 1.5e-4), (12, 384, 2.0, 8e-4)])
+def test_latent_decoding_rounds_no_large_weight(H, rank, spread, bound):
+    """Scores with a deviation of `spread`: of the weights in bfloat16 the largest of every tile is one, so that a softmax that picks a few keys loses
+    less than 2^-9 of them.  (With a maximum kept over the tiles, so that the largest weights lie between powers of two: 8.1e-4, 5.6e-4, 1.0e-3.)"""
+    o, rot, page, T, n = ops(), 64, 64, 16, 4000
+    g = torch.Generator().manual_seed(H + n)
+    pages = -(-n // page)
+    pool = torch.randn(T * pages, page, rank + rot, generator=g).to(DEV, torch.bfloat16)
+    q_lat = (spread * torch.randn(H, T, rank, generator=g)).to(torch.bfloat16).float().to(DEV)
+    q_raw = (spread * torch.randn(T, H * (8 + rot), generator=g)).to(DEV, torch.bfloat16)
+    status, out, scale = o.new_status(DEV), torch.full((H, T, rank), NAN, device=DEV), (rank + rot) ** -0.5
+    table = torch.arange(T * pages, dtype=torch.int32, device=DEV).view(T, pages)
+    o.latent_attention(q_lat, q_raw, 8, rot, 0, None, pool, table, i32([n - 1] * T), i32([[r, r, 1] for r in range(T)]), T, n - 1, 1, min(H, 32), 64, 256, scale, out,
+                       status, mma_stages=1)
+    o.raise_on_status(status)
+    keys = pool.view(T, -1, rank + rot)[:, :n].double()
+    q = torch.cat([q_lat.transpose(0, 1), q_raw.view(T, H, -1)[:, :, 8:].float()], -1).double()
+    want = torch.einsum("ths,tsd->htd", torch.softmax(torch.einsum("thd,tsd->ths", q, keys) * scale, -1), keys[:, :, :rank])
+    assert float((out.double() - want).norm() / want.norm()) < bound
