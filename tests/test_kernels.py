@@ -424,15 +424,20 @@ def test_attention_float32_in_blocks_of_any_rows(ops, nh, nkv, hd, vd, options):
     assert all(torch.equal(outs[0], o) for o in outs[1:])
     at, key = positions.long()[:, None], torch.arange(total, device=DEV)[None, :]
     seen = (key <= at) & ((key > at - window) | (key < keep) if window else key >= 0)
-    s = torch.einsum("thd,shd->hts", q.double(), k.double().repeat_interleave(group, 1)) * hd ** -0.5
-    if cap:
-        s = cap * torch.tanh(s / cap)
-    if slopes is not None:
-        s = s - slopes.double()[:, None, None] * (at - key)
-    want = torch.einsum("hts,shd->thd", torch.softmax(s.masked_fill(~seen, -math.inf), -1), v.double().repeat_interleave(group, 1)).reshape(n, -1)
-    # a score's rounding (a chain of hd products, |q||k| at most, and the exponent's) moves a weight by as much, relatively
-    bound = (hd + 16) * 2.0 ** -24 * float((q.abs().sum(-1).max() * k.abs().max() * hd ** -0.5).double() + 4) * float(v.abs().max())
+
+    def attend(q, k, v):
+        s = torch.einsum("thd,shd->hts", q.double(), k.double().repeat_interleave(group, 1)) * hd ** -0.5
+        if cap:
+            s = cap * torch.tanh(s / cap)
+        if slopes is not None:
+            s = s - slopes.double()[:, None, None] * (at - key)
+        return torch.einsum("hts,shd->thd", torch.softmax(s.masked_fill(~seen, -math.inf), -1), v.double().repeat_interleave(group, 1)).reshape(n, -1)
+
+    want = attend(q, k, v)
+    bound = 1e-5 * max(1.0, float(want.abs().max()))               # as the other float tests
     assert float((outs[0].double() - want).abs().max()) < bound
+    short = lambda t: ((t.contiguous().view(torch.int32) + 0x1000) & ~0x1fff).view(torch.float32)      # operands of eleven bits fail it
+    assert float((attend(short(q), short(k), short(v)) - want).abs().max()) > 3 * bound
 
 
 @pytest.mark.parametrize("nh,nkv,hd,vd,window,keep", [(6, 1, 128, 128, 0, 0), (2, 2, 64, 64, 40, 3), (3, 1, 36, 132, 70, 0), (1, 1, 256, 256, 0, 0), (4, 2, 30, 30, 50, 0)])
