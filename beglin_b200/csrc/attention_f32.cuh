@@ -18,29 +18,13 @@
 #pragma once
 
 #include "common.cuh"
+#include "float_pairs.cuh"
 
 namespace bg {
 
 constexpr int AF_ROWS = 64, AF_KEYS = 64, AF_THREADS = 256;
 constexpr int AF_NARROW = 32;              // features of a head up to which a score is one chain of sums
 
-__device__ __forceinline__ unsigned long long af_fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
-    unsigned long long d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;\n" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-    return d;
-}
-__device__ __forceinline__ unsigned long long af_pair(float a, float b) {
-    return (unsigned long long)__float_as_uint(a) | ((unsigned long long)__float_as_uint(b) << 32);
-}
-__device__ __forceinline__ float af_low(unsigned long long v) { return __uint_as_float((unsigned)v); }
-__device__ __forceinline__ float af_high(unsigned long long v) { return __uint_as_float((unsigned)(v >> 32)); }
-__device__ __forceinline__ void af_async16(float* dst, const float* src, bool in) {
-    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(src), "r"(in ? 16 : 0) : "memory");
-}
-__device__ __forceinline__ void af_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-template <int LEFT>
-__device__ __forceinline__ void af_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(LEFT) : "memory"); }
 // reductions over a row's sixteen threads (half a warp)
 __device__ __forceinline__ float af_max16(float v) {
 #pragma unroll
@@ -110,18 +94,18 @@ __device__ __forceinline__ void af_walk(const P& p, const AfShared& s, int req, 
         for (int idx = tid; idx < AF_KEYS * n4; idx += AF_THREADS) {
             const int j = idx / n4, c = idx - j * n4, page = s.page[j];
             const float* src = pool + (page >= 0 ? (size_t)page * page_elems + ((size_t)kvh * p.page_size + (t0 + j) % p.page_size) * hd + c * 4 : 0);
-            af_async16(s.k + j * s.kld + ((c & ~7) | ((c ^ j) & 7)) * 4, src, page >= 0);
+            async_copy<16>(s.k + j * s.kld + ((c & ~7) | ((c ^ j) & 7)) * 4, src, page >= 0);
         }
-        af_commit();
+        async_commit();
     };
     auto fetch_values = [&](int t0) {
         const int n4 = vd >> 2;
         for (int idx = tid; idx < AF_KEYS * n4; idx += AF_THREADS) {
             const int j = idx / n4, c = idx - j * n4, page = s.page[j];
             const float* src = pool + (page >= 0 ? (size_t)page * page_elems + v_off + ((size_t)kvh * p.page_size + (t0 + j) % p.page_size) * vd + c * 4 : 0);
-            af_async16(s.v + j * s.vld + c * 4, src, page >= 0);
+            async_copy<16>(s.v + j * s.vld + c * 4, src, page >= 0);
         }
-        af_commit();
+        async_commit();
     };
 
     int t0 = k_first;
@@ -133,7 +117,7 @@ __device__ __forceinline__ void af_walk(const P& p, const AfShared& s, int req, 
     }
     while (t0 < k_end) {
         fetch_values(t0);
-        af_wait<1>();                      // the keys are there
+        async_wait<1>();                      // the keys are there
         __syncthreads();
         // ---- scores of the thread's rows against keys t0 + tx + 16 j
         unsigned long long sc[RI][4];
@@ -155,7 +139,7 @@ __device__ __forceinline__ void af_walk(const P& p, const AfShared& s, int req, 
                 for (int i = 0; i < RI; ++i)
 #pragma unroll
                     for (int j = 0; j < 4; ++j)            // (in the low half; the high one stays nought)
-                        sc[i][j] = __float_as_uint(fmaf(a[i].w, b[j].w, fmaf(a[i].z, b[j].z, fmaf(a[i].y, b[j].y, fmaf(a[i].x, b[j].x, af_low(sc[i][j]))))));
+                        sc[i][j] = __float_as_uint(fmaf(a[i].w, b[j].w, fmaf(a[i].z, b[j].z, fmaf(a[i].y, b[j].y, fmaf(a[i].x, b[j].x, __uint_as_float((unsigned)sc[i][j]))))));
             }
         } else if (p.maps == 1) {
 #pragma unroll 4
@@ -168,11 +152,11 @@ __device__ __forceinline__ void af_walk(const P& p, const AfShared& s, int req, 
 #pragma unroll
                 for (int j = 0; j < 4; ++j)
 #pragma unroll
-                    for (int u = 0; u < RI; ++u) { const int i = j & 1 ? RI - 1 - u : u; sc[i][j] = af_fma2(a[i].x, b[j].x, sc[i][j]); }
+                    for (int u = 0; u < RI; ++u) { const int i = j & 1 ? RI - 1 - u : u; sc[i][j] = fma2(a[i].x, b[j].x, sc[i][j]); }
 #pragma unroll
                 for (int j = 3; j >= 0; --j)
 #pragma unroll
-                    for (int u = 0; u < RI; ++u) { const int i = j & 1 ? u : RI - 1 - u; sc[i][j] = af_fma2(a[i].y, b[j].y, sc[i][j]); }
+                    for (int u = 0; u < RI; ++u) { const int i = j & 1 ? u : RI - 1 - u; sc[i][j] = fma2(a[i].y, b[j].y, sc[i][j]); }
             }
         } else {                           // rows of different maps meet different columns of a key row: one row's keys at a time
             for (int c = 0; c < (qhd >> 2); ++c) {
@@ -183,7 +167,7 @@ __device__ __forceinline__ void af_walk(const P& p, const AfShared& s, int req, 
 #pragma unroll
                     for (int j = 0; j < 4; ++j) {
                         const ulonglong2 b = *reinterpret_cast<const ulonglong2*>(kr + j * 16 * s.kld + ((kc & ~7) | ((kc ^ sw) & 7)) * 4);
-                        sc[i][j] = af_fma2(a.y, b.y, af_fma2(a.x, b.x, sc[i][j]));
+                        sc[i][j] = fma2(a.y, b.y, fma2(a.x, b.x, sc[i][j]));
                     }
                 }
             }
@@ -198,7 +182,7 @@ __device__ __forceinline__ void af_walk(const P& p, const AfShared& s, int req, 
                 const int key = t0 + tx + 16 * j;
                 w[j] = -INFINITY;
                 if (key <= pos[i] && key < k_end && key_seen(key, lo[i], p.keep) && s.page[tx + 16 * j] >= 0) {
-                    w[j] = (af_low(sc[i][j]) + af_high(sc[i][j])) * p.scale;
+                    w[j] = sum2(sc[i][j]) * p.scale;
                     if (p.softcap > 0.0f) w[j] = p.softcap * tanhf(w[j] / p.softcap);
                     if (p.slopes) w[j] = fmaf(-slope[i], (float)(pos[i] - key), w[j]);
                 }
@@ -218,12 +202,12 @@ __device__ __forceinline__ void af_walk(const P& p, const AfShared& s, int req, 
             if (m_new != -INFINITY) {      // (else no key of this tile or of one before is seen: everything is still nought)
                 m[i] = m_new;
                 l[i] = fmaf(l[i], corr, sum);
-                const unsigned long long cc = af_pair(corr, corr);
+                const unsigned long long cc = pair2(corr, corr);
 #pragma unroll
-                for (int c = 0; c < 2 * NC; ++c) acc[i][c] = af_fma2(acc[i][c], cc, 0ull);
+                for (int c = 0; c < 2 * NC; ++c) acc[i][c] = fma2(acc[i][c], cc, 0ull);
             }
         }
-        af_wait<0>();                      // the values are there; every warp is done with the keys and their pages
+        async_wait<0>();                      // the values are there; every warp is done with the keys and their pages
         __syncthreads();
         const int t1 = next_tile(t0);
         if (t1 < k_end) look_up(t1);
@@ -245,11 +229,11 @@ __device__ __forceinline__ void af_walk(const P& p, const AfShared& s, int req, 
                     const int i = e & 1 ? RI - 1 - u : u;
                     const float f = e == 0 ? a[i].x : e == 1 ? a[i].y : e == 2 ? a[i].z : a[i].w;
                     if (decltype(ask)::value && f == 0.0f) continue;
-                    const unsigned long long ff = af_pair(f, f);
+                    const unsigned long long ff = pair2(f, f);
 #pragma unroll
                     for (int c = 0; c < NC; ++c) {
-                        acc[i][2 * c] = af_fma2(ff, b[c].x, acc[i][2 * c]);
-                        acc[i][2 * c + 1] = af_fma2(ff, b[c].y, acc[i][2 * c + 1]);
+                        acc[i][2 * c] = fma2(ff, b[c].x, acc[i][2 * c]);
+                        acc[i][2 * c + 1] = fma2(ff, b[c].y, acc[i][2 * c + 1]);
                     }
                 }
             }
@@ -313,9 +297,9 @@ __global__ void __launch_bounds__(AF_THREADS, NC <= 2 ? 2 : 1) attention_f32_ker
         const int r = idx / n4, c = idx - r * n4, qi = r / p.group, g = r - qi * p.group;
         const bool in = r < n_rows;
         const float* src = (const float*)p.q + (in ? (size_t)(row0 + qi) * p.q_stride + (size_t)(kvh * p.group + g) * qhd + c * 4 : 0);
-        af_async16(s.q + r * s.qld + c * 4, src, in);
+        async_copy<16>(s.q + r * s.qld + c * 4, src, in);
     }
-    af_commit();                           // (complete when the first keys are)
+    async_commit();                           // (complete when the first keys are)
     if (s.vld > p.vd)
         for (int idx = threadIdx.x; idx < AF_KEYS * (s.vld - p.vd); idx += AF_THREADS)
             s.v[idx / (s.vld - p.vd) * s.vld + p.vd + idx % (s.vld - p.vd)] = 0.0f;

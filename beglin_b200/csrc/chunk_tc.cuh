@@ -319,7 +319,10 @@ __global__ void __launch_bounds__(CT_THREADS, 2) chunk_out_tc_kernel(R r) {
 // (a block behind the tiles: the score product reads 128 rows from a tile of 64)
 constexpr size_t CT_SMEM = 1024 + 2 * (size_t)CT_TILE + CT_BLOCK;
 // Heads whose sizes fill whole MMA steps and most of a row's threads: n and nv multiples of 16 from 48 to 128.  (Four heads of 32 x 16: 23 us
-// for 194 tokens on the float units, 23 to 33 here.)
+// for 194 tokens on the float units, 23 to 33 here.)  Decayed attention of 12 heads, one chunk and 2,048 rows, all three kernels, float units and
+// here: 48 x 48 30 and 20, 70 and 45 us; 64 x 64 53 and 21, 86 and 47; 96 x 96 66 and 34, 154 and 73; a chunk of 16 rows 27 and 20 (64 x 64), 39
+// and 34 (128 x 128).  Per-channel decay of 16 heads: 48 x 48 46 and 39, 89 and 77; 64 x 64 50 and 39, 100 and 84.  Against 64 bits outputs and
+// states are off by as much or less than on the float units at each of them.
 __host__ inline bool ct_takes(int n, int nv) { return n >= 48 && n <= 128 && nv >= 48 && nv <= 128 && n % 16 == 0 && nv % 16 == 0; }
 
 template <typename K, typename R>

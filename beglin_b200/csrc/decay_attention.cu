@@ -459,7 +459,6 @@ struct DecayTc {
         __device__ float4 score_key(const float4& x, int, int) const { return silu(x, 1.0f); }
         __device__ float weight(float score, int t, int j) const { return score * pw[t - j]; }
         __device__ float factor(int t) const { return pw[t + 1]; }
-        template <typename W> __device__ void weights(W) const {}
         __device__ void finish(const float* o) const {
             const int w4 = r.nv >> 2;
             for (int idx = threadIdx.x; idx < rows * w4; idx += blockDim.x) {

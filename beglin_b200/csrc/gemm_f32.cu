@@ -20,6 +20,7 @@
 //   gemm_f32_few_kernel    up to 16 rows: the product is a stream of weights
 //   gemm_f32_ranges_kernel adds the sums of ranges that went to CTAs of their own
 #include "common.cuh"
+#include "float_pairs.cuh"
 
 namespace bg {
 
@@ -36,27 +37,6 @@ struct GfParams {
     int lda, ldw, ldc, M, N, K, accumulate, ranges, batch;
 };
 
-// c + a b for the two floats of each pair
-__device__ __forceinline__ unsigned long long gf_fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
-    unsigned long long d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;\n" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-    return d;
-}
-__device__ __forceinline__ float gf_sum2(unsigned long long v) {
-    return __uint_as_float((unsigned)v) + __uint_as_float((unsigned)(v >> 32));
-}
-
-template <int BYTES>
-__device__ __forceinline__ void gf_async(float* dst, const float* src, bool in) {
-    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-    const int n = in ? BYTES : 0;          // (nothing is read where n is 0; the destination gets zeros)
-    if constexpr (BYTES == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(src), "r"(n) : "memory");
-    else asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(d), "l"(src), "r"(n) : "memory");
-}
-template <int LEFT>
-__device__ __forceinline__ void gf_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(LEFT) : "memory"); }
-__device__ __forceinline__ void gf_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-
 // ROWS rows of GF_BK values from column k on into a tile of row stride GF_LD (`src`: the tile's first row, of which `rows` exist);
 // what lies behind `rows` or K becomes zeros.
 template <int ROWS, bool VEC>
@@ -66,7 +46,7 @@ __device__ __forceinline__ void gf_fetch(float* dst, const float* src, int ld, i
     for (int i = 0; i < ROWS * PER_ROW / GF_THREADS; ++i) {
         const int r = threadIdx.x / PER_ROW + i * (GF_THREADS / PER_ROW), c = threadIdx.x % PER_ROW * W;
         const bool in = r < rows && k + c < K;
-        gf_async<W * 4>(dst + r * GF_LD + c, src + (in ? (size_t)((unsigned)r * (unsigned)ld + (unsigned)(k + c)) : 0), in);
+        async_copy<W * 4>(dst + r * GF_LD + c, src + (in ? (size_t)((unsigned)r * (unsigned)ld + (unsigned)(k + c)) : 0), in);
     }
 }
 
@@ -157,7 +137,7 @@ __global__ void __launch_bounds__(GF_THREADS, 1) gemm_f32_tile_kernel(GfParams p
                 gf_fetch<BM, VEC>(st, A, p.lda, p.M - m0, k_begin + s * GF_BK, k_end);
                 gf_fetch<GF_BN, VEC>(st + BM * GF_LD, W, p.ldw, p.N - n0, k_begin + s * GF_BK, k_end);
             }
-            gf_commit();
+            async_commit();
         };
         unsigned long long acc[RI][8];
 #pragma unroll
@@ -168,7 +148,7 @@ __global__ void __launch_bounds__(GF_THREADS, 1) gemm_f32_tile_kernel(GfParams p
 #pragma unroll
         for (int s = 0; s < GF_STAGES - 1; ++s) fetch(s);
         for (int s = 0; s < steps; ++s) {
-            gf_wait<GF_STAGES - 2>();
+            async_wait<GF_STAGES - 2>();
             __syncthreads();
             fetch(s + GF_STAGES - 1);      // into the stage that was read in the step before
             const float* As = gf_s + (s % GF_STAGES) * STAGE + ty * GF_LD;
@@ -184,21 +164,21 @@ __global__ void __launch_bounds__(GF_THREADS, 1) gemm_f32_tile_kernel(GfParams p
 #pragma unroll
                 for (int j = 0; j < 8; ++j)
 #pragma unroll
-                    for (int u = 0; u < RI; ++u) { const int i = j & 1 ? RI - 1 - u : u; acc[i][j] = gf_fma2(a[i].x, w[j].x, acc[i][j]); }
+                    for (int u = 0; u < RI; ++u) { const int i = j & 1 ? RI - 1 - u : u; acc[i][j] = fma2(a[i].x, w[j].x, acc[i][j]); }
 #pragma unroll
                 for (int j = 7; j >= 0; --j)
 #pragma unroll
-                    for (int u = 0; u < RI; ++u) { const int i = j & 1 ? u : RI - 1 - u; acc[i][j] = gf_fma2(a[i].y, w[j].y, acc[i][j]); }
+                    for (int u = 0; u < RI; ++u) { const int i = j & 1 ? u : RI - 1 - u; acc[i][j] = fma2(a[i].y, w[j].y, acc[i][j]); }
             }
         }
-        gf_wait<0>();
+        async_wait<0>();
         if (range + 1 < r_end) {           // more ranges follow in this CTA
 #pragma unroll
             for (int i = 0; i < RI; ++i)
 #pragma unroll
                 for (int j = 0; j < 8; ++j) {
                     float* t = total + (i * 8 + j) * GF_THREADS;
-                    *t = range == r_begin ? gf_sum2(acc[i][j]) : *t + gf_sum2(acc[i][j]);
+                    *t = range == r_begin ? sum2(acc[i][j]) : *t + sum2(acc[i][j]);
                 }
             continue;
         }
@@ -210,7 +190,7 @@ __global__ void __launch_bounds__(GF_THREADS, 1) gemm_f32_tile_kernel(GfParams p
             for (int j = 0; j < 8; ++j) {
                 const int n = n0 + tx + 16 * j;
                 if (n >= p.N) continue;
-                float v = gf_sum2(acc[i][j]);
+                float v = sum2(acc[i][j]);
                 if (p.part) {
                     p.part[(((size_t)range * p.batch + b) * p.M + m) * p.N + n] = v;
                     continue;
@@ -283,7 +263,7 @@ __global__ void __launch_bounds__(GW_WARPS * 32) gemm_f32_few_kernel(GfParams p,
 #pragma unroll
             for (int r = 0; r < GW_COLS; r += 4) {
                 const bool in = n0 + r + fr < p.N && k < k_end;
-                gf_async<16>(st + r * GW_LD, in ? W + (size_t)(n0 + r + fr) * p.ldw + k : W, in);
+                async_copy<16>(st + r * GW_LD, in ? W + (size_t)(n0 + r + fr) * p.ldw + k : W, in);
             }
         };
         auto fetch_a = [&](int s) {
@@ -293,7 +273,7 @@ __global__ void __launch_bounds__(GW_WARPS * 32) gemm_f32_few_kernel(GfParams p,
             for (int r = 0; r < 2 * RPL; r += 4) {
                 if (r + fr >= 2 * RPL) continue;
                 const bool in = r + fr < p.M && k < k_end;
-                gf_async<16>(st + r * GW_LD, in ? A + (size_t)(r + fr) * p.lda + k : A, in);
+                async_copy<16>(st + r * GW_LD, in ? A + (size_t)(r + fr) * p.lda + k : A, in);
             }
         };
         __syncwarp();                      // (the last job's ring has been read)
@@ -304,16 +284,16 @@ __global__ void __launch_bounds__(GW_WARPS * 32) gemm_f32_few_kernel(GfParams p,
 #pragma unroll
         for (int s = 0; s < GW_STAGES - 1; ++s) {                          // (the first group holds all the weights asked for above)
             if (s < steps) fetch_a(s);
-            gf_commit();
+            async_commit();
         }
         unsigned long long acc[2][RPL];
 #pragma unroll
         for (int r = 0; r < RPL; ++r) acc[0][r] = acc[1][r] = 0ull;
         for (int s = 0; s < steps; ++s) {
-            gf_wait<GW_STAGES - 2>();
+            async_wait<GW_STAGES - 2>();
             __syncwarp();
             if (s + GW_STAGES - 1 < steps) { fetch_w(s + GW_STAGES - 1); fetch_a(s + GW_STAGES - 1); }
-            gf_commit();
+            async_commit();
             const float* ws = ring + (s % GW_STAGES) * STAGE + c * GW_LD;
             const float* as = ring + (s % GW_STAGES) * STAGE + (GW_COLS + g * RPL) * GW_LD;
             // (k behind the range's end: zeros on both sides)
@@ -324,15 +304,15 @@ __global__ void __launch_bounds__(GW_WARPS * 32) gemm_f32_few_kernel(GfParams p,
 #pragma unroll
                 for (int r = 0; r < RPL; ++r) a[r] = *reinterpret_cast<const ulonglong2*>(as + r * GW_LD + k);
 #pragma unroll
-                for (int r = 0; r < RPL; ++r) { acc[0][r] = gf_fma2(a[r].x, w0.x, acc[0][r]); acc[1][r] = gf_fma2(a[r].x, w1.x, acc[1][r]); }
+                for (int r = 0; r < RPL; ++r) { acc[0][r] = fma2(a[r].x, w0.x, acc[0][r]); acc[1][r] = fma2(a[r].x, w1.x, acc[1][r]); }
 #pragma unroll
-                for (int r = 0; r < RPL; ++r) { acc[0][r] = gf_fma2(a[r].y, w0.y, acc[0][r]); acc[1][r] = gf_fma2(a[r].y, w1.y, acc[1][r]); }
+                for (int r = 0; r < RPL; ++r) { acc[0][r] = fma2(a[r].y, w0.y, acc[0][r]); acc[1][r] = fma2(a[r].y, w1.y, acc[1][r]); }
             }
         }
-        gf_wait<0>();
+        async_wait<0>();
         float* out = sums + (size_t)((group * n_ranges + range) * 2 * RPL + g * RPL) * GW_COLS + c;
 #pragma unroll
-        for (int r = 0; r < RPL; ++r) { out[r * GW_COLS] = gf_sum2(acc[0][r]); out[r * GW_COLS + 16] = gf_sum2(acc[1][r]); }
+        for (int r = 0; r < RPL; ++r) { out[r * GW_COLS] = sum2(acc[0][r]); out[r * GW_COLS + 16] = sum2(acc[1][r]); }
     }
     if (!waited) pdl_wait();               // (no warp goes on to the sums before it)
     __syncthreads();

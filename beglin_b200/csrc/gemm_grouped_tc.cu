@@ -188,6 +188,8 @@ extern "C" int bg_gemm_grouped_tc(const void* W, int E, int n_out, int K, int ld
         case 32: return grouped_launch<32, 4>(mw, mx, p, rows, stream);
         case 64: return grouped_launch<64, 4>(mw, mx, p, rows, stream);
         case 128: return grouped_launch<128, 3>(mw, mx, p, rows, stream);
-        default: return grouped_launch<256, 2>(mw, mx, p, rows, stream);      // (two CTAs an SM: one's epilogue under the other's MMAs)
+        // (more than 128 rows each of more than 512 experts: with fewer, such steps run on pairs of CTAs.  Two CTAs an SM, one's epilogue under
+        // the other's MMAs.)
+        default: return grouped_launch<256, 2>(mw, mx, p, rows, stream);
     }
 }

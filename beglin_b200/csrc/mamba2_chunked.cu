@@ -297,7 +297,9 @@ __global__ void __launch_bounds__(128) ssm_chunk_out_kernel(SsmChunkParams p) {
     }
 }
 
-// The chunks' sums and outputs on the tensor cores, from operands in three bfloat16 parts (chunk_tc.cuh).
+// The chunks' sums and outputs on the tensor cores, from operands in three bfloat16 parts (chunk_tc.cuh).  Off by, of 64 bits, outputs and
+// states over 2,048 rows of 24 heads: 128 x 128 2.6e-7 and 3.3e-7 (the walk 2.9e-7 and 3.6e-7, chunks on the float units 3.0e-7 and 3.5e-7), 96 x 128
+// 3.7e-7 and 3.1e-7 (4.3e-7 and 3.7e-7; 4.0e-7 and 3.2e-7), 80 x 80 1.06e-7 and 1.28e-7 (0.91e-7 and 1.27e-7; 1.19e-7 and 1.41e-7).
 template <typename TI, typename TW>
 struct SsmTc {
     static constexpr bool SCORES = false;
@@ -336,9 +338,6 @@ struct SsmTc {
         __device__ float4 out_value(const float4& x, int, int) const { return x; }
         __device__ float4 query_raw(int t, int i) const { return at(t, r.p.H * r.nv + (r.p.G + g) * r.n + i); }
         __device__ float4 query(const float4& x, int, int) const { return x; }
-        __device__ float4 score_key_raw(int, int) const { return make_float4(0.0f, 0.0f, 0.0f, 0.0f); }
-        __device__ float4 score_key(const float4& x, int, int) const { return x; }
-        __device__ float weight(float score, int, int) const { return score; }
         __device__ float factor(int t) const { return (t >= MC / 2 ? s.pre[MC / 2 - 1] : 1.0f) * s.pre[t]; }
         // the weight of key j at query t: score x (product of the decays behind j up to t) x step.  Threads 0 .. 63: the queries of the
         // key's own half of the chunk, one decay after the other; 64 .. 127: those of the second half for keys of the first; 128 ..

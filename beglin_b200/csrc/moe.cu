@@ -210,8 +210,8 @@ route_vec8_kernel(const TI* __restrict__ h, int ldh, const float* __restrict__ W
 }
 
 // Routing, layout and gather of a step of few tokens as ONE kernel: three dependent launches cost more than their work, on
-// the device (eight tokens, ten router outputs: 7.9 us as three kernels, 6.8 as one) and most of all, outside a graph, on the host (a
-// gated layer with identity and shared experts: 140 -> 126 us).  A cluster of eight CTAs, a token each, routed as in the kernel above
+// the device (eight tokens, ten router outputs: 8.0 us as three kernels, 6.4 as one) and most of all, outside a graph, on the host (a
+// gated layer with identity and shared experts: 138 -> 125 us).  A cluster of eight CTAs, a token each, routed as in the kernel above
 // (the same sums, so the same choice); with two tokens a CTA, one after the other, it lost (10.7 against 8.1 us).  The CTAs read each other's choices through the cluster, each lays out all
 // assignments for itself (an assignment's row: those of smaller experts and the earlier ones of its own, counted) and gathers its own
 // tokens' rows.  Inside an expert the rows stand in the order of the assignments.
