@@ -112,8 +112,8 @@ __global__ void __launch_bounds__(GF_THREADS) gemm_f32_short_kernel(GfParams p) 
 // lie in shared memory as they do in memory, k innermost, so they come by 16-byte asynchronous copies and a thread reads four k of a
 // row at a time: 16 reads of 16 bytes for 128 packed multiply-adds.  A warp covers 4 x 8 (ty, tx); rows 20 floats apart put eight
 // neighbouring rows into different banks.  One CTA an SM (the sums take 128 registers).  550 rows of 1,536 x 17,920: 930 us, 32.5
-// TFLOP/s, where tiles of 64 x 64 with 4-byte loads and no pipeline took 1,720 us; what it waits for is the reads of shared memory,
-// which at this ratio take as long as the multiply-adds.
+// TFLOP/s, where tiles of 64 x 64 with 4-byte loads and no pipeline took 1,720 us; its two warps a scheduler wait for the FMA pipe's
+// queue and for fixed latencies as long as they issue (FMA pipe 54 %, reads of shared memory 40 % of their rates).
 template <int BM, bool VEC>
 __global__ void __launch_bounds__(GF_THREADS, 1) gemm_f32_tile_kernel(GfParams p) {
     extern __shared__ __align__(16) float gf_s[];
