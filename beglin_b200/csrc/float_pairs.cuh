@@ -13,6 +13,8 @@ __device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigne
 __device__ __forceinline__ unsigned long long pair2(float a, float b) {
     return (unsigned long long)__float_as_uint(a) | ((unsigned long long)__float_as_uint(b) << 32);
 }
+__device__ __forceinline__ float low2(unsigned long long v) { return __uint_as_float((unsigned)v); }
+__device__ __forceinline__ float high2(unsigned long long v) { return __uint_as_float((unsigned)(v >> 32)); }
 __device__ __forceinline__ float sum2(unsigned long long v) { return __uint_as_float((unsigned)v) + __uint_as_float((unsigned)(v >> 32)); }
 
 // 16 or 4 bytes, or zeros where `in` is false (nothing is read then)

@@ -15,7 +15,7 @@
 // Inner sizes of up to GF_SHORT are summed in one chain, k = 0 .. K-1 in order, whatever the rows: two chains and a pipeline over k gain
 // nothing there.
 //
-//   gemm_f32_short_kernel  inner sizes of up to 64
+//   gemm_f32_short_kernel  inner sizes of up to 64, and of up to 128 with more than 16 rows
 //   gemm_f32_tile_kernel   tiles of 128 (or 64) rows x 128 columns, for more than 16 rows
 //   gemm_f32_few_kernel    up to 16 rows: the product is a stream of weights
 //   gemm_f32_ranges_kernel adds the sums of ranges that went to CTAs of their own
@@ -50,15 +50,19 @@ __device__ __forceinline__ void gf_fetch(float* dst, const float* src, int ld, i
     }
 }
 
-// Inner sizes of up to GF_SHORT (narrow models, small heads): both operands come whole, BM rows and 64 columns, and a thread sums
-// rows ty + 16 i and columns tx + 16 j, four k of a row at a read (rows 68 floats apart: eight neighbouring ones in different banks).
+// Short inner sizes (narrow models, small heads): both operands come whole, BM rows and 64 columns, and a thread sums rows ty + 16 i
+// and columns tx + 16 j, four k of a row at a read (rows 68 or 132 floats apart: eight neighbouring ones in different banks).  Above GF_SHORT
+// in two chains, as the kernels of larger inner sizes, whose bits these are.
 // Bound by its reads of shared memory and by the results it writes.  2,048 x 4,096 with k of 64: 36 us, 51 in two chains by the pipelined
-// tiles; sixteen products of 2,048 x 512: 71 and 89, with k of 32 43 and 63.
-constexpr int GS_BN = 64, GS_LD = GF_SHORT + 4;
-template <int BM>
+// tiles; sixteen products of 2,048 x 512: 71 and 89, with k of 32 43 and 63; 64 x 640 with k of 72 5.4 and 8.8 (7.5 in tiles of 64 x 64 without
+// a pipeline), 2,048 x 640 10.4 and 16.8, 8,192 x 2,048 with k of 128 121 and 141, 300 x 2,048 14.0 and 12.0.
+constexpr int GS_BN = 64;
+template <int BM, bool TWO>
 __global__ void __launch_bounds__(GF_THREADS) gemm_f32_short_kernel(GfParams p) {
     constexpr int RI = BM / 16, CJ = GS_BN / 16, EACH = GF_THREADS / 32;          // EACH: rows that the threads bring at a time
-    __shared__ __align__(16) float As[BM * GS_LD], Ws[GS_BN * GS_LD];
+    constexpr int MOST = TWO ? 2 * GF_SHORT : GF_SHORT, LD = MOST + 4;
+    extern __shared__ __align__(16) float gf_s[];
+    float *As = gf_s, *Ws = gf_s + BM * LD;
     pdl_launch();
     pdl_wait();
     const int m0 = blockIdx.y * BM, n0 = blockIdx.x * GS_BN, tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
@@ -66,32 +70,35 @@ __global__ void __launch_bounds__(GF_THREADS) gemm_f32_short_kernel(GfParams p) 
     const float* A = p.A + (size_t)blockIdx.z * p.batch_a;
     const float* W = p.W + (size_t)blockIdx.z * p.batch_w;
 #pragma unroll
-    for (int h = 0; h < GF_SHORT; h += 32) {             // (zeros behind K, the rows and the columns)
+    for (int h = 0; h < MOST; h += 32) {                 // (zeros behind K, the rows and the columns)
         const int k = h + lane;
         if (h >= p.K) break;
 #pragma unroll
-        for (int r = warp; r < BM; r += EACH) As[r * GS_LD + k] = k < p.K && m0 + r < p.M ? A[(size_t)(m0 + r) * p.lda + k] : 0.0f;
+        for (int r = warp; r < BM; r += EACH) As[r * LD + k] = k < p.K && m0 + r < p.M ? A[(size_t)(m0 + r) * p.lda + k] : 0.0f;
 #pragma unroll
-        for (int r = warp; r < GS_BN; r += EACH) Ws[r * GS_LD + k] = k < p.K && n0 + r < p.N ? W[(size_t)(n0 + r) * p.ldw + k] : 0.0f;
+        for (int r = warp; r < GS_BN; r += EACH) Ws[r * LD + k] = k < p.K && n0 + r < p.N ? W[(size_t)(n0 + r) * p.ldw + k] : 0.0f;
     }
     __syncthreads();
-    float acc[RI][CJ];
+    unsigned long long acc[RI][CJ];                      // (one chain: in the low half, the high one stays nought)
 #pragma unroll
     for (int i = 0; i < RI; ++i)
 #pragma unroll
-        for (int j = 0; j < CJ; ++j) acc[i][j] = 0.0f;
+        for (int j = 0; j < CJ; ++j) acc[i][j] = 0ull;
 #pragma unroll 4
     for (int k = 0; k < p.K; k += 4) {
-        float4 a[RI], w[CJ];
+        ulonglong2 a[RI], w[CJ];
 #pragma unroll
-        for (int i = 0; i < RI; ++i) a[i] = *reinterpret_cast<const float4*>(As + (ty + 16 * i) * GS_LD + k);
+        for (int i = 0; i < RI; ++i) a[i] = *reinterpret_cast<const ulonglong2*>(As + (ty + 16 * i) * LD + k);
 #pragma unroll
-        for (int j = 0; j < CJ; ++j) w[j] = *reinterpret_cast<const float4*>(Ws + (tx + 16 * j) * GS_LD + k);
+        for (int j = 0; j < CJ; ++j) w[j] = *reinterpret_cast<const ulonglong2*>(Ws + (tx + 16 * j) * LD + k);
 #pragma unroll
         for (int i = 0; i < RI; ++i)
 #pragma unroll
-            for (int j = 0; j < CJ; ++j)
-                acc[i][j] = fmaf(a[i].w, w[j].w, fmaf(a[i].z, w[j].z, fmaf(a[i].y, w[j].y, fmaf(a[i].x, w[j].x, acc[i][j]))));
+            for (int j = 0; j < CJ; ++j) {
+                if constexpr (TWO) acc[i][j] = fma2(a[i].y, w[j].y, fma2(a[i].x, w[j].x, acc[i][j]));
+                else acc[i][j] = __float_as_uint(fmaf(high2(a[i].y), high2(w[j].y), fmaf(low2(a[i].y), low2(w[j].y),
+                                                 fmaf(high2(a[i].x), high2(w[j].x), fmaf(low2(a[i].x), low2(w[j].x), low2(acc[i][j]))))));
+            }
     }
 #pragma unroll
     for (int i = 0; i < RI; ++i) {
@@ -101,7 +108,8 @@ __global__ void __launch_bounds__(GF_THREADS) gemm_f32_short_kernel(GfParams p) 
         for (int j = 0; j < CJ; ++j) {
             const int n = n0 + tx + 16 * j;
             if (n >= p.N) continue;
-            const float v = p.bias ? acc[i][j] + p.bias[n] : acc[i][j];
+            float v = TWO ? sum2(acc[i][j]) : low2(acc[i][j]);
+            if (p.bias) v += p.bias[n];
             float* c = p.C + (size_t)blockIdx.z * p.batch_c + (size_t)m * p.ldc + n;
             *c = p.accumulate ? *c + v : v;
         }
@@ -114,15 +122,15 @@ __global__ void __launch_bounds__(GF_THREADS) gemm_f32_short_kernel(GfParams p) 
 // neighbouring rows into different banks.  One CTA an SM (the sums take 128 registers).  550 rows of 1,536 x 17,920: 930 us, 32.5
 // TFLOP/s, where tiles of 64 x 64 with 4-byte loads and no pipeline took 1,720 us; its two warps a scheduler wait for the FMA pipe's
 // queue and for fixed latencies as long as they issue (FMA pipe 54 %, reads of shared memory 40 % of their rates).
-template <int BM, bool VEC>
+template <int BM, int BN, bool VEC>
 __global__ void __launch_bounds__(GF_THREADS, 1) gemm_f32_tile_kernel(GfParams p) {
     extern __shared__ __align__(16) float gf_s[];
-    constexpr int RI = BM / 16, STAGE = (BM + GF_BN) * GF_LD;
-    float* total = gf_s + GF_STAGES * STAGE + threadIdx.x;       // [RI * 8][GF_THREADS]: the ranges' sums so far, a thread's own
+    constexpr int RI = BM / 16, CJ = BN / 16, STAGE = (BM + BN) * GF_LD;
+    float* total = gf_s + GF_STAGES * STAGE + threadIdx.x;       // [RI * CJ][GF_THREADS]: the ranges' sums so far, a thread's own
     pdl_launch();
     pdl_wait();
     const int b = blockIdx.z % p.batch, own = blockIdx.z / p.batch;
-    const int m0 = blockIdx.y * BM, n0 = blockIdx.x * GF_BN;
+    const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
     const float* A = p.A + (size_t)b * p.batch_a + (size_t)m0 * p.lda;
     const float* W = p.W + (size_t)b * p.batch_w + (size_t)n0 * p.ldw;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -135,15 +143,15 @@ __global__ void __launch_bounds__(GF_THREADS, 1) gemm_f32_tile_kernel(GfParams p
             if (s < steps) {
                 float* st = gf_s + (s % GF_STAGES) * STAGE;
                 gf_fetch<BM, VEC>(st, A, p.lda, p.M - m0, k_begin + s * GF_BK, k_end);
-                gf_fetch<GF_BN, VEC>(st + BM * GF_LD, W, p.ldw, p.N - n0, k_begin + s * GF_BK, k_end);
+                gf_fetch<BN, VEC>(st + BM * GF_LD, W, p.ldw, p.N - n0, k_begin + s * GF_BK, k_end);
             }
             async_commit();
         };
-        unsigned long long acc[RI][8];
+        unsigned long long acc[RI][CJ];
 #pragma unroll
         for (int i = 0; i < RI; ++i)
 #pragma unroll
-            for (int j = 0; j < 8; ++j) acc[i][j] = 0ull;
+            for (int j = 0; j < CJ; ++j) acc[i][j] = 0ull;
         __syncthreads();                   // (the last range's tiles have been read)
 #pragma unroll
         for (int s = 0; s < GF_STAGES - 1; ++s) fetch(s);
@@ -155,18 +163,18 @@ __global__ void __launch_bounds__(GF_THREADS, 1) gemm_f32_tile_kernel(GfParams p
             const float* Ws = gf_s + (s % GF_STAGES) * STAGE + (BM + tx) * GF_LD;
 #pragma unroll
             for (int k = 0; k < GF_BK; k += 4) {
-                ulonglong2 a[RI], w[8];
+                ulonglong2 a[RI], w[CJ];
 #pragma unroll
                 for (int i = 0; i < RI; ++i) a[i] = *reinterpret_cast<const ulonglong2*>(As + i * 16 * GF_LD + k);
 #pragma unroll
-                for (int j = 0; j < 8; ++j) w[j] = *reinterpret_cast<const ulonglong2*>(Ws + j * 16 * GF_LD + k);
+                for (int j = 0; j < CJ; ++j) w[j] = *reinterpret_cast<const ulonglong2*>(Ws + j * 16 * GF_LD + k);
                 // rows to and fro under the columns
 #pragma unroll
-                for (int j = 0; j < 8; ++j)
+                for (int j = 0; j < CJ; ++j)
 #pragma unroll
                     for (int u = 0; u < RI; ++u) { const int i = j & 1 ? RI - 1 - u : u; acc[i][j] = fma2(a[i].x, w[j].x, acc[i][j]); }
 #pragma unroll
-                for (int j = 7; j >= 0; --j)
+                for (int j = CJ - 1; j >= 0; --j)
 #pragma unroll
                     for (int u = 0; u < RI; ++u) { const int i = j & 1 ? u : RI - 1 - u; acc[i][j] = fma2(a[i].y, w[j].y, acc[i][j]); }
             }
@@ -176,8 +184,8 @@ __global__ void __launch_bounds__(GF_THREADS, 1) gemm_f32_tile_kernel(GfParams p
 #pragma unroll
             for (int i = 0; i < RI; ++i)
 #pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                    float* t = total + (i * 8 + j) * GF_THREADS;
+                for (int j = 0; j < CJ; ++j) {
+                    float* t = total + (i * CJ + j) * GF_THREADS;
                     *t = range == r_begin ? sum2(acc[i][j]) : *t + sum2(acc[i][j]);
                 }
             continue;
@@ -187,7 +195,7 @@ __global__ void __launch_bounds__(GF_THREADS, 1) gemm_f32_tile_kernel(GfParams p
             const int m = m0 + ty + 16 * i;
             if (m >= p.M) continue;
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
+            for (int j = 0; j < CJ; ++j) {
                 const int n = n0 + tx + 16 * j;
                 if (n >= p.N) continue;
                 float v = sum2(acc[i][j]);
@@ -195,7 +203,7 @@ __global__ void __launch_bounds__(GF_THREADS, 1) gemm_f32_tile_kernel(GfParams p
                     p.part[(((size_t)range * p.batch + b) * p.M + m) * p.N + n] = v;
                     continue;
                 }
-                if (range > r_begin) v = total[(i * 8 + j) * GF_THREADS] + v;
+                if (range > r_begin) v = total[(i * CJ + j) * GF_THREADS] + v;
                 if (p.bias) v += p.bias[n];
                 float* c = p.C + (size_t)b * p.batch_c + (size_t)m * p.ldc + n;
                 *c = p.accumulate ? *c + v : v;
@@ -362,6 +370,8 @@ static int gf_cuts(int M, int N, int ranges, int batch, int bm) {
     return rows >= M ? M : (int)(rows / bm * bm);
 }
 
+// Inner sizes that go to the short kernel; from 16 rows down, longer than GF_SHORT, the product is a stream of weights as others.
+static bool gf_short(int M, int K) { return K <= GF_SHORT || (K <= 2 * GF_SHORT && M > GF_FEW); }
 static bool gf_few(int M, int ranges, bool vec) { return vec && M <= GF_FEW && ranges <= 64; }
 // Tiles of 64 rows where 128 would be half empty, or leave SMs without a tile.
 static int gf_bm(int M, int N, int ranges, int batch) {
@@ -383,14 +393,24 @@ static cudaError_t gf_launch_few(const GfParams& p, cudaStream_t stream) {
     const unsigned x = (unsigned)((p.N + groups * GW_COLS - 1) / (groups * GW_COLS));
     return launch(gemm_f32_few_kernel<RPL>, dim3(x, p.batch, shares), dim3(warps * 32), smem, stream, p, groups);
 }
-template <int BM, bool VEC>
+template <int BM, int BN, bool VEC>
 static cudaError_t gf_launch_tile(const GfParams& p, cudaStream_t stream) {
-    constexpr size_t tiles = (size_t)GF_STAGES * (BM + GF_BN) * GF_LD * sizeof(float), totals = (size_t)BM * GF_BN * sizeof(float);
+    constexpr size_t tiles = (size_t)GF_STAGES * (BM + BN) * GF_LD * sizeof(float), totals = (size_t)BM * BN * sizeof(float);
     const size_t smem = p.part || p.ranges == 1 ? tiles : tiles + totals;
-    cudaError_t e = cudaFuncSetAttribute(gemm_f32_tile_kernel<BM, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(tiles + totals));
+    cudaError_t e = cudaFuncSetAttribute(gemm_f32_tile_kernel<BM, BN, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(tiles + totals));
     if (e != cudaSuccess) return e;
-    const dim3 grid((p.N + GF_BN - 1) / GF_BN, (p.M + BM - 1) / BM, p.batch * (p.part ? p.ranges : 1));
-    return launch(gemm_f32_tile_kernel<BM, VEC>, grid, dim3(GF_THREADS), smem, stream, p);
+    const dim3 grid((p.N + BN - 1) / BN, (p.M + BM - 1) / BM, p.batch * (p.part ? p.ranges : 1));
+    return launch(gemm_f32_tile_kernel<BM, BN, VEC>, grid, dim3(GF_THREADS), smem, stream, p);
+}
+
+template <int BM, bool TWO>
+static cudaError_t gf_launch_short(const GfParams& p, cudaStream_t stream) {
+    constexpr size_t smem = (size_t)(BM + GS_BN) * ((TWO ? 2 * GF_SHORT : GF_SHORT) + 4) * sizeof(float);
+    const dim3 grid((p.N + GS_BN - 1) / GS_BN, (p.M + BM - 1) / BM, p.batch);
+    if (grid.y > 65535) return cudaErrorInvalidConfiguration;
+    cudaError_t e = cudaFuncSetAttribute(gemm_f32_short_kernel<BM, TWO>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    return launch(gemm_f32_short_kernel<BM, TWO>, grid, dim3(GF_THREADS), smem, stream, p);
 }
 
 static cudaError_t gf_add_ranges(const GfParams& p, cudaStream_t stream) {
@@ -402,12 +422,9 @@ static int gf_run(GfParams p, cudaStream_t stream) {
     const bool vec = p.K % 4 == 0 && p.lda % 4 == 0 && p.ldw % 4 == 0 && p.batch_a % 4 == 0 && p.batch_w % 4 == 0 &&
                      (uintptr_t)p.A % 16 == 0 && (uintptr_t)p.W % 16 == 0;
     p.ranges = (p.K + GF_RANGE - 1) / GF_RANGE;
-    if (p.K <= GF_SHORT) {
-        const int bm = p.M <= 16 ? 16 : 64;
-        const dim3 grid((p.N + GS_BN - 1) / GS_BN, (p.M + bm - 1) / bm, p.batch);
-        if (grid.y > 65535) return BG_ERR_SHAPE;
-        const cudaError_t e = bm == 16 ? launch(gemm_f32_short_kernel<16>, grid, dim3(GF_THREADS), 0, stream, p)
-                                       : launch(gemm_f32_short_kernel<64>, grid, dim3(GF_THREADS), 0, stream, p);
+    if (gf_short(p.M, p.K)) {
+        const cudaError_t e = p.K > GF_SHORT ? gf_launch_short<64, true>(p, stream)
+                            : p.M <= 16 ? gf_launch_short<16, false>(p, stream) : gf_launch_short<64, false>(p, stream);
         return e == cudaSuccess ? BG_OK : (int)e;
     }
     if (gf_few(p.M, p.ranges, vec)) {
@@ -424,8 +441,13 @@ static int gf_run(GfParams p, cudaStream_t stream) {
     if ((rows + bm - 1) / bm > 65535 || (long long)p.batch * (cut > 0 ? p.ranges : 1) > 65535) return BG_ERR_SHAPE;
     for (int m0 = 0; m0 < M; m0 += rows) {
         p.M = M - m0 < rows ? M - m0 : rows;
-        cudaError_t e = bm == 64 ? (vec ? gf_launch_tile<64, true>(p, stream) : gf_launch_tile<64, false>(p, stream))
-                                 : (vec ? gf_launch_tile<128, true>(p, stream) : gf_launch_tile<128, false>(p, stream));
+        cudaError_t e;
+        if (p.N <= 64)                     // (as many columns as there are: 32 products of 2,048 x 64, k of 192, 61 us, 105 half empty; 300 x 64, k of 4,096, 39 and 67)
+            e = bm == 64 ? (vec ? gf_launch_tile<64, 64, true>(p, stream) : gf_launch_tile<64, 64, false>(p, stream))
+                         : (vec ? gf_launch_tile<128, 64, true>(p, stream) : gf_launch_tile<128, 64, false>(p, stream));
+        else
+            e = bm == 64 ? (vec ? gf_launch_tile<64, GF_BN, true>(p, stream) : gf_launch_tile<64, GF_BN, false>(p, stream))
+                         : (vec ? gf_launch_tile<128, GF_BN, true>(p, stream) : gf_launch_tile<128, GF_BN, false>(p, stream));
         if (e == cudaSuccess && cut > 0) e = gf_add_ranges(p, stream);
         if (e != cudaSuccess) return (int)e;
         p.A += (size_t)rows * p.lda;

@@ -191,9 +191,10 @@ def test_gemm_f32_kernels_agree_bit_for_bit(ops, N, K):
             assert torch.equal(out[e], f * plain)
 
 
-@pytest.mark.parametrize("K", [1, 31, 32, 33, 63, 64, 65])                # on both sides of what is summed in one chain
+@pytest.mark.parametrize("K", [1, 31, 32, 33, 63, 64, 65, 72, 127, 128, 129])       # on both sides of what is summed in one chain, and comes whole
 def test_gemm_f32_short_inner_sizes(ops, K):
-    test_gemm_f32_kernels_agree_bit_for_bit(ops, 130, K)
+    for N in (130, 64, 40):
+        test_gemm_f32_kernels_agree_bit_for_bit(ops, N, K)
     a, w = rnd(70, K, seed=1), rnd(67, K, seed=2)
     if K <= 64:                                                           # the chain itself: products are exact in 64 bits
         chain = torch.zeros((70, 67), dtype=torch.float64, device=DEV)
