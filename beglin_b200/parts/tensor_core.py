@@ -104,11 +104,12 @@ class TensorCoreProduct:
         add inside a cluster; 1: the plain kernel, one CTA a tile.  As `fused_splits`, but no more CTAs than run side by side: some
         256 with up to 32 rows (two share an SM), one an SM with 64.  4,096 x 4,096: 20.8 us on 32 CTAs -> 8.7 in eight ranges (32
         rows), 21.9 -> 11.1 in four (64 rows; in eight 20.9); 9,216 x 1,536: 10.4 -> 9.8 in two (32 rows; in four 13.3), 11.4 and
-        11.5 (64 rows)."""
+        11.5 (64 rows).  From 16 blocks of 64 of the inner size on: below, a CTA's stream is too short for the exchange (6,152 x 520: 4.7 us and
+        5.0 in two for 8 rows, 6.5 and 8.3 for 64; 576 x 1,024: 6.1 and 3.5, 7.6 and 5.1)."""
         s = self._splits.get(("complete", T))
         if s is None:
             s = 1
-            if self.ctx.fuse and 0 < T <= FEW_TOKENS and self.k % 8 == 0:
+            if self.ctx.fuse and 0 < T <= FEW_TOKENS and self.k % 8 == 0 and self.k_blocks >= 16:
                 s, most = self.fused_splits(T), 256 if T <= 32 else self.sms
                 while s > 1 and (self.tiles * s > most or (s - 1) * -(-self.k_blocks // s) >= self.k_blocks):
                     s //= 2

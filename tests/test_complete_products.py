@@ -39,3 +39,11 @@ def test_complete_product_of_no_rows():
     lin = Linear(torch.randn(264, 72), None, ctx)
     out = lin(torch.empty(0, 72, dtype=torch.bfloat16, device=DEV))
     assert out.shape == (0, 264) and out.dtype == torch.bfloat16
+
+
+def test_short_inner_sizes_are_not_cut():
+    from beglin_b200.parts import BuildContext
+    from beglin_b200.parts.tensor_core import TensorCoreProduct
+    for k, cut in ((72, False), (520, False), (960, False), (1024, True), (4096, True)):
+        p = TensorCoreProduct(torch.empty((576, k), dtype=torch.bfloat16, device=DEV), BuildContext(device=DEV, compute_dtype=torch.bfloat16))
+        assert all((p.complete_splits(T) > 1) == cut for T in (1, 16, 33, 64)), k
