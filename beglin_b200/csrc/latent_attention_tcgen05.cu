@@ -316,13 +316,13 @@ __global__ void __launch_bounds__(LT_THREADS, 1) latent_attention_tc_kernel(cons
                     l[h] = fmaf(l[h], f.x, u.x); l[h + 1] = fmaf(l[h + 1], f.y, u.y);
                     l[h + 2] = fmaf(l[h + 2], f.z, v.x); l[h + 3] = fmaf(l[h + 3], f.w, v.y);
                 }
-                if (ti == n_tiles - 1 && key >= k_end) { // rows that this request has not written (the scores have read them)
+                if (ti == n_tiles - 1) {                 // rows that this request has not written (the scores have read them), side by side
+                    const unsigned from = (unsigned)(k_end - k_begin - ti * LT_KEYS) * 128;
                     for (int i = 0; i < pairs; ++i) {
-                        unsigned char* row = ring + (size_t)((ti * pairs + i) % p.slots) * LT_SLOT + kk * 128;
-#pragma unroll
-                        for (int c = 0; c < 8; ++c) {
-                            *reinterpret_cast<uint4*>(row + c * 16) = make_uint4(0u, 0u, 0u, 0u);
-                            *reinterpret_cast<uint4*>(row + LT_BLOCK + c * 16) = make_uint4(0u, 0u, 0u, 0u);
+                        unsigned char* slot = ring + (size_t)((ti * pairs + i) % p.slots) * LT_SLOT;
+                        for (unsigned o = from + kk * 16; o < LT_BLOCK; o += 128 * 16) {
+                            *reinterpret_cast<uint4*>(slot + o) = make_uint4(0u, 0u, 0u, 0u);
+                            *reinterpret_cast<uint4*>(slot + LT_BLOCK + o) = make_uint4(0u, 0u, 0u, 0u);
                         }
                     }
                 }

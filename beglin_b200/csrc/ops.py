@@ -1242,6 +1242,8 @@ def latent_append(src: torch.Tensor, col0: int, rank: int, rot: int, rot_dims: i
 
 
 LATENT_TC_KEYS = 128          # keys of a tile of the tcgen05 kernel
+LATENT_TC_FROM = 64           # the longest row's position from which it runs: shorter ones are half a tile and less (64 rows of 32 heads,
+                              # kernel and merge: 64 keys 18.9 us with mma.sync and 22.1 here, 128 keys 25.4 and 19.5)
 
 
 @functools.lru_cache(maxsize=1024)
@@ -1284,7 +1286,7 @@ def latent_attention(q_lat: torch.Tensor, q_raw: torch.Tensor, dim: int, rot: in
     # one row per block (decoding) on tcgen05 where it takes the sizes: a row's own keys spread over the SMs
     tc = bool(mma_stages) and bq == 1 and q_raw.dtype == pool.dtype == torch.bfloat16 \
         and q_lat.stride(0) % 4 == 0 and q_lat.stride(1) % 4 == 0 and q_lat.data_ptr() % 16 == 0 and pool.data_ptr() % 16 == 0 \
-        and (cos_sin is None or cos_sin.data_ptr() % 8 == 0) and pool.shape[0] * pool.shape[1] <= 0x7fffffff \
+        and max_position >= LATENT_TC_FROM and (cos_sin is None or cos_sin.data_ptr() % 8 == 0) and pool.shape[0] * pool.shape[1] <= 0x7fffffff \
         and L.bg_latent_attention_tc_plan(H, rank, rot, pool.shape[1]) == 0
     if tc:
         keys = min(max_position + 1, window + LATENT_TC_KEYS) if window > 0 else max_position + 1
