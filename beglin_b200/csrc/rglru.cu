@@ -49,7 +49,8 @@ __device__ __forceinline__ float gelu_tanh32(float z) {
 // (a, b) of S <- a S + b from the gates' arguments and the convolved input
 __device__ __forceinline__ void lru_values(float gr, float gi, float u, float spc, float* a, float* b) {
     const float log_a = -sigmoid32(gr) * spc, e = expm1f(log_a);
-    *a = e > -0.5f ? 1.0f + e : expf(log_a);
+    const float strong = expf(log_a);          // (always: under a branch it costs more than it takes)
+    *a = e > -0.5f ? 1.0f + e : strong;
     *b = sqrtf(fmaf(-e, e, -2.0f * e)) * (sigmoid32(gi) * u);
 }
 
