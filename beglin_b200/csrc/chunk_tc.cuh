@@ -269,12 +269,14 @@ __global__ void __launch_bounds__(CT_THREADS, 2) chunk_out_tc_kernel(R r) {
         split = split && ct_splits(y.x) && ct_splits(y.y) && ct_splits(y.z) && ct_splits(y.w);
         return y;
     });
-    if (!split) {                            // (out of the way of the usual tile: once more, with noughts)
+    if (!split) {                            // (out of the way of the usual tile, and in few instructions: once more, with noughts)
         s.odd = 1;
-        ct_put<SV>(xt, part, raw, r.nv, [&](const float4& x, int j, int v) {
-            const float4 y = c.out_value(x, j, v);
-            return make_float4(ct_splits(y.x) ? y.x : 0.0f, ct_splits(y.y) ? y.y : 0.0f, ct_splits(y.z) ? y.z : 0.0f, ct_splits(y.w) ? y.w : 0.0f);
-        });
+        const int v = (threadIdx.x & ((1 << SV) - 1)) * 4;
+#pragma unroll 1
+        for (int j = threadIdx.x >> SV; j < CT; j += CT_THREADS >> SV) {
+            const float4 y = c.out_value(c.value_raw(j, v), j, v);
+            ct_put4(xt, part, j, v, make_float4(ct_splits(y.x) ? y.x : 0.0f, ct_splits(y.y) ? y.y : 0.0f, ct_splits(y.z) ? y.z : 0.0f, ct_splits(y.w) ? y.w : 0.0f));
+        }
     }
     ct_issue(s, [&] { ct_mma<true, false>(d, d + 64, x_a, part, q_a, part, CT / 16, CT / 32, ct_idesc(CT, true, false), true); });
     ct_wait(s, phase);

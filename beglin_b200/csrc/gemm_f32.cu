@@ -442,7 +442,8 @@ static int gf_run(GfParams p, cudaStream_t stream) {
     for (int m0 = 0; m0 < M; m0 += rows) {
         p.M = M - m0 < rows ? M - m0 : rows;
         cudaError_t e;
-        if (p.N <= 64)                     // (as many columns as there are: 32 products of 2,048 x 64, k of 192, 61 us, 105 half empty; 300 x 64, k of 4,096, 39 and 67)
+        // (as many columns as there are: 32 products of 2,048 x 64, k of 192, 61 us, half empty 105; 300 x 64, k of 4,096, 39 and 67)
+        if (p.N <= 64)
             e = bm == 64 ? (vec ? gf_launch_tile<64, 64, true>(p, stream) : gf_launch_tile<64, 64, false>(p, stream))
                          : (vec ? gf_launch_tile<128, 64, true>(p, stream) : gf_launch_tile<128, 64, false>(p, stream));
         else
