@@ -1,0 +1,21 @@
+// What the two files of the float product share: its parameters, the length of a range of k, and the tensor-core part's host interface.
+#pragma once
+
+#include "common.cuh"
+
+namespace bg {
+
+constexpr int GF_RANGE = 512;              // k of a range: the ranges lie at the same places whatever the call
+
+struct GfParams {
+    const float* A; const float* W; const float* bias; float* C;
+    float* scratch;                        // as many floats as gt_scratch asks for (with `accumulate` and several ranges M N more)
+    long long batch_a, batch_w, batch_c;   // a batch of independent products
+    int lda, ldw, ldc, M, N, K, accumulate, batch;
+    unsigned* status;
+};
+
+long long gt_scratch(int M, int N, int K, int batch);
+int gt_run(const GfParams& p, cudaStream_t stream);
+
+}  // namespace bg

@@ -115,7 +115,7 @@ _SIGNATURES = {
                              _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_float, _c_int, _c_void_p, _c_void_p],
     "bg_gemm_f32_scratch": [_c_int, _c_int, _c_int, _c_int],
     "bg_gemm_f32_nt": [_c_void_p, _c_int, _c_void_p, _c_int, _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int,
-                       _c_int, _c_void_p, _c_void_p],
+                       _c_int, _c_void_p, _c_void_p, _c_void_p],
     "bg_gemm_bf16_tn": [_c_void_p, _c_int, _c_int, _c_int, _c_void_p, _c_int, _c_int, _c_void_p, _c_void_p, _c_int,
                         _c_int, _c_int, _c_void_p, _c_void_p],
     "bg_gemm_pair": [_c_void_p, _c_int, _c_int, _c_int, _c_void_p, _c_int, _c_int, _c_void_p, _c_void_p, _c_int, _c_int,
@@ -171,7 +171,7 @@ _SIGNATURES = {
     "bg_gated_group_rmsnorm": [_c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_void_p, _c_int, _c_float, _c_void_p, _c_int,
                                _c_int, _c_int, _c_int, _c_int, _c_void_p],
     "bg_gemm_f32_nt_batched": [_c_void_p, _c_int, _c_ll, _c_void_p, _c_int, _c_ll, _c_void_p, _c_int, _c_ll, _c_int, _c_int,
-                               _c_int, _c_int, _c_void_p, _c_void_p],
+                               _c_int, _c_int, _c_void_p, _c_void_p, _c_void_p],
     "bg_sample": [_c_void_p, _c_int, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p],
     "bg_sample_feed": [_c_void_p, _c_int, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p,
                        _c_void_p],
@@ -822,8 +822,9 @@ def _difference_attention(q: torch.Tensor, kv_pool: torch.Tensor, block_table: t
 
 
 def gemm_f32_nt(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], out: torch.Tensor,
-                accumulate: bool = False) -> None:
-    """out[M, N] (+)= a[M, K] @ w[N, K]^T (+ bias), all float32, CUDA cores only."""
+                accumulate: bool = False, status: Optional[torch.Tensor] = None) -> None:
+    """out[M, N] (+)= a[M, K] @ w[N, K]^T (+ bias), all float32: no operand and no sum in fewer bits.  `status` learns of a wait
+    inside the kernel that ran out (the outputs are then no numbers)."""
     _cuda(a, w, bias, out)
     for t in (a, w, out) + ((bias,) if bias is not None else ()):
         if t.dtype != torch.float32:
@@ -834,14 +835,14 @@ def gemm_f32_nt(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], 
         raise KernelError(f"gemm_f32_nt: shapes a{tuple(a.shape)} w{tuple(w.shape)} out{tuple(out.shape)} do not fit")
     if bias is not None and (bias.numel() != N or not bias.is_contiguous()):
         raise KernelError("gemm_f32_nt: bias must have one value per output feature")
-    scratch = _gemm_f32_scratch(M, N, K, 1, out.device)
+    scratch = _gemm_f32_scratch(M, N, K, 1, out.device, M * N if accumulate else 0)
     _check(lib().bg_gemm_f32_nt(_p(a), a.stride(0), _p(w), w.stride(0), _p(bias), _p(out), out.stride(0), M, N, K,
-                                1 if accumulate else 0, _p(scratch), _stream()), "gemm_f32_nt")
+                                1 if accumulate else 0, _p(scratch), _p(status), _stream()), "gemm_f32_nt")
 
 
-def _gemm_f32_scratch(M: int, N: int, K: int, batch: int, device) -> Optional[torch.Tensor]:
-    """Room for the sums of the ranges of K, where the float32 product cuts it."""
-    n = lib().bg_gemm_f32_scratch(M, N, K, batch)
+def _gemm_f32_scratch(M: int, N: int, K: int, batch: int, device, more: int = 0) -> Optional[torch.Tensor]:
+    """Room for the parts of the operands and the sums of the ranges of K of the float32 product, and for `more` floats."""
+    n = lib().bg_gemm_f32_scratch(M, N, K, batch) + more
     return torch.empty((n,), dtype=torch.float32, device=device) if n > 0 else None
 
 
@@ -1169,9 +1170,9 @@ def gate_heads(src: torch.Tensor, gate: Optional[torch.Tensor], gate_col0: int, 
                "gate_heads")
 
 
-def gemm_f32_nt_batched(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None:
+def gemm_f32_nt_batched(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, status: Optional[torch.Tensor] = None) -> None:
     """out[b] = a[b] @ w[b]^T for a [B, M, K], w [B, N, K], out [B, M, N], float32 views of any batch and row
-    strides with unit inner stride.  CUDA cores only."""
+    strides with unit inner stride.  `status` as for gemm_f32_nt."""
     _cuda(a, w, out)
     for t in (a, w, out):
         if t.dtype != torch.float32 or t.dim() != 3 or (t.stride(2) != 1 and t.shape[2] != 1):
@@ -1182,7 +1183,8 @@ def gemm_f32_nt_batched(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> 
         raise KernelError(f"gemm_f32_nt_batched: shapes a{tuple(a.shape)} w{tuple(w.shape)} out{tuple(out.shape)} do not fit")
     scratch = _gemm_f32_scratch(M, N, K, B, out.device)
     _check(lib().bg_gemm_f32_nt_batched(_p(a), a.stride(1), a.stride(0), _p(w), w.stride(1), w.stride(0), _p(out),
-                                        out.stride(1), out.stride(0), B, M, N, K, _p(scratch), _stream()), "gemm_f32_nt_batched")
+                                        out.stride(1), out.stride(0), B, M, N, K, _p(scratch), _p(status), _stream()),
+           "gemm_f32_nt_batched")
 
 
 # ------------------------------------------------------------------------------------------------
