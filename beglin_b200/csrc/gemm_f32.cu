@@ -112,7 +112,7 @@ static int gf_run(const GfParams& p, cudaStream_t stream) {
 
 }  // namespace bg
 
-// Floats of scratch that a product of these sizes wants (0: none); one that accumulates over more than GF_RANGE of k wants M N more.
+// Floats of scratch that a product of these sizes wants (0: none); one that accumulates wants M N more.
 extern "C" long long bg_gemm_f32_scratch(int M, int N, int K, int batch) {
     if (M <= 0 || N <= 0 || K <= 0 || batch <= 0) return 0;
     return K > 2 * bg::GF_SHORT ? bg::gt_scratch(M, N, K, batch) : 0;

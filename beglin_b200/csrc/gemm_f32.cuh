@@ -5,11 +5,9 @@
 
 namespace bg {
 
-constexpr int GF_RANGE = 512;              // k of a range: the ranges lie at the same places whatever the call
-
 struct GfParams {
     const float* A; const float* W; const float* bias; float* C;
-    float* scratch;                        // as many floats as gt_scratch asks for (with `accumulate` and several ranges M N more)
+    float* scratch;                        // as many floats as gt_scratch asks for (with `accumulate` M N more)
     long long batch_a, batch_w, batch_c;   // a batch of independent products
     int lda, ldw, ldc, M, N, K, accumulate, batch;
     unsigned* status;
