@@ -25,6 +25,7 @@
 // t >= first_visible(pos, window) or t < k, the tiles and splits between the two ranges being passed over.
 #include "common.cuh"
 #include "attention_f32.cuh"
+#include "attention_f32_tc.cuh"
 
 namespace bg {
 
@@ -329,6 +330,7 @@ static bool attention_f32_takes(int rows, int hd, int vd, int maps) {
 // (`hd` counts a whole key row; with two maps in it, it may be twice as wide; `f32`: queries and cache are float)
 extern "C" int bg_attention_plan(int group, int hd, int vd, int maps, int f32, int* bq_out, int* tile_out) {
     if (maps < 1 || hd <= 0 || hd > 32 * ATT_MAX_DPL * maps || vd <= 0 || vd > 32 * ATT_MAX_DPL || group <= 0) return BG_ERR_UNSUPPORTED;
+    if (f32 && ax_takes(group, hd, vd, maps)) { *bq_out = AX_ROWS / group; *tile_out = AX_KEYS; return BG_OK; }
     if (f32 && attention_f32_takes(group, hd, vd, maps)) { *bq_out = AF_ROWS / group; *tile_out = AF_KEYS; return BG_OK; }
     const size_t limit = 200 * 1024;
     for (int tile = 64; tile >= 32; tile >>= 1) {
@@ -356,8 +358,23 @@ extern "C" int bg_attention_partial(const void* q, int q_dtype, int q_stride, co
     p.group = nh / nkv; p.window = window; p.split = split; p.tile = tile; p.bq = bq; p.scale = scale; p.softcap = softcap; p.status = status;
     p.keep = keep; p.slopes = slopes; p.maps = maps;
     dim3 grid(n_qblk, nkv, n_splits_launch);
+    const bool pieces = q_stride % 4 == 0 && (uintptr_t)q % 16 == 0 && (uintptr_t)kv_pool % 16 == 0 && (uintptr_t)part_o % 16 == 0;
+    if (q_dtype == BG_DTYPE_F32 && cache_dtype == BG_DTYPE_F32 && ax_takes(bq * p.group, hd, vd, maps) && split % AX_KEYS == 0 && pieces) {
+        constexpr int need = 2 * AX_TILE + 1024;
+        auto kern = attention_f32_tc_kernel<AttnParams>;
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, need);
+        if (e != cudaSuccess) return (int)e;
+        static const bool fits = [] {                      // (the split of the registers counts on as many at launch)
+            cudaFuncAttributes a;
+            return cudaFuncGetAttributes(&a, attention_f32_tc_kernel<AttnParams>) == cudaSuccess && a.numRegs >= AX_REGS;
+        }();
+        if (!fits) return (int)cudaErrorInvalidConfiguration;
+        launch(kern, grid, dim3(AX_THREADS), need, stream, p);
+        BG_LAUNCH_CHECK();
+        return BG_OK;
+    }
     if (q_dtype == BG_DTYPE_F32 && cache_dtype == BG_DTYPE_F32 && bq * p.group <= AF_ROWS && attention_f32_takes(p.group, hd, vd, maps) &&
-        split % AF_KEYS == 0 && q_stride % 4 == 0 && (uintptr_t)q % 16 == 0 && (uintptr_t)kv_pool % 16 == 0 && (uintptr_t)part_o % 16 == 0) {
+        split % AF_KEYS == 0 && pieces) {
         const size_t need = af_smem(hd / maps, hd, vd);
 #define BG_AF_LAUNCH(NC)                                                                                                    \
         do {                                                                                                                \

@@ -1,0 +1,400 @@
+// The partial results of float queries over a float cache on the tensor cores: heads of 48 to 128 features, a multiple of 16
+// (attention_f32.cuh runs the other sizes, attention_partial_kernel in attention.cu the other types).
+//
+// No precision is given up: queries, keys, values and weights are cut into three bfloat16 numbers each, exactly, and a product of two floats is
+// the six products of parts that are not below 2^-24 of it, the small ones added up before the large ones (gemm_f32_tc.cu says more).
+// A CTA takes up to 128 rows (queries x query heads of a kv head), a lane of tensor memory each, and one split of keys, 64 at a time:
+// eight warps cut the keys and values of a tile into swizzled shared memory, one issues the MMAs, and eight warps, two threads a row with
+// 32 keys each, make the weights and keep the row's sums of values in registers (a tile's sums leave tensor memory and are added in float).
+// Queries and weights are left operands in tensor memory.  The scores of a tile are multiplied while the weights of the one before are made,
+// its values while those of the one behind are.
+//
+// A row's arithmetic depends on nothing but its own keys: tiles and splits lie at absolute positions, and an MMA's rows do not meet.  What has no
+// three parts (infinite, not a number, below some 2^-110) is noticed where it is cut: scores of such queries or keys, and those that are
+// not finite, are summed by floats instead; such values go into the tile as nought and are added by floats to the rows whose weight for them
+// is not nought, so that an infinite one at a position that a row does not see does not reach it.
+#pragma once
+
+#include "float_parts.cuh"
+
+namespace bg {
+
+constexpr int AX_ROWS = 128, AX_KEYS = 64;
+constexpr int AX_THREADS = 640;                        // two warpgroups of rows, two that cut, one with the warp that issues
+constexpr unsigned AX_BLOCK = AX_KEYS * 128, AX_PART = 2 * AX_BLOCK, AX_TILE = 3 * AX_PART;       // 64 keys x 64 features; x 128; three parts
+constexpr unsigned AX_Q = 0, AX_S = 192, AX_P = 256, AX_O = 352;                      // columns of tensor memory
+constexpr int AX_REGS = 96, AX_REGS_ROW = 152, AX_REGS_CUT = 64, AX_REGS_OTHER = 48;
+static_assert(2 * AX_REGS_ROW + 2 * AX_REGS_CUT + AX_REGS_OTHER <= 5 * AX_REGS);
+
+__host__ __device__ __forceinline__ bool ax_takes(int rows, int hd, int vd, int maps) {
+    return maps == 1 && rows <= AX_ROWS && hd >= 48 && hd <= 128 && hd % 16 == 0 && vd >= 16 && vd <= 128 && vd % 16 == 0;
+}
+__device__ __forceinline__ bool ax_odd(float x) {      // no three parts
+    unsigned h, m, l, left = 0;
+    gt_split(pair2(x, 0.0f), h, m, l, left);
+    return (left & 0xffffu) != 0;
+}
+// all 256 threads of the rows meet
+__device__ __forceinline__ void ax_rows_meet() { asm volatile("barrier.cta.sync 1, 256;\n" ::: "memory"); }
+
+template <typename P>
+__global__ void __launch_bounds__(AX_THREADS, 1) attention_f32_tc_kernel(P p) {
+    extern __shared__ unsigned char ax_raw[];
+    unsigned char* kt = (unsigned char*)(((uintptr_t)ax_raw + 1023) & ~(uintptr_t)1023);
+    unsigned char* vt = kt + AX_TILE;
+    __shared__ __align__(8) unsigned long long q_full, k_full, k_empty, v_full, v_empty, s_full, s_empty, p_full, o_full, o_empty;
+    __shared__ unsigned tmem_sh;
+    __shared__ int failed;
+    __shared__ int page_s[4][AX_KEYS];                 // pages of a tile's keys, -1: none (they are asked for again when its values have been summed)
+    __shared__ unsigned char key_odd[2][AX_KEYS], value_odd[2][AX_KEYS], row_odd[2][AX_ROWS];
+    __shared__ float row_max[2][AX_ROWS];
+
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int qb = blockIdx.x, kvh = blockIdx.y, sp = blockIdx.z;
+    if (tid == 0) {
+        mbar_init(&q_full, 8); mbar_init(&k_full, 8); mbar_init(&k_empty, 1); mbar_init(&v_full, 8); mbar_init(&v_empty, 1);
+        mbar_init(&s_full, 1); mbar_init(&s_empty, 8); mbar_init(&p_full, 8); mbar_init(&o_full, 1); mbar_init(&o_empty, 8);
+        failed = 0;
+        mbar_init_fence();
+    }
+    if (warp == 16) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(&tmem_sh)), "r"(512u) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    pdl_launch();                                      // (the columns are held)
+    const unsigned tmem = tmem_sh;
+    pdl_wait();
+    const int req = p.qblk[qb * 3 + 0], row0 = p.qblk[qb * 3 + 1], nq = p.qblk[qb * 3 + 2];
+    const int lo_first = nq > 0 ? first_visible(p.positions[row0], p.window) : 0;
+    const int k_first = sp * p.split, k_end = nq > 0 ? min((sp + 1) * p.split, p.positions[row0 + nq - 1] + 1) : 0;       // exclusive
+    const bool seen = nq > 0 && k_first < k_end && !(lo_first >= k_end && k_first >= p.keep);       // (else no key of the split is seen)
+    const int hd = p.hd, vd = p.vd, group = p.group, n_rows = nq * group;
+    const float* pool = (const float*)p.kv_pool;
+    const size_t page_elems = (size_t)p.nkv * p.page_size * (hd + vd), v_off = (size_t)p.nkv * p.page_size * hd;
+    auto skipped = [&](int t0) { return t0 + AX_KEYS <= lo_first && t0 >= p.keep; };
+    auto next_tile = [&](int t0) { do t0 += AX_KEYS; while (t0 < k_end && skipped(t0)); return t0; };
+    const int t_first = skipped(k_first) ? next_tile(k_first) : k_first;
+
+    if (warp >= 16) gt_regs<AX_REGS, AX_REGS_OTHER>();
+    if (warp == 16) {
+        // ---------------- the MMAs: a tile's scores before the values of the tile in front of it
+        if (seen && t_first < k_end) {
+            const unsigned s_desc = instr_desc_bf16(AX_ROWS, AX_KEYS), o_desc = instr_desc_bf16(AX_ROWS, vd, 1);
+            const unsigned ka = smem_u32(kt), va = smem_u32(vt);
+            bool ok = mbar_wait(&q_full, 0, &failed);
+            int i = 0;
+            auto scores = [&](int tile) {
+                ok = ok && mbar_wait(&k_full, tile & 1, &failed) && (tile == 0 || mbar_wait(&s_empty, (tile - 1) & 1, &failed));
+                if (!ok) return;
+                tc_fence_after();
+                if (elect_one()) {
+#pragma unroll
+                    for (int e = 0; e < 6; ++e) {
+                        constexpr int PA[6] = {2, 1, 0, 1, 0, 0}, PB[6] = {0, 1, 2, 0, 1, 0};
+                        for (int j = 0; j < hd / 16; ++j)
+                            tc_mma_ts(tmem + AX_S, tmem + AX_Q + PA[e] * 64 + j * 8, smem_desc_sw128(ka + PB[e] * AX_PART + (j >> 2) * AX_BLOCK + (j & 3) * 32), s_desc, e || j ? 1u : 0u);
+                    }
+                    tc_commit(&s_full);
+                    tc_commit(&k_empty);
+                }
+                __syncwarp();
+            };
+            scores(0);
+            for (int t0 = t_first; t0 < k_end && ok; ++i) {
+                const int t1 = next_tile(t0);
+                if (t1 < k_end) scores(i + 1);
+                ok = ok && mbar_wait(&v_full, i & 1, &failed) && mbar_wait(&p_full, i & 1, &failed) && (i == 0 || mbar_wait(&o_empty, (i - 1) & 1, &failed));
+                if (!ok) break;
+                tc_fence_after();
+                if (elect_one()) {
+#pragma unroll
+                    for (int e = 0; e < 6; ++e) {
+                        constexpr int PA[6] = {2, 1, 0, 1, 0, 0}, PB[6] = {0, 1, 2, 0, 1, 0};
+#pragma unroll
+                        for (int j = 0; j < AX_KEYS / 16; ++j)
+                            tc_mma_ts(tmem + AX_O, tmem + AX_P + PA[e] * 32 + j * 8, smem_desc_sw128_nmajor(va + PB[e] * AX_PART + j * 2048, AX_BLOCK, 1024), o_desc, e || j ? 1u : 0u);
+                    }
+                    tc_commit(&o_full);
+                    tc_commit(&v_empty);
+                }
+                __syncwarp();
+                t0 = t1;
+            }
+        }
+    } else if (warp >= 8 && warp < 16) {
+        // ---------------- keys and values into parts: four threads a key, pieces of eight features
+        gt_regs<AX_REGS, AX_REGS_CUT>();
+        const int c0 = tid & 3, key = (tid - 256) >> 2;
+        if (seen) {
+            int i = 0;
+            for (int t0 = t_first; t0 < k_end; ++i) {
+                const int at = t0 + key;
+                int page = -1;
+                if (at < k_end && key_seen(at, lo_first, p.keep)) {
+                    page = p.block_table[(size_t)req * p.max_pages + at / p.page_size];
+                    if (page < 0 || page >= p.num_pages) {
+                        if (p.status && c0 == 0) atomicOr(p.status, BG_STATUS_BAD_PAGE);
+                        page = -1;
+                    }
+                }
+                const size_t slot = (size_t)kvh * p.page_size + at % p.page_size;
+                const float* ks = pool + (page >= 0 ? (size_t)page * page_elems + slot * hd : 0);
+                const float* vs = pool + (page >= 0 ? (size_t)page * page_elems + v_off + slot * vd : 0);
+                auto fetch = [&](const float* src, int width, float4 (&v)[8]) {
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const int c = c0 + 4 * j;
+                        v[2 * j] = v[2 * j + 1] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                        if (page >= 0 && c * 8 < width) {
+                            v[2 * j] = *reinterpret_cast<const float4*>(src + c * 8);
+                            v[2 * j + 1] = *reinterpret_cast<const float4*>(src + c * 8 + 4);
+                        }
+                    }
+                };
+                auto store = [&](unsigned char* tile, int c, const uint4& h, const uint4& m, const uint4& l) {
+                    unsigned char* d = tile + (c >> 3) * AX_BLOCK + key * 128 + (((c ^ key) & 7) << 4);
+                    *reinterpret_cast<uint4*>(d) = h;
+                    *reinterpret_cast<uint4*>(d + AX_PART) = m;
+                    *reinterpret_cast<uint4*>(d + 2 * AX_PART) = l;
+                };
+                auto split8 = [&](const float4& a, const float4& b, uint4& h, uint4& m, uint4& l, unsigned& left) {
+                    gt_split(pair2(a.x, a.y), h.x, m.x, l.x, left);
+                    gt_split(pair2(a.z, a.w), h.y, m.y, l.y, left);
+                    gt_split(pair2(b.x, b.y), h.z, m.z, l.z, left);
+                    gt_split(pair2(b.z, b.w), h.w, m.w, l.w, left);
+                };
+                float4 v[8];
+                fetch(ks, hd, v);
+                if (i > 0) mbar_wait(&k_empty, (i - 1) & 1, &failed);
+                unsigned left = 0;
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    uint4 h, m, l;
+                    split8(v[2 * j], v[2 * j + 1], h, m, l, left);
+                    if ((c0 + 4 * j) * 8 < hd) store(kt, c0 + 4 * j, h, m, l);
+                }
+                left &= 0xffffu;
+                left |= __shfl_xor_sync(0xffffffffu, left, 1);
+                left |= __shfl_xor_sync(0xffffffffu, left, 2);
+                if (c0 == 0) { page_s[i & 3][key] = page; key_odd[i & 1][key] = left != 0; }
+                fence_proxy_async();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&k_full);
+                fetch(vs, vd, v);
+                if (i > 0) mbar_wait(&v_empty, (i - 1) & 1, &failed);
+                left = 0;
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    uint4 h, m, l;
+                    unsigned mine = 0;
+                    split8(v[2 * j], v[2 * j + 1], h, m, l, mine);
+                    if (mine & 0xffffu) {              // what has no three parts is nought here
+                        float* x = reinterpret_cast<float*>(&v[2 * j]);
+#pragma unroll
+                        for (int e = 0; e < 8; ++e)
+                            if (ax_odd(x[e])) x[e] = 0.0f;
+                        unsigned none = 0;
+                        split8(v[2 * j], v[2 * j + 1], h, m, l, none);
+                    }
+                    left |= mine;
+                    if ((c0 + 4 * j) * 8 < vd) store(vt, c0 + 4 * j, h, m, l);
+                }
+                left &= 0xffffu;
+                left |= __shfl_xor_sync(0xffffffffu, left, 1);
+                left |= __shfl_xor_sync(0xffffffffu, left, 2);
+                if (c0 == 0) value_odd[i & 1][key] = left != 0;
+                fence_proxy_async();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&v_full);
+                t0 = next_tile(t0);
+            }
+        }
+    } else if (warp < 8) {
+        // ---------------- the rows: lane and quarter are the row, the half says which keys and which output features
+        gt_regs<AX_REGS, AX_REGS_ROW>();
+        const int quarter = warp & 3, half = warp >> 2, row = quarter * 32 + lane;
+        const unsigned lanes = tmem + ((unsigned)(quarter * 32) << 16);
+        const bool in = row < n_rows;
+        const int qi = in ? row / group : 0, head = kvh * group + (in ? row - qi * group : 0);
+        const int pos = in ? p.positions[row0 + qi] : -1, lo = first_visible(pos < 0 ? 0 : pos, p.window);
+        const float* q = (const float*)p.q + (size_t)(row0 + qi) * p.q_stride + (size_t)head * hd;
+        const float slope = p.slopes && in ? p.slopes[head] : 0.0f;
+        const int od = vd / 2;                         // output features of a thread, a multiple of 8
+        float out[64];
+        float m = -INFINITY, sum = 0.0f;
+#pragma unroll
+        for (int d = 0; d < 64; ++d) out[d] = 0.0f;
+        if (seen && t_first < k_end) {
+            // the row's queries, half of their features a thread
+            unsigned left = 0;
+            for (int d = half * (hd / 2); d < (half + 1) * (hd / 2); d += 8) {
+                unsigned h[4], mm[4], l[4];
+                float4 a = make_float4(0.0f, 0.0f, 0.0f, 0.0f), b = a;
+                if (in) { a = *reinterpret_cast<const float4*>(q + d); b = *reinterpret_cast<const float4*>(q + d + 4); }
+                gt_split(pair2(a.x, a.y), h[0], mm[0], l[0], left);
+                gt_split(pair2(a.z, a.w), h[1], mm[1], l[1], left);
+                gt_split(pair2(b.x, b.y), h[2], mm[2], l[2], left);
+                gt_split(pair2(b.z, b.w), h[3], mm[3], l[3], left);
+                gt_st4(lanes + AX_Q + d / 2, h); gt_st4(lanes + AX_Q + 64 + d / 2, mm); gt_st4(lanes + AX_Q + 128 + d / 2, l);
+            }
+            row_odd[half][row] = (left & 0xffffu) != 0;
+            tc_wait_st();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&q_full);
+            ax_rows_meet();
+            const bool q_odd = row_odd[0][row] || row_odd[1][row];
+            float corr_before = 0.0f;                  // of the tile whose values are still being summed
+            // adds the tile's sums of values to the row's
+            auto add_values = [&](int i, int t0, float corr) {
+                mbar_wait(&o_full, i & 1, &failed);
+                tc_fence_after();
+#pragma unroll
+                for (int c = 0; c < 64; c += 16) {
+                    if (c >= od) break;
+                    unsigned r[16];
+                    if (c + 16 <= od) gt_ld16(lanes + AX_O + half * od + c, r);
+                    else gt_ld8(lanes + AX_O + half * od + c, r);
+                    tc_wait_ld();
+#pragma unroll
+                    for (int e = 0; e < 16; ++e)
+                        if (c + e < od) out[c + e] = fmaf(out[c + e], corr, __uint_as_float(r[e]));
+                }
+                bool odd = false;
+#pragma unroll
+                for (int j = 0; j < 2; ++j) odd |= value_odd[i & 1][j * 32 + lane] != 0;
+                if (__any_sync(0xffffffffu, odd)) {    // values without three parts: the weights come back from their own
+                    for (int j = 0; j < AX_KEYS; ++j) {
+                        if (!value_odd[i & 1][j]) continue;
+                        unsigned w[3];
+#pragma unroll
+                        for (int e = 0; e < 3; ++e)
+                            asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];\n" : "=r"(w[e]) : "r"(lanes + AX_P + e * 32 + (j >> 1)));
+                        tc_wait_ld();
+                        float f = 0.0f;
+#pragma unroll
+                        for (int e = 2; e >= 0; --e) f += __uint_as_float(j & 1 ? w[e] & 0xffff0000u : w[e] << 16);
+                        const int page = page_s[i & 3][j];
+                        if (f == 0.0f || page < 0) continue;
+                        const float* src = pool + (size_t)page * page_elems + v_off + ((size_t)kvh * p.page_size + (t0 + j) % p.page_size) * vd + half * od;
+#pragma unroll
+                        for (int d = 0; d < 64; ++d)
+                            if (d < od && ax_odd(src[d])) out[d] = fmaf(f, src[d], out[d]);
+                    }
+                }
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&o_empty);
+            };
+            int i = 0, t_before = 0;
+            for (int t0 = t_first; t0 < k_end; ++i) {
+                mbar_wait(&s_full, i & 1, &failed);
+                tc_fence_after();
+                float w[32];
+                {
+                    unsigned r[32];
+                    tc_ld32_nowait(lanes + AX_S + half * 32, r);
+                    tc_wait_ld();
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) w[j] = __uint_as_float(r[j]);
+                }
+                // the keys that the row sees, a bit each, and the scores that the parts cannot make
+                const int base = t0 + half * 32, last = min(pos, k_end - 1) - base;
+                auto below = [](int n) { return n <= 0 ? 0u : n >= 32 ? 0xffffffffu : (1u << n) - 1; };       // bits 0 .. n - 1
+                unsigned visible = __ballot_sync(0xffffffffu, page_s[i & 3][half * 32 + lane] >= 0) & below(last + 1) & (~below(lo - base) | below(p.keep - base));
+                unsigned bad = __ballot_sync(0xffffffffu, key_odd[i & 1][half * 32 + lane] != 0);
+                if (q_odd) bad = 0xffffffffu;
+                float nought = 0.0f;
+#pragma unroll
+                for (int j = 0; j < 32; ++j) nought = fmaf(w[j], 0.0f, nought);
+                if (!(nought == 0.0f)) {
+#pragma unroll
+                    for (int j = 0; j < 32; ++j)
+                        if (!(fabsf(w[j]) <= 3.402823466e38f)) bad |= 1u << j;
+                }
+                bad &= visible;
+                while (bad) {
+                    const int jb = __ffs(bad) - 1, at = t0 + half * 32 + jb, page = page_s[i & 3][half * 32 + jb];
+                    bad &= bad - 1;
+                    const float* src = pool + (size_t)page * page_elems + ((size_t)kvh * p.page_size + at % p.page_size) * hd;
+                    float even = 0.0f, odd = 0.0f;
+                    for (int d = 0; d < hd; d += 2) { even = fmaf(q[d], src[d], even); odd = fmaf(q[d + 1], src[d + 1], odd); }
+                    even += odd;
+#pragma unroll
+                    for (int j = 0; j < 32; ++j)
+                        if (j == jb) w[j] = even;
+                }
+                __syncwarp();
+                float most = -INFINITY;
+#pragma unroll
+                for (int j = 0; j < 32; ++j) {
+                    w[j] *= p.scale;
+                    if (p.softcap > 0.0f) w[j] = p.softcap * tanhf(w[j] / p.softcap);
+                    if (p.slopes) w[j] = fmaf(-slope, (float)(pos - (t0 + half * 32 + j)), w[j]);
+                    if (!(visible >> j & 1)) w[j] = -INFINITY;
+                    most = fmaxf(most, w[j]);
+                }
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&s_empty);  // (the scores and the tile's pages have been read)
+                row_max[half][row] = most;
+                ax_rows_meet();
+                const float m_new = fmaxf(m, fmaxf(row_max[0][row], row_max[1][row]));
+                const float corr = m == -INFINITY ? 0.0f : expf(m - m_new);
+                float s = 0.0f;
+#pragma unroll
+                for (int j = 0; j < 32; ++j) {
+                    w[j] = w[j] == -INFINITY || m_new == -INFINITY ? 0.0f : expf(w[j] - m_new);
+                    s += w[j];
+                }
+                sum = fmaf(sum, corr, s);
+                m = m_new;
+                if (i > 0) add_values(i - 1, t_before, corr_before);
+                else ax_rows_meet();                   // (as often as below)
+                corr_before = corr;
+                // the weights' parts, where the values' products before have read theirs
+                unsigned none = 0;
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    unsigned h[4], mm[4], l[4];
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) gt_split(pair2(w[8 * c + 2 * e], w[8 * c + 2 * e + 1]), h[e], mm[e], l[e], none);
+                    const unsigned a = lanes + AX_P + half * 16 + 4 * c;
+                    gt_st4(a, h); gt_st4(a + 32, mm); gt_st4(a + 64, l);
+                }
+                tc_wait_st();
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&p_full);
+                if (i > 0) ax_rows_meet();             // (row_max is free again)
+                t_before = t0;
+                t0 = next_tile(t0);
+            }
+            add_values(i - 1, t_before, corr_before);
+            row_max[half][row] = sum;
+            ax_rows_meet();
+            // partial results of the rows that see at least one key of this split
+            if (in && !(pos < sp * p.split || (lo >= (sp + 1) * p.split && sp * p.split >= p.keep))) {
+                const bool lost = *(volatile int*)&failed != 0;                // (a wait ran out)
+                const size_t prow = ((size_t)(row0 + qi) * p.nh + head) * p.max_splits + sp;
+                float* o = p.part_o + prow * vd + half * od;
+#pragma unroll
+                for (int d = 0; d < 64; d += 4)
+                    if (d < od) *reinterpret_cast<float4*>(o + d) = lost ? make_float4(NAN, NAN, NAN, NAN) : make_float4(out[d], out[d + 1], out[d + 2], out[d + 3]);
+                if (half == 0) { p.part_ml[prow * 2 + 0] = m; p.part_ml[prow * 2 + 1] = row_max[0][row] + row_max[1][row]; }
+            }
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 16) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(512u) : "memory");
+    }
+    if (tid == 0 && failed && p.status) atomicOr(p.status, BG_STATUS_TIMEOUT);
+}
+
+}  // namespace bg

@@ -18,8 +18,7 @@
 // bandwidth the right operands need.  The tokens' parts are made once by gf_parts_kernel and come by bulk copies (the weights' tiles would each
 // make them again); up to 16 tokens a warp of the CTA's own makes them.  Other warpgroups add up the stages' sums.
 #include "gemm_f32.cuh"
-#include "float_pairs.cuh"
-#include "ptx.cuh"
+#include "float_parts.cuh"
 
 namespace bg {
 
@@ -40,31 +39,6 @@ struct GtParams {
     int lda, ldw, ldc, ldr, M, N, K, accumulate, range_len, ranges, r0, r1, batch, tok_tiles, feat_tiles, units, map_batch;      // (ranges: of all k; r0 to r1: of this launch)
     unsigned* status;
 };
-
-// Two floats into their three parts, two bfloat16 a word (the first one low).  `odd` collects what is left over in the low halves:
-// nought there if the third part is exact.  (An infinity leaves a NaN, whose low half is not nought.)
-__device__ __forceinline__ unsigned gt_pack(unsigned long long v) {
-    unsigned r;
-    asm("cvt.rn.bf16x2.f32 %0, %1, %2;\n" : "=r"(r) : "f"(high2(v)), "f"(low2(v)));
-    return r;
-}
-__device__ __forceinline__ unsigned long long gt_unpack(unsigned p) {
-    return (unsigned long long)(p << 16) | ((unsigned long long)(p & 0xffff0000u) << 32);
-}
-__device__ __forceinline__ void gt_split(unsigned long long v, unsigned& h, unsigned& m, unsigned& l, unsigned& odd) {
-    const unsigned long long minus = pair2(-1.0f, -1.0f);
-    h = gt_pack(v);
-    const unsigned long long r = fma2(gt_unpack(h), minus, v);
-    m = gt_pack(r);
-    const unsigned long long q = fma2(gt_unpack(m), minus, r);
-    l = __byte_perm((unsigned)q, (unsigned)(q >> 32), 0x7632);
-    odd |= (unsigned)q | (unsigned)(q >> 32);
-}
-__device__ __forceinline__ unsigned long long gt_add2(unsigned long long a, unsigned long long b) {
-    unsigned long long d;
-    asm("add.rn.f32x2 %0, %1, %2;\n" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
 
 // The tokens' parts as the images of the stages' right operands, [batch][tile of nt tokens][stage][part][token][64 of k] with the swizzle of
 // shared memory, noughts behind the last token and behind K; and whether a row has an operand without three parts.  One part of a stage is
@@ -106,19 +80,6 @@ __global__ void __launch_bounds__(256) gf_parts_kernel(GtParams p, unsigned char
     if (threadIdx.x == 0) odd[blockIdx.x] = any != 0;
 }
 
-// Loads and stores of tensor memory; the caller waits.
-__device__ __forceinline__ void gt_ld8(unsigned taddr, unsigned* r) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "r"(taddr));
-}
-__device__ __forceinline__ void gt_ld16(unsigned taddr, unsigned* r) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-                   "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]) : "r"(taddr));
-}
-__device__ __forceinline__ void gt_st4(unsigned taddr, const unsigned (&v)[4]) {
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1,%2,%3,%4};\n" ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]) : "memory");
-}
 // `bytes` contiguous ones (a multiple of 16, both sides on 16 bytes)
 __device__ __forceinline__ void bulk_load(void* dst, const void* src, unsigned bytes, unsigned long long* bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n"
@@ -128,12 +89,6 @@ __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, i
     asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];\n"
                  ::"r"(smem_u32(dst)), "l"(map), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar)) : "memory");
 }
-template <int HAS, int WANTS>
-__device__ __forceinline__ void gt_regs() {
-    if constexpr (WANTS > HAS) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;\n" ::"n"(WANTS));
-    if constexpr (WANTS < HAS) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;\n" ::"n"(WANTS));
-}
-
 // Whether any of the THREADS that add says so; they all meet.
 template <int THREADS>
 __device__ __forceinline__ bool gt_any(bool mine) {
