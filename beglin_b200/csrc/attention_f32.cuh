@@ -1,5 +1,6 @@
 // The partial results of float queries over a float cache in blocks of registers: the float path's attention for head sizes that
-// are multiples of 4 (attention_partial_kernel in attention.cu runs the other sizes and types, and says what a partial result is).
+// are multiples of 4 and that the tensor cores' kernel does not take (attention_f32_tc.cuh: 48 to 128 features in sixteens, one map;
+// attention_partial_kernel in attention.cu runs the other sizes and types, and says what a partial result is).
 //
 // A CTA takes up to 64 rows (queries x query heads of a kv head) and one split of keys, 64 keys at a time.  Thread (ty, tx) of
 // 16 x 16 owns rows ty + 16 i (i < RI, as many sixteens as the block has rows), of the scores keys tx + 16 j, of the output columns

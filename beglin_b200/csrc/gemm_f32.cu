@@ -1,24 +1,11 @@
-// C[M, N] (+)= A[M, K] * W[N, K]^T (+ bias[N]) in true float: CUDA-core FFMA, no tensor cores and no
-// reduced-precision mode (the tensor cores have no float x float kind; their tf32 kind drops
-// mantissa bits).  This is the reference's linear, y[o] = bias[o] + sum_i W[o,i] x[i] with W
-// row-major [out, in] (qwen_infer.c:688-691), for a batch of rows.
+// C[M, N] (+)= A[M, K] * W[N, K]^T (+ bias[N]) in true float: no operand and no sum in fewer bits.  This is the
+// reference's linear, y[o] = bias[o] + sum_i W[o,i] x[i] with W row-major [out, in] (qwen_infer.c:688-691), for a batch of rows.
 //
-// K is cut into ranges of GF_RANGE, at the same places whatever the call.  Every output is, per range, TWO chains of fused
-// multiply-adds, over the even and over the odd k in order, each starting from nought, and their sum; the ranges' sums are added in
-// order, then the bias.  Which kernel runs, how its tiles lie and whether the ranges go to CTAs of their own changes none of that, so
-// a row's result does not depend on how many other rows the call has or where the row stands among them: all the kernels here give
-// the same bits.  Two chains because an even k and the odd one behind it lie side by side in both operands, which is what the packed
-// multiply-add takes (fma.rn.f32x2: two independent float multiply-adds).  In a product's inner loop the register file, not the
-// float units, is what an 8 x 8 block of single multiply-adds waits for: 51 TFLOP/s on 148 SMs from registers alone, 68 with packed
-// ones whose rows are walked to and fro, so that each shares an operand with the one before.
-//
-// Inner sizes of up to GF_SHORT are summed in one chain, k = 0 .. K-1 in order, whatever the rows: two chains and a pipeline over k gain
-// nothing there.
-//
-//   gemm_f32_short_kernel  inner sizes of up to 64, and of up to 128 with more than 16 rows
-//   gemm_f32_tile_kernel   tiles of 128 (or 64) rows x 128 columns, for more than 16 rows
-//   gemm_f32_few_kernel    up to 16 rows: the product is a stream of weights
-//   gemm_f32_ranges_kernel adds the sums of ranges that went to CTAs of their own
+// Inner sizes above 2 GF_SHORT run on the tensor cores, every operand in three bfloat16 parts (gemm_f32_tc.cu).  Shorter ones come whole and
+// are summed on the float units here: up to GF_SHORT in one chain of fused multiply-adds, k = 0 .. K-1 in order, above it in two, over
+// the even and over the odd k, each starting from nought, and their sum (an even k and the odd one behind it lie side by side in both
+// operands, which is what the packed multiply-add takes: fma.rn.f32x2, two independent float multiply-adds).  Which way a product goes is
+// its K's alone, so a row's result does not depend on how many other rows the call has or where the row stands among them.
 #include "gemm_f32.cuh"
 #include "float_pairs.cuh"
 
@@ -29,8 +16,8 @@ constexpr int GF_SHORT = 64;               // inner sizes up to which a product 
 
 // Short inner sizes (narrow models, small heads): both operands come whole, BM rows and 64 columns, and a thread sums rows ty + 16 i
 // and columns tx + 16 j, four k of a row at a read (rows 68 or 132 floats apart: eight neighbouring ones in different banks).  Above GF_SHORT
-// in two chains, as the kernels of larger inner sizes, whose bits these are.
-// Bound by its reads of shared memory and by the results it writes.  2,048 x 4,096 with k of 64: 36 us, 51 in two chains by the pipelined
+// in two chains.  Tiles of 16 rows for up to as many, of 64 else.
+// Bound by its reads of shared memory and by the results it writes.  2,048 x 4,096 with k of 64: 36 us, 51 in two chains by pipelined
 // tiles; sixteen products of 2,048 x 512: 71 and 89, with k of 32 43 and 63; 64 x 640 with k of 72 5.4 and 8.8 (7.5 in tiles of 64 x 64 without
 // a pipeline), 2,048 x 640 10.4 and 16.8, 8,192 x 2,048 with k of 128 121 and 141, 300 x 2,048 14.0 and 12.0.
 constexpr int GS_BN = 64;

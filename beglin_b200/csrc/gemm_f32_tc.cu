@@ -4,19 +4,26 @@
 // the six products of parts that are not below 2^-24 of it (one with a single bit set times any float is exact).  64 of k are one
 // stage: its five kinds of small products go into an accumulator in tensor memory first, so that their sums are not cut off at the size of
 // the large ones, then h h; the stage's sum leaves tensor memory and is added to the range's in float, rounded to nearest.  (An
-// accumulator cuts off instead of rounding, always towards nought: four MMAs on a large sum are four such cuts.)  Ranges of GF_RANGE of k lie
-// at fixed places; their sums are added in order, then the bias.  None of this depends on the number of rows, on tiles or on who
-// adds the ranges, so a row's result does not depend on how many other rows the call has: all forms here give the same bits.
+// accumulator cuts off instead of rounding, always towards nought: four MMAs on a large sum are four such cuts.)  Ranges of k lie at places that
+// follow from N and K alone (gt_range); their sums are added in order, then the bias.  None of this depends on the number of rows, on
+// tiles or on who adds the ranges, so a row's result does not depend on how many other rows the call has: all forms here give the
+// same bits.  Error against 64 bits (2-norm, normal operands): 1.0e-7 for K of 1,536 and 1.3e-7 for 9,000, where two chains of float
+// multiply-adds over 1,024 of k had 3.7e-7 and 4.1e-7; 0.9e-7 for K of 200 (1.8e-7).
 //
 // An operand that has no three parts (infinite, not a number, next to the largest float, or below some 2^-110) is noticed where it is cut;
 // the outputs of its row and range, and those whose sum is not finite, are summed by floats in two chains (even and odd k) instead, which
 // makes of them what floats make.  That, too, depends on the output's own row and column only.
 //
 // The weights' rows are the M side (128 a CTA), so a lane of tensor memory is an output feature and results leave in rows of 128 bytes;
-// the tokens are the N side (NT = 16 to 192).  Weights come as floats (TMA, two boxes of 128 rows x 32 of k a stage); a warpgroup or two read them, a row a
-// lane, cut them and put the parts into tensor memory (`tcgen05.st`) as left operands: they never return to shared memory, whose
-// bandwidth the right operands need.  The tokens' parts are made once by gf_parts_kernel and come by bulk copies (the weights' tiles would each
-// make them again); up to 16 tokens a warp of the CTA's own makes them.  Other warpgroups add up the stages' sums.
+// the tokens are the N side (NT = 16 to 160).  Weights come as floats (TMA, two boxes of 128 rows x 32 of k a stage); a warpgroup or
+// several read them, a row a lane, cut them and put the parts into tensor memory (`tcgen05.st`) as left operands: they never return to
+// shared memory, whose bandwidth the right operands need.  The tokens' parts are made once by gf_parts_kernel and come by bulk copies
+// (the weights' tiles would each make them again).  Other warpgroups add up the stages' sums.
+//
+// What bounds it: with 144 and 160 tokens the tensor cores (a stage of 160 tokens takes 1,980 cycles, its MMAs 1,920; with 32 of k a stage, one
+// warp that issued and one set of warps that cut and added it was 5,000), with fewer the instructions of the cut (some 12 a value: 1,600
+// cycles a stage, weights at 4 TB/s for 8 rows).  In us, the float units' kernels in brackets: 550 x 17,920 with k of 1,536 142 (930),
+// 550 x 1,536 with 8,960 99 (498), 64 x 17,920 with 1,536 33 (116), 8 x 17,920 27 (32), 1 x 2,048 with 768 8.1 (13.3).
 #include "gemm_f32.cuh"
 #include "float_parts.cuh"
 

@@ -146,7 +146,7 @@ class LatentAttention:
         H, T, _ = x.shape
         if self.f32:
             out = torch.empty((H, T, w.shape[1]), dtype=torch.float32, device=x.device)
-            ops.gemm_f32_nt_batched(x, w, out)
+            ops.gemm_f32_nt_batched(x, w, out, status=self.ctx.status)
             return out
         with ops.phase("proj_heads"):
             if out_dtype == x.dtype:

@@ -1,6 +1,7 @@
 """y = x W^T (+ bias), W row-major [out, in] as in the checkpoint (qwen_infer.c:688-691).
 
-float32: the hand-written CUDA-core kernel (true 32-bit, no tensor-core mode).
+float32: the hand-written product whose operands keep all their bits (on the tensor cores in three bfloat16 parts each, summed in
+float; small inner sizes on the float units).
 bfloat16: the tcgen05 tensor-core kernel of this package where it is the faster one (or everywhere,
 with gemm="tcgen05"), else the vendor library's product, which is where the reference calls its own
 platform's library (cblas_sgemv, qwen_infer.c:690).  Accumulation is float in every case: the library
@@ -43,7 +44,7 @@ class Linear:
         T = x.shape[0]
         if self.f32:
             out = torch.empty((T, self.out_features), dtype=torch.float32, device=x.device)
-            ops.gemm_f32_nt(x, self.weight, self.bias_f32, out)
+            ops.gemm_f32_nt(x, self.weight, self.bias_f32, out, status=self.ctx.status)
             return out
         if self._tc is not None and (self._tc_always or self._tc.wins(T)):
             return self._tc(x, self.bias_f32, out_dtype, partial)

@@ -10,7 +10,7 @@ The state S and the last taps - 1 inputs of the convolution are per-request stat
 manager's slab, float32, zero when the request starts): a step continues each request from its slot, however the request's
 tokens are cut into steps and whatever else the step holds.  Everything that enters the recurrence is float in both number
 formats: the input product comes out as float, the convolution, the gates' products, sigmoids, softplus, decay, step and
-state are float.  The gates' products run on the CUDA cores in float32 steps (every output summed in index order); in
+state are float.  The gates' products keep all bits in float32 steps (every output's sum has one order); in
 bfloat16 steps on the tensor cores, with u cut into two bfloat16 numbers that together hold sixteen bits of it, against the
 matrices in bfloat16, accumulated in float.  Portions of at least `CHUNK_FROM` rows of a request walk
 the recurrence in chunks that are joined by a scan over the chunks' (product of decays, sum); shorter ones and single
@@ -99,7 +99,7 @@ class RGLRU:
                 gates = torch.bmm(x2, self.gate_w2, out_dtype=torch.float32)
         else:
             gates = torch.empty((B, T, 2 * (W // B)), dtype=torch.float32, device=h.device)
-            ops.gemm_f32_nt_batched(u.view(T, B, W // B).transpose(0, 1), self.gate_w, gates)
+            ops.gemm_f32_nt_batched(u.view(T, B, W // B).transpose(0, 1), self.gate_w, gates, status=ctx.status)
         out = torch.empty((T, W), dtype=ctx.compute_dtype, device=h.device)
         if max(batch.lens) < self.CHUNK_FROM:
             ops.rglru_scan(gates, u, proj, 0, self.bias_r, self.bias_i, self.decay, cache.state, cache.slots, reqs, n_req, out,

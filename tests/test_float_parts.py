@@ -1,0 +1,95 @@
+"""The float products and float attention on the tensor cores: operands without three bfloat16 parts, exact products, and the
+tiles that the product chooses by its sizes."""
+import math
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+@pytest.fixture(scope="module")
+def ops():
+    from beglin_b200.csrc import ops as o
+    o.lib()
+    return o
+
+
+def rnd(*shape, seed=0):
+    g = torch.Generator(device=DEV).manual_seed(seed)
+    return torch.empty(shape, device=DEV).normal_(generator=g)
+
+
+def product(ops, a, w, bias=None):
+    out = torch.empty((a.shape[0], w.shape[0]), device=DEV)
+    ops.gemm_f32_nt(a, w, bias, out)
+    return out
+
+
+@pytest.mark.parametrize("K", [129, 600, 1100])
+@pytest.mark.parametrize("M", [3, 40, 200])
+def test_operands_without_three_parts(ops, M, K):
+    """Infinities, NaN, numbers next to the largest float and below 2^-110, on either side: what floats make of them, row by row."""
+    a, w = rnd(M, K, seed=1) * 0.125, rnd(130, K, seed=2) * 0.125
+    a[0, 5], a[1, K - 1], a[2, 70] = math.inf, math.nan, 3.4e38
+    w[7, 3], w[129, 128] = -math.inf, 3.4e38
+    if M > 3:
+        a[5] = rnd(K, seed=3) * 1e-38                       # a row of small numbers beside ones of the usual size
+        a[6, :] = 0.0
+    out, want = product(ops, a, w), a.double() @ w.double().t()
+    lost = want.abs() > 3.4028234e38
+    same = torch.isnan(out) == torch.isnan(want)
+    assert bool((same | lost).all()) and bool((torch.isinf(out) | torch.isnan(out))[lost].all())
+    fine = torch.isfinite(want) & ~lost
+    # a chain of K rounded sums, and the smallest float for what lies below it
+    bound = (K + 8) * 2.0 ** -24 * (a.abs().double() @ w.abs().double().t()) + K * 2.0 ** -149
+    assert bool(((out.double() - want).abs() <= bound)[fine].all())
+    for m in range(min(M, 8)):
+        assert torch.equal(product(ops, a[m:m + 1].contiguous(), w).view(torch.int32), out[m:m + 1].view(torch.int32)), m
+
+
+def test_small_numbers_keep_their_digits(ops):
+    a, w = rnd(20, 300, seed=4) * 1e-38, rnd(70, 300, seed=5) * 1e37
+    out, want = product(ops, a, w), a.double() @ w.double().t()
+    assert bool(((out.double() - want).abs() <= 308 * 2.0 ** -24 * (a.abs().double() @ w.abs().double().t())).all())
+
+
+def test_single_numbers_come_through_whole(ops):
+    w = rnd(200, 300, seed=6)
+    assert torch.equal(product(ops, torch.eye(300, device=DEV), w), w.t())
+
+
+@pytest.mark.parametrize("M,N,K", [(16, 130, 1100), (31, 17920, 200), (64, 9000, 320), (96, 9472, 260), (128, 9472, 200), (143, 18944, 192), (160, 18944, 192),
+                                   (300, 9472, 136), (161, 257, 8200)])
+def test_tiles_of_all_sizes(ops, M, N, K):
+    a, w, b = rnd(M, K, seed=7), rnd(N, K, seed=8), rnd(N, seed=9)
+    out = product(ops, a, w, b)
+    want = a.double() @ w.double().t() + b.double()
+    assert bool(((out.double() - want).abs() <= (K + 8) * 2.0 ** -24 * (a.abs().double() @ w.abs().double().t() + b.abs().double())).all())
+    for m in (0, M // 2, M - 1):
+        assert torch.equal(product(ops, a[m:m + 1].contiguous(), w, b)[0], out[m]), m
+
+
+@pytest.mark.parametrize("hd", [48, 80, 128])
+def test_attention_of_queries_without_three_parts(ops, hd):
+    """Queries below 2^-110 against keys as large: scores of the usual size, every digit of them needed."""
+    n, nh, page = 70, 2, 16
+    pages = -(-n // page)
+    pool = rnd(pages, 2, 1, page, hd, seed=10)
+    pool[:, 0] *= 1e37
+    q = rnd(n, nh * hd, seed=11) * 1e-37
+    pos = torch.arange(n, dtype=torch.int32, device=DEV)
+    _, bq, tile = ops.attention_plan(nh, hd, torch.float32, False, "generic", page)
+    blocks = torch.tensor([(0, r, min(bq, n - r)) for r in range(0, n, bq)], dtype=torch.int32, device=DEV)
+    out, status = torch.empty((n, nh * hd), device=DEV), ops.new_status(DEV)
+    table = torch.arange(pages, dtype=torch.int32, device=DEV).view(1, -1)
+    ops.attention(q, nh * hd, pool, table, pos, blocks, len(blocks), n - 1, n, nh, 1, hd, 0, 256, tile, bq, hd ** -0.5, out, status, "generic")
+    ops.raise_on_status(status)
+    k, v = (pool[:, i, 0].reshape(-1, hd)[:n].double() for i in (0, 1))
+    for h in range(nh):
+        s = (q[:, h * hd:(h + 1) * hd].double() @ k.t()) * hd ** -0.5
+        s = s.masked_fill(torch.triu(torch.ones(n, n, dtype=torch.bool, device=DEV), 1), -math.inf)
+        want = torch.softmax(s, -1) @ v
+        # a score's error moves a weight by as much: hd + 8 roundings of the largest sum of products
+        assert (out[:, h * hd:(h + 1) * hd].double() - want).abs().max() <= (hd + 8) * 2.0 ** -23 * float(s.abs()[s > -math.inf].max() + 1) * float(v.abs().max())
