@@ -361,12 +361,15 @@ extern "C" int bg_attention_partial(const void* q, int q_dtype, int q_stride, co
     const bool pieces = q_stride % 4 == 0 && (uintptr_t)q % 16 == 0 && (uintptr_t)kv_pool % 16 == 0 && (uintptr_t)part_o % 16 == 0;
     if (q_dtype == BG_DTYPE_F32 && cache_dtype == BG_DTYPE_F32 && ax_takes(bq * p.group, hd, vd, maps) && split % AX_KEYS == 0 && pieces) {
         constexpr int need = 2 * AX_TILE + 1024;
-        auto kern = attention_f32_tc_kernel<AttnParams>;
+        auto kern = vd == 128 ? attention_f32_tc_kernel<AttnParams, 64> : vd == 64 ? attention_f32_tc_kernel<AttnParams, 32> : attention_f32_tc_kernel<AttnParams, 0>;
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, need);
         if (e != cudaSuccess) return (int)e;
         static const bool fits = [] {                      // (the split of the registers counts on as many at launch)
-            cudaFuncAttributes a;
-            return cudaFuncGetAttributes(&a, attention_f32_tc_kernel<AttnParams>) == cudaSuccess && a.numRegs >= AX_REGS;
+            for (auto k : {attention_f32_tc_kernel<AttnParams, 64>, attention_f32_tc_kernel<AttnParams, 32>, attention_f32_tc_kernel<AttnParams, 0>}) {
+                cudaFuncAttributes a;
+                if (cudaFuncGetAttributes(&a, k) != cudaSuccess || a.numRegs < AX_REGS) return false;
+            }
+            return true;
         }();
         if (!fits) return (int)cudaErrorInvalidConfiguration;
         launch(kern, grid, dim3(AX_THREADS), need, stream, p);

@@ -37,7 +37,8 @@ __device__ __forceinline__ bool ax_odd(float x) {      // no three parts
 // all 256 threads of the rows meet
 __device__ __forceinline__ void ax_rows_meet() { asm volatile("barrier.cta.sync 1, 256;\n" ::: "memory"); }
 
-template <typename P>
+// OD: output features of a thread where they are a constant (half a value's: 64 or 32), or 0.
+template <typename P, int OD>
 __global__ void __launch_bounds__(AX_THREADS, 1) attention_f32_tc_kernel(P p) {
     extern __shared__ unsigned char ax_raw[];
     unsigned char* kt = (unsigned char*)(((uintptr_t)ax_raw + 1023) & ~(uintptr_t)1023);
@@ -48,6 +49,7 @@ __global__ void __launch_bounds__(AX_THREADS, 1) attention_f32_tc_kernel(P p) {
     __shared__ int page_s[4][AX_KEYS];                 // pages of a tile's keys, -1: none (they are asked for again when its values have been summed)
     __shared__ unsigned char key_odd[2][AX_KEYS], value_odd[2][AX_KEYS], row_odd[2][AX_ROWS];
     __shared__ float row_max[2][AX_ROWS];
+    __shared__ int row_at[AX_ROWS];                    // a row's place among the partial results, -1: none
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int qb = blockIdx.x, kvh = blockIdx.y, sp = blockIdx.z;
@@ -186,23 +188,27 @@ __global__ void __launch_bounds__(AX_THREADS, 1) attention_f32_tc_kernel(P p) {
                 fetch(vs, vd, v);
                 if (i > 0) mbar_wait(&v_empty, (i - 1) & 1, &failed);
                 left = 0;
+                auto values = [&]() {
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    uint4 h, m, l;
-                    unsigned mine = 0;
-                    split8(v[2 * j], v[2 * j + 1], h, m, l, mine);
-                    if (mine & 0xffffu) {              // what has no three parts is nought here
-                        float* x = reinterpret_cast<float*>(&v[2 * j]);
-#pragma unroll
-                        for (int e = 0; e < 8; ++e)
-                            if (ax_odd(x[e])) x[e] = 0.0f;
-                        unsigned none = 0;
-                        split8(v[2 * j], v[2 * j + 1], h, m, l, none);
+                    for (int j = 0; j < 4; ++j) {
+                        uint4 h, m, l;
+                        split8(v[2 * j], v[2 * j + 1], h, m, l, left);
+                        if ((c0 + 4 * j) * 8 < vd) store(vt, c0 + 4 * j, h, m, l);
                     }
-                    left |= mine;
-                    if ((c0 + 4 * j) * 8 < vd) store(vt, c0 + 4 * j, h, m, l);
-                }
+                };
+                values();
                 left &= 0xffffu;
+                if (left) {                            // what has no three parts is nought here
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) {
+                        if (ax_odd(v[j].x)) v[j].x = 0.0f;
+                        if (ax_odd(v[j].y)) v[j].y = 0.0f;
+                        if (ax_odd(v[j].z)) v[j].z = 0.0f;
+                        if (ax_odd(v[j].w)) v[j].w = 0.0f;
+                    }
+                    values();
+                    left = 1;
+                }
                 left |= __shfl_xor_sync(0xffffffffu, left, 1);
                 left |= __shfl_xor_sync(0xffffffffu, left, 2);
                 if (c0 == 0) value_odd[i & 1][key] = left != 0;
@@ -222,23 +228,28 @@ __global__ void __launch_bounds__(AX_THREADS, 1) attention_f32_tc_kernel(P p) {
         const int pos = in ? p.positions[row0 + qi] : -1, lo = first_visible(pos < 0 ? 0 : pos, p.window);
         const float* q = (const float*)p.q + (size_t)(row0 + qi) * p.q_stride + (size_t)head * hd;
         const float slope = p.slopes && in ? p.slopes[head] : 0.0f;
-        const int od = vd / 2;                         // output features of a thread, a multiple of 8
-        float out[64];
+        const int od = OD ? OD : vd / 2;               // output features of a thread, a multiple of 8
+        constexpr int MOST = OD ? OD : 64;
+        float out[MOST];
         float m = -INFINITY, sum = 0.0f;
 #pragma unroll
-        for (int d = 0; d < 64; ++d) out[d] = 0.0f;
+        for (int d = 0; d < MOST; ++d) out[d] = 0.0f;
         if (seen && t_first < k_end) {
             // the row's queries, half of their features a thread
             unsigned left = 0;
-            for (int d = half * (hd / 2); d < (half + 1) * (hd / 2); d += 8) {
+            float4 x[16];                              // (all on their way together)
+#pragma unroll
+            for (int c = 0; c < 16; ++c) x[c] = in && c * 4 < hd / 2 ? *reinterpret_cast<const float4*>(q + half * (hd / 2) + c * 4) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+            for (int c = 0; c < 8; ++c) {
+                if (c * 8 >= hd / 2) break;
                 unsigned h[4], mm[4], l[4];
-                float4 a = make_float4(0.0f, 0.0f, 0.0f, 0.0f), b = a;
-                if (in) { a = *reinterpret_cast<const float4*>(q + d); b = *reinterpret_cast<const float4*>(q + d + 4); }
-                gt_split(pair2(a.x, a.y), h[0], mm[0], l[0], left);
-                gt_split(pair2(a.z, a.w), h[1], mm[1], l[1], left);
-                gt_split(pair2(b.x, b.y), h[2], mm[2], l[2], left);
-                gt_split(pair2(b.z, b.w), h[3], mm[3], l[3], left);
-                gt_st4(lanes + AX_Q + d / 2, h); gt_st4(lanes + AX_Q + 64 + d / 2, mm); gt_st4(lanes + AX_Q + 128 + d / 2, l);
+                gt_split(pair2(x[2 * c].x, x[2 * c].y), h[0], mm[0], l[0], left);
+                gt_split(pair2(x[2 * c].z, x[2 * c].w), h[1], mm[1], l[1], left);
+                gt_split(pair2(x[2 * c + 1].x, x[2 * c + 1].y), h[2], mm[2], l[2], left);
+                gt_split(pair2(x[2 * c + 1].z, x[2 * c + 1].w), h[3], mm[3], l[3], left);
+                const unsigned a = lanes + AX_Q + half * (hd / 4) + c * 4;
+                gt_st4(a, h); gt_st4(a + 64, mm); gt_st4(a + 128, l);
             }
             row_odd[half][row] = (left & 0xffffu) != 0;
             tc_wait_st();
@@ -252,16 +263,20 @@ __global__ void __launch_bounds__(AX_THREADS, 1) attention_f32_tc_kernel(P p) {
             auto add_values = [&](int i, int t0, float corr) {
                 mbar_wait(&o_full, i & 1, &failed);
                 tc_fence_after();
+                const unsigned long long cc = pair2(corr, corr);
 #pragma unroll
-                for (int c = 0; c < 64; c += 16) {
-                    if (c >= od) break;
+                for (int c = 0; c < MOST; c += 16) {
+                    if (!OD && c >= od) break;
                     unsigned r[16];
-                    if (c + 16 <= od) gt_ld16(lanes + AX_O + half * od + c, r);
+                    if (OD || c + 16 <= od) gt_ld16(lanes + AX_O + half * od + c, r);
                     else gt_ld8(lanes + AX_O + half * od + c, r);
                     tc_wait_ld();
 #pragma unroll
-                    for (int e = 0; e < 16; ++e)
-                        if (c + e < od) out[c + e] = fmaf(out[c + e], corr, __uint_as_float(r[e]));
+                    for (int e = 0; e < 16; e += 2)
+                        if (OD || c + e < od) {
+                            const unsigned long long y = fma2(pair2(out[c + e], out[c + e + 1]), cc, (unsigned long long)r[e] | ((unsigned long long)r[e + 1] << 32));
+                            out[c + e] = low2(y); out[c + e + 1] = high2(y);
+                        }
                 }
                 bool odd = false;
 #pragma unroll
@@ -281,7 +296,7 @@ __global__ void __launch_bounds__(AX_THREADS, 1) attention_f32_tc_kernel(P p) {
                         if (f == 0.0f || page < 0) continue;
                         const float* src = pool + (size_t)page * page_elems + v_off + ((size_t)kvh * p.page_size + (t0 + j) % p.page_size) * vd + half * od;
 #pragma unroll
-                        for (int d = 0; d < 64; ++d)
+                        for (int d = 0; d < MOST; ++d)
                             if (d < od && ax_odd(src[d])) out[d] = fmaf(f, src[d], out[d]);
                     }
                 }
@@ -328,15 +343,27 @@ __global__ void __launch_bounds__(AX_THREADS, 1) attention_f32_tc_kernel(P p) {
                         if (j == jb) w[j] = even;
                 }
                 __syncwarp();
+                // (the way that most tiles go is short: a warp's instructions are fetched once a tile, and with every option in one unrolled
+                // loop the fetches were most of a tile's 12,500 cycles)
                 float most = -INFINITY;
+                if (p.softcap > 0.0f || p.slopes) {
 #pragma unroll
-                for (int j = 0; j < 32; ++j) {
-                    w[j] *= p.scale;
-                    if (p.softcap > 0.0f) w[j] = p.softcap * tanhf(w[j] / p.softcap);
-                    if (p.slopes) w[j] = fmaf(-slope, (float)(pos - (t0 + half * 32 + j)), w[j]);
-                    if (!(visible >> j & 1)) w[j] = -INFINITY;
-                    most = fmaxf(most, w[j]);
+                    for (int j = 0; j < 32; ++j) {
+                        w[j] *= p.scale;
+                        if (p.softcap > 0.0f) w[j] = p.softcap * tanhf(w[j] / p.softcap);
+                        if (p.slopes) w[j] = fmaf(-slope, (float)(pos - (base + j)), w[j]);
+                    }
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) w[j] *= p.scale;
                 }
+                if (!__all_sync(0xffffffffu, visible == 0xffffffffu)) {
+#pragma unroll
+                    for (int j = 0; j < 32; ++j)
+                        if (!(visible >> j & 1)) w[j] = -INFINITY;
+                }
+#pragma unroll
+                for (int j = 0; j < 32; ++j) most = fmaxf(most, w[j]);
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&s_empty);  // (the scores and the tile's pages have been read)
@@ -344,12 +371,10 @@ __global__ void __launch_bounds__(AX_THREADS, 1) attention_f32_tc_kernel(P p) {
                 ax_rows_meet();
                 const float m_new = fmaxf(m, fmaxf(row_max[0][row], row_max[1][row]));
                 const float corr = m == -INFINITY ? 0.0f : expf(m - m_new);
+                const float from = m_new == -INFINITY ? 0.0f : m_new;          // (no key seen so far: every weight is nought)
                 float s = 0.0f;
 #pragma unroll
-                for (int j = 0; j < 32; ++j) {
-                    w[j] = w[j] == -INFINITY || m_new == -INFINITY ? 0.0f : expf(w[j] - m_new);
-                    s += w[j];
-                }
+                for (int j = 0; j < 32; ++j) { w[j] = expf(w[j] - from); s += w[j]; }
                 sum = fmaf(sum, corr, s);
                 m = m_new;
                 if (i > 0) add_values(i - 1, t_before, corr_before);
@@ -374,17 +399,24 @@ __global__ void __launch_bounds__(AX_THREADS, 1) attention_f32_tc_kernel(P p) {
                 t0 = next_tile(t0);
             }
             add_values(i - 1, t_before, corr_before);
+            // partial results of the rows that see at least one key of this split, through the tiles' room (their products are complete)
             row_max[half][row] = sum;
-            ax_rows_meet();
-            // partial results of the rows that see at least one key of this split
-            if (in && !(pos < sp * p.split || (lo >= (sp + 1) * p.split && sp * p.split >= p.keep))) {
-                const bool lost = *(volatile int*)&failed != 0;                // (a wait ran out)
-                const size_t prow = ((size_t)(row0 + qi) * p.nh + head) * p.max_splits + sp;
-                float* o = p.part_o + prow * vd + half * od;
+            if (half == 0) row_at[row] = in && !(pos < sp * p.split || (lo >= (sp + 1) * p.split && sp * p.split >= p.keep)) ? (row0 + qi) * p.nh + head : -1;
+            float* stage = (float*)kt;
+            const int ld = vd + 4;
 #pragma unroll
-                for (int d = 0; d < 64; d += 4)
-                    if (d < od) *reinterpret_cast<float4*>(o + d) = lost ? make_float4(NAN, NAN, NAN, NAN) : make_float4(out[d], out[d + 1], out[d + 2], out[d + 3]);
-                if (half == 0) { p.part_ml[prow * 2 + 0] = m; p.part_ml[prow * 2 + 1] = row_max[0][row] + row_max[1][row]; }
+            for (int d = 0; d < MOST; d += 4)
+                if (OD || d < od) *reinterpret_cast<float4*>(stage + row * ld + half * od + d) = make_float4(out[d], out[d + 1], out[d + 2], out[d + 3]);
+            ax_rows_meet();
+            const bool lost = *(volatile int*)&failed != 0;                    // (a wait ran out)
+            if (half == 0 && row_at[row] >= 0) {
+                float* ml = p.part_ml + ((size_t)row_at[row] * p.max_splits + sp) * 2;
+                ml[0] = m; ml[1] = lost ? NAN : row_max[0][row] + row_max[1][row];
+            }
+            for (int r = warp; r < n_rows; r += 8) {
+                const int place = row_at[r];
+                if (place >= 0 && lane * 4 < vd)
+                    *reinterpret_cast<float4*>(p.part_o + ((size_t)place * p.max_splits + sp) * vd + lane * 4) = *reinterpret_cast<const float4*>(stage + r * ld + lane * 4);
             }
         }
     }
