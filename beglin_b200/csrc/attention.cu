@@ -360,7 +360,7 @@ extern "C" int bg_attention_partial(const void* q, int q_dtype, int q_stride, co
     dim3 grid(n_qblk, nkv, n_splits_launch);
     const bool pieces = q_stride % 4 == 0 && (uintptr_t)q % 16 == 0 && (uintptr_t)kv_pool % 16 == 0 && (uintptr_t)part_o % 16 == 0;
     if (q_dtype == BG_DTYPE_F32 && cache_dtype == BG_DTYPE_F32 && ax_takes(bq * p.group, hd, vd, maps) && split % AX_KEYS == 0 && pieces) {
-        constexpr int need = 2 * AX_TILE + 1024;
+        constexpr int need = 4 * AX_TILE + 1024;
         auto kern = vd == 128 ? attention_f32_tc_kernel<AttnParams, 64> : vd == 64 ? attention_f32_tc_kernel<AttnParams, 32> : attention_f32_tc_kernel<AttnParams, 0>;
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, need);
         if (e != cudaSuccess) return (int)e;

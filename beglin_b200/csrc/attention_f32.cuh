@@ -9,8 +9,8 @@
 // are two chains whose sums are added; heads of up to AF_NARROW features are one chain, which takes no longer there: 2,048 rows of 8 heads of
 // 32, 188 and 194 us).  A row's sixteen threads lie in one half of a warp: maximum and sum are shuffles, and the weights pass through
 // shared memory behind a warp's barrier only.  The keys of the next tile come (cp.async) under the value product, the values under the scores.  112 KB of shared memory for heads of 128, so that two CTAs share an SM.  FMA pipe, shared
-// memory and issue are each used by half, a tile's phases in turn: the mixer of 550 rows of 12 heads of 128 over 1,536 to 3,000 held
-// positions takes 570 us with its products, 2,818 us with a key a lane and two reads of shared memory for every multiply-add.
+// memory and issue are each used by half, a tile's phases in turn: heads of 128, which the tensor cores have taken over since, took 307 us for
+// 550 rows of 12 heads over 1,536 to 3,000 held positions, 2,200 with a key a lane and two reads of shared memory for every multiply-add.
 //
 // A row's arithmetic depends on nothing but its own keys: tiles and splits lie at absolute positions, every sum has one order, and a
 // value whose weight is nought is left out, so that an infinite one at a position that a row does not see does not reach it.  A warp

@@ -8,6 +8,10 @@
 // 32 keys each, make the weights and keep the row's sums of values in registers (a tile's sums leave tensor memory and are added in float).
 // Queries and weights are left operands in tensor memory.  The scores of a tile are multiplied while the weights of the one before are made,
 // its values while those of the one behind are.
+// 550 rows of 12 heads of 128 (2 kv heads) behind 1,500 positions: 82 us, 87 with one tile of keys and of values in shared memory, 120 with
+// all options in one unrolled loop and results stored a row a thread; the mixer of 550 rows over 1,536 to 3,000 held positions takes 179 us
+// with its products, 399 with the float units' attention and the same products.  What bounds it: a tile's some 8,000 cycles are a chain of
+// hand-overs and of instructions that are fetched once a tile (its MMAs take 3,072), on one CTA an SM.
 //
 // A row's arithmetic depends on nothing but its own keys: tiles and splits lie at absolute positions, and an MMA's rows do not meet.  What has no
 // three parts (infinite, not a number, below some 2^-110) is noticed where it is cut: scores of such queries or keys, and those that are
@@ -20,6 +24,7 @@
 namespace bg {
 
 constexpr int AX_ROWS = 128, AX_KEYS = 64;
+constexpr int AX_NONE = -2147483647 - 1;               // no key here (not an entry of a block table)
 constexpr int AX_THREADS = 640;                        // two warpgroups of rows, two that cut, one with the warp that issues
 constexpr unsigned AX_BLOCK = AX_KEYS * 128, AX_PART = 2 * AX_BLOCK, AX_TILE = 3 * AX_PART;       // 64 keys x 64 features; x 128; three parts
 constexpr unsigned AX_Q = 0, AX_S = 192, AX_P = 256, AX_O = 352;                      // columns of tensor memory
@@ -42,19 +47,21 @@ template <typename P, int OD>
 __global__ void __launch_bounds__(AX_THREADS, 1) attention_f32_tc_kernel(P p) {
     extern __shared__ unsigned char ax_raw[];
     unsigned char* kt = (unsigned char*)(((uintptr_t)ax_raw + 1023) & ~(uintptr_t)1023);
-    unsigned char* vt = kt + AX_TILE;
-    __shared__ __align__(8) unsigned long long q_full, k_full, k_empty, v_full, v_empty, s_full, s_empty, p_full, o_full, o_empty;
+    unsigned char* vt = kt + 2 * AX_TILE;              // two tiles of keys, two of values
+    __shared__ __align__(8) unsigned long long q_full, k_full[2], k_empty[2], v_full[2], v_empty[2], s_full, s_empty, p_full, o_full, o_empty;
     __shared__ unsigned tmem_sh;
     __shared__ int failed;
-    __shared__ int page_s[4][AX_KEYS];                 // pages of a tile's keys, -1: none (they are asked for again when its values have been summed)
-    __shared__ unsigned char key_odd[2][AX_KEYS], value_odd[2][AX_KEYS], row_odd[2][AX_ROWS];
+    // of the last tiles, as many as cutting can be ahead of reading: pages of the keys, -1: none (asked for again when a tile's values have been summed), ..
+    __shared__ int page_s[8][AX_KEYS];
+    __shared__ unsigned char key_odd[4][AX_KEYS], value_odd[4][AX_KEYS], row_odd[2][AX_ROWS];
     __shared__ float row_max[2][AX_ROWS];
     __shared__ int row_at[AX_ROWS];                    // a row's place among the partial results, -1: none
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int qb = blockIdx.x, kvh = blockIdx.y, sp = blockIdx.z;
     if (tid == 0) {
-        mbar_init(&q_full, 8); mbar_init(&k_full, 8); mbar_init(&k_empty, 1); mbar_init(&v_full, 8); mbar_init(&v_empty, 1);
+        mbar_init(&q_full, 8);
+        for (int b = 0; b < 2; ++b) { mbar_init(&k_full[b], 8); mbar_init(&k_empty[b], 1); mbar_init(&v_full[b], 8); mbar_init(&v_empty[b], 1); }
         mbar_init(&s_full, 1); mbar_init(&s_empty, 8); mbar_init(&p_full, 8); mbar_init(&o_full, 1); mbar_init(&o_empty, 8);
         failed = 0;
         mbar_init_fence();
@@ -85,22 +92,24 @@ __global__ void __launch_bounds__(AX_THREADS, 1) attention_f32_tc_kernel(P p) {
         // ---------------- the MMAs: a tile's scores before the values of the tile in front of it
         if (seen && t_first < k_end) {
             const unsigned s_desc = instr_desc_bf16(AX_ROWS, AX_KEYS), o_desc = instr_desc_bf16(AX_ROWS, vd, 1);
-            const unsigned ka = smem_u32(kt), va = smem_u32(vt);
+            const unsigned k0 = smem_u32(kt), v0 = smem_u32(vt);
             bool ok = mbar_wait(&q_full, 0, &failed);
             int i = 0;
             auto scores = [&](int tile) {
-                ok = ok && mbar_wait(&k_full, tile & 1, &failed) && (tile == 0 || mbar_wait(&s_empty, (tile - 1) & 1, &failed));
+                ok = ok && mbar_wait(&k_full[tile & 1], (tile >> 1) & 1, &failed) && (tile == 0 || mbar_wait(&s_empty, (tile - 1) & 1, &failed));
                 if (!ok) return;
                 tc_fence_after();
+                const unsigned ka = k0 + (tile & 1) * AX_TILE;
                 if (elect_one()) {
 #pragma unroll
                     for (int e = 0; e < 6; ++e) {
                         constexpr int PA[6] = {2, 1, 0, 1, 0, 0}, PB[6] = {0, 1, 2, 0, 1, 0};
-                        for (int j = 0; j < hd / 16; ++j)
-                            tc_mma_ts(tmem + AX_S, tmem + AX_Q + PA[e] * 64 + j * 8, smem_desc_sw128(ka + PB[e] * AX_PART + (j >> 2) * AX_BLOCK + (j & 3) * 32), s_desc, e || j ? 1u : 0u);
+#pragma unroll
+                        for (int j = 0; j < 8; ++j)
+                            if (j < hd / 16) tc_mma_ts(tmem + AX_S, tmem + AX_Q + PA[e] * 64 + j * 8, smem_desc_sw128(ka + PB[e] * AX_PART + (j >> 2) * AX_BLOCK + (j & 3) * 32), s_desc, e || j ? 1u : 0u);
                     }
                     tc_commit(&s_full);
-                    tc_commit(&k_empty);
+                    tc_commit(&k_empty[tile & 1]);
                 }
                 __syncwarp();
             };
@@ -108,9 +117,10 @@ __global__ void __launch_bounds__(AX_THREADS, 1) attention_f32_tc_kernel(P p) {
             for (int t0 = t_first; t0 < k_end && ok; ++i) {
                 const int t1 = next_tile(t0);
                 if (t1 < k_end) scores(i + 1);
-                ok = ok && mbar_wait(&v_full, i & 1, &failed) && mbar_wait(&p_full, i & 1, &failed) && (i == 0 || mbar_wait(&o_empty, (i - 1) & 1, &failed));
+                ok = ok && mbar_wait(&v_full[i & 1], (i >> 1) & 1, &failed) && mbar_wait(&p_full, i & 1, &failed) && (i == 0 || mbar_wait(&o_empty, (i - 1) & 1, &failed));
                 if (!ok) break;
                 tc_fence_after();
+                const unsigned va = v0 + (i & 1) * AX_TILE;
                 if (elect_one()) {
 #pragma unroll
                     for (int e = 0; e < 6; ++e) {
@@ -120,7 +130,7 @@ __global__ void __launch_bounds__(AX_THREADS, 1) attention_f32_tc_kernel(P p) {
                             tc_mma_ts(tmem + AX_O, tmem + AX_P + PA[e] * 32 + j * 8, smem_desc_sw128_nmajor(va + PB[e] * AX_PART + j * 2048, AX_BLOCK, 1024), o_desc, e || j ? 1u : 0u);
                     }
                     tc_commit(&o_full);
-                    tc_commit(&v_empty);
+                    tc_commit(&v_empty[i & 1]);
                 }
                 __syncwarp();
                 t0 = t1;
@@ -132,16 +142,20 @@ __global__ void __launch_bounds__(AX_THREADS, 1) attention_f32_tc_kernel(P p) {
         const int c0 = tid & 3, key = (tid - 256) >> 2;
         if (seen) {
             int i = 0;
+            auto page_of = [&](int t0) {
+                const int at = t0 + key;
+                return at < k_end && key_seen(at, lo_first, p.keep) ? p.block_table[(size_t)req * p.max_pages + at / p.page_size] : AX_NONE;
+            };
+            int page_next = page_of(t_first);          // (asked for a tile ahead)
             for (int t0 = t_first; t0 < k_end; ++i) {
                 const int at = t0 + key;
-                int page = -1;
-                if (at < k_end && key_seen(at, lo_first, p.keep)) {
-                    page = p.block_table[(size_t)req * p.max_pages + at / p.page_size];
-                    if (page < 0 || page >= p.num_pages) {
-                        if (p.status && c0 == 0) atomicOr(p.status, BG_STATUS_BAD_PAGE);
-                        page = -1;
-                    }
+                int page = page_next;
+                if (page != AX_NONE && (page < 0 || page >= p.num_pages)) {
+                    if (p.status && c0 == 0) atomicOr(p.status, BG_STATUS_BAD_PAGE);
+                    page = -1;
                 }
+                if (page < 0) page = -1;
+                unsigned char *kb = kt + (i & 1) * AX_TILE, *vb = vt + (i & 1) * AX_TILE;
                 const size_t slot = (size_t)kvh * p.page_size + at % p.page_size;
                 const float* ks = pool + (page >= 0 ? (size_t)page * page_elems + slot * hd : 0);
                 const float* vs = pool + (page >= 0 ? (size_t)page * page_elems + v_off + slot * vd : 0);
@@ -170,30 +184,32 @@ __global__ void __launch_bounds__(AX_THREADS, 1) attention_f32_tc_kernel(P p) {
                 };
                 float4 v[8];
                 fetch(ks, hd, v);
-                if (i > 0) mbar_wait(&k_empty, (i - 1) & 1, &failed);
+                const int t1 = next_tile(t0);
+                page_next = t1 < k_end ? page_of(t1) : AX_NONE;
+                if (i > 1) mbar_wait(&k_empty[i & 1], ((i >> 1) - 1) & 1, &failed);
                 unsigned left = 0;
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
                     uint4 h, m, l;
                     split8(v[2 * j], v[2 * j + 1], h, m, l, left);
-                    if ((c0 + 4 * j) * 8 < hd) store(kt, c0 + 4 * j, h, m, l);
+                    if ((c0 + 4 * j) * 8 < hd) store(kb, c0 + 4 * j, h, m, l);
                 }
                 left &= 0xffffu;
                 left |= __shfl_xor_sync(0xffffffffu, left, 1);
                 left |= __shfl_xor_sync(0xffffffffu, left, 2);
-                if (c0 == 0) { page_s[i & 3][key] = page; key_odd[i & 1][key] = left != 0; }
+                if (c0 == 0) { page_s[i & 7][key] = page; key_odd[i & 3][key] = left != 0; }
                 fence_proxy_async();
                 __syncwarp();
-                if (lane == 0) mbar_arrive(&k_full);
+                if (lane == 0) mbar_arrive(&k_full[i & 1]);
                 fetch(vs, vd, v);
-                if (i > 0) mbar_wait(&v_empty, (i - 1) & 1, &failed);
+                if (i > 1) mbar_wait(&v_empty[i & 1], ((i >> 1) - 1) & 1, &failed);
                 left = 0;
                 auto values = [&]() {
 #pragma unroll
                     for (int j = 0; j < 4; ++j) {
                         uint4 h, m, l;
                         split8(v[2 * j], v[2 * j + 1], h, m, l, left);
-                        if ((c0 + 4 * j) * 8 < vd) store(vt, c0 + 4 * j, h, m, l);
+                        if ((c0 + 4 * j) * 8 < vd) store(vb, c0 + 4 * j, h, m, l);
                     }
                 };
                 values();
@@ -211,11 +227,11 @@ __global__ void __launch_bounds__(AX_THREADS, 1) attention_f32_tc_kernel(P p) {
                 }
                 left |= __shfl_xor_sync(0xffffffffu, left, 1);
                 left |= __shfl_xor_sync(0xffffffffu, left, 2);
-                if (c0 == 0) value_odd[i & 1][key] = left != 0;
+                if (c0 == 0) value_odd[i & 3][key] = left != 0;
                 fence_proxy_async();
                 __syncwarp();
-                if (lane == 0) mbar_arrive(&v_full);
-                t0 = next_tile(t0);
+                if (lane == 0) mbar_arrive(&v_full[i & 1]);
+                t0 = t1;
             }
         }
     } else if (warp < 8) {
@@ -280,10 +296,10 @@ __global__ void __launch_bounds__(AX_THREADS, 1) attention_f32_tc_kernel(P p) {
                 }
                 bool odd = false;
 #pragma unroll
-                for (int j = 0; j < 2; ++j) odd |= value_odd[i & 1][j * 32 + lane] != 0;
+                for (int j = 0; j < 2; ++j) odd |= value_odd[i & 3][j * 32 + lane] != 0;
                 if (__any_sync(0xffffffffu, odd)) {    // values without three parts: the weights come back from their own
                     for (int j = 0; j < AX_KEYS; ++j) {
-                        if (!value_odd[i & 1][j]) continue;
+                        if (!value_odd[i & 3][j]) continue;
                         unsigned w[3];
 #pragma unroll
                         for (int e = 0; e < 3; ++e)
@@ -292,7 +308,7 @@ __global__ void __launch_bounds__(AX_THREADS, 1) attention_f32_tc_kernel(P p) {
                         float f = 0.0f;
 #pragma unroll
                         for (int e = 2; e >= 0; --e) f += __uint_as_float(j & 1 ? w[e] & 0xffff0000u : w[e] << 16);
-                        const int page = page_s[i & 3][j];
+                        const int page = page_s[i & 7][j];
                         if (f == 0.0f || page < 0) continue;
                         const float* src = pool + (size_t)page * page_elems + v_off + ((size_t)kvh * p.page_size + (t0 + j) % p.page_size) * vd + half * od;
 #pragma unroll
@@ -319,8 +335,8 @@ __global__ void __launch_bounds__(AX_THREADS, 1) attention_f32_tc_kernel(P p) {
                 // the keys that the row sees, a bit each, and the scores that the parts cannot make
                 const int base = t0 + half * 32, last = min(pos, k_end - 1) - base;
                 auto below = [](int n) { return n <= 0 ? 0u : n >= 32 ? 0xffffffffu : (1u << n) - 1; };       // bits 0 .. n - 1
-                unsigned visible = __ballot_sync(0xffffffffu, page_s[i & 3][half * 32 + lane] >= 0) & below(last + 1) & (~below(lo - base) | below(p.keep - base));
-                unsigned bad = __ballot_sync(0xffffffffu, key_odd[i & 1][half * 32 + lane] != 0);
+                unsigned visible = __ballot_sync(0xffffffffu, page_s[i & 7][half * 32 + lane] >= 0) & below(last + 1) & (~below(lo - base) | below(p.keep - base));
+                unsigned bad = __ballot_sync(0xffffffffu, key_odd[i & 3][half * 32 + lane] != 0);
                 if (q_odd) bad = 0xffffffffu;
                 float nought = 0.0f;
 #pragma unroll
@@ -332,7 +348,7 @@ __global__ void __launch_bounds__(AX_THREADS, 1) attention_f32_tc_kernel(P p) {
                 }
                 bad &= visible;
                 while (bad) {
-                    const int jb = __ffs(bad) - 1, at = t0 + half * 32 + jb, page = page_s[i & 3][half * 32 + jb];
+                    const int jb = __ffs(bad) - 1, at = t0 + half * 32 + jb, page = page_s[i & 7][half * 32 + jb];
                     bad &= bad - 1;
                     const float* src = pool + (size_t)page * page_elems + ((size_t)kvh * p.page_size + at % p.page_size) * hd;
                     float even = 0.0f, odd = 0.0f;
