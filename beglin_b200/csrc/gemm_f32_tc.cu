@@ -560,7 +560,7 @@ static int gt_piece(const GfParams& f, const GtPlan& g, int r0, int r1, cudaStre
     }
     const long long padded = (long long)p.tok_tiles * g.nt * f.batch;
     unsigned char *images = (unsigned char*)f.scratch, *odd = (unsigned char*)(f.scratch + padded * (r1 - r0) * (g.range_len * 3 / 2));
-    float* behind = f.scratch + gt_token_floats(g, padded, r1 - r0);
+    float* behind = f.scratch + gt_token_floats(g, padded, g.at_once);         // (the running sums stay in one place from launch to launch)
     p.images = images;
     p.odd = odd;
     p.feat_tiles = (f.N + GT_BM - 1) / GT_BM;

@@ -71,6 +71,19 @@ def test_tiles_of_all_sizes(ops, M, N, K):
         assert torch.equal(product(ops, a[m:m + 1].contiguous(), w, b)[0], out[m]), m
 
 
+@pytest.mark.parametrize("accumulate", [False, True])
+def test_ranges_in_several_launches(ops, accumulate):
+    """An inner size whose ranges take more than one launch, the last of fewer ranges than the first (146 of 960, 145 at a time).  Whole
+    numbers: every sum is exact."""
+    M, N, K = 160, 64, 140000
+    g = torch.Generator(device=DEV).manual_seed(12)
+    a, w = (torch.randint(-1, 2, (n, K), device=DEV, generator=g).float() for n in (M, N))
+    old = torch.randint(-99, 100, (M, N), device=DEV, generator=g).float()
+    out = old.clone()
+    ops.gemm_f32_nt(a, w, None, out, accumulate=accumulate)
+    assert torch.equal(out.double(), a.double() @ w.double().t() + (old.double() if accumulate else 0.0))
+
+
 @pytest.mark.parametrize("hd", [48, 80, 128])
 def test_attention_of_queries_without_three_parts(ops, hd):
     """Queries below 2^-110 against keys as large: scores of the usual size, every digit of them needed."""
