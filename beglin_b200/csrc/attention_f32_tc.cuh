@@ -278,6 +278,7 @@ __global__ void __launch_bounds__(AX_THREADS, 1) attention_f32_tc_kernel(P p) {
             // adds the tile's sums of values to the row's
             auto add_values = [&](int i, int t0, float corr) {
                 mbar_wait(&o_full, i & 1, &failed);
+                __syncwarp();
                 tc_fence_after();
                 const unsigned long long cc = pair2(corr, corr);
 #pragma unroll
@@ -300,6 +301,7 @@ __global__ void __launch_bounds__(AX_THREADS, 1) attention_f32_tc_kernel(P p) {
                 if (__any_sync(0xffffffffu, odd)) {    // values without three parts: the weights come back from their own
                     for (int j = 0; j < AX_KEYS; ++j) {
                         if (!value_odd[i & 3][j]) continue;
+                        __syncwarp();                  // (lanes come from the sums of the key before)
                         unsigned w[3];
 #pragma unroll
                         for (int e = 0; e < 3; ++e)
@@ -309,11 +311,12 @@ __global__ void __launch_bounds__(AX_THREADS, 1) attention_f32_tc_kernel(P p) {
 #pragma unroll
                         for (int e = 2; e >= 0; --e) f += __uint_as_float(j & 1 ? w[e] & 0xffff0000u : w[e] << 16);
                         const int page = page_s[i & 7][j];
-                        if (f == 0.0f || page < 0) continue;
-                        const float* src = pool + (size_t)page * page_elems + v_off + ((size_t)kvh * p.page_size + (t0 + j) % p.page_size) * vd + half * od;
+                        if (f != 0.0f && page >= 0) {
+                            const float* src = pool + (size_t)page * page_elems + v_off + ((size_t)kvh * p.page_size + (t0 + j) % p.page_size) * vd + half * od;
 #pragma unroll
-                        for (int d = 0; d < MOST; ++d)
-                            if (d < od && ax_odd(src[d])) out[d] = fmaf(f, src[d], out[d]);
+                            for (int d = 0; d < MOST; ++d)
+                                if (d < od && ax_odd(src[d])) out[d] = fmaf(f, src[d], out[d]);
+                        }
                     }
                 }
                 tc_fence_before();
@@ -323,6 +326,7 @@ __global__ void __launch_bounds__(AX_THREADS, 1) attention_f32_tc_kernel(P p) {
             int i = 0, t_before = 0;
             for (int t0 = t_first; t0 < k_end; ++i) {
                 mbar_wait(&s_full, i & 1, &failed);
+                __syncwarp();
                 tc_fence_after();
                 float w[32];
                 {
@@ -394,7 +398,10 @@ __global__ void __launch_bounds__(AX_THREADS, 1) attention_f32_tc_kernel(P p) {
                 sum = fmaf(sum, corr, s);
                 m = m_new;
                 if (i > 0) add_values(i - 1, t_before, corr_before);
-                else ax_rows_meet();                   // (as often as below)
+                // row_max is free again; and neither of a row's two threads puts weights where the other may still read those of the tile before
+                // (add_values, values without three parts)
+                ax_rows_meet();
+                tc_fence_after();
                 corr_before = corr;
                 // the weights' parts, where the values' products before have read theirs
                 unsigned none = 0;
@@ -410,7 +417,6 @@ __global__ void __launch_bounds__(AX_THREADS, 1) attention_f32_tc_kernel(P p) {
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&p_full);
-                if (i > 0) ax_rows_meet();             // (row_max is free again)
                 t_before = t0;
                 t0 = next_tile(t0);
             }

@@ -106,3 +106,42 @@ def test_attention_of_queries_without_three_parts(ops, hd):
         want = torch.softmax(s, -1) @ v
         # a score's error moves a weight by as much: hd + 8 roundings of the largest sum of products
         assert (out[:, h * hd:(h + 1) * hd].double() - want).abs().max() <= (hd + 8) * 2.0 ** -23 * float(s.abs()[s > -math.inf].max() + 1) * float(v.abs().max())
+
+
+def attend(ops, q, k, v, split=256, window=0, slopes=None, softcap=0.0, keep=0, page=16, scale=None):
+    """q [n, heads, features], k and v [n, kv heads, features]: a prompt's rows over themselves, one block table."""
+    n, nh, hd = q.shape
+    nkv, vd = v.shape[1], v.shape[2]
+    pages = -(-n // page)
+    pad = lambda t: torch.cat([t, torch.zeros((pages * page - n,) + t.shape[1:], device=DEV)]).view(pages, page, nkv, -1).transpose(1, 2).reshape(pages, -1)
+    pool = torch.cat([pad(k), pad(v)], dim=1)
+    if vd == hd:
+        pool = pool.view(pages, 2, nkv, page, hd)
+    pos, table = torch.arange(n, dtype=torch.int32, device=DEV), torch.arange(pages, dtype=torch.int32, device=DEV).view(1, -1)
+    _, bq, tile = ops.attention_plan(nh // nkv, hd, torch.float32, False, "generic", page, vd=vd)
+    blocks = torch.tensor([(0, r, min(bq, n - r)) for r in range(0, n, bq)], dtype=torch.int32, device=DEV)
+    out, status = torch.full((n, nh * vd), -7.0, device=DEV), ops.new_status(DEV)
+    ops.attention(q.reshape(n, -1), nh * hd, pool, table, pos, blocks, len(blocks), n - 1, n, nh, nkv, hd, window, split, tile, bq,
+                  hd ** -0.5 if scale is None else scale, out, status, "generic", softcap=softcap, vd=vd, keep=keep, slopes=slopes)
+    ops.raise_on_status(status)
+    return out.view(n, nh, vd)
+
+
+@pytest.mark.parametrize("nh,nkv,hd,vd,window,keep", [(6, 1, 128, 128, 0, 0), (2, 2, 64, 64, 40, 3), (3, 1, 80, 48, 100, 0)])
+@pytest.mark.parametrize("split", [64, 256, 1024])
+def test_attention_of_several_values_without_three_parts(ops, nh, nkv, hd, vd, window, keep, split):
+    """Infinities and NaN in both halves of tiles one behind the other: they reach the rows that see them, and the same ones each time."""
+    n, bad_at = 330, [3, 40, 61, 70, 97, 99, 127, 128, 200, 255, 256, 300]
+    q, k, v = rnd(n, nh, hd, seed=20), rnd(n, nkv, hd, seed=21), rnd(n, nkv, vd, seed=22)
+    v[bad_at, :, 1] = 0.25
+    fine = attend(ops, q, k, v, split, window, keep=keep)
+    for i, at in enumerate(bad_at):
+        v[at, :, 1] = (math.inf, math.nan, -math.inf)[i % 3]
+    pos = torch.arange(n, device=DEV)[:, None]
+    at = torch.tensor(bad_at, device=DEV)[None, :]
+    sees = ((at <= pos) & ((at > pos - window) if window else (at >= 0)) | ((at < keep) & (at <= pos))).any(1)
+    other = torch.arange(vd, device=DEV) != 1
+    for _ in range(8):
+        out = attend(ops, q, k, v, split, window, keep=keep)
+        assert torch.isfinite(fine).all() and torch.equal(out[~sees], fine[~sees]) and torch.equal(out[..., other], fine[..., other])
+        assert not torch.isfinite(out[sees][..., 1]).any()
