@@ -292,6 +292,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, GtParams p) {
                 for (int c = 0; c < AHEAD; ++c) cut(c, c);
                 if (g >= DA) {                                 // (the products of stage g - DA have read its parts)
                     mbar_wait(&a_empty[g % DA], (g / DA - 1) & 1, &failed);
+                    __syncwarp();
                     tc_fence_after();
                 }
 #pragma unroll
@@ -329,6 +330,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, GtParams p) {
             const bool first = e % STAGES == 0, last = (e + 1) % STAGES == 0 || e + 1 == n;
             const unsigned acc = sums + g % DS * NT;
             mbar_wait(&done[g % DS], (g / DS) & 1, &failed);
+            __syncwarp();                                      // (the loads of tensor memory want the whole warp: not all lanes store a range's sums)
             tc_fence_after();
             auto add = [&](int c, const unsigned* r, int count) {
 #pragma unroll
@@ -382,44 +384,46 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, GtParams p) {
                 }
                 gt_any<ADDERS>(false);
             }
-            if (feature >= p.N) continue;
-            const int rows = min(CG, p.M - t0 - group * CG);
-            const bool end = !p.part && range + 1 == p.ranges, sums_before = !p.part && range > 0, add_old = end && p.accumulate;
-            const size_t at = (size_t)(t0 + group * CG);
-            float* run = p.run + (size_t)b * p.batch_r + at * p.ldr + feature;
-            float* out = p.part ? p.part + (((size_t)range * p.batch + b) * p.M + at) * p.N + feature : end ? p.C + (size_t)b * p.batch_c + at * p.ldc + feature : run;
-            size_t step = p.part ? p.N : end ? p.ldc : p.ldr, step_r = p.ldr;
-            const float bias = end && p.bias ? p.bias[feature] : 0.0f;
+            if (feature < p.N) {
+                const int rows = min(CG, p.M - t0 - group * CG);
+                const bool end = !p.part && range + 1 == p.ranges, sums_before = !p.part && range > 0, add_old = end && p.accumulate;
+                const size_t at = (size_t)(t0 + group * CG);
+                float* run = p.run + (size_t)b * p.batch_r + at * p.ldr + feature;
+                float* out = p.part ? p.part + (((size_t)range * p.batch + b) * p.M + at) * p.N + feature : end ? p.C + (size_t)b * p.batch_c + at * p.ldc + feature : run;
+                size_t step = p.part ? p.N : end ? p.ldc : p.ldr, step_r = p.ldr;
+                const float bias = end && p.bias ? p.bias[feature] : 0.0f;
 #pragma unroll
-            for (int j0 = 0; j0 < CG; j0 += 8) {               // (eight loads on their way at a time)
-                asm volatile("" : "+l"(run), "+l"(out), "+l"(step), "+l"(step_r));         // (no address is made ahead and kept)
-                float y[8];
+                for (int j0 = 0; j0 < CG; j0 += 8) {           // (eight loads on their way at a time)
+                    asm volatile("" : "+l"(run), "+l"(out), "+l"(step), "+l"(step_r));         // (no address is made ahead and kept)
+                    float y[8];
 #pragma unroll
-                for (int j = 0; j < 8; ++j) y[j] = j & 1 ? high2(total[(j0 + j) / 2]) : low2(total[(j0 + j) / 2]);
-                if (sums_before) {
-                    float old[8];
+                    for (int j = 0; j < 8; ++j) y[j] = j & 1 ? high2(total[(j0 + j) / 2]) : low2(total[(j0 + j) / 2]);
+                    if (sums_before) {
+                        float old[8];
 #pragma unroll
-                    for (int j = 0; j < 8; ++j) old[j] = j0 + j < rows ? run[j * step_r] : 0.0f;
+                        for (int j = 0; j < 8; ++j) old[j] = j0 + j < rows ? run[j * step_r] : 0.0f;
 #pragma unroll
-                    for (int j = 0; j < 8; ++j) y[j] = old[j] + y[j];
+                        for (int j = 0; j < 8; ++j) y[j] = old[j] + y[j];
+                    }
+                    if (end && p.bias) {
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) y[j] += bias;
+                    }
+                    if (add_old) {
+                        float old[8];
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) old[j] = j0 + j < rows ? out[j * step] : 0.0f;
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) y[j] = old[j] + y[j];
+                    }
+#pragma unroll
+                    for (int j = 0; j < 8; ++j)
+                        if (j0 + j < rows) out[j * step] = y[j];
+                    run += 8 * step_r;
+                    out += 8 * step;
                 }
-                if (end && p.bias) {
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) y[j] += bias;
-                }
-                if (add_old) {
-                    float old[8];
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) old[j] = j0 + j < rows ? out[j * step] : 0.0f;
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) y[j] = old[j] + y[j];
-                }
-#pragma unroll
-                for (int j = 0; j < 8; ++j)
-                    if (j0 + j < rows) out[j * step] = y[j];
-                run += 8 * step_r;
-                out += 8 * step;
             }
+            __syncwarp();
           }
         }
     }

@@ -71,6 +71,16 @@ def test_tiles_of_all_sizes(ops, M, N, K):
         assert torch.equal(product(ops, a[m:m + 1].contiguous(), w, b)[0], out[m]), m
 
 
+@pytest.mark.parametrize("M", [5, 40, 100, 150])
+@pytest.mark.parametrize("N", [1, 15, 130, 203])
+def test_features_that_fill_no_warp(ops, M, N):
+    """Several ranges, walked and added, whose sums some lanes of a warp do not store: the same bits each time."""
+    a, w, b = rnd(M, 4000, seed=13), rnd(N, 4000, seed=14), rnd(N, seed=15)
+    out, want = product(ops, a, w, b), a.double() @ w.double().t() + b.double()
+    assert bool(((out.double() - want).abs() <= 4008 * 2.0 ** -24 * (a.abs().double() @ w.abs().double().t() + b.abs().double())).all())
+    assert all(torch.equal(product(ops, a, w, b), out) for _ in range(5))
+
+
 @pytest.mark.parametrize("accumulate", [False, True])
 def test_ranges_in_several_launches(ops, accumulate):
     """An inner size whose ranges take more than one launch, the last of fewer ranges than the first (146 of 960, 145 at a time).  Whole
