@@ -8,15 +8,16 @@
 // 32 keys each, make the weights and keep the row's sums of values in registers (a tile's sums leave tensor memory and are added in float).
 // Queries and weights are left operands in tensor memory.  The scores of a tile are multiplied while the weights of the one before are made,
 // its values while those of the one behind are.
-// 550 rows of 12 heads of 128 (2 kv heads) behind 1,500 positions: 82 us, 87 with one tile of keys and of values in shared memory, 120 with
+// 550 rows of 12 heads of 128 (2 kv heads) behind 1,500 positions: 79 us, 87 with one tile of keys and of values in shared memory, 120 with
 // all options in one unrolled loop and results stored a row a thread; the mixer of 550 rows over 1,536 to 3,000 held positions takes 179 us
 // with its products, 399 with the float units' attention and the same products.  What bounds it: a tile's some 8,000 cycles are a chain of
 // hand-overs and of instructions that are fetched once a tile (its MMAs take 3,072), on one CTA an SM.
 //
-// A row's arithmetic depends on nothing but its own keys: tiles and splits lie at absolute positions, and an MMA's rows do not meet.  What has no
-// three parts (infinite, not a number, below some 2^-110) is noticed where it is cut: scores of such queries or keys, and those that are
-// not finite, are summed by floats instead; such values go into the tile as nought and are added by floats to the rows whose weight for them
-// is not nought, so that an infinite one at a position that a row does not see does not reach it.
+// A row's arithmetic depends on nothing but its own keys: tiles and splits lie at absolute positions, and an MMA's rows do not meet.  Scores that
+// are not finite (an operand that is infinite or not a number, a query above 2^90) are summed by floats instead.  Values of 2^72 and more go into
+// the tile as nought and are added by floats to the rows whose weight for them is not nought, so that an infinite one at a position that a row
+// does not see does not reach it.  Small operands take the usual way (see AX_Q_UP): 550 rows with a key, a query or a value of 1e-36 in every eighth
+// row or less, 79 us; noticed where they are cut and summed by floats they took 940 to 980.
 #pragma once
 
 #include "float_parts.cuh"
@@ -28,17 +29,18 @@ constexpr int AX_NONE = -2147483647 - 1;               // no key here (not an en
 constexpr int AX_THREADS = 640;                        // two warpgroups of rows, two that cut, one with the warp that issues
 constexpr unsigned AX_BLOCK = AX_KEYS * 128, AX_PART = 2 * AX_BLOCK, AX_TILE = 3 * AX_PART;       // 64 keys x 64 features; x 128; three parts
 constexpr unsigned AX_Q = 0, AX_S = 192, AX_P = 256, AX_O = 352;                      // columns of tensor memory
-constexpr int AX_REGS = 96, AX_REGS_ROW = 152, AX_REGS_CUT = 64, AX_REGS_OTHER = 48;
+constexpr int AX_REGS = 96, AX_REGS_ROW = 144, AX_REGS_CUT = 72, AX_REGS_OTHER = 48;
 static_assert(2 * AX_REGS_ROW + 2 * AX_REGS_CUT + AX_REGS_OTHER <= 5 * AX_REGS);
 
 __host__ __device__ __forceinline__ bool ax_takes(int rows, int hd, int vd, int maps) {
     return maps == 1 && rows <= AX_ROWS && hd >= 48 && hd <= 128 && hd % 16 == 0 && vd >= 16 && vd <= 128 && vd % 16 == 0;
 }
-__device__ __forceinline__ bool ax_odd(float x) {      // no three parts
-    unsigned h, m, l, left = 0;
-    gt_split(pair2(x, 0.0f), h, m, l, left);
-    return (left & 0xffffu) != 0;
-}
+// Powers of two that queries, weights and values are cut with.  Every weight and value has exact parts then (the smallest bit of a float times
+// 2^24 is 2^-125), and so has every query below 2^90; larger ones have parts that are not numbers, which the scores show.  Keys are cut as they
+// are: what is lost of the smallest, below 2^-133, moves a score of smaller queries by less than 2^-36.
+constexpr float AX_Q_UP = 274877906944.0f, AX_PV_UP = 16777216.0f;     // 2^38, 2^24
+// Values that are added by floats: 64 of the others times their weights stay finite.
+__device__ __forceinline__ bool ax_large(float x) { return !(fabsf(x) < 4.722366e21f); }       // 2^72
 // all 256 threads of the rows meet
 __device__ __forceinline__ void ax_rows_meet() { asm volatile("barrier.cta.sync 1, 256;\n" ::: "memory"); }
 
@@ -53,7 +55,7 @@ __global__ void __launch_bounds__(AX_THREADS, 1) attention_f32_tc_kernel(P p) {
     __shared__ int failed;
     // of the last tiles, as many as cutting can be ahead of reading: pages of the keys, -1: none (asked for again when a tile's values have been summed), ..
     __shared__ int page_s[8][AX_KEYS];
-    __shared__ unsigned char key_odd[4][AX_KEYS], value_odd[4][AX_KEYS], row_odd[2][AX_ROWS];
+    __shared__ unsigned char value_large[4][AX_KEYS];
     __shared__ float row_max[2][AX_ROWS];
     __shared__ int row_at[AX_ROWS];                    // a row's place among the partial results, -1: none
 
@@ -176,58 +178,58 @@ __global__ void __launch_bounds__(AX_THREADS, 1) attention_f32_tc_kernel(P p) {
                     *reinterpret_cast<uint4*>(d + AX_PART) = m;
                     *reinterpret_cast<uint4*>(d + 2 * AX_PART) = l;
                 };
-                auto split8 = [&](const float4& a, const float4& b, uint4& h, uint4& m, uint4& l, unsigned& left) {
-                    gt_split(pair2(a.x, a.y), h.x, m.x, l.x, left);
-                    gt_split(pair2(a.z, a.w), h.y, m.y, l.y, left);
-                    gt_split(pair2(b.x, b.y), h.z, m.z, l.z, left);
-                    gt_split(pair2(b.z, b.w), h.w, m.w, l.w, left);
+                auto split8 = [&](const float4& a, const float4& b, uint4& h, uint4& m, uint4& l, float up) {
+                    gt_split(gt_up(pair2(a.x, a.y), up), h.x, m.x, l.x);
+                    gt_split(gt_up(pair2(a.z, a.w), up), h.y, m.y, l.y);
+                    gt_split(gt_up(pair2(b.x, b.y), up), h.z, m.z, l.z);
+                    gt_split(gt_up(pair2(b.z, b.w), up), h.w, m.w, l.w);
                 };
                 float4 v[8];
                 fetch(ks, hd, v);
                 const int t1 = next_tile(t0);
                 page_next = t1 < k_end ? page_of(t1) : AX_NONE;
                 if (i > 1) mbar_wait(&k_empty[i & 1], ((i >> 1) - 1) & 1, &failed);
-                unsigned left = 0;
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
                     uint4 h, m, l;
-                    split8(v[2 * j], v[2 * j + 1], h, m, l, left);
+                    split8(v[2 * j], v[2 * j + 1], h, m, l, 1.0f);
                     if ((c0 + 4 * j) * 8 < hd) store(kb, c0 + 4 * j, h, m, l);
                 }
-                left &= 0xffffu;
-                left |= __shfl_xor_sync(0xffffffffu, left, 1);
-                left |= __shfl_xor_sync(0xffffffffu, left, 2);
-                if (c0 == 0) { page_s[i & 7][key] = page; key_odd[i & 3][key] = left != 0; }
+                if (c0 == 0) page_s[i & 7][key] = page;
                 fence_proxy_async();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&k_full[i & 1]);
                 fetch(vs, vd, v);
                 if (i > 1) mbar_wait(&v_empty[i & 1], ((i >> 1) - 1) & 1, &failed);
-                left = 0;
+                unsigned long long squares = 0ull;     // not finite with a value of 2^64 and more
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    const unsigned long long a = pair2(v[j].x, v[j].y), b = pair2(v[j].z, v[j].w);
+                    squares = fma2(b, b, fma2(a, a, squares));
+                }
                 auto values = [&]() {
 #pragma unroll
                     for (int j = 0; j < 4; ++j) {
                         uint4 h, m, l;
-                        split8(v[2 * j], v[2 * j + 1], h, m, l, left);
+                        split8(v[2 * j], v[2 * j + 1], h, m, l, AX_PV_UP);
                         if ((c0 + 4 * j) * 8 < vd) store(vb, c0 + 4 * j, h, m, l);
                     }
                 };
                 values();
-                left &= 0xffffu;
-                if (left) {                            // what has no three parts is nought here
+                unsigned large = !(sum2(squares) <= 3.402823466e38f);
+                large |= __shfl_xor_sync(0xffffffffu, large, 1);
+                large |= __shfl_xor_sync(0xffffffffu, large, 2);
+                if (large) {                           // large values are nought here
 #pragma unroll
                     for (int j = 0; j < 8; ++j) {
-                        if (ax_odd(v[j].x)) v[j].x = 0.0f;
-                        if (ax_odd(v[j].y)) v[j].y = 0.0f;
-                        if (ax_odd(v[j].z)) v[j].z = 0.0f;
-                        if (ax_odd(v[j].w)) v[j].w = 0.0f;
+                        if (ax_large(v[j].x)) v[j].x = 0.0f;
+                        if (ax_large(v[j].y)) v[j].y = 0.0f;
+                        if (ax_large(v[j].z)) v[j].z = 0.0f;
+                        if (ax_large(v[j].w)) v[j].w = 0.0f;
                     }
                     values();
-                    left = 1;
                 }
-                left |= __shfl_xor_sync(0xffffffffu, left, 1);
-                left |= __shfl_xor_sync(0xffffffffu, left, 2);
-                if (c0 == 0) value_odd[i & 3][key] = left != 0;
+                if (c0 == 0) value_large[i & 3][key] = large != 0;
                 fence_proxy_async();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&v_full[i & 1]);
@@ -243,7 +245,7 @@ __global__ void __launch_bounds__(AX_THREADS, 1) attention_f32_tc_kernel(P p) {
         const int qi = in ? row / group : 0, head = kvh * group + (in ? row - qi * group : 0);
         const int pos = in ? p.positions[row0 + qi] : -1, lo = first_visible(pos < 0 ? 0 : pos, p.window);
         const float* q = (const float*)p.q + (size_t)(row0 + qi) * p.q_stride + (size_t)head * hd;
-        const float slope = p.slopes && in ? p.slopes[head] : 0.0f;
+        const float slope = p.slopes && in ? p.slopes[head] : 0.0f, scale_down = p.scale / AX_Q_UP;
         const int od = OD ? OD : vd / 2;               // output features of a thread, a multiple of 8
         constexpr int MOST = OD ? OD : 64;
         float out[MOST];
@@ -252,7 +254,6 @@ __global__ void __launch_bounds__(AX_THREADS, 1) attention_f32_tc_kernel(P p) {
         for (int d = 0; d < MOST; ++d) out[d] = 0.0f;
         if (seen && t_first < k_end) {
             // the row's queries, half of their features a thread
-            unsigned left = 0;
             float4 x[16];                              // (all on their way together)
 #pragma unroll
             for (int c = 0; c < 16; ++c) x[c] = in && c * 4 < hd / 2 ? *reinterpret_cast<const float4*>(q + half * (hd / 2) + c * 4) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
@@ -260,27 +261,24 @@ __global__ void __launch_bounds__(AX_THREADS, 1) attention_f32_tc_kernel(P p) {
             for (int c = 0; c < 8; ++c) {
                 if (c * 8 >= hd / 2) break;
                 unsigned h[4], mm[4], l[4];
-                gt_split(pair2(x[2 * c].x, x[2 * c].y), h[0], mm[0], l[0], left);
-                gt_split(pair2(x[2 * c].z, x[2 * c].w), h[1], mm[1], l[1], left);
-                gt_split(pair2(x[2 * c + 1].x, x[2 * c + 1].y), h[2], mm[2], l[2], left);
-                gt_split(pair2(x[2 * c + 1].z, x[2 * c + 1].w), h[3], mm[3], l[3], left);
+                gt_split(gt_up(pair2(x[2 * c].x, x[2 * c].y), AX_Q_UP), h[0], mm[0], l[0]);
+                gt_split(gt_up(pair2(x[2 * c].z, x[2 * c].w), AX_Q_UP), h[1], mm[1], l[1]);
+                gt_split(gt_up(pair2(x[2 * c + 1].x, x[2 * c + 1].y), AX_Q_UP), h[2], mm[2], l[2]);
+                gt_split(gt_up(pair2(x[2 * c + 1].z, x[2 * c + 1].w), AX_Q_UP), h[3], mm[3], l[3]);
                 const unsigned a = lanes + AX_Q + half * (hd / 4) + c * 4;
                 gt_st4(a, h); gt_st4(a + 64, mm); gt_st4(a + 128, l);
             }
-            row_odd[half][row] = (left & 0xffffu) != 0;
             tc_wait_st();
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(&q_full);
-            ax_rows_meet();
-            const bool q_odd = row_odd[0][row] || row_odd[1][row];
             float corr_before = 0.0f;                  // of the tile whose values are still being summed
             // adds the tile's sums of values to the row's
             auto add_values = [&](int i, int t0, float corr) {
                 mbar_wait(&o_full, i & 1, &failed);
                 __syncwarp();
                 tc_fence_after();
-                const unsigned long long cc = pair2(corr, corr);
+                const unsigned long long cc = pair2(corr, corr), down = pair2(1.0f / AX_PV_UP / AX_PV_UP, 1.0f / AX_PV_UP / AX_PV_UP);
 #pragma unroll
                 for (int c = 0; c < MOST; c += 16) {
                     if (!OD && c >= od) break;
@@ -291,16 +289,16 @@ __global__ void __launch_bounds__(AX_THREADS, 1) attention_f32_tc_kernel(P p) {
 #pragma unroll
                     for (int e = 0; e < 16; e += 2)
                         if (OD || c + e < od) {
-                            const unsigned long long y = fma2(pair2(out[c + e], out[c + e + 1]), cc, (unsigned long long)r[e] | ((unsigned long long)r[e + 1] << 32));
+                            const unsigned long long y = fma2(pair2(out[c + e], out[c + e + 1]), cc, fma2((unsigned long long)r[e] | ((unsigned long long)r[e + 1] << 32), down, 0ull));
                             out[c + e] = low2(y); out[c + e + 1] = high2(y);
                         }
                 }
-                bool odd = false;
+                bool large = false;
 #pragma unroll
-                for (int j = 0; j < 2; ++j) odd |= value_odd[i & 3][j * 32 + lane] != 0;
-                if (__any_sync(0xffffffffu, odd)) {    // values without three parts: the weights come back from their own
+                for (int j = 0; j < 2; ++j) large |= value_large[i & 3][j * 32 + lane] != 0;
+                if (__any_sync(0xffffffffu, large)) {  // the weights come back from their parts
                     for (int j = 0; j < AX_KEYS; ++j) {
-                        if (!value_odd[i & 3][j]) continue;
+                        if (!value_large[i & 3][j]) continue;
                         __syncwarp();                  // (lanes come from the sums of the key before)
                         unsigned w[3];
 #pragma unroll
@@ -310,12 +308,13 @@ __global__ void __launch_bounds__(AX_THREADS, 1) attention_f32_tc_kernel(P p) {
                         float f = 0.0f;
 #pragma unroll
                         for (int e = 2; e >= 0; --e) f += __uint_as_float(j & 1 ? w[e] & 0xffff0000u : w[e] << 16);
+                        f *= 1.0f / AX_PV_UP;
                         const int page = page_s[i & 7][j];
                         if (f != 0.0f && page >= 0) {
                             const float* src = pool + (size_t)page * page_elems + v_off + ((size_t)kvh * p.page_size + (t0 + j) % p.page_size) * vd + half * od;
 #pragma unroll
                             for (int d = 0; d < MOST; ++d)
-                                if (d < od && ax_odd(src[d])) out[d] = fmaf(f, src[d], out[d]);
+                                if (d < od && ax_large(src[d])) out[d] = fmaf(f, src[d], out[d]);
                         }
                     }
                 }
@@ -340,8 +339,7 @@ __global__ void __launch_bounds__(AX_THREADS, 1) attention_f32_tc_kernel(P p) {
                 const int base = t0 + half * 32, last = min(pos, k_end - 1) - base;
                 auto below = [](int n) { return n <= 0 ? 0u : n >= 32 ? 0xffffffffu : (1u << n) - 1; };       // bits 0 .. n - 1
                 unsigned visible = __ballot_sync(0xffffffffu, page_s[i & 7][half * 32 + lane] >= 0) & below(last + 1) & (~below(lo - base) | below(p.keep - base));
-                unsigned bad = __ballot_sync(0xffffffffu, key_odd[i & 3][half * 32 + lane] != 0);
-                if (q_odd) bad = 0xffffffffu;
+                unsigned bad = 0;
                 float nought = 0.0f;
 #pragma unroll
                 for (int j = 0; j < 32; ++j) nought = fmaf(w[j], 0.0f, nought);
@@ -350,6 +348,8 @@ __global__ void __launch_bounds__(AX_THREADS, 1) attention_f32_tc_kernel(P p) {
                     for (int j = 0; j < 32; ++j)
                         if (!(fabsf(w[j]) <= 3.402823466e38f)) bad |= 1u << j;
                 }
+#pragma unroll
+                for (int j = 0; j < 32; ++j) w[j] *= scale_down;
                 bad &= visible;
                 while (bad) {
                     const int jb = __ffs(bad) - 1, at = t0 + half * 32 + jb, page = page_s[i & 7][half * 32 + jb];
@@ -357,7 +357,7 @@ __global__ void __launch_bounds__(AX_THREADS, 1) attention_f32_tc_kernel(P p) {
                     const float* src = pool + (size_t)page * page_elems + ((size_t)kvh * p.page_size + at % p.page_size) * hd;
                     float even = 0.0f, odd = 0.0f;
                     for (int d = 0; d < hd; d += 2) { even = fmaf(q[d], src[d], even); odd = fmaf(q[d + 1], src[d + 1], odd); }
-                    even += odd;
+                    even = (even + odd) * p.scale;
 #pragma unroll
                     for (int j = 0; j < 32; ++j)
                         if (j == jb) w[j] = even;
@@ -369,13 +369,9 @@ __global__ void __launch_bounds__(AX_THREADS, 1) attention_f32_tc_kernel(P p) {
                 if (p.softcap > 0.0f || p.slopes) {
 #pragma unroll
                     for (int j = 0; j < 32; ++j) {
-                        w[j] *= p.scale;
                         if (p.softcap > 0.0f) w[j] = p.softcap * tanhf(w[j] / p.softcap);
                         if (p.slopes) w[j] = fmaf(-slope, (float)(pos - (base + j)), w[j]);
                     }
-                } else {
-#pragma unroll
-                    for (int j = 0; j < 32; ++j) w[j] *= p.scale;
                 }
                 if (!__all_sync(0xffffffffu, visible == 0xffffffffu)) {
 #pragma unroll
@@ -404,12 +400,11 @@ __global__ void __launch_bounds__(AX_THREADS, 1) attention_f32_tc_kernel(P p) {
                 tc_fence_after();
                 corr_before = corr;
                 // the weights' parts, where the values' products before have read theirs
-                unsigned none = 0;
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {
                     unsigned h[4], mm[4], l[4];
 #pragma unroll
-                    for (int e = 0; e < 4; ++e) gt_split(pair2(w[8 * c + 2 * e], w[8 * c + 2 * e + 1]), h[e], mm[e], l[e], none);
+                    for (int e = 0; e < 4; ++e) gt_split(gt_up(pair2(w[8 * c + 2 * e], w[8 * c + 2 * e + 1]), AX_PV_UP), h[e], mm[e], l[e]);
                     const unsigned a = lanes + AX_P + half * 16 + 4 * c;
                     gt_st4(a, h); gt_st4(a + 32, mm); gt_st4(a + 64, l);
                 }

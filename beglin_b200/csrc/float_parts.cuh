@@ -26,6 +26,13 @@ __device__ __forceinline__ void gt_split(unsigned long long v, unsigned& h, unsi
     l = __byte_perm((unsigned)q, (unsigned)(q >> 32), 0x7632);
     odd |= (unsigned)q | (unsigned)(q >> 32);
 }
+// The same where what is left over is told otherwise, or is no matter.
+__device__ __forceinline__ void gt_split(unsigned long long v, unsigned& h, unsigned& m, unsigned& l) {
+    unsigned odd = 0;
+    gt_split(v, h, m, l, odd);
+}
+// Both floats times a power of two (one by one: packed, the multiplication makes the kernels around it slower by a tenth).
+__device__ __forceinline__ unsigned long long gt_up(unsigned long long v, float up) { return pair2(low2(v) * up, high2(v) * up); }
 __device__ __forceinline__ unsigned long long gt_add2(unsigned long long a, unsigned long long b) {
     unsigned long long d;
     asm("add.rn.f32x2 %0, %1, %2;\n" : "=l"(d) : "l"(a), "l"(b));

@@ -155,3 +155,44 @@ def test_attention_of_several_values_without_three_parts(ops, nh, nkv, hd, vd, w
         out = attend(ops, q, k, v, split, window, keep=keep)
         assert torch.isfinite(fine).all() and torch.equal(out[~sees], fine[~sees]) and torch.equal(out[..., other], fine[..., other])
         assert not torch.isfinite(out[sees][..., 1]).any()
+
+
+@pytest.mark.parametrize("size", [1e20, 1e36])
+@pytest.mark.parametrize("hd", [64, 128])
+def test_attention_of_small_weights_beside_large_values(ops, hd, size):
+    """Weights down to the smallest float, which large values make count: a key's share is off by a few roundings of the weight."""
+    n = 50
+    q, k, v = torch.zeros((n, 1, hd), device=DEV), torch.zeros((n, 1, hd), device=DEV), rnd(n, 1, hd, seed=30) * size
+    away = torch.linspace(70, 103, n, device=DEV).mul(8).round().div(8)
+    away[0], v[0] = 0.0, 0.0
+    q[:, :, 0], k[:, 0, 0] = 1.0, -8.0 * away
+    out = attend(ops, q, k, v, scale=0.125)[-1, 0].double()
+    w = torch.exp(-away.double())
+    bound = (w * 2.0 ** -21 + 2.0 ** -149) @ v[:, 0].abs().double() + n * 2.0 ** -24 * (w @ v[:, 0].abs().double())
+    assert bool(((out * w.sum() - w @ v[:, 0].double()).abs() <= bound).all())
+    v[40, 0, 5] = math.inf                                 # a weight of some 1e-42 is not nought
+    out = attend(ops, q, k, v, scale=0.125)
+    assert away[40] > 96 and torch.isinf(out[40:, 0, 5]).all() and torch.isfinite(out[:40]).all()
+
+
+@pytest.mark.parametrize("hd", [48, 80, 128])
+def test_attention_of_small_operands(ops, hd):
+    """Powers of two that go from the queries to the keys change no bit, however small the queries get; small keys and values keep theirs."""
+    q, k, v = rnd(150, 4, hd, seed=31), rnd(150, 2, hd, seed=32), rnd(150, 2, hd, seed=33)
+    out = attend(ops, q, k, v)
+    assert torch.equal(attend(ops, q * 2.0 ** -95, k * 2.0 ** 95, v), out)
+    s = torch.einsum("thd,shd->hts", q.double(), k.double().repeat_interleave(2, 1)) * hd ** -0.5
+    s = s.masked_fill(torch.ones(150, 150, dtype=torch.bool, device=DEV).triu(1), -math.inf)
+    want = torch.einsum("hts,shd->thd", torch.softmax(s, -1), v.double().repeat_interleave(2, 1))
+    # a score's error moves a weight by as much: hd + 8 roundings of the largest sum of products
+    bound = (hd + 8) * 2.0 ** -23 * float(s.abs()[s > -math.inf].max() + 1) * float(v.abs().max())
+    for power in (80, 95, 120):                            # (queries below and above 2^90)
+        kk = k * 2.0 ** -power
+        exact = (kk * 2.0 ** power).double()               # (what is left of keys below the smallest normal float)
+        s2 = torch.einsum("thd,shd->hts", q.double(), exact.repeat_interleave(2, 1)) * hd ** -0.5
+        want2 = torch.einsum("hts,shd->thd", torch.softmax(s2.masked_fill(s == -math.inf, -math.inf), -1), v.double().repeat_interleave(2, 1))
+        assert (attend(ops, q * 2.0 ** power, kk, v).double() - want2).abs().max() <= bound, power
+    small = attend(ops, q, k, v * 2.0 ** -100).double() * 2.0 ** 100
+    assert (small - want).abs().max() <= bound
+    top = attend(ops, q, k, v * 2.0 ** 100).double() * 2.0 ** -100
+    assert (top - want).abs().max() <= bound
