@@ -10,9 +10,11 @@
 // same bits.  Error against 64 bits (2-norm, normal operands): 1.0e-7 for K of 1,536 and 1.3e-7 for 9,000, where two chains of float
 // multiply-adds over 1,024 of k had 3.7e-7 and 4.1e-7; 0.9e-7 for K of 200 (1.8e-7).
 //
-// An operand that has no three parts (infinite, not a number, next to the largest float, or below some 2^-110) is noticed where it is cut;
-// the outputs of its row and range, and those whose sum is not finite, are summed by floats in two chains (even and odd k) instead, which
-// makes of them what floats make.  That, too, depends on the output's own row and column only.
+// Operands are cut times 2^24 (GT_UP) and sums are scaled back, so that small ones keep their parts.  A range's sum that is not finite (an operand
+// that is infinite, not a number or above some 2^103, or a sum above some 2^80) is made by floats instead, in two chains (even and odd k), which makes of
+// it what floats make.  That, too, depends on the output's own row and column only.  550 x 1,536 with k of 8,960: 103 us, with an infinity in one
+// row 180, with NaN in every row 2,510.  (Small operands noticed where they are cut and summed by floats: 1,900 us with one weight of 1e-36, 510 with one
+// in a row of tokens, 30,000 with one in every row.)
 //
 // The weights' rows are the M side (128 a CTA), so a lane of tensor memory is an output feature and results leave in rows of 128 bytes;
 // the tokens are the N side (NT = 16 to 160).  Weights come as floats (TMA, two boxes of 128 rows x 32 of k a stage); a warpgroup or
@@ -21,9 +23,9 @@
 // (the weights' tiles would each make them again).  Other warpgroups add up the stages' sums.
 //
 // What bounds it: with 144 and 160 tokens the tensor cores (a stage of 160 tokens takes 1,980 cycles, its MMAs 1,920; with 32 of k a stage, one
-// warp that issued and one set of warps that cut and added it was 5,000), with fewer the instructions of the cut (some 12 a value: 1,600
-// cycles a stage, weights at 4 TB/s for 8 rows).  In us, the float units' kernels in brackets: 550 x 17,920 with k of 1,536 142 (930),
-// 550 x 1,536 with 8,960 99 (498), 64 x 17,920 with 1,536 33 (116), 8 x 17,920 27 (32), 1 x 2,048 with 768 8.1 (13.3).
+// warp that issued and one set of warps that cut and added it was 5,000), with fewer the instructions of the cut (some 12 a value:
+// weights at 4.6 TB/s for 8 rows).  In us, the float units' kernels in brackets: 550 x 17,920 with k of 1,536 142 (930),
+// 550 x 1,536 with 8,960 99 (498), 64 x 17,920 with 1,536 33 (116), 8 x 17,920 24 (32), 1 x 2,048 with 768 8.1 (13.3).
 #include "gemm_f32.cuh"
 #include "float_parts.cuh"
 
@@ -31,7 +33,9 @@ namespace bg {
 
 constexpr int GT_BM = 128, GT_BK = 64;     // output features of a CTA; k of a stage
 constexpr unsigned GT_W_BYTES = GT_BM * GT_BK * 4;
-constexpr int GT_RING = 8;                 // entries of the operands' marks, by range: cutting is at most DA + DS + 1 stages ahead of adding
+// Tokens and weights are cut times 2^24: no float is so small then that its parts are not exact (the smallest bit of any is 2^-125); what is
+// infinite, not a number or above some 2^103 has parts that are not numbers, which every sum that they enter shows.
+constexpr float GT_UP = 16777216.0f;
 constexpr long long GT_SCRATCH = 32 << 20; // floats that a call's scratch may take
 // Warpgroups: those that cut the weights, those that add the stages' sums, one for copies, MMAs and tokens.
 constexpr int gt_threads(int gc, int gd) { return (gc + gd + 1) * 128; }
@@ -41,18 +45,16 @@ struct GtParams {
     float* part;                           // [ranges][batch][M][N]: a CTA has one range and leaves its sums here; or null: it walks them all
     float* run;                            // where a walk keeps the ranges' sum so far, [batch][M] rows of ldr
     const unsigned char* images;           // the tokens' parts (gf_parts_kernel)
-    const unsigned char* odd;              // [batch][tokens of all tiles]: rows with an operand that has no three parts
     long long batch_a, batch_w, batch_c, batch_r;
     int lda, ldw, ldc, ldr, M, N, K, accumulate, range_len, ranges, r0, r1, batch, tok_tiles, feat_tiles, units, map_batch;      // (ranges: of all k; r0 to r1: of this launch)
     unsigned* status;
 };
 
 // The tokens' parts as the images of the stages' right operands, [batch][tile of nt tokens][stage][part][token][64 of k] with the swizzle of
-// shared memory, noughts behind the last token and behind K; and whether a row has an operand without three parts.  One part of a stage is
-// then one copy of contiguous bytes: boxes of a tensor map, 64 bytes a row, took the copy engine 2.4 cycles a row, 1,750 for 32 of k of 192 tokens.
+// shared memory, noughts behind the last token and behind K.  One part of a stage is then one copy of contiguous bytes: boxes of a tensor map, 64 bytes a row, took the copy engine 2.4 cycles a row, 1,750 for 32 of k of 192 tokens.
 // A CTA per row, a warp per 512 of k, 16 values a lane.
 template <bool VEC>
-__global__ void __launch_bounds__(256) gf_parts_kernel(GtParams p, unsigned char* images, unsigned char* odd, int nt) {
+__global__ void __launch_bounds__(256) gf_parts_kernel(GtParams p, unsigned char* images, int nt) {
     pdl_launch();
     const int padded = p.tok_tiles * nt, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int k_first = p.r0 * p.range_len, k_all = min(p.K, p.r1 * p.range_len) - k_first, stages = (k_all + GT_BK - 1) / GT_BK;
@@ -60,7 +62,6 @@ __global__ void __launch_bounds__(256) gf_parts_kernel(GtParams p, unsigned char
     const float* src = p.A + (size_t)b * p.batch_a + (size_t)m * p.lda + k_first;
     unsigned char* tile = images + ((size_t)b * p.tok_tiles + m / nt) * stages * 3 * nt * 128 + in * 128 + (((lane >> 1 & 7) ^ (in & 7)) << 4) + (lane & 1) * 8;
     pdl_wait();
-    unsigned left = 0;
     for (int k0 = warp * 512; k0 < stages * GT_BK; k0 += blockDim.x / 32 * 512) {
         float4 v[4];
 #pragma unroll
@@ -73,8 +74,8 @@ __global__ void __launch_bounds__(256) gf_parts_kernel(GtParams p, unsigned char
         for (int i = 0; i < 4; ++i) {
             const int stage = (k0 + i * 128) / GT_BK + (lane >> 4);
             uint2 h, q, l;
-            gt_split(pair2(v[i].x, v[i].y), h.x, q.x, l.x, left);
-            gt_split(pair2(v[i].z, v[i].w), h.y, q.y, l.y, left);
+            gt_split(gt_up(pair2(v[i].x, v[i].y), GT_UP), h.x, q.x, l.x);
+            gt_split(gt_up(pair2(v[i].z, v[i].w), GT_UP), h.y, q.y, l.y);
             if (stage < stages) {
                 unsigned char* d = tile + (size_t)stage * 3 * nt * 128;
                 *reinterpret_cast<uint2*>(d) = h;
@@ -83,8 +84,6 @@ __global__ void __launch_bounds__(256) gf_parts_kernel(GtParams p, unsigned char
             }
         }
     }
-    const int any = __syncthreads_or((left & 0xffffu) != 0);
-    if (threadIdx.x == 0) odd[blockIdx.x] = any != 0;
 }
 
 // `bytes` contiguous ones (a multiple of 16, both sides on 16 bytes)
@@ -96,22 +95,21 @@ __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, i
     asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];\n"
                  ::"r"(smem_u32(dst)), "l"(map), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar)) : "memory");
 }
-// Whether any of the THREADS that add says so; they all meet.
-template <int THREADS>
-__device__ __forceinline__ bool gt_any(bool mine) {
-    unsigned r;
-    asm volatile("{\n .reg .pred p, q;\n setp.ne.u32 p, %1, 0;\n barrier.cta.red.or.pred q, 1, %2, p;\n selp.u32 %0, 1, 0, q;\n}\n"
-                 : "=r"(r) : "r"(mine ? 1u : 0u), "n"(THREADS) : "memory");
-    return r != 0;
-}
-
-// Two chains of multiply-adds over n of k, and their sum.
+// Two chains of multiply-adds over n of k (the even and the odd ones), and their sum.
 __device__ __forceinline__ float gt_chain(const float* a, const float* w, int n) {
-    float even = 0.0f, odd = 0.0f;
+    unsigned long long sum = 0ull;
     int k = 0;
-    for (; k + 1 < n; k += 2) { even = fmaf(a[k], w[k], even); odd = fmaf(a[k + 1], w[k + 1], odd); }
-    if (k < n) even = fmaf(a[k], w[k], even);
-    return even + odd;
+    if ((((uintptr_t)a | (uintptr_t)w) & 15) == 0) {
+#pragma unroll 8
+        for (; k + 3 < n; k += 4) {
+            const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(a + k), y = *reinterpret_cast<const ulonglong2*>(w + k);
+            sum = fma2(x.y, y.y, fma2(x.x, y.x, sum));
+        }
+    }
+#pragma unroll 8
+    for (; k + 1 < n; k += 2) sum = fma2(pair2(a[k], a[k + 1]), pair2(w[k], w[k + 1]), sum);
+    if (k < n) sum = fma2(pair2(a[k], 0.0f), pair2(w[k], 0.0f), sum);
+    return sum2(sum);
 }
 
 // What a form of the kernel takes: tokens NT; warpgroups that cut (GC: 64 / GC of a stage's k each) and that add (GD: NT / GD columns each);
@@ -137,7 +135,6 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, GtParams p) {
     __shared__ __align__(8) unsigned long long w_full[WS], w_empty[WS], b_full[BS * 3], b_empty[BS * 3], a_full[DA], a_empty[DA], done[DS], sum_empty[DS];
     __shared__ unsigned tmem_sh;
     __shared__ int failed;
-    __shared__ unsigned char row_odd[GT_RING][GC][GT_BM], tok_odd[NT];
 
     constexpr int W_WARP = 4 * (GC + GD), MMA_WARP = W_WARP + 1, TOKEN_WARP = W_WARP + 2;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, STAGES = p.range_len / GT_BK;
@@ -255,7 +252,6 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, GtParams p) {
         const int quarter = warp & 3, group = warp >> 2, row = quarter * 32 + lane;
         const unsigned parts = tmem + ((unsigned)(quarter * 32) << 16) + PARTS0 + group * (KG / 2);
         unsigned long long v[KG / 2];
-        unsigned left = 0;
         auto fetch = [&](int g) {
             mbar_wait(&w_full[g % WS], (g / WS) & 1, &failed);
             const unsigned char* src = wt + (g % WS) * GT_W_BYTES + group * KG / 32 * (GT_W_BYTES / 2) + row * 128;
@@ -267,7 +263,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, GtParams p) {
         };
         if (DIRECT && NT > 16) pdl_wait();
         if (!DIRECT && (int)blockIdx.x < p.units) fetch(0);
-        for (int u = blockIdx.x, g = 0, ring = 0; u < p.units; u += gridDim.x) {
+        for (int u = blockIdx.x, g = 0; u < p.units; u += gridDim.x) {
             const Unit x = unit_of(u);
 #pragma unroll 1
             for (int s = 0; s < x.n; ++s, ++g) {
@@ -284,7 +280,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, GtParams p) {
                 unsigned h[AHEAD][4], m[AHEAD][4], l[AHEAD][4];
                 auto cut = [&](int c, int to) {
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) gt_split(v[4 * c + i], h[to][i], m[to][i], l[to][i], left);
+                    for (int i = 0; i < 4; ++i) gt_split(gt_up(v[4 * c + i], GT_UP), h[to][i], m[to][i], l[to][i]);
                 };
                 const unsigned a = parts + g % DA * 96;
                 auto put = [&](int c, int from) { gt_st4(a + 4 * c, h[from]); gt_st4(a + 32 + 4 * c, m[from]); gt_st4(a + 64 + 4 * c, l[from]); };
@@ -302,11 +298,6 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, GtParams p) {
                 __syncwarp();
                 if (lane == 0 && !DIRECT) mbar_arrive(&w_empty[g % WS]);
                 const bool more = s + 1 < x.n;
-                if ((s + 1) % STAGES == 0 || !more) {
-                    row_odd[ring % GT_RING][group][row] = (left & 0xffffu) != 0;
-                    left = 0;
-                    ++ring;
-                }
                 tc_wait_st();
                 tc_fence_before();
                 __syncwarp();
@@ -317,14 +308,13 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, GtParams p) {
     } else if (warp < W_WARP) {
         // ---------------- the stages' sums
         gt_regs<F::REGS, F::RD>();
-        const int quarter = warp & 3, group = (warp >> 2) - GC, row = quarter * 32 + lane, adder = threadIdx.x - 128 * GC;
+        const int quarter = warp & 3, group = (warp >> 2) - GC, row = quarter * 32 + lane;
         const unsigned sums = tmem + ((unsigned)(quarter * 32) << 16) + group * CG;
         unsigned long long total[CG / 2];
         pdl_wait();
-        for (int u = blockIdx.x, g = 0, ring = 0; u < p.units; u += gridDim.x) {
+        for (int u = blockIdx.x, g = 0; u < p.units; u += gridDim.x) {
           const Unit x = unit_of(u);
           const int t0 = x.t0, b = x.b, n = x.n, feature = x.n0 + row;
-          const bool t_odd = adder < NT && p.odd[(size_t)b * p.tok_tiles * NT + t0 + adder] != 0;
 #pragma unroll 1
           for (int e = 0; e < n; ++e, ++g) {
             const bool first = e % STAGES == 0, last = (e + 1) % STAGES == 0 || e + 1 == n;
@@ -356,16 +346,14 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, GtParams p) {
             if (!last) continue;
             // ---- the sums of a range
             const int range = x.range + e / STAGES;
-            const int slot = ring++ % GT_RING;
-            bool w_odd = false;
-#pragma unroll
-            for (int c = 0; c < GC; ++c) w_odd |= row_odd[slot][c][row] != 0;
             unsigned long long nought = 0ull;                  // not nought if a sum is not finite
 #pragma unroll
-            for (int j = 0; j < CG / 2; ++j) nought = fma2(total[j], 0ull, nought);
-            if (gt_any<ADDERS>(w_odd || t_odd || !(sum2(nought) == 0.0f) || *(volatile int*)&failed)) {
-                if (adder < NT) tok_odd[adder] = t_odd;
-                gt_any<ADDERS>(false);
+            for (int j = 0; j < CG / 2; ++j) {
+                nought = fma2(total[j], 0ull, nought);
+                total[j] = gt_up(total[j], 1.0f / GT_UP / GT_UP);
+            }
+            const bool lost = *(volatile int*)&failed != 0;    // (a wait ran out)
+            if (!(sum2(nought) == 0.0f) || lost) {
                 const int kr = range * p.range_len, nr = min(p.K - kr, p.range_len);
                 const float* w_row = p.W + (size_t)b * p.batch_w + (size_t)(feature < p.N ? feature : 0) * p.ldw;
 #pragma unroll 1
@@ -375,14 +363,12 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, GtParams p) {
                     float y = 0.0f;
 #pragma unroll
                     for (int j = 0; j < CG; ++j) y = j == c ? (j & 1 ? high2(total[j / 2]) : low2(total[j / 2])) : y;
-                    if (feature < p.N && (w_odd || tok_odd[group * CG + c] || !(fabsf(y) <= 3.402823466e38f)))
-                        y = gt_chain(p.A + (size_t)b * p.batch_a + (size_t)t * p.lda + kr, w_row + kr, nr);
-                    if (*(volatile int*)&failed) y = __uint_as_float(0x7fffffffu);         // (a wait ran out)
+                    if (feature < p.N && !(fabsf(y) <= 3.402823466e38f)) y = gt_chain(p.A + (size_t)b * p.batch_a + (size_t)t * p.lda + kr, w_row + kr, nr);
+                    if (lost) y = __uint_as_float(0x7fffffffu);
 #pragma unroll
                     for (int j = 0; j < CG; ++j)
                         if (j == c) total[j / 2] = j & 1 ? pair2(low2(total[j / 2]), y) : pair2(y, high2(total[j / 2]));
                 }
-                gt_any<ADDERS>(false);
             }
             if (feature < p.N) {
                 const int rows = min(CG, p.M - t0 - group * CG);
@@ -497,8 +483,8 @@ static GtPlan gt_plan(int M, int N, int K, int batch) {
         }
     }
     const long long part = (long long)g.ranges * N, all = (M + g.nt - 1) / g.nt * (long long)g.nt, token = (long long)g.range_len * 3 / 2;
-    if (g.cut && all * (token * g.ranges + 1) + M * part > GT_SCRATCH) g.cut = false;
-    const long long each = all * (token * g.ranges + 1) + (g.cut ? M * part : 0), tile = g.nt * (token * g.ranges + 1);
+    if (g.cut && all * token * g.ranges + M * part > GT_SCRATCH) g.cut = false;
+    const long long each = all * token * g.ranges + (g.cut ? M * part : 0), tile = g.nt * token * g.ranges;
     g.rows = M;
     g.batches = batch;
     if (each > GT_SCRATCH) {                               // (never a cut one: the tokens' parts)
@@ -506,13 +492,13 @@ static GtPlan gt_plan(int M, int N, int K, int batch) {
         g.rows = (int)(GT_SCRATCH / tile * g.nt);
         if (g.rows == 0) {
             g.rows = g.nt;
-            g.at_once = (int)(GT_SCRATCH / (g.nt * (token + 1)));
+            g.at_once = (int)(GT_SCRATCH / (g.nt * token));
             if (g.at_once < 1) g.at_once = 1;
         }
     } else if (GT_SCRATCH / each < batch) g.batches = (int)(GT_SCRATCH / each);
     return g;
 }
-static long long gt_token_floats(const GtPlan& g, long long padded, int ranges) { return padded * ranges * (g.range_len * 3 / 2) + (padded + 15) / 16 * 4; }
+static long long gt_token_floats(const GtPlan& g, long long padded, int ranges) { return padded * ranges * (g.range_len * 3 / 2); }
 long long gt_scratch(int M, int N, int K, int batch) {
     const GtPlan g = gt_plan(M, N, K, batch);
     const long long padded = (long long)(g.rows + g.nt - 1) / g.nt * g.nt * g.batches;
@@ -563,18 +549,17 @@ static int gt_piece(const GfParams& f, const GtPlan& g, int r0, int r1, cudaStre
         if (rc != BG_OK) return rc;
     }
     const long long padded = (long long)p.tok_tiles * g.nt * f.batch;
-    unsigned char *images = (unsigned char*)f.scratch, *odd = (unsigned char*)(f.scratch + padded * (r1 - r0) * (g.range_len * 3 / 2));
+    unsigned char* images = (unsigned char*)f.scratch;
     float* behind = f.scratch + gt_token_floats(g, padded, g.at_once);         // (the running sums stay in one place from launch to launch)
     p.images = images;
-    p.odd = odd;
     p.feat_tiles = (f.N + GT_BM - 1) / GT_BM;
     const long long units = (long long)p.tok_tiles * p.feat_tiles * f.batch * (g.cut ? r1 - r0 : 1);
     if (units > 0x3fffffff) return BG_ERR_SHAPE;
     p.units = (int)units;
     const bool vec = f.K % 4 == 0 && f.lda % 4 == 0 && f.batch_a % 4 == 0 && (uintptr_t)f.A % 16 == 0 && p.r0 * (long long)g.range_len % 4 == 0;
     const int pieces = ((r1 - r0) * g.range_len + 511) / 512, threads = 32 * (pieces < 8 ? pieces : 8);
-    cudaError_t e = vec ? launch(gf_parts_kernel<true>, dim3((unsigned)padded), dim3(threads), 0, stream, p, images, odd, g.nt)
-                        : launch(gf_parts_kernel<false>, dim3((unsigned)padded), dim3(threads), 0, stream, p, images, odd, g.nt);
+    cudaError_t e = vec ? launch(gf_parts_kernel<true>, dim3((unsigned)padded), dim3(threads), 0, stream, p, images, g.nt)
+                        : launch(gf_parts_kernel<false>, dim3((unsigned)padded), dim3(threads), 0, stream, p, images, g.nt);
     if (e != cudaSuccess) return (int)e;
     if (g.cut) p.part = behind;
     else if (f.accumulate && g.ranges > 1) { p.run = behind; p.ldr = f.N; p.batch_r = (long long)f.M * f.N; }

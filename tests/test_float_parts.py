@@ -55,6 +55,19 @@ def test_small_numbers_keep_their_digits(ops):
     assert bool(((out.double() - want).abs() <= 308 * 2.0 ** -24 * (a.abs().double() @ w.abs().double().t())).all())
 
 
+@pytest.mark.parametrize("M,N,K", [(3, 130, 600), (40, 64, 1100), (200, 203, 300)])
+def test_powers_of_two_change_no_bit(ops, M, N, K):
+    """Small operands are summed as those of the usual size are, all of them or one in a row."""
+    a, w = rnd(M, K, seed=16), rnd(N, K, seed=17)
+    out = product(ops, a, w)
+    assert torch.equal(product(ops, a * 2.0 ** -100, w) * 2.0 ** 100, out) and torch.equal(product(ops, a, w * 2.0 ** -100) * 2.0 ** 100, out)
+    assert torch.equal(product(ops, a * 2.0 ** -100, w * 2.0 ** 80) * 2.0 ** 20, out)
+    a[:, 70], w[:, 100] = 0.0, 0.0
+    out = product(ops, a, w)
+    a[:, 70], w[:, 100] = 1e-36, 1e-36
+    assert torch.equal(product(ops, a, w), out)
+
+
 def test_single_numbers_come_through_whole(ops):
     w = rnd(200, 300, seed=6)
     assert torch.equal(product(ops, torch.eye(300, device=DEV), w), w.t())
