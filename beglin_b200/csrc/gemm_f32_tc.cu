@@ -261,7 +261,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, GtParams p) {
                 v[2 * i] = x.x; v[2 * i + 1] = x.y;
             }
         };
-        if (DIRECT && NT > 16) pdl_wait();
+        if (DIRECT) pdl_wait();
         if (!DIRECT && (int)blockIdx.x < p.units) fetch(0);
         for (int u = blockIdx.x, g = 0; u < p.units; u += gridDim.x) {
             const Unit x = unit_of(u);

@@ -68,6 +68,17 @@ def test_powers_of_two_change_no_bit(ops, M, N, K):
     assert torch.equal(product(ops, a, w), out)
 
 
+def test_weights_that_the_kernel_before_makes(ops):
+    """Weights off 16 bytes are read behind the kernel before, for few rows too."""
+    a = rnd(3, 201, seed=18)
+    for i in range(4):
+        w, made = rnd(64, 201, seed=19 + i), torch.empty(64 * 201 + 1, device=DEV)[1:].view(64, 201)
+        ops.gemm_f32_nt(w, torch.eye(201, device=DEV), None, made)
+        out = product(ops, a, made)
+        torch.cuda.synchronize()
+        assert torch.equal(made, w) and torch.equal(out, product(ops, a, made))
+
+
 def test_single_numbers_come_through_whole(ops):
     w = rnd(200, 300, seed=6)
     assert torch.equal(product(ops, torch.eye(300, device=DEV), w), w.t())
