@@ -325,6 +325,19 @@ static bool attention_f32_takes(int rows, int hd, int vd, int maps) {
     return rows <= AF_ROWS && hd % (4 * maps) == 0 && vd % 4 == 0 && vd <= 256 && af_smem(hd / maps, hd, vd) <= 226 * 1024;
 }
 
+// Whether the compiler gave attention_f32_tc_kernel the registers at launch that its split among the warpgroups counts on (else its calls go on
+// to the kernels of other sizes).
+static bool ax_fits() {
+    static const bool fits = [] {
+        for (auto k : {attention_f32_tc_kernel<AttnParams, 64>, attention_f32_tc_kernel<AttnParams, 32>, attention_f32_tc_kernel<AttnParams, 0>}) {
+            cudaFuncAttributes a;
+            if (cudaFuncGetAttributes(&a, k) != cudaSuccess || a.numRegs < AX_REGS) return false;
+        }
+        return true;
+    }();
+    return fits;
+}
+
 // Rows per query block and keys per tile that fit the shared memory of one CTA for these sizes.
 // Returns 0 and fills bq and tile, or BG_ERR_UNSUPPORTED.
 // (`hd` counts a whole key row; with two maps in it, it may be twice as wide; `f32`: queries and cache are float)
@@ -359,19 +372,11 @@ extern "C" int bg_attention_partial(const void* q, int q_dtype, int q_stride, co
     p.keep = keep; p.slopes = slopes; p.maps = maps;
     dim3 grid(n_qblk, nkv, n_splits_launch);
     const bool pieces = q_stride % 4 == 0 && (uintptr_t)q % 16 == 0 && (uintptr_t)kv_pool % 16 == 0 && (uintptr_t)part_o % 16 == 0;
-    if (q_dtype == BG_DTYPE_F32 && cache_dtype == BG_DTYPE_F32 && ax_takes(bq * p.group, hd, vd, maps) && split % AX_KEYS == 0 && pieces) {
+    if (q_dtype == BG_DTYPE_F32 && cache_dtype == BG_DTYPE_F32 && ax_takes(bq * p.group, hd, vd, maps) && split % AX_KEYS == 0 && pieces && ax_fits()) {
         constexpr int need = 4 * AX_TILE + 1024;
         auto kern = vd == 128 ? attention_f32_tc_kernel<AttnParams, 64> : vd == 64 ? attention_f32_tc_kernel<AttnParams, 32> : attention_f32_tc_kernel<AttnParams, 0>;
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, need);
         if (e != cudaSuccess) return (int)e;
-        static const bool fits = [] {                      // (the split of the registers counts on as many at launch)
-            for (auto k : {attention_f32_tc_kernel<AttnParams, 64>, attention_f32_tc_kernel<AttnParams, 32>, attention_f32_tc_kernel<AttnParams, 0>}) {
-                cudaFuncAttributes a;
-                if (cudaFuncGetAttributes(&a, k) != cudaSuccess || a.numRegs < AX_REGS) return false;
-            }
-            return true;
-        }();
-        if (!fits) return (int)cudaErrorInvalidConfiguration;
         launch(kern, grid, dim3(AX_THREADS), need, stream, p);
         BG_LAUNCH_CHECK();
         return BG_OK;
@@ -395,7 +400,7 @@ extern "C" int bg_attention_partial(const void* q, int q_dtype, int q_stride, co
         return BG_OK;
     }
     size_t smem = attention_smem_bytes(bq, p.group, hd / maps, hd, vd, tile);
-    // blocks that were cut for attention_f32_kernel, which does not take the rows as they lie: its 64 rows fit beside tiles of half as many keys
+    // blocks that were cut for the float kernels above, which do not take the rows as they lie: up to 128 rows fit beside tiles of half as many keys
     if (smem > 227 * 1024 && tile == 64) smem = attention_smem_bytes(bq, p.group, hd / maps, hd, vd, p.tile = tile = 32);
     if (smem > 227 * 1024) return BG_ERR_UNSUPPORTED;
 #define BG_ATT_LAUNCH(TQ, TC)                                                                              \

@@ -14,6 +14,7 @@ import fcntl
 import glob
 import hashlib
 import os
+import re
 import shutil
 import subprocess
 import sys
@@ -25,7 +26,7 @@ from typing import List, Optional
 HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_NAME = "libbeglin_b200.so"
 ARCH_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a"]
-NVCC_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "--threads", "2"] + ARCH_FLAGS
+NVCC_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xptxas", "-v", "-Xcompiler", "-fPIC", "--threads", "2"] + ARCH_FLAGS
 
 _lib: Optional[ctypes.CDLL] = None
 
@@ -90,6 +91,23 @@ def _say(msg: str) -> None:
     print(f"[beglin_b200] {msg}", file=sys.stderr, flush=True)
 
 
+def registers_short(log: str, attention: int) -> List[str]:
+    """Kernels of the compiler's report (`-Xptxas -v`) that get fewer registers at launch than the split among their warpgroups counts on: the
+    float product's forms say how many (the eighth number of GtForm), float attention wants `attention`.  Such a kernel refuses to run."""
+    short = []
+    for name, used in re.findall(r"Compiling entry function '(\S+)'.*?Used (\d+) registers", log, re.S):
+        form = re.search(r"gemm_f32_tc_kernel.*?GtFormI((?:Li\d+E)+)", name)
+        want = int(re.findall(r"Li(\d+)E", form.group(1))[7]) if form else attention if "attention_f32_tc_kernel" in name else 0
+        if int(used) < want:
+            short.append(f"{name}: {used} registers of {want}")
+    return short
+
+
+def _attention_registers() -> int:
+    with open(os.path.join(HERE, "attention_f32_tc.cuh")) as f:
+        return int(re.search(r"AX_REGS = (\d+)", f.read()).group(1))
+
+
 def _compile_one(nvcc: str, src: str, obj: str) -> None:
     _say(f"compiling {os.path.basename(src)} for sm_100a ...")
     t0 = time.time()
@@ -97,6 +115,8 @@ def _compile_one(nvcc: str, src: str, obj: str) -> None:
     r = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
     if r.returncode != 0:
         raise BuildError(f"nvcc failed on {src}:\n{r.stdout}")
+    for line in registers_short(r.stdout, _attention_registers()):
+        _say(f"WARNING: float32 steps will lose a kernel with this compiler: {line}")
     _say(f"compiled {os.path.basename(src)} in {time.time() - t0:.1f} s")
 
 
