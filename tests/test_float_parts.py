@@ -220,3 +220,50 @@ def test_attention_of_small_operands(ops, hd):
     assert (small - want).abs().max() <= bound
     top = attend(ops, q, k, v * 2.0 ** 100).double() * 2.0 ** -100
     assert (top - want).abs().max() <= bound
+
+
+def plain_attention(q, k, v, slopes=None, softcap=0.0, window=0):
+    """In 64 bits, with the largest |score|."""
+    n, nh, hd = q.shape
+    group = nh // k.shape[1]
+    s = torch.einsum("thd,shd->hts", q.double(), k.double().repeat_interleave(group, 1)) * hd ** -0.5
+    if softcap:
+        s = softcap * torch.tanh(s / softcap)
+    pos = torch.arange(n, device=DEV)
+    away = (pos[:, None] - pos[None, :]).double()
+    if slopes is not None:
+        s = s - slopes.double()[:, None, None] * away
+    hidden = (away < 0) | ((away >= window) if window else (away < 0))
+    most = float(s.masked_fill(hidden, 0.0).abs().max())
+    return torch.einsum("hts,shd->thd", torch.softmax(s.masked_fill(hidden, -math.inf), -1), v.double().repeat_interleave(group, 1)), most
+
+
+@pytest.mark.parametrize("hd,vd", [(48, 48), (80, 112), (128, 128), (64, 16)])
+@pytest.mark.parametrize("how", ["slopes", "softcap", "both", "window"])
+def test_attention_options_over_a_portion(ops, hd, vd, how):
+    """Slopes, bounds of scores and windows over several tiles and splits of a portion."""
+    n, nh, nkv = 300, 6, 2
+    q, k, v = rnd(n, nh, hd, seed=40), rnd(n, nkv, hd, seed=41), rnd(n, nkv, vd, seed=42)
+    slopes = torch.tensor([2.0 ** -i for i in range(nh)], device=DEV) if how in ("slopes", "both") else None
+    softcap, window = (3.0 if how in ("softcap", "both") else 0.0), (70 if how == "window" else 0)
+    want, most = plain_attention(q, k, v, slopes, softcap, window)
+    out = attend(ops, q, k, v, 128, window, slopes, softcap)
+    # a score's error moves a weight by as much: hd + 8 roundings of the largest score (slopes reach n), and those of the row's sums
+    assert (out.double() - want).abs().max() <= ((hd + 8) * (most + 1) + n) * 2.0 ** -24 * float(v.abs().max())
+
+
+@pytest.mark.parametrize("hd", [48, 128])
+@pytest.mark.parametrize("split", [64, 256])
+def test_attention_of_keys_that_are_not_finite(ops, hd, split):
+    """Infinite keys and ones that are no numbers, in both halves of tiles: rows that see one are what 64 bits make of them, others are
+    untouched."""
+    n, nh, nkv = 300, 4, 2
+    q, k, v = rnd(n, nh, hd, seed=43), rnd(n, nkv, hd, seed=44), rnd(n, nkv, hd, seed=45)
+    fine = attend(ops, q, k, v, split)
+    k[40, 0, 3], k[100, 1, 0], k[170, 0, 5], k[255, 1, 1] = -math.inf, math.inf, math.nan, 1e37
+    want, _ = plain_attention(q, k, v)
+    out = attend(ops, q, k, v, split)
+    assert torch.equal(out[:40], fine[:40]) and torch.equal(torch.isnan(out), torch.isnan(want))
+    same = torch.isfinite(want)
+    # (row 255 on: keys next to the largest float, whose scores decide alone)
+    assert float(((out.double() - want).abs())[same].max()) <= (hd + 8) * 2.0 ** -20 * float(v.abs().max())
