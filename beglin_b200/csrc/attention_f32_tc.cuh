@@ -1,8 +1,9 @@
 // The partial results of float queries over a float cache on the tensor cores: heads of 48 to 128 features, a multiple of 16
 // (attention_f32.cuh runs the other sizes, attention_partial_kernel in attention.cu the other types).
 //
-// No precision is given up: queries, keys, values and weights are cut into three bfloat16 numbers each, exactly, and a product of two floats is
-// the six products of parts that are not below 2^-24 of it, the small ones added up before the large ones (gemm_f32_tc.cu says more).
+// Queries, keys, values and weights are cut into three bfloat16 numbers each, and of the nine products of the parts of two floats the six are
+// made that are not below 2^-24 of theirs, the small ones added up before the large ones; gemm_f32_tc.cu says what that leaves out, and how far the sums
+// are off (a row that sees few keys is a sum of few terms).
 // A CTA takes up to 128 rows (queries x query heads of a kv head), a lane of tensor memory each, and one split of keys, 64 at a time:
 // eight warps cut the keys and values of a tile into swizzled shared memory, one issues the MMAs, and eight warps, two threads a row with
 // 32 keys each, make the weights and keep the row's sums of values in registers (a tile's sums leave tensor memory and are added in float).

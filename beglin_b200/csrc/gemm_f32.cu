@@ -1,4 +1,4 @@
-// C[M, N] (+)= A[M, K] * W[N, K]^T (+ bias[N]) in true float: no operand and no sum in fewer bits.  This is the
+// C[M, N] (+)= A[M, K] * W[N, K]^T (+ bias[N]) of floats, no operand in fewer bits.  This is the
 // reference's linear, y[o] = bias[o] + sum_i W[o,i] x[i] with W row-major [out, in] (qwen_infer.c:688-691), for a batch of rows.
 //
 // Inner sizes above 2 GF_SHORT run on the tensor cores, every operand in three bfloat16 parts (gemm_f32_tc.cu).  Shorter ones come whole and

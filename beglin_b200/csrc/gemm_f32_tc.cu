@@ -1,14 +1,18 @@
 // The float product C[M, N] (+)= A[M, K] W[N, K]^T (+ bias) on the tensor cores, for inner sizes above those of gemm_f32.cu's own kernel.
 //
-// No precision is given up for it: every operand is cut into three bfloat16 numbers, x = h + m + l exactly, and a product of two floats is
-// the six products of parts that are not below 2^-24 of it (one with a single bit set times any float is exact).  64 of k are one
+// Every operand is cut into three bfloat16 numbers, x = h + m + l exactly, and of the nine products of the parts of two floats the six are made
+// that are not below 2^-24 of theirs (m l, l m and l l are left out; one with a single bit set times any float is exact).  64 of k are one
 // stage: its five kinds of small products go into an accumulator in tensor memory first, so that their sums are not cut off at the size of
 // the large ones, then h h; the stage's sum leaves tensor memory and is added to the range's in float, rounded to nearest.  (An
 // accumulator cuts off instead of rounding, always towards nought: four MMAs on a large sum are four such cuts.)  Ranges of k lie at places that
 // follow from N and K alone (gt_range); their sums are added in order, then the bias.  None of this depends on the number of rows, on
 // tiles or on who adds the ranges, so a row's result does not depend on how many other rows the call has: all forms here give the
-// same bits.  Error against 64 bits (2-norm, normal operands): 1.0e-7 for K of 1,536 and 1.3e-7 for 9,000, where two chains of float
-// multiply-adds over 1,024 of k had 3.7e-7 and 4.1e-7; 0.9e-7 for K of 200 (1.8e-7).
+// same bits.
+//
+// Error against 64 bits (2-norm, normal operands), two chains of float multiply-adds over 1,024 of k in brackets: K of 192 0.85e-7 (1.8e-7),
+// 1,536 1.0e-7 (3.7e-7), 9,000 1.3e-7 (4.1e-7).  It is smaller for dense rows and larger for those of few terms, whose chains have few
+// roundings: one term in a row 4.5e-8 (2.5e-8), four 5.6e-8 (4.2e-8), sixteen 6.3e-8 (6.1e-8), 64 7.0e-8 (1.07e-7).  And sums of one sign lean
+// towards nought, by 0.6 (one term) to 1.4 (dense) x 2^-24 of themselves, where the chains' do not lean.
 //
 // Operands are cut times 2^24 (GT_UP) and sums are scaled back, so that small ones keep their parts.  A range's sum that is not finite (an operand
 // that is infinite, not a number or above some 2^103, or a sum above some 2^80) is made by floats instead, in two chains (even and odd k), which makes of

@@ -823,8 +823,8 @@ def _difference_attention(q: torch.Tensor, kv_pool: torch.Tensor, block_table: t
 
 def gemm_f32_nt(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], out: torch.Tensor,
                 accumulate: bool = False, status: Optional[torch.Tensor] = None) -> None:
-    """out[M, N] (+)= a[M, K] @ w[N, K]^T (+ bias), all float32: no operand and no sum in fewer bits.  `status` learns of a wait
-    inside the kernel that ran out (the outputs are then no numbers)."""
+    """out[M, N] (+)= a[M, K] @ w[N, K]^T (+ bias), all float32: no operand in fewer bits, sums as csrc/gemm_f32_tc.cu says.
+    `status` learns of a wait inside the kernel that ran out (the outputs are then no numbers)."""
     _cuda(a, w, bias, out)
     for t in (a, w, out) + ((bias,) if bias is not None else ()):
         if t.dtype != torch.float32:

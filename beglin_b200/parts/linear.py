@@ -1,7 +1,7 @@
 """y = x W^T (+ bias), W row-major [out, in] as in the checkpoint (qwen_infer.c:688-691).
 
-float32: the hand-written product whose operands keep all their bits (on the tensor cores in three bfloat16 parts each, summed in
-float; small inner sizes on the float units).
+float32: the hand-written product whose operands keep all their bits (on the tensor cores in three bfloat16 parts each, six of the nine
+products of parts; small inner sizes on the float units).  csrc/gemm_f32_tc.cu says how far its sums are off.
 bfloat16: the tcgen05 tensor-core kernel of this package where it is the faster one (or everywhere,
 with gemm="tcgen05"), else the vendor library's product, which is where the reference calls its own
 platform's library (cblas_sgemv, qwen_infer.c:690).  Accumulation is float in every case: the library

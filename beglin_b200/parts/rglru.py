@@ -10,7 +10,7 @@ The state S and the last taps - 1 inputs of the convolution are per-request stat
 manager's slab, float32, zero when the request starts): a step continues each request from its slot, however the request's
 tokens are cut into steps and whatever else the step holds.  Everything that enters the recurrence is float in both number
 formats: the input product comes out as float, the convolution, the gates' products, sigmoids, softplus, decay, step and
-state are float.  The gates' products keep all bits in float32 steps (every output's sum has one order); in
+state are float.  The gates' products keep their operands' bits in float32 steps (every output's sum has one order); in
 bfloat16 steps on the tensor cores, with u cut into two bfloat16 numbers that together hold sixteen bits of it, against the
 matrices in bfloat16, accumulated in float.  Portions of at least `CHUNK_FROM` rows of a request walk
 the recurrence in chunks that are joined by a scan over the chunks' (product of decays, sum); shorter ones and single
