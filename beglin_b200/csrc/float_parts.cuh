@@ -7,8 +7,8 @@
 
 namespace bg {
 
-// Two floats into their three parts, two bfloat16 a word (the first one low).  `odd` collects what is left over in the low halves:
-// nought there if the third part is exact.  (An infinity leaves a NaN, whose low half is not nought.)
+// Two floats into their three parts, two bfloat16 a word (the first one low): exact for multiples of 2^-133, parts that are not numbers for
+// what is infinite, not a number, or next to the largest float.
 __device__ __forceinline__ unsigned gt_pack(unsigned long long v) {
     unsigned r;
     asm("cvt.rn.bf16x2.f32 %0, %1, %2;\n" : "=r"(r) : "f"(high2(v)), "f"(low2(v)));
@@ -17,21 +17,15 @@ __device__ __forceinline__ unsigned gt_pack(unsigned long long v) {
 __device__ __forceinline__ unsigned long long gt_unpack(unsigned p) {
     return (unsigned long long)(p << 16) | ((unsigned long long)(p & 0xffff0000u) << 32);
 }
-__device__ __forceinline__ void gt_split(unsigned long long v, unsigned& h, unsigned& m, unsigned& l, unsigned& odd) {
+__device__ __forceinline__ void gt_split(unsigned long long v, unsigned& h, unsigned& m, unsigned& l) {
     const unsigned long long minus = pair2(-1.0f, -1.0f);
     h = gt_pack(v);
     const unsigned long long r = fma2(gt_unpack(h), minus, v);
     m = gt_pack(r);
     const unsigned long long q = fma2(gt_unpack(m), minus, r);
     l = __byte_perm((unsigned)q, (unsigned)(q >> 32), 0x7632);
-    odd |= (unsigned)q | (unsigned)(q >> 32);
 }
-// The same where what is left over is told otherwise, or is no matter.
-__device__ __forceinline__ void gt_split(unsigned long long v, unsigned& h, unsigned& m, unsigned& l) {
-    unsigned odd = 0;
-    gt_split(v, h, m, l, odd);
-}
-// Both floats times a power of two (one by one: packed, the multiplication makes the kernels around it slower by a tenth).
+// Both floats times a power of two (one by one: packed, the multiplication makes float attention slower by a tenth).
 __device__ __forceinline__ unsigned long long gt_up(unsigned long long v, float up) { return pair2(low2(v) * up, high2(v) * up); }
 __device__ __forceinline__ unsigned long long gt_add2(unsigned long long a, unsigned long long b) {
     unsigned long long d;

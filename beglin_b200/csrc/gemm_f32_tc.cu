@@ -29,7 +29,7 @@
 // What bounds it: with 144 and 160 tokens the tensor cores (a stage of 160 tokens takes 1,980 cycles, its MMAs 1,920; with 32 of k a stage, one
 // warp that issued and one set of warps that cut and added it was 5,000), with fewer the instructions of the cut (some 12 a value:
 // weights at 4.6 TB/s for 8 rows).  In us, the float units' kernels in brackets: 550 x 17,920 with k of 1,536 142 (930),
-// 550 x 1,536 with 8,960 99 (498), 64 x 17,920 with 1,536 33 (116), 8 x 17,920 24 (32), 1 x 2,048 with 768 8.1 (13.3).
+// 550 x 1,536 with 8,960 103 (498), 64 x 17,920 with 1,536 34 (116), 8 x 17,920 24 to 26 (31), 1 x 2,048 with 768 8.0 (13.2).
 #include "gemm_f32.cuh"
 #include "float_parts.cuh"
 
@@ -282,9 +282,13 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, GtParams p) {
                 // (what the registers hold is cut before the wait for room)
                 constexpr int AHEAD = 2;
                 unsigned h[AHEAD][4], m[AHEAD][4], l[AHEAD][4];
+                // (packed or one by one: 550 x 17,920 with k of 1,536 143.4 and 145.2 us; sixteen products of 8 x 512 with 256 8.0 and 7.3)
                 auto cut = [&](int c, int to) {
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) gt_split(gt_up(v[4 * c + i], GT_UP), h[to][i], m[to][i], l[to][i]);
+                    for (int i = 0; i < 4; ++i) {
+                        const unsigned long long x = v[4 * c + i];
+                        gt_split(GC == 2 ? fma2(x, pair2(GT_UP, GT_UP), 0ull) : gt_up(x, GT_UP), h[to][i], m[to][i], l[to][i]);
+                    }
                 };
                 const unsigned a = parts + g % DA * 96;
                 auto put = [&](int c, int from) { gt_st4(a + 4 * c, h[from]); gt_st4(a + 32 + 4 * c, m[from]); gt_st4(a + 64 + 4 * c, l[from]); };
@@ -545,6 +549,8 @@ static int gt_piece(const GfParams& f, const GtPlan& g, int r0, int r1, cudaStre
     p.lda = f.lda; p.ldw = f.ldw; p.ldc = f.ldc; p.M = f.M; p.N = f.N; p.K = f.K; p.accumulate = f.accumulate; p.batch = f.batch;
     p.range_len = g.range_len; p.ranges = g.ranges; p.r0 = r0; p.r1 = r1; p.status = f.status;
     p.tok_tiles = (f.M + g.nt - 1) / g.nt;
+    // (Weights off 16 bytes are read value by value, a row a lane.  In us, by 4-byte asynchronous copies on the float units in brackets:
+    // 1 x 768 with k of 201 11.6 (16.1), 8 x 2,048 with 513 11.8 (38.4), 8 x 8,192 with 1,537 36.6 (76), 64 x 2,048 36.3 (78), 550 x 4,096 104 (281).)
     const bool direct = !(f.ldw % 4 == 0 && f.batch_w % 4 == 0 && (uintptr_t)f.W % 16 == 0);
     p.map_batch = f.batch > 1 && f.batch_w != 0;
     CUtensorMap mw = {};
