@@ -18,7 +18,8 @@
 // are not finite (an operand that is infinite or not a number, a query above 2^90) are summed by floats instead.  Values of 2^72 and more go into
 // the tile as nought and are added by floats to the rows whose weight for them is not nought, so that an infinite one at a position that a row
 // does not see does not reach it.  Small operands take the usual way (see AX_Q_UP): 550 rows with a key, a query or a value of 1e-36 in every eighth
-// row or less, 79 us; noticed where they are cut and summed by floats they took 940 to 980.
+// row or less, 79 us; noticed where they are cut and summed by floats they took 940 to 980.  With NaN in every eighth key 330 us (16 bytes a load; a value
+// a load 940), in one query 845, in every eighth value 183 (the float units' kernel: 293 to 308).
 #pragma once
 
 #include "float_parts.cuh"
@@ -357,7 +358,12 @@ __global__ void __launch_bounds__(AX_THREADS, 1) attention_f32_tc_kernel(P p) {
                     bad &= bad - 1;
                     const float* src = pool + (size_t)page * page_elems + ((size_t)kvh * p.page_size + at % p.page_size) * hd;
                     float even = 0.0f, odd = 0.0f;
-                    for (int d = 0; d < hd; d += 2) { even = fmaf(q[d], src[d], even); odd = fmaf(q[d + 1], src[d + 1], odd); }
+#pragma unroll 2
+                    for (int d = 0; d < hd; d += 4) {
+                        const float4 x = *reinterpret_cast<const float4*>(q + d), y = *reinterpret_cast<const float4*>(src + d);
+                        even = fmaf(x.z, y.z, fmaf(x.x, y.x, even));
+                        odd = fmaf(x.w, y.w, fmaf(x.y, y.y, odd));
+                    }
                     even = (even + odd) * p.scale;
 #pragma unroll
                     for (int j = 0; j < 32; ++j)
