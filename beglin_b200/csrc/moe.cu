@@ -9,6 +9,7 @@
 //                  src_of[row] the assignment that row holds.  ONE CTA; the order inside an expert is whatever the
 //                  atomics give, which no result depends on (a row's product is a function of that row alone).
 //   route_rows     the three above and below for a step of few tokens in one kernel, a cluster of CTAs.
+//   route_place    route_sort and route_gather in one kernel, from counts that the router's kernel leaves.
 //   route_gather   xp[row] = (weight * x[token]) rounded to the compute type (or x[token] as it is).
 //   gemm_grouped   yp[row] = act(xp[row] W[e]^T) on CUDA cores, float accumulation, every output summed over k in index
 //                  order by one thread: the float32 path, and the sizes the tensor-core product does not take.
@@ -148,65 +149,166 @@ route_kernel(const TI* __restrict__ h, int ldh, const float* __restrict__ W, int
     if (warp < n) choose_experts(logit_s + warp * E, E, top, rule, ids, weights, (size_t)(t0 + warp), lane);
 }
 
-// The logits of one token's row by `warps` warps of a block (this is the `warp`-th), each a group of G experts at a time: a lane walks the
-// features in chunks of eight, 32 chunks apart (16-byte loads), and the warp adds up.
-template <typename TI, int G>
-__device__ __forceinline__ void route_logits_of(const TI* row, const float* __restrict__ W, int d8, int d, int E, float* sc, float* logits_out,
-                                                int warp, int warps, int lane) {
+// The logits of TPW tokens' rows (row, row + ldh, ..; those from `live` on are the first one's again and not stored) by `warps` warps of a block
+// (this is the `warp`-th), each a group of G experts at a time: a lane walks the features in chunks of eight, 32 chunks apart (16-byte
+// loads), and the warp adds up.  An expert's row is fetched once for all the tokens; a logit's sum does not depend on TPW, G or `warps`.
+// Experts from E on are the last one again and not stored: a condition on the loads keeps them from being on their way together.
+template <typename TI, int TPW, int G>
+__device__ __forceinline__ void route_logits_of(const TI* row, int ldh, int live, const float* __restrict__ W, int d8, int d, int E, float* sc,
+                                                float* logits_out, int warp, int warps, int lane) {
     for (int e0 = warp * G; e0 < E; e0 += warps * G) {
-        float acc[G];
+        float acc[TPW][G];
 #pragma unroll
-        for (int u = 0; u < G; ++u) acc[u] = 0.0f;
+        for (int q = 0; q < TPW; ++q)
+#pragma unroll
+            for (int u = 0; u < G; ++u) acc[q][u] = 0.0f;
 #pragma unroll 2
         for (int c = lane; c < d8; c += 32) {
-            float hv[8];
-            load8(row + 8 * c, hv);
+            float hv[TPW][8], wv[G][8];
+#pragma unroll
+            for (int q = 0; q < TPW; ++q) load8(row + (size_t)(q < live ? q : 0) * ldh + 8 * c, hv[q]);
+#pragma unroll
+            for (int u = 0; u < G; ++u) load8(W + (size_t)min(e0 + u, E - 1) * d + 8 * c, wv[u]);
+#pragma unroll
+            for (int u = 0; u < G; ++u)
+#pragma unroll
+                for (int q = 0; q < TPW; ++q)
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) acc[q][u] = fmaf(hv[q][i], wv[u][i], acc[q][u]);
+        }
+#pragma unroll
+        for (int q = 0; q < TPW; ++q)
 #pragma unroll
             for (int u = 0; u < G; ++u) {
-                if (e0 + u < E) {
-                    float wv[8];
-                    load8(W + (size_t)(e0 + u) * d + 8 * c, wv);
-#pragma unroll
-                    for (int i = 0; i < 8; ++i) acc[u] = fmaf(hv[i], wv[i], acc[u]);
+                const float v = warp_sum(acc[q][u]);
+                if (lane == 0 && e0 + u < E && q < live) {
+                    sc[q * E + e0 + u] = v;
+                    if (logits_out) logits_out[(size_t)q * E + e0 + u] = v;
                 }
             }
-        }
-#pragma unroll
-        for (int u = 0; u < G; ++u) {
-            const float v = warp_sum(acc[u]);
-            if (lane == 0 && e0 + u < E) {
-                sc[e0 + u] = v;
-                if (logits_out) logits_out[e0 + u] = v;
-            }
-        }
     }
 }
 
-// The same for a width that is a multiple of 8 and 16-byte aligned rows.  A block of eight warps takes TPB tokens, 8 / TPB
-// warps to a token, which share the experts in groups of G; a lane walks the token's features in chunks of eight, 32 chunks
-// apart (16-byte loads: one of the token's row, which stays in the first-level cache from expert to expert, and two of
-// each expert's row), and the warp adds up; the first warp of a token then chooses.  Steps of many tokens: a warp per token,
-// four experts at a time.  Steps of few tokens: a block per token and an expert per warp at a time, so that a decoding step
-// spreads over as many SMs as it has tokens and a warp's chain of loads is one expert long.  (The walk through the features
-// one at a time above cost 53 us for 1,536 features whatever the number of tokens.)
-template <typename TI, int TPB, int G>
+// The same for a width that is a multiple of 8 and 16-byte aligned rows.  A block of eight warps takes TPW x 8 / wpt tokens: `wpt` warps share
+// TPW tokens' experts in groups of G, and every warp then chooses for some of the block's tokens.  Steps of few tokens: a block per token and
+// an expert per warp at a time, so that a decoding step spreads over as many SMs as it has tokens and a warp's chain of loads is one
+// expert long.  Steps of many: four tokens a warp, four experts at a time.  What bounds it is the router's float rows, which every token needs
+// whole: with a warp to one token they came through the first-level cache once a token (2,048 tokens, 8 experts, 1,536 features: 17.0 -> 8.9 us).
+// `hist`, when given, receives how many of the block's assignments each expert has, [blocks][E].
+template <typename TI, int TPW, int G>
 __global__ void __launch_bounds__(32 * ROUTE_TOKENS)
-route_vec8_kernel(const TI* __restrict__ h, int ldh, const float* __restrict__ W, int T, int d, int E, int top, RouteRule rule,
-                  int* __restrict__ ids, float* __restrict__ weights, float* __restrict__ logits_out) {
-    constexpr int WPT = ROUTE_TOKENS / TPB;                // warps per token
-    extern __shared__ float logit_s[];                     // [TPB][E]
+route_vec8_kernel(const TI* __restrict__ h, int ldh, const float* __restrict__ W, int T, int d, int E, int top, RouteRule rule, int wpt,
+                  int* __restrict__ ids, float* __restrict__ weights, float* __restrict__ logits_out, int* __restrict__ hist) {
+    extern __shared__ float logit_s[];                     // [tokens][E], then the experts' counts
     pdl_launch();
     pdl_wait();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int tl = warp / WPT, wq = warp % WPT;
-    const int t = blockIdx.x * TPB + tl;
-    const bool live = t < T;
-    const TI* row = h + (size_t)(live ? t : 0) * ldh;
-    float* sc = logit_s + tl * E;
-    const int d8 = d >> 3;
-    if (live) route_logits_of<TI, G>(row, W, d8, d, E, sc, logits_out ? logits_out + (size_t)t * E : nullptr, wq, WPT, lane);
+    const int tokens = TPW * (ROUTE_TOKENS / wpt), t0 = blockIdx.x * tokens, n = min(tokens, T - t0);
+    const int first = warp / wpt * TPW;                    // of this warp's tokens, in the block
+    const int live = min(TPW, n - first);
+    int* count_s = (int*)(logit_s + tokens * E);
+    if (hist) for (int e = threadIdx.x; e < E; e += blockDim.x) count_s[e] = 0;
+    if (live > 0)
+        route_logits_of<TI, TPW, G>(h + (size_t)(t0 + first) * ldh, ldh, live, W, d >> 3, d, E, logit_s + first * E,
+                                    logits_out ? logits_out + (size_t)(t0 + first) * E : nullptr, warp % wpt, wpt, lane);
     __syncthreads();                                       // every warp comes here, with or without a token
-    if (live && wq == 0) choose_experts(sc, E, top, rule, ids, weights, (size_t)t, lane);
+    for (int tl = warp; tl < n; tl += ROUTE_TOKENS) {
+        choose_experts(logit_s + tl * E, E, top, rule, ids, weights, (size_t)(t0 + tl), lane);
+        if (hist) {
+            __syncwarp();
+            if (lane < top) atomicAdd(&count_s[ids[(size_t)(t0 + tl) * top + lane]], 1);
+        }
+    }
+    if (!hist) return;
+    __syncthreads();
+    for (int e = threadIdx.x; e < E; e += blockDim.x) hist[(size_t)blockIdx.x * E + e] = count_s[e];
+}
+
+// What route_sort and route_gather do, for the same blocks of `tokens` tokens as the router's kernel ahead, from its counts: every block adds up the
+// counts (RL_MAX of them at most) for itself, so an expert's rows begin behind those of smaller experts, a block's behind those of the
+// blocks before it, and inside a block they stand in the order of the assignments.  No atomics: the order is the same every time.
+// gridDim.y blocks share the columns of a block's rows.  Bound by bytes and by the chain of counts, prefix and rows in front of them (2,048
+// tokens, two of 8 experts, 1,536 features: sort and gather 11.4 us -> 9.0; the whole case of perf/cases.py 122 -> 116).
+constexpr int RL_MAX = 8192, RL_MAX_E = 256, RL_MAX_A = 512;
+template <typename TI>
+__global__ void __launch_bounds__(256)
+route_place_kernel(const TI* __restrict__ h, int ldh, const float* __restrict__ weights, const int* __restrict__ ids, const int* __restrict__ hist,
+                   int T, int d, int E, int top, int tokens, int* __restrict__ offsets, int* __restrict__ row_of, int* __restrict__ src_of,
+                   TI* __restrict__ xp, int scale) {
+    __shared__ int before_s[RL_MAX_E], total_s[RL_MAX_E], expert_s[RL_MAX_A], row_s[RL_MAX_A];
+    __shared__ float weight_s[RL_MAX_A];
+    pdl_launch();
+    const int tid = threadIdx.x, t0 = blockIdx.x * tokens, n = min(tokens, T - t0), A = n * top, a0 = t0 * top;
+    for (int e = tid; e < E; e += blockDim.x) { before_s[e] = 0; total_s[e] = 0; }
+    pdl_wait();
+    for (int a = tid; a < A; a += blockDim.x) { expert_s[a] = ids[a0 + a]; weight_s[a] = scale ? weights[a0 + a] : 1.0f; }
+    __syncthreads();
+    {
+        int ep = 1;                                        // threads of the same expert: ep apart
+        while (ep < E) ep *= 2;
+        const int e = tid & (ep - 1), step = 256 / ep;
+        int total = 0, before = 0;
+        if (e < E) {
+#pragma unroll 8
+            for (int b = tid / ep; b < (int)gridDim.x; b += step) {
+                const int c = hist[b * E + e];
+                total += c;
+                before += b < (int)blockIdx.x ? c : 0;
+            }
+        }
+        for (int o = ep; o < 32; o *= 2) { total += __shfl_xor_sync(0xffffffffu, total, o); before += __shfl_xor_sync(0xffffffffu, before, o); }
+        if (e < E && (tid & 31) < ep) { atomicAdd(&total_s[e], total); atomicAdd(&before_s[e], before); }
+    }
+    __syncthreads();
+    if (tid < 32) {                                        // totals become the experts' first rows
+        int run = 0;
+        for (int e0 = 0; e0 < E; e0 += 32) {
+            const int c = e0 + tid < E ? total_s[e0 + tid] : 0;
+            int up = c;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int u = __shfl_up_sync(0xffffffffu, up, o);
+                if (tid >= o) up += u;
+            }
+            if (e0 + tid < E) {
+                total_s[e0 + tid] = run + up - c;
+                if (blockIdx.x == 0 && blockIdx.y == 0) offsets[e0 + tid] = run + up - c;
+            }
+            run += __shfl_sync(0xffffffffu, up, 31);
+        }
+        if (tid == 0 && blockIdx.x == 0 && blockIdx.y == 0) offsets[E] = run;
+    }
+    __syncthreads();
+    for (int a = tid; a < A; a += blockDim.x) {
+        const int e = expert_s[a];
+        int row = total_s[e] + before_s[e];
+#pragma unroll 8
+        for (int b = 0; b < a; ++b) row += expert_s[b] == e ? 1 : 0;
+        row_s[a] = row;
+        if (blockIdx.y == 0) { row_of[a0 + a] = row; src_of[row] = a0 + a; }
+    }
+    __syncthreads();
+    // a warp to a token at a time, its share of the columns four pieces a lane on their way together
+    const int d8 = d >> 3, c0 = (int)((long long)d8 * blockIdx.y / gridDim.y), c1 = (int)((long long)d8 * (blockIdx.y + 1) / gridDim.y);
+    for (int tl = tid >> 5; tl < n; tl += 8) {
+        const TI* from = h + (size_t)(t0 + tl) * ldh;
+        for (int c = c0 + (tid & 31); c < c1; c += 128) {
+            float x[4][8];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) load8(from + 8 * min(c + 32 * u, c1 - 1), x[u]);
+            for (int j = 0; j < top; ++j) {
+                const float wt = weight_s[tl * top + j];
+                TI* to = xp + (size_t)row_s[tl * top + j] * d;
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    float v[8];
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) v[q] = wt * x[u][q];
+                    if (c + 32 * u < c1) store8(to + 8 * (c + 32 * u), v);
+                }
+            }
+        }
+    }
 }
 
 // Routing, layout and gather of a step of few tokens as ONE kernel: three dependent launches cost more than their work, on
@@ -229,7 +331,7 @@ route_rows_kernel(const TI* __restrict__ h, int ldh, const float* __restrict__ W
     const int rank = blockIdx.z, A = T * top, d8 = d >> 3;
     const int t = rank;                                    // this CTA's token
     if (t < T) {
-        route_logits_of<TI, G>(h + (size_t)t * ldh, W, d8, d, E, logit_s, nullptr, warp, ROUTE_TOKENS, lane);
+        route_logits_of<TI, 1, G>(h + (size_t)t * ldh, ldh, 1, W, d8, d, E, logit_s, nullptr, warp, ROUTE_TOKENS, lane);
         __syncthreads();
         if (warp == 0) {
             choose_experts(logit_s, E, top, rule, ids, weights, (size_t)t, lane);
@@ -646,6 +748,36 @@ extern "C" int bg_route_topk(const float* logits, int T, int E, int top, int mod
     return BG_OK;
 }
 
+// How the router's kernel of 16-byte loads cuts a step: `tpw` tokens and `g` experts a warp at a time, `wpt` warps to the same tokens, `tokens` a
+// block.  Few tokens: a block each, and as many experts a warp as let them go through in one pass (the loads of a pass are all on their way
+// together; ten router outputs: 9.3 -> 7.8 us).  More than 256: four tokens a warp.
+struct RouteCut { int tpw, g, wpt, tokens; };
+static RouteCut route_cut(int T, int E) {
+    if (T <= 256) return {1, E <= ROUTE_TOKENS ? 1 : E <= 2 * ROUTE_TOKENS ? 2 : 4, ROUTE_TOKENS, 1};
+    int wpt = 1;
+    while (wpt < ROUTE_TOKENS && wpt * 4 < E) wpt *= 2;
+    return {4, 4, wpt, 4 * (ROUTE_TOKENS / wpt)};
+}
+static bool route_vec(const void* h, int ldh, const float* W, int d) {
+    return d % 8 == 0 && ldh % 8 == 0 && (uintptr_t)h % 16 == 0 && (uintptr_t)W % 16 == 0;
+}
+static int route_launch(const void* h, int h_dtype, int ldh, const float* W, int T, int d, int E, int top, RouteRule rule, int* ids,
+                        float* weights, float* logits_out, int* hist, cudaStream_t stream) {
+    const RouteCut c = route_cut(T, E);
+    const size_t smem = (size_t)(c.tokens + (hist ? 1 : 0)) * E * sizeof(float);
+    if (smem > 40 * 1024) return BG_ERR_UNSUPPORTED;
+#define BG_ROUTE_VEC(TPW, G)                                                                                                     \
+    BG_DISPATCH_DTYPE(h_dtype, TI, launch(route_vec8_kernel<TI, TPW, G>, dim3((T + c.tokens - 1) / c.tokens), dim3(32 * ROUTE_TOKENS), smem, \
+                                          stream, (const TI*)h, ldh, W, T, d, E, top, rule, c.wpt, ids, weights, logits_out, hist))
+    if (c.tpw == 4) BG_ROUTE_VEC(4, 4);
+    else if (c.g == 1) BG_ROUTE_VEC(1, 1);
+    else if (c.g == 2) BG_ROUTE_VEC(1, 2);
+    else BG_ROUTE_VEC(1, 4);
+#undef BG_ROUTE_VEC
+    BG_LAUNCH_CHECK();
+    return BG_OK;
+}
+
 // The router in one kernel: float logits of h [T, d] (either type, row stride ldh) against W [E, d] float, and the choice.
 extern "C" int bg_route(const void* h, int h_dtype, int ldh, const float* W, int T, int d, int E, int top, int mode, int renorm,
                         const float* bias, float scale, const float* logit_bias, int* ids, float* weights, float* logits_out,
@@ -655,25 +787,32 @@ extern "C" int bg_route(const void* h, int h_dtype, int ldh, const float* W, int
     const RouteRule rule = {mode, renorm, bias, scale, logit_bias};
     const size_t smem = (size_t)ROUTE_TOKENS * E * sizeof(float);
     if (smem > 40 * 1024) return BG_ERR_UNSUPPORTED;
-    const dim3 grid((T + ROUTE_TOKENS - 1) / ROUTE_TOKENS), block(32 * ROUTE_TOKENS);
-    // experts a warp takes at a time in steps of few tokens: as many as let a token's experts go through in one pass (the loads
-    // of a pass are all on their way together; every expert's sum keeps its own order, so the logits are the same bits: 9.3 ->
-    // 7.8 us for ten router outputs)
-    const bool vec = d % 8 == 0 && ldh % 8 == 0 && (uintptr_t)h % 16 == 0 && (uintptr_t)W % 16 == 0;
-#define BG_ROUTE_VEC(TPB, G, GRID, SMEM)                                                                                \
-    BG_DISPATCH_DTYPE(h_dtype, TI, launch(route_vec8_kernel<TI, TPB, G>, GRID, block, SMEM, stream, (const TI*)h, ldh, W, T, d, E, \
-                                          top, rule, ids, weights, logits_out))
-    if (vec && T <= 256) {
-        const size_t one = (size_t)E * sizeof(float);
-        if (E <= ROUTE_TOKENS) BG_ROUTE_VEC(1, 1, dim3(T), one);
-        else if (E <= 2 * ROUTE_TOKENS) BG_ROUTE_VEC(1, 2, dim3(T), one);
-        else BG_ROUTE_VEC(1, 4, dim3(T), one);
-    } else if (vec) {
-        BG_ROUTE_VEC(ROUTE_TOKENS, 4, grid, smem);     // (sixteen at a time: 39.7 against 25.3 us for 2,048 tokens and ten experts)
-    } else
-#undef BG_ROUTE_VEC
-        BG_DISPATCH_DTYPE(h_dtype, TI, launch(route_kernel<TI>, grid, block, smem, stream, (const TI*)h, ldh, W, T, d, E, top, rule,
-                                              ids, weights, logits_out));
+    if (route_vec(h, ldh, W, d)) return route_launch(h, h_dtype, ldh, W, T, d, E, top, rule, ids, weights, logits_out, nullptr, stream);
+    BG_DISPATCH_DTYPE(h_dtype, TI, launch(route_kernel<TI>, dim3((T + ROUTE_TOKENS - 1) / ROUTE_TOKENS), dim3(32 * ROUTE_TOKENS), smem, stream,
+                                          (const TI*)h, ldh, W, T, d, E, top, rule, ids, weights, logits_out));
+    BG_LAUNCH_CHECK();
+    return BG_OK;
+}
+
+// bg_route, bg_route_sort and bg_route_gather (xp in h's type) of a step of any number of tokens as two kernels; hist: `n_hist` integers of
+// scratch.  BG_ERR_UNSUPPORTED, with nothing launched, where they do not take the sizes: rows that are not whole 16-byte pieces, more than
+// RL_MAX counts (every block of the second kernel adds them all up: 2,048 tokens of 8 experts are 1,024), more assignments to a block than fit.
+extern "C" int bg_route_layout(const void* h, int h_dtype, int ldh, const float* W, int T, int d, int E, int top, int mode, int renorm,
+                               const float* bias, float scale, const float* logit_bias, int* ids, float* weights, int* offsets, int* row_of,
+                               int* src_of, void* xp, int scale_input, int* hist, int n_hist, cudaStream_t stream) {
+    if (T <= 0) return BG_OK;
+    if (E <= 0 || top <= 0 || top > E || top > 32 || d <= 0 || mode < 0 || mode > 3 || (mode == 3 && bias)) return BG_ERR_SHAPE;
+    const RouteCut c = route_cut(T, E);
+    const int blocks = (T + c.tokens - 1) / c.tokens;
+    if (!route_vec(h, ldh, W, d) || (uintptr_t)xp % 16 || E > RL_MAX_E || c.tokens * top > RL_MAX_A || (long long)blocks * E > RL_MAX ||
+        (long long)blocks * E > n_hist)
+        return BG_ERR_UNSUPPORTED;
+    const RouteRule rule = {mode, renorm, bias, scale, logit_bias};
+    const int rc = route_launch(h, h_dtype, ldh, W, T, d, E, top, rule, ids, weights, nullptr, hist, stream);
+    if (rc != BG_OK) return rc;
+    const int cols = blocks >= 296 || d < 1024 ? 1 : 2;
+    BG_DISPATCH_DTYPE(h_dtype, TI, launch(route_place_kernel<TI>, dim3(blocks, cols), dim3(256), 0, stream, (const TI*)h, ldh, weights, ids, hist, T, d,
+                                          E, top, c.tokens, offsets, row_of, src_of, (TI*)xp, scale_input));
     BG_LAUNCH_CHECK();
     return BG_OK;
 }

@@ -74,6 +74,8 @@ _SIGNATURES = {
     "bg_rglru_split": [_c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_void_p],
     "bg_route_rows": [_c_void_p, _c_int, _c_int, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void_p, _c_float, _c_void_p,
                       _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_void_p],
+    "bg_route_layout": [_c_void_p, _c_int, _c_int, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void_p, _c_float, _c_void_p,
+                        _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_void_p, _c_int, _c_void_p],
     "bg_route_sort": [_c_void_p, _c_int, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_void_p],
     "bg_route_gather": [_c_void_p, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void_p],
     "bg_route_combine": [_c_void_p, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_void_p],
@@ -1864,26 +1866,54 @@ def route_rows(h: torch.Tensor, router: torch.Tensor, top: int, ids: torch.Tenso
                bias: Optional[torch.Tensor] = None, scale: float = 1.0, logit_bias: Optional[torch.Tensor] = None) -> bool:
     """`route`, `route_sort` and `route_gather` (out of h's type) of a step of few tokens as one kernel; False, with nothing done, where
     it does not take the sizes."""
+    if h.shape[0] > ROUTE_ROWS_TOKENS:
+        return False
+    return _route_and_place("route_rows", h, router, top, ids, weights, offsets, row_of, src_of, out, scale_input, None, sigmoid, renorm, bias,
+                            scale, logit_bias)
+
+
+ROUTE_LAYOUT_COUNTS = 8192    # integers of scratch that `route_layout` can use
+
+
+def route_layout(h: torch.Tensor, router: torch.Tensor, top: int, ids: torch.Tensor, weights: torch.Tensor, offsets: torch.Tensor,
+                 row_of: torch.Tensor, src_of: torch.Tensor, out: torch.Tensor, scale_input: bool, counts: torch.Tensor, sigmoid=True,
+                 renorm: bool = False, bias: Optional[torch.Tensor] = None, scale: float = 1.0,
+                 logit_bias: Optional[torch.Tensor] = None) -> bool:
+    """The same for any number of tokens, as two kernels, with `counts` int32 as scratch (T * E integers suffice, and no more than
+    ROUTE_LAYOUT_COUNTS are used); False, with nothing done, where they do not take the sizes."""
+    _i32(counts, "counts")
+    return _route_and_place("route_layout", h, router, top, ids, weights, offsets, row_of, src_of, out, scale_input, counts, sigmoid, renorm, bias,
+                            scale, logit_bias)
+
+
+def _route_and_place(what, h, router, top, ids, weights, offsets, row_of, src_of, out, scale_input, counts, sigmoid, renorm, bias, scale,
+                     logit_bias) -> bool:
     T, d = h.shape
     E, A = router.shape[0], T * top
-    if T > ROUTE_ROWS_TOKENS or out.dtype != h.dtype or h.dtype not in (torch.float32, torch.bfloat16) or not h.is_contiguous():
+    if out.dtype != h.dtype or h.dtype not in (torch.float32, torch.bfloat16) or not h.is_contiguous():
         return False
-    _cuda(h, router, ids, weights, offsets, row_of, src_of, out, bias, logit_bias)
+    _cuda(h, router, ids, weights, offsets, row_of, src_of, out, counts, bias, logit_bias)
     for t, n in ((ids, "ids"), (offsets, "offsets"), (row_of, "row_of"), (src_of, "src_of")):
         _i32(t, n)
     if router.dtype != torch.float32 or router.shape[1] != d or not router.is_contiguous() or tuple(ids.shape) != (T, top) \
             or tuple(weights.shape) != (T, top) or weights.dtype != torch.float32 or not weights.is_contiguous() \
             or not ids.is_contiguous() or offsets.numel() != E + 1 or row_of.numel() != A or src_of.numel() != A \
             or tuple(out.shape) != (A, d) or not out.is_contiguous():
-        raise KernelError("route_rows: h [T, d], router float32 [E, d], ids and weights [T, top], offsets [E + 1], row_of and src_of [T * top], "
+        raise KernelError(f"{what}: h [T, d], router float32 [E, d], ids and weights [T, top], offsets [E + 1], row_of and src_of [T * top], "
                           "out [T * top, d]")
-    rule = _route_rule(E, sigmoid, bias, "route_rows", logit_bias)
+    rule = _route_rule(E, sigmoid, bias, what, logit_bias)
     with phase("router"):
-        rc = lib().bg_route_rows(_p(h), _dt(h), h.stride(0), _p(router), T, d, E, top, rule, 1 if renorm else 0, _p(bias), float(scale),
-                                 _p(logit_bias), _p(ids), _p(weights), _p(offsets), _p(row_of), _p(src_of), _p(out), 1 if scale_input else 0, _stream())
+        args = (_p(h), _dt(h), h.stride(0), _p(router), T, d, E, top, rule, 1 if renorm else 0, _p(bias), float(scale), _p(logit_bias), _p(ids),
+                _p(weights), _p(offsets), _p(row_of), _p(src_of), _p(out), 1 if scale_input else 0)
+        if counts is None:
+            rc = lib().bg_route_rows(*args, _stream())
+        else:
+            rc = lib().bg_route_layout(*args, _p(counts), counts.numel(), _stream())
         if rc == _UNSUPPORTED:
             return False
-        _check(rc, "route_rows")
+        _check(rc, what)
+    if counts is not None:
+        count_launches(1)
     return True
 
 

@@ -134,12 +134,15 @@ class RoutedExperts:
         s, dev, ct = self.spec, h.device, self.ctx.compute_dtype
         T, A = h.shape[0], h.shape[0] * s.top
         outputs = s.experts + s.identity
-        ints = torch.empty((3 * A + outputs + 1,), dtype=torch.int32, device=dev)
-        ids, row_of, src_of, offsets = ints[:A].view(T, s.top), ints[A:2 * A], ints[2 * A:3 * A], ints[3 * A:]
+        few = T <= ops.ROUTE_ROWS_TOKENS
+        counts = 0 if few else min(T * outputs, ops.ROUTE_LAYOUT_COUNTS)
+        ints = torch.empty((3 * A + outputs + 1 + counts,), dtype=torch.int32, device=dev)
+        ids, row_of, src_of, offsets = ints[:A].view(T, s.top), ints[A:2 * A], ints[2 * A:3 * A], ints[3 * A:3 * A + outputs + 1]
         weights = torch.empty((T, s.top), dtype=torch.float32, device=dev)
         xp = torch.empty((A, s.hidden), dtype=ct, device=dev)
         how = dict(sigmoid=s.router_activation, renorm=s.renormalize, bias=self.choice_bias, scale=s.route_scale, logit_bias=self.logit_bias)
-        if T > ops.ROUTE_ROWS_TOKENS or not ops.route_rows(h, self.router, s.top, ids, weights, offsets, row_of, src_of, xp, s.scale_input, **how):
+        place = (h, self.router, s.top, ids, weights, offsets, row_of, src_of, xp, s.scale_input)
+        if not (ops.route_rows(*place, **how) if few else ops.route_layout(*place, ints[3 * A + outputs + 1:], **how)):
             ops.route(h, self.router, s.top, ids, weights, **how)
             ops.route_sort(ids.view(-1), outputs, offsets, row_of, src_of)
             ops.route_gather(h, weights.view(-1), src_of, xp, s.top, scale=s.scale_input)

@@ -85,3 +85,38 @@ def test_routing_of_few_tokens_in_one_kernel(ops, T, E, top, d, dtype):
             assert ((row_of.long() >= starts[chosen]) & (row_of.long() < starts[chosen + 1])).all()
             ops.route_gather(h, weights.view(-1), src_of, xp2, top, scale=scale_input)
             assert torch.equal(xp, xp2)
+
+
+@pytest.mark.parametrize("T,E,top,d", [(9, 10, 2, 1536), (40, 8, 8, 64), (33, 200, 5, 2056), (256, 17, 3, 264), (257, 8, 2, 1536), (300, 40, 32, 72), (261, 120, 2, 136),
+                                       (1003, 4, 2, 64), (700, 3, 3, 8), (2048, 16, 1, 1024), (2000, 9, 4, 520)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_routing_of_many_tokens_in_two_kernels(ops, T, E, top, d, dtype):
+    """The same for steps of more tokens: edges of a warp's four tokens, of a block's, of a group of four experts, few columns and many."""
+    g = torch.Generator().manual_seed(T * E)
+    h, W = torch.randn(T, d, generator=g).to(DEV, dtype), torch.randn(E, d, generator=g).to(DEV)
+    bias, A = torch.randn(E, generator=g).to(DEV), T * top
+    i32 = lambda *n: torch.full(n, -7, dtype=torch.int32, device=DEV)
+    for scale_input, how in ((False, dict(sigmoid="sigmoid", renorm=True)), (True, dict(sigmoid="softmax", bias=bias, scale=2.5))):
+        ids, weights, offsets, row_of, src_of = i32(T, top), torch.zeros((T, top), device=DEV), i32(E + 1), i32(A), i32(A)
+        xp = torch.full((A, d), float("nan"), dtype=dtype, device=DEV)
+        assert ops.route_layout(h, W, top, ids, weights, offsets, row_of, src_of, xp, scale_input, i32(min(T * E, ops.ROUTE_LAYOUT_COUNTS)), **how)
+        ids2, weights2, xp2, logits = i32(T, top), torch.zeros((T, top), device=DEV), torch.full_like(xp, float("nan")), torch.zeros((T, E), device=DEV)
+        ops.route(h, W, top, ids2, weights2, logits=logits, **how)
+        assert torch.equal(ids, ids2) and torch.equal(weights, weights2)
+        assert ((logits.double() - h.double() @ W.double().T).abs() <= d * 2.0 ** -24 * (h.double().abs() @ W.double().abs().T)).all()
+        chosen, starts = ids.view(-1).long(), offsets.long()
+        assert torch.equal(starts, torch.cat([torch.zeros(1, device=DEV), torch.bincount(chosen, minlength=E).cumsum(0)]).long())
+        assert torch.equal(src_of.long(), torch.sort(chosen, stable=True).indices)           # inside an expert: the order of the assignments
+        assert torch.equal(row_of[src_of.long()].long(), torch.arange(A, device=DEV))
+        ops.route_gather(h, weights.view(-1), src_of, xp2, top, scale=scale_input)
+        assert torch.equal(xp, xp2)
+
+
+def test_routing_of_many_tokens_refuses_what_it_does_not_take(ops):
+    for T, E, d, n in ((2500, 256, 64, 8192), (300, 8, 36, 8192), (300, 8, 64, 100)):       # too many counts, rows of odd pieces, too little scratch
+        h, W = torch.randn(T, d, device=DEV), torch.randn(E, d, device=DEV)
+        i32 = lambda *n: torch.full(n, -7, dtype=torch.int32, device=DEV)
+        ids = i32(T, 2)
+        assert not ops.route_layout(h, W, 2, ids, torch.zeros((T, 2), device=DEV), i32(E + 1), i32(2 * T), i32(2 * T), torch.empty((2 * T, d), device=DEV),
+                                    False, i32(n))
+        assert (ids == -7).all()
