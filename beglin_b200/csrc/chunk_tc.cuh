@@ -20,7 +20,7 @@
 // other multiplies.
 #pragma once
 
-#include "ptx.cuh"
+#include "float_parts.cuh"
 
 namespace bg {
 
@@ -51,15 +51,12 @@ __device__ __forceinline__ unsigned ct_at(int row, int col) {
 }
 // four neighbouring columns (of a multiple of four) into the three parts, `part` bytes apart; two values a conversion
 __device__ __forceinline__ void ct_put4(unsigned char* tile, unsigned part, int row, int col, const float4& x) {
-    float2 a = make_float2(x.x, x.y), b = make_float2(x.z, x.w);
     unsigned char* d = tile + ct_at(row, col);
+    unsigned p[3], q[3];
+    gt_split(pair2(x.x, x.y), p[0], p[1], p[2]);
+    gt_split(pair2(x.z, x.w), q[0], q[1], q[2]);
 #pragma unroll
-    for (int i = 0; i < 3; ++i) {
-        const __nv_bfloat162 p = __floats2bfloat162_rn(a.x, a.y), q = __floats2bfloat162_rn(b.x, b.y);
-        *reinterpret_cast<uint2*>(d + i * part) = make_uint2(*reinterpret_cast<const unsigned*>(&p), *reinterpret_cast<const unsigned*>(&q));
-        const float2 pf = __bfloat1622float2(p), qf = __bfloat1622float2(q);
-        a.x -= pf.x; a.y -= pf.y; b.x -= qf.x; b.y -= qf.y;
-    }
+    for (int i = 0; i < 3; ++i) *reinterpret_cast<uint2*>(d + i * part) = make_uint2(p[i], q[i]);
 }
 __device__ __forceinline__ void ct_put1(unsigned char* tile, unsigned part, int row, int col, float x) {
     __nv_bfloat16 h, m, l;
@@ -104,6 +101,7 @@ __device__ __forceinline__ void ct_mma(unsigned d1, unsigned d2, unsigned a, uns
         return B_N ? smem_desc_sw128_nmajor(b + p * b_part + ks * 2048, CT_BLOCK, 1024)
                    : smem_desc_sw128(b + p * b_part + (ks >> 2) * CT_BLOCK + (ks & 3) * 32);
     };
+#pragma unroll 1
     for (int ks = 0; ks < steps; ++ks) {
         const unsigned long long ah = da(0, ks), am = da(1, ks), al = da(2, ks), bh = db(0, ks), bm = db(1, ks), bl = db(2, ks);
         tc_mma(d2, al, bh, idesc, first && ks == 0 ? 0u : 1u);
@@ -112,6 +110,7 @@ __device__ __forceinline__ void ct_mma(unsigned d1, unsigned d2, unsigned a, uns
         tc_mma(d2, am, bh, idesc, 1u);
         tc_mma(d2, ah, bm, idesc, 1u);
     }
+#pragma unroll 1
     for (int ks = 0; ks < steps; ++ks) tc_mma(ks < split ? d1 : d2, da(0, ks), db(0, ks), idesc, first && ks == 0 && split > 0 ? 0u : 1u);
 }
 __host__ __device__ constexpr unsigned ct_idesc(int n, bool a_m, bool b_n) { return instr_desc_bf16(128, n, b_n ? 1 : 0) | (a_m ? 1u << 15 : 0u); }
@@ -156,8 +155,9 @@ __device__ __forceinline__ void ct_wait(CtShared& s, unsigned& phase) {
     tc_fence_after();
 }
 
-// R: the policy.  R::Chunk c(r, h, ch, shared): what a CTA needs of its head and chunk (constructed by all threads, may meet at
-// barriers); c.rows; c.key_raw / c.key, c.value_raw / c.value; r.n, r.nv; r.sum_out(h, ch): A of the head and chunk, [n][r.nv_ld].
+// R: the policy.  R::Chunk c(r, h, ch, shared): a CTA's head and chunk; c.begin(): what else it makes for them, while the first fetches are on their
+// way (by all threads, ends with a barrier if it writes); c.rows; c.key_raw / c.key, c.value_raw / c.value; r.n, r.nv; r.sum_out(h, ch): A of
+// the head and chunk, [n][r.nv_ld].
 // (SN, SV: 4 for up to 64 features of keys, of values, 5 for up to 128)
 template <typename R, int SN, int SV>
 __global__ void __launch_bounds__(CT_THREADS, 2) chunk_sum_tc_kernel(R r) {
@@ -170,10 +170,11 @@ __global__ void __launch_bounds__(CT_THREADS, 2) chunk_sum_tc_kernel(R r) {
     ct_begin(s);
     pdl_wait();
     typename R::Chunk c(r, blockIdx.x, blockIdx.y, rs);
-    c.sum_begin();
     float4 raw[8], vals[8];
     ct_fetch<SN>(raw, r.n, [&](int j, int i) { return c.key_raw(j, i); });
     ct_fetch<SV>(vals, r.nv, [&](int j, int v) { return c.value_raw(j, v); });
+    c.begin();
+    c.sum_begin();
     ct_put<SN>(kt, part, raw, r.n, [&](const float4& x, int j, int i) { return c.key(x, j, i); });
     ct_put<SV>(vt, part, vals, r.nv, [&](const float4& x, int j, int v) { return c.value(x, j, v); });
     unsigned phase = 0;
@@ -186,8 +187,9 @@ __global__ void __launch_bounds__(CT_THREADS, 2) chunk_sum_tc_kernel(R r) {
         const unsigned lanes = (unsigned)((warp & 3) * 32) << 16;
         for (int i0 = (warp >> 2) * 16; i0 < r.n; i0 += 32) {
             unsigned a[16], b[16];
-            tc_ld16(d1 + lanes + i0, a);
-            tc_ld16(d2 + lanes + i0, b);
+            gt_ld16(d1 + lanes + i0, a);
+            gt_ld16(d2 + lanes + i0, b);
+            tc_wait_ld();
             if (v < r.nv) {
 #pragma unroll
                 for (int e = 0; e < 16; ++e) A[(size_t)(i0 + e) * r.nv_ld + v] = __uint_as_float(a[e]) + __uint_as_float(b[e]);
@@ -198,8 +200,16 @@ __global__ void __launch_bounds__(CT_THREADS, 2) chunk_sum_tc_kernel(R r) {
 }
 
 // Further members of R::Chunk: c.query_raw / c.query; with R::SCORES the weights are scores of this kernel's own: c.score_key_raw /
-// c.score_key, and c.weight(score, t, j) for j <= t; else c.weights(put) calls put(t, j, P) for every t, j < CT; r.state(h, ch): S;
-// c.factor(t); c.finish(values): values(t, v) gives o_t[v] from a float tile [CT][CT_OUT_LD] in shared memory, all threads call.
+// c.score_key, and c.weight(score, t, j) for j <= t; else c.weight_raw(x) fetches a thread's CT_WEIGHTS scores and c.weights(x, put) calls put(t, j, P)
+// for every t, j < CT, over all threads; r.state(h, ch): S; c.factor(t); c.finish_raw(t, v): what the results in columns v .. v + 3 need from
+// memory besides, c.finish(t, v, y, raw): their end, from the products' float4 y (lanes whose columns are there; t may be behind the rows).
+//
+// What a CTA waits for is hidden by the other one on its SM, not within it, so each phase's loads leave before the wait ahead of it.  Read at the
+// end (the values once more, the gate) or in a chain (the scores under their decays), they took a third to a half of a CTA's life: 33,600
+// cycles for Mamba-2, of which weights 7,300 and end 4,900, and 49,600 for the decay per channel, of which 21,200 were its norm and gate (2,048 tokens:
+// 59 -> 50 us for 24 heads of 128 x 128, 107 -> 88 for 32).  What is left is latency: without its MMAs the kernel takes 49 us of 58, without the
+// splits 50; loops stay rolled, since a CTA runs its 60 to 100 KB of straight code once.
+constexpr int CT_WEIGHTS = CT * CT / CT_THREADS;
 constexpr int CT_OUT_LD = 132;
 template <typename R, int SN, int SV>
 __global__ void __launch_bounds__(CT_THREADS, 2) chunk_out_tc_kernel(R r) {
@@ -214,7 +224,6 @@ __global__ void __launch_bounds__(CT_THREADS, 2) chunk_out_tc_kernel(R r) {
     ct_begin(s);
     pdl_wait();
     typename R::Chunk c(r, blockIdx.x, blockIdx.y, rs);
-    c.out_begin();
     const unsigned d = s.tmem, q_a = smem_u32(qt), x_a = smem_u32(xt);
     unsigned phase = 0;
     float4 raw[8];
@@ -225,7 +234,9 @@ __global__ void __launch_bounds__(CT_THREADS, 2) chunk_out_tc_kernel(R r) {
         });
     };
     auto value_fetch = [&] { ct_fetch<SV>(raw, r.nv, [&](int j, int v) { return c.value_raw(j, v); }); };
+    float weight_raw[R::SCORES ? 1 : CT_WEIGHTS];
     ct_fetch<SN>(raw, r.n, [&](int t, int i) { return c.query_raw(t, i); });
+    c.begin();
     ct_put<SN>(qt, part, raw, r.n, [&](const float4& x, int t, int i) { return c.query(x, t, i); });
     if constexpr (R::SCORES) {
         // S^T [key][query]: rows 64 to 127 of the left operand are whatever follows its tile and their results are not read
@@ -237,6 +248,7 @@ __global__ void __launch_bounds__(CT_THREADS, 2) chunk_out_tc_kernel(R r) {
     } else {
         state_fetch(0);
     }
+#pragma unroll 1
     for (int i0 = 0; i0 < r.n; i0 += 64) {
         const int w = min(64, r.n - i0);
         ct_put<SV>(xt, part, raw, r.nv, [&](const float4& x, int, int) { return x; });
@@ -245,7 +257,10 @@ __global__ void __launch_bounds__(CT_THREADS, 2) chunk_out_tc_kernel(R r) {
                                 ct_idesc(CT, true, false), i0 == 0);
         });
         if (i0 + 64 < r.n) state_fetch(i0 + 64);
-        else value_fetch();
+        else {
+            value_fetch();
+            if constexpr (!R::SCORES) c.weight_raw(weight_raw);
+        }
         ct_wait(s, phase);
     }
     if constexpr (R::SCORES) {
@@ -253,15 +268,16 @@ __global__ void __launch_bounds__(CT_THREADS, 2) chunk_out_tc_kernel(R r) {
             const int j = (warp & 3) * 32 + lane;
             for (int t0 = (warp >> 2) * 32; t0 < (warp >> 2) * 32 + 32; t0 += 16) {
                 unsigned a[16], b[16];
-                tc_ld16(d + lanes + t0, a);
-                tc_ld16(d + 64 + lanes + t0, b);
+                gt_ld16(d + lanes + t0, a);
+                gt_ld16(d + 64 + lanes + t0, b);
+                tc_wait_ld();
 #pragma unroll
                 for (int e = 0; e < 16; ++e)
                     ct_put1(qt, part, t0 + e, j, j <= t0 + e ? c.weight(__uint_as_float(a[e]) + __uint_as_float(b[e]), t0 + e, j) : 0.0f);
             }
         }
     } else {
-        c.weights([&](int t, int j, float w) { ct_put1(qt, part, t, j, w); });
+        c.weights(weight_raw, [&](int t, int j, float w) { ct_put1(qt, part, t, j, w); });
     }
     bool split = true;
     ct_put<SV>(xt, part, raw, r.nv, [&](const float4& x, int j, int v) {
@@ -279,19 +295,22 @@ __global__ void __launch_bounds__(CT_THREADS, 2) chunk_out_tc_kernel(R r) {
         }
     }
     ct_issue(s, [&] { ct_mma<true, false>(d, d + 64, x_a, part, q_a, part, CT / 16, CT / 32, ct_idesc(CT, true, false), true); });
+    ct_fetch<SV>(raw, r.nv, [&](int t, int v) { return c.finish_raw(t, v); });
     ct_wait(s, phase);
     float* out = reinterpret_cast<float*>(xt);               // [CT][CT_OUT_LD] (the weights stay where they are)
     {
         const int v = (warp & 3) * 32 + lane;
-        for (int t0 = (warp >> 2) * 32; t0 < (warp >> 2) * 32 + 32; t0 += 16) {
-            unsigned a[16], b[16], f[16], g[16];
-            tc_ld16(d + 128 + lanes + t0, a);
-            tc_ld16(d + 192 + lanes + t0, b);
-            tc_ld16(d + lanes + t0, f);
-            tc_ld16(d + 64 + lanes + t0, g);
+#pragma unroll 1
+        for (int t0 = (warp >> 2) * 32; t0 < (warp >> 2) * 32 + 32; t0 += 8) {
+            unsigned a[8], b[8], f[8], g[8];
+            gt_ld8(d + 128 + lanes + t0, a);
+            gt_ld8(d + 192 + lanes + t0, b);
+            gt_ld8(d + lanes + t0, f);
+            gt_ld8(d + 64 + lanes + t0, g);
+            tc_wait_ld();
             if (v < r.nv) {
 #pragma unroll
-                for (int e = 0; e < 16; ++e)
+                for (int e = 0; e < 8; ++e)
                     out[(t0 + e) * CT_OUT_LD + v] = fmaf(c.factor(t0 + e), __uint_as_float(a[e]) + __uint_as_float(b[e]),
                                                          __uint_as_float(f[e]) + __uint_as_float(g[e]));
             }
@@ -314,7 +333,16 @@ __global__ void __launch_bounds__(CT_THREADS, 2) chunk_out_tc_kernel(R r) {
         }
         __syncthreads();
     }
-    if (!s.failed) c.finish(out);
+    {                                        // the threads that fetched `raw`; a row's lanes all call, with or without columns
+        const int v = (threadIdx.x & ((1 << SV) - 1)) * 4, row = threadIdx.x >> SV;
+        if (!s.failed) {
+#pragma unroll
+            for (int u = 0; u < CT_PASSES<SV>; ++u) {
+                const int t = row + u * (CT_THREADS >> SV);
+                c.template finish<SV>(t, v, v < r.nv ? *reinterpret_cast<const float4*>(out + t * CT_OUT_LD + v) : make_float4(0.0f, 0.0f, 0.0f, 0.0f), raw[u]);
+            }
+        }
+    }
     ct_end(s, r.status);
 }
 

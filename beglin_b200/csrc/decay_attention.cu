@@ -430,17 +430,19 @@ struct DecayTc {
     __device__ const float* state(int h, int ch) const { return sum_out(h, ch); }
     struct Chunk {
         const DecayTc& r;
+        Shared& s;
         const float* src;
         const float* pw;
         int h, row0, rows;
-        __device__ Chunk(const DecayTc& r_, int h_, int ch, Shared& s) : r(r_), pw(s.pw), h(h_) {
+        __device__ Chunk(const DecayTc& r_, int h_, int ch, Shared& s_) : r(r_), s(s_), pw(s_.pw), h(h_) {
             row0 = r.p.chunks[ch * 4 + 1]; rows = r.p.chunks[ch * 4 + 2];
             src = (const float*)r.p.src + (size_t)row0 * r.p.src_stride;
+        }
+        __device__ void begin() {
             decay_powers(s.pw, r.p.decay[h]);
             __syncthreads();
         }
         __device__ void sum_begin() {}
-        __device__ void out_begin() {}
         // Rows that are not there are ones: a nought would send silu's division its slow way (12 heads of 128 x 128, a chunk of 16 rows: 47.9 us,
         // of 64 rows 34.6; as ones 34.0 and 35.3).  Their keys are multiplied by nought, their values by weights of nought, and their queries' results
         // go nowhere.
@@ -459,12 +461,9 @@ struct DecayTc {
         __device__ float4 score_key(const float4& x, int, int) const { return silu(x, 1.0f); }
         __device__ float weight(float score, int t, int j) const { return score * pw[t - j]; }
         __device__ float factor(int t) const { return pw[t + 1]; }
-        __device__ void finish(const float* o) const {
-            const int w4 = r.nv >> 2;
-            for (int idx = threadIdx.x; idx < rows * w4; idx += blockDim.x) {
-                const int t = idx / w4, v = (idx - t * w4) * 4;
-                *reinterpret_cast<float4*>(r.p.y + (size_t)(row0 + t) * r.p.H * r.nv + (size_t)h * r.nv + v) = *reinterpret_cast<const float4*>(o + t * CT_OUT_LD + v);
-            }
+        __device__ float4 finish_raw(int, int) const { return make_float4(0.0f, 0.0f, 0.0f, 0.0f); }
+        template <int SV> __device__ void finish(int t, int v, const float4& y, const float4&) const {
+            if (v < r.nv && t < rows) *reinterpret_cast<float4*>(r.p.y + (size_t)(row0 + t) * r.p.H * r.nv + (size_t)h * r.nv + v) = y;
         }
     };
 };

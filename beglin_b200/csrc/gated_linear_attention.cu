@@ -612,6 +612,7 @@ struct GlaTc {
     GlaParams p;
     int n, nv, nv_ld;
     unsigned* status;
+    int gate16;                                 // the gate's rows lie on 16-byte boundaries
     __device__ const float* state(int h, int ch) const { return p.work + ((size_t)ch * p.H + h) * n * nv; }
     struct Chunk {
         const GlaTc& r;
@@ -619,7 +620,7 @@ struct GlaTc {
         __device__ Chunk(const GlaTc& r_, int h_, int ch_, Shared&) : r(r_), h(h_), ch(ch_) {
             row0 = r.p.chunks[ch * 4 + 1]; rows = r.p.chunks[ch * 4 + 2];
         }
-        __device__ void out_begin() {}
+        __device__ void begin() {}
         __device__ float4 made(const float* x, int t, int i) const {         // of the prepared queries or keys
             return t < rows ? *reinterpret_cast<const float4*>(x + ((size_t)(row0 + t) * r.p.H + h) * r.n + i) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         }
@@ -631,34 +632,39 @@ struct GlaTc {
         __device__ float4 query_raw(int t, int i) const { return made(r.p.qd, t, i); }
         __device__ float4 query(const float4& x, int, int) const { return x; }
         __device__ float factor(int) const { return 1.0f; }
-        template <typename W> __device__ void weights(W put) const {
+        __device__ void weight_raw(float (&x)[CT_WEIGHTS]) const {
             const float* sc = r.p.scores + ((size_t)ch * r.p.H + h) * GC * GC;
-            float x[GC * GC / CT_THREADS];
 #pragma unroll
-            for (int u = 0; u < GC * GC / CT_THREADS; ++u) {
+            for (int u = 0; u < CT_WEIGHTS; ++u) {
                 const int idx = u * CT_THREADS + threadIdx.x, t = idx / GC, j = idx % GC;
                 x[u] = j <= t && t < rows ? sc[idx] : 0.0f;
             }
+        }
+        template <typename W> __device__ void weights(const float (&x)[CT_WEIGHTS], W put) const {
 #pragma unroll
-            for (int u = 0; u < GC * GC / CT_THREADS; ++u) {
+            for (int u = 0; u < CT_WEIGHTS; ++u) {
                 const int idx = u * CT_THREADS + threadIdx.x;
                 put(idx / GC, idx % GC, x[u]);
             }
         }
-        // the head's norm and gate: a warp per token, four columns a lane
-        __device__ void finish(const float* o) const {
-            const int warp = threadIdx.x >> 5, c = (threadIdx.x & 31) * 4;
-            for (int t = warp; t < rows; t += CT_THREADS / 32) {
-                const float4 x = c < r.nv ? *reinterpret_cast<const float4*>(o + t * CT_OUT_LD + c) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                const float total = warp_sum(x.x * x.x + x.y * x.y + x.z * x.z + x.w * x.w);
-                if (c >= r.nv) continue;
-                const float inv = 1.0f / sqrtf(total / (float)r.nv + r.p.eps);
-                const float* row = r.p.src + (size_t)(row0 + t) * r.p.src_stride;
-                const size_t at = (size_t)(row0 + t) * r.p.H * r.nv + (size_t)h * r.nv + c;
-                const float xs[4] = {x.x, x.y, x.z, x.w};
+        // the head's norm and gate: the 2^SV lanes of a row add up its squares
+        __device__ float4 finish_raw(int t, int v) const {
+            if (r.p.g_col < 0 || t >= rows) return make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            const float* g = r.p.src + (size_t)(row0 + t) * r.p.src_stride + r.p.g_col + h * r.nv + v;
+            return r.gate16 ? *reinterpret_cast<const float4*>(g) : make_float4(g[0], g[1], g[2], g[3]);
+        }
+        template <int SV> __device__ void finish(int t, int v, const float4& y, const float4& gate) const {
+            float total = y.x * y.x + y.y * y.y + y.z * y.z + y.w * y.w;
 #pragma unroll
-                for (int v = 0; v < 4; ++v) gla_store(r.p, at + v, xs[v] * inv * r.p.norm_w[c + v] * gla_gate(r.p, row, h, c + v));
-            }
+            for (int o = (1 << SV) / 2; o > 0; o >>= 1) total += __shfl_xor_sync(0xffffffffu, total, o);
+            if (v >= r.nv || t >= rows) return;
+            const float inv = 1.0f / sqrtf(total / (float)r.nv + r.p.eps);
+            const float4 w = make_float4(r.p.norm_w[v], r.p.norm_w[v + 1], r.p.norm_w[v + 2], r.p.norm_w[v + 3]);
+            float4 o = make_float4(y.x * inv * w.x, y.y * inv * w.y, y.z * inv * w.z, y.w * inv * w.w);
+            if (r.p.g_col >= 0) o = make_float4(o.x * gla_silu(gate.x), o.y * gla_silu(gate.y), o.z * gla_silu(gate.z), o.w * gla_silu(gate.w));
+            const __nv_bfloat162 a = __floats2bfloat162_rn(o.x, o.y), b = __floats2bfloat162_rn(o.z, o.w);
+            *reinterpret_cast<uint2*>((__nv_bfloat16*)r.p.out + (size_t)(row0 + t) * r.p.H * r.nv + (size_t)h * r.nv + v) =
+                make_uint2(*reinterpret_cast<const unsigned*>(&a), *reinterpret_cast<const unsigned*>(&b));
         }
     };
 };
@@ -771,9 +777,9 @@ extern "C" int bg_gla_chunked(const GlaArgs* args, const int* chunks, int n_chun
     BG_LAUNCH_CHECK();
     // (the float32 path, whose results leave as floats, uses no tensor cores; the sums that become the state stay on the float units, whose
     // error against 64 bits is the smaller: 1.20e-7 against 1.25e-7 for 2,048 rows of 16 heads of 128 x 128)
-    if (!p.out_float && ct_takes(p.n, p.nv) && p.vec) {
+    if (!p.out_float && ct_takes(p.n, p.nv) && p.vec && (uintptr_t)p.out % 8 == 0) {
         GlaTc r;
-        r.p = p; r.n = p.n; r.nv = r.nv_ld = p.nv; r.status = status;
+        r.p = p; r.n = p.n; r.nv = r.nv_ld = p.nv; r.status = status; r.gate16 = p.g_col % 4 == 0;
         launch(gla_chunk_sum_kernel, dim3(p.H, n_chunks, tiles), dim3(256), s_sum, stream, p);
         BG_LAUNCH_CHECK();
         launch(gla_chunk_scan_kernel, dim3((p.n * p.nv + 255) / 256, p.H, n_long), dim3(256), 0, stream, p);

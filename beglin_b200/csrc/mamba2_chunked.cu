@@ -74,6 +74,43 @@ __device__ __forceinline__ void sc_steps(const SsmChunkParams& p, int h, int row
     dt_s[t] = dt; a_s[t] = a; pre[t] = up; suf[t] = lane == 31 ? 1.0f : behind;
 }
 
+// The same for the tensor cores' kernels, by blocks of 16 tokens: in[t] = product from the block's start up to and with t; upto[t] = product from the chunk's
+// start up to and with t; behind[j] = product behind j to the chunk's end; to_end[j] the same to the block's end.  All threads call.
+template <typename TI, typename TW>
+__device__ __forceinline__ void sc_steps16(const SsmChunkParams& p, int h, int row0, int rows, float* dt_s, float* a_s, float* in, float* to_end,
+                                           float* upto, float* behind) {
+    const int t = threadIdx.x, lane = t & 15;
+    float up = 1.0f, down = 1.0f;
+    if (t < MC) {
+        float dt = 0.0f, a = 1.0f;
+        if (t < rows) {
+            dt = sc_softplus(to_float(((const TI*)p.src)[(size_t)(row0 + t) * p.src_stride + p.dt_col + h]) + to_float(((const TW*)p.dt_bias)[h]));
+            a = expf(-expf(to_float(((const TW*)p.A_log)[h])) * dt);
+        }
+        up = a; down = a;
+#pragma unroll
+        for (int o = 1; o < 16; o <<= 1) {
+            const float u = __shfl_up_sync(0xffffffffu, up, o), d = __shfl_down_sync(0xffffffffu, down, o);
+            if (lane >= o) up *= u;
+            if (lane + o < 16) down *= d;
+        }
+        down = __shfl_down_sync(0xffffffffu, down, 1);
+        if (lane == 15) down = 1.0f;
+        dt_s[t] = dt; a_s[t] = a; in[t] = up; to_end[t] = down;
+    }
+    __syncthreads();
+    if (t < MC) {
+        float before = 1.0f, after = 1.0f;
+        for (int b = 0; b < MC / 16; ++b) {
+            const float whole = in[b * 16 + 15];
+            if (b < t / 16) before *= whole;
+            if (b > t / 16) after *= whole;
+        }
+        upto[t] = before * up; behind[t] = down * after;
+    }
+    __syncthreads();
+}
+
 __global__ void __launch_bounds__(256) ssm_chunk_scores_kernel(SsmChunkParams p) {
     extern __shared__ __align__(16) float sc_s[];
     const int ld = p.N + 4;
@@ -303,7 +340,7 @@ __global__ void __launch_bounds__(128) ssm_chunk_out_kernel(SsmChunkParams p) {
 template <typename TI, typename TW>
 struct SsmTc {
     static constexpr bool SCORES = false;
-    struct Shared { float dt[MC], a[MC], pre[MC], suf[MC]; };
+    struct Shared { float dt[MC], a[MC], in[MC], to_end[MC], upto[MC], behind[MC]; };
     SsmChunkParams p;
     int n, nv, nv_ld;
     unsigned* status;
@@ -318,13 +355,11 @@ struct SsmTc {
             row0 = r.p.chunks[ch * 4 + 1]; rows = r.p.chunks[ch * 4 + 2];
             g = h / (r.p.H / r.p.G);
             row = r.p.xbc + (size_t)row0 * r.p.channels;
-            sc_steps<TI, TW>(r.p, h, row0, rows, s.dt, s.a, s.pre, s.suf);
-            __syncthreads();
         }
+        __device__ void begin() { sc_steps16<TI, TW>(r.p, h, row0, rows, s.dt, s.a, s.in, s.to_end, s.upto, s.behind); }
         __device__ void sum_begin() {
-            if (threadIdx.x == 0) r.p.decay[(size_t)ch * r.p.H + h] = s.pre[MC / 2 - 1] * s.pre[MC - 1];
+            if (threadIdx.x == 0) r.p.decay[(size_t)ch * r.p.H + h] = s.upto[MC - 1];
         }
-        __device__ void out_begin() {}
         __device__ float4 at(int t, int c) const {
             return t < rows ? *reinterpret_cast<const float4*>(row + (size_t)t * r.p.channels + c) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         }
@@ -332,43 +367,41 @@ struct SsmTc {
         __device__ float4 key(const float4& x, int, int) const { return x; }
         __device__ float4 value_raw(int j, int v) const { return at(j, h * r.nv + v); }
         __device__ float4 value(const float4& x, int j, int) const {       // times the step and the decay behind the token
-            const float w = s.dt[j] * (j < MC / 2 ? s.suf[j] * s.pre[MC - 1] : s.suf[j]);
+            const float w = s.dt[j] * s.behind[j];
             return make_float4(x.x * w, x.y * w, x.z * w, x.w * w);
         }
         __device__ float4 out_value(const float4& x, int, int) const { return x; }
         __device__ float4 query_raw(int t, int i) const { return at(t, r.p.H * r.nv + (r.p.G + g) * r.n + i); }
         __device__ float4 query(const float4& x, int, int) const { return x; }
-        __device__ float factor(int t) const { return (t >= MC / 2 ? s.pre[MC / 2 - 1] : 1.0f) * s.pre[t]; }
-        // the weight of key j at query t: score x (product of the decays behind j up to t) x step.  Threads 0 .. 63: the queries of the
-        // key's own half of the chunk, one decay after the other; 64 .. 127: those of the second half for keys of the first; 128 ..
-        // 191: noughts at the queries of the first half for keys of the second
-        template <typename W> __device__ void weights(W put) const {
-            const int j = threadIdx.x & (MC - 1), part = threadIdx.x / MC, half = j / (MC / 2);
-            const float* sc = r.p.scores + ((size_t)ch * r.p.G + g) * MC * MC + j;
-            if (part > 2 || (part == 1 && half == 1) || (part == 2 && half == 0)) return;
-            const int t_begin = part == 0 ? half * (MC / 2) : part == 1 ? MC / 2 : 0;
-            float l = part == 0 ? s.dt[j] : s.suf[j] * s.dt[j];
-            for (int t0 = t_begin; t0 < t_begin + MC / 2; t0 += 8) {
-                float x[8];
+        __device__ float factor(int t) const { return s.upto[t]; }
+        // the weight of key j at query t: score x (product of the decays behind j up to t) x step, for the 16 queries of one block: of the key's own
+        // block one decay after the other, of a later one with the key's product to its block's end and the blocks between
+        __device__ void weight_raw(float (&x)[CT_WEIGHTS]) const {
+            const int j = threadIdx.x & (MC - 1), t0 = threadIdx.x / MC * 16;
+            const float* sc = r.p.scores + (((size_t)ch * r.p.G + g) * MC + t0) * MC + j;
 #pragma unroll
-                for (int u = 0; u < 8; ++u) x[u] = part != 2 && t0 + u >= j ? sc[(size_t)(t0 + u) * MC] : 0.0f;
+            for (int u = 0; u < 16; ++u) x[u] = t0 + u >= j ? sc[(size_t)u * MC] : 0.0f;
+        }
+        template <typename W> __device__ void weights(const float (&x)[CT_WEIGHTS], W put) const {
+            const int j = threadIdx.x & (MC - 1), block = threadIdx.x / MC, t0 = block * 16;
+            float l = s.dt[j];
+            if (block > j / 16) {
+                l *= s.to_end[j];
+                for (int b = j / 16 + 1; b < block; ++b) l *= s.in[b * 16 + 15];
+            }
 #pragma unroll
-                for (int u = 0; u < 8; ++u) {
-                    const int t = t0 + u;
-                    if (part == 0 && t > j) l *= s.a[t];
-                    put(t, j, part == 1 ? x[u] * (l * s.pre[t]) : x[u] * l);
-                }
+            for (int u = 0; u < 16; ++u) {
+                const int t = t0 + u;
+                if (block == j / 16 && t > j) l *= s.a[t];
+                put(t, j, x[u] * (block > j / 16 ? l * s.in[t] : l));
             }
         }
-        __device__ void finish(const float* o) const {
-            const int w4 = r.nv >> 2;
+        __device__ float4 finish_raw(int t, int v) const { return value_raw(t, v); }
+        template <int SV> __device__ void finish(int t, int v, const float4& y, const float4& x) const {
+            if (v >= r.nv || t >= rows) return;
             const float D = to_float(((const TW*)r.p.D)[h]);
-            for (int idx = threadIdx.x; idx < rows * w4; idx += blockDim.x) {
-                const int t = idx / w4, v = (idx - t * w4) * 4;
-                const float4 x = at(t, h * r.nv + v), y = *reinterpret_cast<const float4*>(o + t * CT_OUT_LD + v);
-                *reinterpret_cast<float4*>(r.p.y + (size_t)(row0 + t) * r.p.H * r.nv + (size_t)h * r.nv + v) =
-                    make_float4(fmaf(D, x.x, y.x), fmaf(D, x.y, y.y), fmaf(D, x.z, y.z), fmaf(D, x.w, y.w));
-            }
+            *reinterpret_cast<float4*>(r.p.y + (size_t)(row0 + t) * r.p.H * r.nv + (size_t)h * r.nv + v) =
+                make_float4(fmaf(D, x.x, y.x), fmaf(D, x.y, y.y), fmaf(D, x.z, y.z), fmaf(D, x.w, y.w));
         }
     };
 };
