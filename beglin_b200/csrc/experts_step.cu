@@ -1,0 +1,134 @@
+// Routed experts of a step as ONE call from the host: the launches of routing, layout, products, activations and the sum per token, one behind the
+// other, on scratch that the caller allocates in one piece.  The kernels and their order are those of the single entries.  Outside a captured
+// step these launches are what bounds a small one: eight tokens with identity experts and a shared one took 121 us as eight entries of some twelve
+// arguments and seven tensors in all, for kernels of 42; as one call 47 (host 29).
+#include "common.cuh"
+
+extern "C" {
+int bg_route_rows(const void*, int, int, const float*, int, int, int, int, int, int, const float*, float, const float*, int*, float*, int*, int*, int*, void*, int,
+                  cudaStream_t);
+int bg_route_layout(const void*, int, int, const float*, int, int, int, int, int, int, const float*, float, const float*, int*, float*, int*, int*, int*, void*, int,
+                    int*, int, cudaStream_t);
+int bg_gemm_grouped_tc(const void*, int, int, int, int, const void*, int, int, void*, int, int, const int*, int, unsigned*, cudaStream_t);
+int bg_gemm_grouped_pair(const void*, int, int, int, int, const void*, int, int, void*, int, int, const int*, int, unsigned*, cudaStream_t);
+int bg_glu_clamped(const void*, int, int, void*, int, int, int, float, float, cudaStream_t);
+int bg_swiglu(const void*, int, int, long long, void*, int, int, int, int, int, float, cudaStream_t);
+int bg_gemm_fused(const void*, int, int, int, const void*, int, const float*, int, const float*, int, int, const void*, float, int, const float*, int, void*, int,
+                  int, float*, int, int, float, unsigned*, cudaStream_t);
+int bg_route_combine(const void*, int, const float*, const int*, float*, int, int, int, int, cudaStream_t);
+int bg_route_combine_ext(const void*, int, const float*, const int*, const int*, int, const void*, int, int, const float*, const void*, int, int, float*, int, int,
+                         int, cudaStream_t);
+}
+
+// A layer's experts, bfloat16: what does not change from step to step.  The host side fills the fields by name.
+struct ExpertsArgs {
+    const float* router; const float* choice_bias; const float* logit_bias;    // [outputs][hidden], [outputs] or null
+    const void* up; const void* down;                                           // [experts][intermediate (twice with a gate)][hidden], [experts][hidden][intermediate]
+    const void* shared_up; const void* shared_down;                             // [shared_rows][hidden], [hidden][shared], or null
+    unsigned* status;
+    int hidden, intermediate, experts, outputs, top, mode, renorm, scale_input;
+    int act;                    // of experts without a gate (gemm_grouped's)
+    int gated;                  // 0: no gate branch; 1: the clamped form; 2: silu
+    int extended;               // the sum per token with ids, identity experts and shared rows
+    int shared, shared_rows, shared_block, shared_gated, few;                  // few: tokens up to which route_rows takes a step
+    float route_scale, limit, shared_limit, alpha;
+};
+
+namespace {
+
+constexpr int EX_COUNTS = 8192;                // of bg_route_layout
+
+struct Scratch {
+    size_t ids, weights, offsets, row_of, src_of, counts, xp, gu, hp, yp, shared_gu, shared_act, shared_out, bytes;
+    int n_counts;
+    Scratch(const ExpertsArgs& a, int T) {
+        const size_t A = (size_t)T * a.top;
+        size_t at = 0;
+        auto take = [&](size_t n) { const size_t p = at; at += (n + 255) & ~(size_t)255; return p; };
+        n_counts = T <= a.few ? 0 : (int)((long long)T * a.outputs < EX_COUNTS ? (long long)T * a.outputs : EX_COUNTS);
+        ids = take(A * 4); weights = take(A * 4); offsets = take((size_t)(a.outputs + 1) * 4); row_of = take(A * 4); src_of = take(A * 4);
+        counts = take((size_t)n_counts * 4);
+        xp = take(A * a.hidden * 2);
+        gu = take(a.gated ? A * 2 * a.intermediate * 2 : 0);
+        hp = take(A * a.intermediate * 2);
+        yp = take(A * a.hidden * 4);
+        shared_gu = take((size_t)T * a.shared_rows * 4); shared_act = take((size_t)T * a.shared * 2); shared_out = take(a.shared ? (size_t)T * a.hidden * 4 : 0);
+        bytes = at;
+    }
+};
+
+}  // namespace
+
+using namespace bg;
+
+extern "C" long long bg_experts_scratch(const ExpertsArgs* a, int T) { return (long long)Scratch(*a, T).bytes; }
+
+// out [T][hidden] float = the step's result for h [T][hidden] bfloat16.  With a shared expert its rows come from the two fused products of few tokens
+// (up_splits and down_splits ranges of their inner sizes), or, with up_splits nought, from the caller: shared [T][hidden] float and, behind a gate, sg
+// (its type and stride).  `launched` counts the kernels.  BG_ERR_UNSUPPORTED, with nothing launched, where the routing does not take the sizes.
+extern "C" int bg_experts_step(const ExpertsArgs* args, const void* h, int T, int pairs, int up_splits, int down_splits, const float* shared,
+                               const void* sg, int sg_dtype, int sg_stride, void* scratch, long long scratch_bytes, float* out, int* launched,
+                               cudaStream_t stream) {
+    if (T <= 0) return BG_OK;
+    const ExpertsArgs& a = *args;
+    if (a.hidden <= 0 || a.hidden % 8 || a.intermediate <= 0 || a.intermediate % 8 || (uintptr_t)h % 16 || (uintptr_t)scratch % 16)
+        return BG_ERR_UNSUPPORTED;
+    const Scratch s(a, T);
+    if (scratch_bytes < (long long)s.bytes) return BG_ERR_SHAPE;
+    char* w = (char*)scratch;
+    int* ids = (int*)(w + s.ids); float* weights = (float*)(w + s.weights); int* offsets = (int*)(w + s.offsets);
+    int* row_of = (int*)(w + s.row_of); int* src_of = (int*)(w + s.src_of);
+    const int A = T * a.top, F = BG_DTYPE_F32, B = BG_DTYPE_BF16;
+    int rc, n = 0;
+    if (T <= a.few) {
+        rc = bg_route_rows(h, B, a.hidden, a.router, T, a.hidden, a.outputs, a.top, a.mode, a.renorm, a.choice_bias, a.route_scale, a.logit_bias, ids, weights,
+                           offsets, row_of, src_of, w + s.xp, a.scale_input, stream);
+        n = 1;
+    } else {
+        rc = bg_route_layout(h, B, a.hidden, a.router, T, a.hidden, a.outputs, a.top, a.mode, a.renorm, a.choice_bias, a.route_scale, a.logit_bias, ids, weights,
+                             offsets, row_of, src_of, w + s.xp, a.scale_input, (int*)(w + s.counts), s.n_counts, stream);
+        n = 2;
+    }
+    if (rc != BG_OK) return rc;
+    auto grouped = pairs ? bg_gemm_grouped_pair : bg_gemm_grouped_tc;
+    auto gate = [&](const void* gu, int dtype, int ld, void* to, int rows, int cols, float limit, int block) {
+        return a.gated == 1 ? bg_glu_clamped(gu, dtype, ld, to, B, rows, cols, limit, a.alpha, stream)
+                            : bg_swiglu(gu, dtype, 1, 0, to, B, rows, cols, block, 0, 0.0f, stream);
+    };
+    // (rows of experts without weights stay empty: the products see the first `experts` offsets only)
+    if (a.gated) {
+        rc = grouped(a.up, a.experts, 2 * a.intermediate, a.hidden, a.hidden, w + s.xp, A, a.hidden, w + s.gu, B, 2 * a.intermediate, offsets, 0, a.status, stream);
+        if (rc == BG_OK) rc = gate(w + s.gu, B, 2 * a.intermediate, w + s.hp, A, a.intermediate, a.limit, 0);
+        n += 2;
+    } else {
+        rc = grouped(a.up, a.experts, a.intermediate, a.hidden, a.hidden, w + s.xp, A, a.hidden, w + s.hp, B, a.intermediate, offsets, a.act, a.status, stream);
+        ++n;
+    }
+    if (rc == BG_OK) rc = grouped(a.down, a.experts, a.hidden, a.intermediate, a.intermediate, w + s.hp, A, a.intermediate, w + s.yp, F, a.hidden, offsets, 0, a.status, stream);
+    ++n;
+    if (rc == BG_OK && a.shared && up_splits) {
+        float* gu = (float*)(w + s.shared_gu);
+        if (a.shared_block) {
+            rc = bg_gemm_fused(a.shared_up, a.shared_rows, a.hidden, a.hidden, h, a.hidden, nullptr, 0, nullptr, 0, 0, nullptr, 0.0f, T, nullptr, 2, w + s.shared_act, B,
+                               a.shared, nullptr, 0, up_splits, 0.0f, a.status, stream);
+        } else {
+            rc = bg_gemm_fused(a.shared_up, a.shared_rows, a.hidden, a.hidden, h, a.hidden, nullptr, 0, nullptr, 0, 0, nullptr, 0.0f, T, nullptr, 0, gu, F, a.shared_rows,
+                               nullptr, 0, up_splits, 0.0f, a.status, stream);
+            if (rc == BG_OK) rc = gate(gu, F, a.shared_rows, w + s.shared_act, T, a.shared, a.shared_limit, 0);
+            ++n;
+        }
+        shared = (const float*)(w + s.shared_out);
+        if (rc == BG_OK)
+            rc = bg_gemm_fused(a.shared_down, a.hidden, a.shared, a.shared, w + s.shared_act, a.shared, nullptr, 0, nullptr, 0, 0, nullptr, 0.0f, T, nullptr, 0,
+                               w + s.shared_out, F, a.hidden, nullptr, 0, down_splits, 0.0f, a.status, stream);
+        n += 2;
+        sg = a.shared_gated ? gu + 2 * a.shared : nullptr;
+        sg_dtype = F; sg_stride = a.shared_rows;
+    }
+    if (rc == BG_OK)
+        rc = a.extended ? bg_route_combine_ext(w + s.yp, F, weights, row_of, ids, a.experts, h, B, a.hidden, a.shared ? shared : nullptr, a.shared ? sg : nullptr, sg_dtype,
+                                               sg_stride, out, T, a.hidden, a.top, stream)
+                        : bg_route_combine(w + s.yp, F, weights, row_of, out, T, a.hidden, a.top, a.scale_input ? 0 : 1, stream);
+    if (launched) *launched = n + 1;
+    return rc;
+}

@@ -76,6 +76,9 @@ _SIGNATURES = {
                       _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_void_p],
     "bg_route_layout": [_c_void_p, _c_int, _c_int, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void_p, _c_float, _c_void_p,
                         _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_void_p, _c_int, _c_void_p],
+    "bg_experts_scratch": [_c_void_p, _c_int],
+    "bg_experts_step": [_c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_void_p, _c_void_p, _c_int, _c_int, _c_void_p, _c_ll, _c_void_p,
+                        _c_void_p, _c_void_p],
     "bg_route_sort": [_c_void_p, _c_int, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_void_p],
     "bg_route_gather": [_c_void_p, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void_p],
     "bg_route_combine": [_c_void_p, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_void_p],
@@ -179,7 +182,7 @@ _SIGNATURES = {
                        _c_void_p],
 }
 
-_RESULTS = {"bg_gemm_f32_scratch": _c_ll}         # what does not return a code
+_RESULTS = {"bg_gemm_f32_scratch": _c_ll, "bg_experts_scratch": _c_ll}         # what does not return a code
 
 _lib = None
 
@@ -291,6 +294,11 @@ class _Outer(_Phase):
             super().__exit__(*exc)
         _depth -= 1
         return False
+
+
+def profiling() -> bool:
+    """Whether a profile is open, so that kernels have to be launched class by class."""
+    return _profile is not None
 
 
 def profile_begin() -> None:
@@ -2129,3 +2137,41 @@ def gemm_grouped(x: torch.Tensor, w: torch.Tensor, offsets: torch.Tensor, out: t
         else:
             _check(lib().bg_gemm_grouped(_p(x), _dt(x), K, _p(w), K, N * K, _p(out), _dt(out), N, _p(offsets), E, A, N, K, act,
                                          _stream()), "gemm_grouped")
+
+
+class ExpertsArgs(ctypes.Structure):
+    """What `experts_step` needs of a layer's experts (csrc/experts_step.cu says what the fields are)."""
+    _fields_ = [("router", _c_void_p), ("choice_bias", _c_void_p), ("logit_bias", _c_void_p), ("up", _c_void_p), ("down", _c_void_p),
+                ("shared_up", _c_void_p), ("shared_down", _c_void_p), ("status", _c_void_p), ("hidden", _c_int), ("intermediate", _c_int),
+                ("experts", _c_int), ("outputs", _c_int), ("top", _c_int), ("mode", _c_int), ("renorm", _c_int), ("scale_input", _c_int),
+                ("act", _c_int), ("gated", _c_int), ("extended", _c_int), ("shared", _c_int), ("shared_rows", _c_int), ("shared_block", _c_int),
+                ("shared_gated", _c_int), ("few", _c_int), ("route_scale", _c_float), ("limit", _c_float), ("shared_limit", _c_float), ("alpha", _c_float)]
+
+
+def experts_scratch(args: ExpertsArgs, T: int) -> int:
+    """Bytes of scratch that `experts_step` wants for T tokens."""
+    return lib().bg_experts_scratch(ctypes.byref(args), T)
+
+
+def experts_step(args: ExpertsArgs, h: torch.Tensor, scratch: torch.Tensor, out: torch.Tensor, up_splits: int = 0, down_splits: int = 0,
+                 shared: Optional[torch.Tensor] = None, sg: Optional[torch.Tensor] = None) -> bool:
+    """A step's routed experts as one call: h bfloat16 [T, hidden], scratch bytes, out float32 [T, hidden], all contiguous.  A shared expert runs
+    inside (`up_splits`, `down_splits`: the ranges of its two fused products) or comes as its rows `shared` float32 [T, hidden] and the gate's
+    numbers `sg` [T].  False, with nothing launched, where the routing does not take the sizes."""
+    T = h.shape[0]
+    if not h.is_cuda or h.dtype != torch.bfloat16 or not h.is_contiguous() or h.shape[1] != args.hidden or out.dtype != torch.float32 \
+            or tuple(out.shape) != (T, args.hidden) or not out.is_contiguous():
+        raise KernelError(f"experts_step: h bfloat16 [T, {args.hidden}], out float32 like it, contiguous on the device")
+    if shared is not None and (shared.dtype != torch.float32 or tuple(shared.shape) != (T, args.hidden) or not shared.is_contiguous()):
+        raise KernelError("experts_step: shared float32 [T, d]")
+    if args.shared and not up_splits and (shared is None or (sg is None) != (not args.shared_gated)):
+        raise KernelError("experts_step: the shared expert's rows (and gate) are missing")
+    n = _c_int(0)
+    rc = lib().bg_experts_step(ctypes.byref(args), h.data_ptr(), T, grouped_pairs(T * args.top, args.experts), up_splits, down_splits, _p(shared), _p(sg),
+                               F32 if sg is None else _dt(sg), 0 if sg is None else sg.stride(0), scratch.data_ptr(), scratch.numel(), out.data_ptr(),
+                               ctypes.byref(n), _stream())
+    if rc == _UNSUPPORTED:
+        return False
+    _check(rc, "experts_step")
+    count_launches(n.value - 1)
+    return True

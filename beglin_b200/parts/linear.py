@@ -79,6 +79,10 @@ class Linear:
         """Whether a step of T rows runs the fused product (bfloat16, few tokens, sizes it takes)."""
         return self._tc is not None and self._tc.fuses(T)
 
+    def fused_splits(self, T: int) -> int:
+        """The ranges of the inner size in which the fused product of T rows runs (only where `fuses`)."""
+        return self._tc.fused_splits(T)
+
     def _check_rows(self, x: torch.Tensor) -> None:
         if x.dtype != torch.bfloat16 or x.stride(1) != 1 or x.shape[1] != self.in_features or x.stride(0) % 8:
             raise ops.KernelError(f"the fused product takes contiguous bfloat16 rows of {self.in_features} features")

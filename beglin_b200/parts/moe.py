@@ -117,6 +117,44 @@ class RoutedExperts:
                 rows += [w, torch.zeros((7, w.shape[1]), dtype=w.dtype, device=w.device)]
             self.shared_up = Linear(torch.cat(rows, dim=0), None, ctx, label="proj_gate_up")
             self.shared_down = Linear(tensors["shared.down.weight"], None, ctx, label="proj_down")
+        self._args, self._scratch = self._step_args(outputs), {}
+
+    def _step_args(self, outputs: int):
+        """The layer as the one-call step takes it (bfloat16, inner sizes of whole 16-byte pieces), or None."""
+        s, sh = self.spec, self.spec.shared
+        if self.ctx.compute_dtype != torch.bfloat16 or not self.tensor_cores or s.hidden % 8 or s.intermediate % 8 or self.up.dtype != torch.bfloat16:
+            return None
+        ptr = lambda t: None if t is None else t.data_ptr()
+        return ops.ExpertsArgs(
+            router=ptr(self.router), choice_bias=ptr(self.choice_bias), logit_bias=ptr(self.logit_bias), up=ptr(self.up), down=ptr(self.down),
+            shared_up=ptr(self.shared_up.weight) if sh else None, shared_down=ptr(self.shared_down.weight) if sh else None, status=ptr(self.ctx.status),
+            hidden=s.hidden, intermediate=s.intermediate, experts=s.experts, outputs=outputs, top=s.top,
+            mode=ops.ROUTER_MODES[s.router_activation], renorm=int(s.renormalize), scale_input=int(s.scale_input),
+            act=0 if self.glu else ops.EXPERT_ACTIVATIONS[s.activation], gated=(1 if self.clamped else 2) if self.glu else 0, extended=int(self.extended),
+            shared=sh.intermediate if sh else 0, shared_rows=self.shared_up.out_features if sh else 0, shared_block=self.shared_block,
+            shared_gated=int(sh.gated) if sh else 0, few=ops.ROUTE_ROWS_TOKENS, route_scale=s.route_scale, limit=s.limit if self.clamped else 0.0,
+            shared_limit=sh.limit if sh and self.clamped else 0.0, alpha=1.702)
+
+    def _one_call(self, h: torch.Tensor):
+        """The whole step as one call, or None where it does not take the step (or kernel classes are being timed)."""
+        if self._args is None or ops.profiling() or h.dtype != torch.bfloat16 or not h.is_contiguous():
+            return None
+        T, s = h.shape[0], self.spec
+        up = down = 0
+        shared = gate = None
+        if s.shared is not None:
+            if s.shared.intermediate % 8 == 0 and self.shared_up.fuses(T) and self.shared_down.fuses(T):
+                up, down = self.shared_up.fused_splits(T), self.shared_down.fused_splits(T)
+            else:
+                shared, gate = self._shared(h)
+        size = self._scratch.get(T)
+        if size is None:
+            if len(self._scratch) >= 4096:
+                self._scratch.clear()
+            size = self._scratch[T] = ops.experts_scratch(self._args, T)
+        out = torch.empty((T, s.hidden), dtype=torch.float32, device=h.device)
+        scratch = torch.empty((size,), dtype=torch.uint8, device=h.device)
+        return out if ops.experts_step(self._args, h, scratch, out, up, down, shared, gate) else None
 
     def _gate(self, gate_up: torch.Tensor, out: torch.Tensor, limit: float, block: int = 0) -> None:
         """The experts' activation: gate_up [rows, >= 2 n] = [gate | up | ...] (or gate and up in turns of `block` columns)
@@ -126,11 +164,26 @@ class RoutedExperts:
         else:
             ops.swiglu(gate_up, out, block)
 
+    def _shared(self, h: torch.Tensor):
+        """The shared expert's rows, float32 [T, hidden], and the numbers of its gate [T] (None without one)."""
+        s, T = self.spec, h.shape[0]
+        im = s.shared.intermediate
+        act = self.shared_up.of(h, swiglu=True) if self.shared_block else None
+        if act is None:
+            # [T, gate | up (| the gate's number, zeros)]: float from the fused product of few rows, else in the compute type
+            gu = self.shared_up.full_f32(h) if self.shared_up.fuses(T) else self.shared_up(h)
+            act = torch.empty((T, im), dtype=self.ctx.compute_dtype, device=h.device)
+            self._gate(gu, act, s.shared.limit, self.shared_block)
+        return self.shared_down.full_f32(act), gu[:, 2 * im] if s.shared.gated else None
+
     def forward(self, h: torch.Tensor, batch, summed: bool = True):
         """h [T, hidden] in the compute type -> the sum of the chosen experts' results, float32 [T, hidden]; or, with
         `summed` False, the results as `RoutedRows`, for a consumer that adds them up itself."""
         if not isinstance(h, torch.Tensor):
             h = h.tensor()
+        out = self._one_call(h) if summed or self.extended else None
+        if out is not None:
+            return out
         s, dev, ct = self.spec, h.device, self.ctx.compute_dtype
         T, A = h.shape[0], h.shape[0] * s.top
         outputs = s.experts + s.identity
@@ -163,17 +216,7 @@ class RoutedExperts:
             out = torch.empty((T, s.hidden), dtype=torch.float32, device=dev)
             ops.route_combine(yp, weights.view(-1), row_of, out, s.top, scale=not s.scale_input)
             return out
-        shared = gate = None
-        if s.shared is not None:
-            im = s.shared.intermediate
-            act = self.shared_up.of(h, swiglu=True) if self.shared_block else None
-            if act is None:
-                # [T, gate | up (| the gate's number, zeros)]: float from the fused product of few rows, else in the compute type
-                gu = self.shared_up.full_f32(h) if self.shared_up.fuses(T) else self.shared_up(h)
-                act = torch.empty((T, im), dtype=ct, device=dev)
-                self._gate(gu, act, s.shared.limit, self.shared_block)
-            shared = self.shared_down.full_f32(act)
-            gate = gu[:, 2 * im] if s.shared.gated else None
+        shared, gate = self._shared(h) if s.shared is not None else (None, None)
         out = torch.empty((T, s.hidden), dtype=torch.float32, device=dev)
         ops.route_combine_ext(yp, weights.view(-1), row_of, ids.view(-1), s.experts, h, out, s.top, shared=shared, sg=gate)
         return out

@@ -1,0 +1,52 @@
+"""A step's routed experts as one call from the host beside the same step entry by entry: every form of layer, steps at the edges of what the
+routing's kernels and the shared expert's products take."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def layer(form, experts, top, gen, hidden=192, ff=136, shared_ff=128):
+    from beglin_b200.parts import registry
+    from beglin_b200.parts.context import BuildContext
+    from beglin_b200.parts.spec import RoutedExpertsSpec, SharedExpertSpec
+    identity = 2 if form == "clamped" else 0
+    how = {"plain": dict(activation="relu2"),
+           "clamped": dict(activation="glu_clamped", limit=7.0, router_activation="softmax", choice_bias=True, route_scale=2.5, identity=identity,
+                           scale_input=False, shared=SharedExpertSpec(intermediate=shared_ff, limit=5.0)),
+           "silu": dict(activation="swiglu", router_activation="softmax_chosen", logit_bias=True, scale_input=False,
+                        shared=SharedExpertSpec(intermediate=shared_ff, gated=False)),
+           "silu_odd": dict(activation="swiglu", scale_input=False, shared=SharedExpertSpec(intermediate=40, gated=False))}[form]
+    spec = RoutedExpertsSpec(hidden=hidden, intermediate=ff, experts=experts, top=top, **how)
+    cls = registry.part_class("feed_forward", spec.kind)
+    w = {r.name: torch.randn(r.shape, generator=gen).to(DEV, torch.bfloat16) * r.shape[-1] ** -0.5 for r in cls.expected_tensors(spec)}
+    return cls(spec, w, BuildContext(device=DEV, compute_dtype=torch.bfloat16, page_size=64, status=torch.zeros(1, dtype=torch.int32, device=DEV)))
+
+
+@pytest.mark.parametrize("form", ["plain", "clamped", "silu", "silu_odd"])
+@pytest.mark.parametrize("T", [1, 8, 9, 16, 17, 65, 300, 1100])
+def test_one_call_gives_the_bits_of_the_single_entries(form, T):
+    gen = torch.Generator().manual_seed(T)
+    part = layer(form, 4, 2, gen)
+    h = torch.randn(T, 192, generator=gen).to(DEV, torch.bfloat16)
+    from beglin_b200.csrc import ops
+    assert part._args is not None
+    before = ops.launch_count()
+    got = part.forward(h, None)
+    counted = ops.launch_count() - before
+    part._args = None
+    before = ops.launch_count()
+    want = part.forward(h, None)
+    assert torch.equal(got, want) and counted == ops.launch_count() - before
+    ops.raise_on_status(part.ctx.status)
+
+
+def test_one_call_leaves_sizes_of_odd_pieces_to_the_single_entries():
+    gen = torch.Generator().manual_seed(0)
+    assert layer("plain", 4, 2, gen, hidden=100)._args is None and layer("plain", 4, 2, gen, ff=36)._args is None
+    part = layer("plain", 300, 2, gen)                      # more experts than the layout's counts take: the routing refuses, the step runs all the same
+    h = torch.randn(40, 192, generator=gen).to(DEV, torch.bfloat16)
+    assert part._one_call(h) is None and part.forward(h, None).shape == (40, 192)
+    wide = torch.randn(8, 400, generator=gen).to(DEV, torch.bfloat16)
+    assert layer("plain", 4, 2, gen)._one_call(wide[:, :192]) is None       # rows that do not lie one behind the other
