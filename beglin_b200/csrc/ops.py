@@ -125,6 +125,8 @@ _SIGNATURES = {
                         _c_int, _c_int, _c_void_p, _c_void_p],
     "bg_gemm_pair": [_c_void_p, _c_int, _c_int, _c_int, _c_void_p, _c_int, _c_int, _c_void_p, _c_void_p, _c_int, _c_int,
                      _c_float, _c_void_p, _c_void_p],
+    "bg_gemm_heads": [_c_void_p, _c_int, _c_int, _c_int, _c_void_p, _c_ll, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void_p, _c_int, _c_ll, _c_int,
+                      _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_void_p, _c_void_p],
     "bg_gemm_fused": [_c_void_p, _c_int, _c_int, _c_int, _c_void_p, _c_int, _c_void_p, _c_int, _c_void_p, _c_int, _c_int,
                       _c_void_p, _c_float, _c_int, _c_void_p, _c_int, _c_void_p, _c_int, _c_int, _c_void_p, _c_int, _c_int,
                       _c_float, _c_void_p, _c_void_p],
@@ -160,6 +162,8 @@ _SIGNATURES = {
     "bg_latent_attention_tc_partial": [_c_void_p, _c_ll, _c_int, _c_void_p, _c_int, _c_int, _c_int, _c_void_p, _c_void_p, _c_int, _c_int,
                                        _c_void_p, _c_int, _c_void_p, _c_void_p, _c_int, _c_void_p, _c_void_p, _c_int, _c_int, _c_int,
                                        _c_int, _c_int, _c_int, _c_float, _c_void_p, _c_void_p],
+    "bg_latent_step_scratch": [_c_void_p, _c_int, _c_int],
+    "bg_latent_step": [_c_void_p, _c_void_p, _c_void_p],
     "bg_latent_gather": [_c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void_p, _c_void_p,
                          _c_void_p],
     "bg_latent_expand": [_c_void_p, _c_int, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_void_p, _c_void_p],
@@ -182,7 +186,7 @@ _SIGNATURES = {
                        _c_void_p],
 }
 
-_RESULTS = {"bg_gemm_f32_scratch": _c_ll, "bg_experts_scratch": _c_ll}         # what does not return a code
+_RESULTS = {"bg_gemm_f32_scratch": _c_ll, "bg_experts_scratch": _c_ll, "bg_latent_step_scratch": _c_ll}         # what does not return a code
 
 _lib = None
 
@@ -1180,6 +1184,36 @@ def gate_heads(src: torch.Tensor, gate: Optional[torch.Tensor], gate_col0: int, 
                "gate_heads")
 
 
+def gemm_heads(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, status: Optional[torch.Tensor] = None, gate: Optional[torch.Tensor] = None,
+               gate_col0: int = 0, per_feature: bool = False) -> None:
+    """The product that every head has of its own, for steps of few rows: x bfloat16 [H, T, K] (a view of a matrix in which a head's rows begin at
+    a column or a row of its own, K a multiple of 64), w bfloat16 [H, N, K] contiguous.  out is [H, T, N] (float32 or bfloat16, unit inner stride)
+    or the heads row by row, [T, H N], and there with `gate` as in `gate_heads`."""
+    _cuda(x, w, out, status, gate)
+    H, T, K = x.shape
+    N = w.shape[1]
+    if x.dtype != torch.bfloat16 or w.dtype != torch.bfloat16 or tuple(w.shape) != (H, N, K) or not w.is_contiguous() or x.stride(2) != 1 or K % 64:
+        raise KernelError("gemm_heads: x bfloat16 [H, T, K] with unit inner stride, w bfloat16 [H, N, K], K a multiple of 64")
+    head, row = x.stride(0), x.stride(1)
+    if T == 1 and row < K:
+        row = head                                  # (the stride of a single row says nothing)
+    if head < row or H == 1:
+        rows, cols, x_row, x_col = T, (H - 1) * head + K, 0, head if H > 1 else 0
+    elif row >= K and head % row == 0:
+        rows, cols, x_row, x_col = (H - 1) * (head // row) + T, K, head // row, 0
+    else:
+        raise KernelError(f"gemm_heads: heads {head} and rows {row} elements apart are not one matrix")
+    by_rows = out.dim() == 2
+    if tuple(out.shape) != ((T, H * N) if by_rows else (H, T, N)) or out.stride(-1) != 1 or (gate is not None and not by_rows):
+        raise KernelError(f"gemm_heads: out is {tuple(out.shape)}, expected {(H, T, N)} or {(T, H * N)} (with gates)")
+    if gate is not None and (gate.stride(1) != 1 or gate.shape[0] < T or gate_col0 + (H * N if per_feature else H) > gate.shape[1]):
+        raise KernelError("gemm_heads: gate rows that hold the gates from gate_col0")
+    with phase("proj_heads"):
+        _check(lib().bg_gemm_heads(_p(w), H, N, K, _p(x), rows, max(cols, K), max(row, cols), x_row, x_col, T, _p(out), _dt(out), N if by_rows else out.stride(0),
+                                   out.stride(0) if by_rows else out.stride(1), _p(gate), F32 if gate is None else _dt(gate),
+                                   0 if gate is None else gate.stride(0), gate_col0, 1 if per_feature else 0, _p(status), _stream()), "gemm_heads")
+
+
 def gemm_f32_nt_batched(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, status: Optional[torch.Tensor] = None) -> None:
     """out[b] = a[b] @ w[b]^T for a [B, M, K], w [B, N, K], out [B, M, N], float32 views of any batch and row
     strides with unit inner stride.  `status` as for gemm_f32_nt."""
@@ -1266,6 +1300,71 @@ def latent_splits(rows: int, keys: int, sms: Optional[int] = None) -> int:
     return lib().bg_latent_attention_tc_ranges(rows, keys, sm_count() if sms is None else sms)
 
 
+def latent_tc(H: int, rank: int, rot: int, pool: torch.Tensor, max_position: int, cos_sin: Optional[torch.Tensor]) -> bool:
+    """Whether a step of one row per request (decoding) runs on tcgen05: where the kernel takes the sizes, and from LATENT_TC_FROM positions on."""
+    return max_position >= LATENT_TC_FROM and pool.dtype == torch.bfloat16 and pool.data_ptr() % 16 == 0 \
+        and (cos_sin is None or cos_sin.data_ptr() % 8 == 0) and pool.shape[0] * pool.shape[1] <= 0x7fffffff \
+        and _latent_tc_plan(H, rank, rot, pool.shape[1])
+
+
+@functools.lru_cache(maxsize=1024)
+def _latent_tc_plan(H: int, rank: int, rot: int, page: int) -> bool:
+    return lib().bg_latent_attention_tc_plan(H, rank, rot, page) == 0
+
+
+def latent_ranges(tc: bool, n_qblk: int, H: int, max_position: int, split: int, window: int) -> Tuple[int, int, int]:
+    """(ranges of keys at most, positions a range or 0, CTAs that share the SMs or 0) of a step's attention through a latent."""
+    if not tc:
+        return max_position // split + 1, split, 0
+    keys = min(max_position + 1, window + LATENT_TC_KEYS) if window > 0 else max_position + 1      # a row's own keys spread over the SMs
+    ctas = n_qblk * -(-H // 32)
+    return latent_splits(ctas, -(-keys // LATENT_TC_KEYS) * LATENT_TC_KEYS, sm_count()), 0, ctas
+
+
+class LatentArgs(ctypes.Structure):
+    """What `latent_step` needs of a layer (csrc/latent_step.cu says what the fields are)."""
+    _fields_ = [(n, _c_void_p) for n in ("down", "q_up", "k_up_t", "v_up", "q_norm", "kv_norm", "sink", "status")] \
+        + [(n, _c_int) for n in ("hidden", "n_down", "q_rank", "kv_rank", "dim", "rot", "rot_dims", "vdim", "heads", "kv_col", "gate_col", "gated",
+                                 "per_feature", "norm_dtype", "window", "hc", "stages")] + [("eps", _c_float), ("scale", _c_float)]
+
+
+class LatentStep(ctypes.Structure):
+    """What a step brings to `latent_step`."""
+    _fields_ = [(n, _c_void_p) for n in ("h", "cos_sin", "positions", "row_req", "block_table", "pool", "qblk", "scratch")] \
+        + [("scratch_bytes", _c_ll), ("out", _c_void_p)] \
+        + [(n, _c_int) for n in ("T", "ldh", "max_pages", "num_pages", "page_size", "n_qblk", "bq", "tc", "n_splits", "split", "ctas", "down_fused",
+                                 "down_splits", "q_fused", "q_splits")]
+
+
+def latent_step(args: LatentArgs, h: torch.Tensor, cos_sin: Optional[torch.Tensor], positions: torch.Tensor, row_req: torch.Tensor,
+                block_table: torch.Tensor, pool: torch.Tensor, qblk: torch.Tensor, n_qblk: int, max_position: int, bq: int, split: int,
+                down: Tuple[bool, int], q: Tuple[bool, int]) -> torch.Tensor:
+    """A step of few rows from the mixer's input h bfloat16 [T, hidden] to its gated heads [T, heads * vdim] as one call: products, append,
+    attention and per-head products, with the arguments of `latent_append` and `latent_attention`.  `down`, `q`: the two products' kernel (fused
+    or plain) and its ranges of the inner size."""
+    _cuda(h, cos_sin, positions, row_req, block_table, pool, qblk)
+    _i32(positions, "positions"); _i32(row_req, "row_req"); _i32(block_table, "block_table"); _i32(qblk, "qblk")
+    T = h.shape[0]
+    if h.dtype != torch.bfloat16 or h.stride(1) != 1 or h.shape[1] != args.hidden or h.stride(0) % 8 or positions.numel() != T \
+            or pool.dtype != torch.bfloat16 or pool.dim() != 3 or pool.shape[2] != args.kv_rank + args.rot or not pool.is_contiguous():
+        raise KernelError("latent_step: h bfloat16 [T, hidden], one position per row, pool bfloat16 [pages, page, kv_rank + rot]")
+    if args.rot_dims > 0 and (cos_sin is None or cos_sin.dtype != torch.float32 or cos_sin.shape[0] < T
+                              or cos_sin.shape[1] != args.rot_dims // 2 or not cos_sin.is_contiguous()):
+        raise KernelError("latent_step: cos_sin must be float32 [T, rot_dims/2, 2]")
+    tc = bq == 1 and latent_tc(args.heads, args.kv_rank, args.rot, pool, max_position, cos_sin)
+    n_splits, split, ctas = latent_ranges(tc, n_qblk, args.heads, max_position, split, args.window)
+    a = ctypes.byref(args)
+    out = torch.empty((T, args.heads * args.vdim), dtype=torch.bfloat16, device=h.device)
+    size = lib().bg_latent_step_scratch(a, T, n_splits)
+    scratch = torch.empty((size,), dtype=torch.uint8, device=h.device)
+    s = LatentStep(h.data_ptr(), _p(cos_sin), positions.data_ptr(), row_req.data_ptr(), block_table.data_ptr(), pool.data_ptr(), qblk.data_ptr(),
+                   scratch.data_ptr(), size, out.data_ptr(), T, h.stride(0), block_table.shape[1], pool.shape[0], pool.shape[1], n_qblk, bq, tc,
+                   n_splits, split, ctas, down[0], down[1], q[0], q[1])
+    _check(_lib.bg_latent_step(a, ctypes.byref(s), _stream()), "latent_step")
+    count_launches(6)
+    return out
+
+
 def latent_attention(q_lat: torch.Tensor, q_raw: torch.Tensor, dim: int, rot: int, rot_dims: int,
                      cos_sin: Optional[torch.Tensor], pool: torch.Tensor, block_table: torch.Tensor,
                      positions: torch.Tensor, qblk: torch.Tensor, n_qblk: int, max_position: int, bq: int, hc: int,
@@ -1295,17 +1394,10 @@ def latent_attention(q_lat: torch.Tensor, q_raw: torch.Tensor, dim: int, rot: in
                          or cos_sin.shape[1] != rot_dims // 2 or not cos_sin.is_contiguous()):
         raise KernelError("latent_attention: cos_sin must be float32 [T, rot_dims/2, 2]")
     L = lib()
-    # one row per block (decoding) on tcgen05 where it takes the sizes: a row's own keys spread over the SMs
-    tc = bool(mma_stages) and bq == 1 and q_raw.dtype == pool.dtype == torch.bfloat16 \
-        and q_lat.stride(0) % 4 == 0 and q_lat.stride(1) % 4 == 0 and q_lat.data_ptr() % 16 == 0 and pool.data_ptr() % 16 == 0 \
-        and max_position >= LATENT_TC_FROM and (cos_sin is None or cos_sin.data_ptr() % 8 == 0) and pool.shape[0] * pool.shape[1] <= 0x7fffffff \
-        and L.bg_latent_attention_tc_plan(H, rank, rot, pool.shape[1]) == 0
-    if tc:
-        keys = min(max_position + 1, window + LATENT_TC_KEYS) if window > 0 else max_position + 1
-        split, ctas = 0, n_qblk * -(-H // 32)
-        n_splits = latent_splits(ctas, -(-keys // LATENT_TC_KEYS) * LATENT_TC_KEYS, sm_count())
-    else:
-        n_splits, ctas = max_position // split + 1, 0
+    tc = bool(mma_stages) and bq == 1 and q_raw.dtype == torch.bfloat16 \
+        and q_lat.stride(0) % 4 == 0 and q_lat.stride(1) % 4 == 0 and q_lat.data_ptr() % 16 == 0 \
+        and latent_tc(H, rank, rot, pool, max_position, cos_sin)
+    n_splits, split, ctas = latent_ranges(tc, n_qblk, H, max_position, split, window)
     part_o = torch.empty((T * H * n_splits, rank), dtype=torch.float32, device=q_lat.device)
     part_ml = torch.empty((T * H * n_splits, 2), dtype=torch.float32, device=q_lat.device)
     with phase("attn"):

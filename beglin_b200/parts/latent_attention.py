@@ -138,6 +138,51 @@ class LatentAttention:
                 self.expand = (bq, tile)
                 self.kv_up = ctx.matrix(torch.cat([tensors["k_up.weight"], tensors["v_up.weight"]], dim=0))
 
+        # steps of few rows: the per-head products as one kernel each, and all of the step as one call where every product is this package's
+        self.heads_tc = not self.f32 and ctx.gemm != "library" and spec.dim % 64 == 0 and spec.kv_rank % 64 == 0 and (spec.dim + spec.rot_dim) % 8 == 0 \
+            and self.k_up_t.dtype == torch.bfloat16
+        self._args = self._step_args()
+
+    def _step_args(self):
+        """The layer as the one-call step takes it, or None: bfloat16 with a query latent and a latent of its own, on the tensor cores."""
+        s, ctx = self.spec, self.ctx
+        if not self.heads_tc or self.mma is None or self.direct_q or not s.own_kv or self.q_norm.dtype != self.kv_norm.dtype:
+            return None
+        ptr = lambda t: None if t is None else t.data_ptr()
+        return ops.LatentArgs(
+            down=ptr(self.down.weight), q_up=ptr(self.q_up.weight), k_up_t=ptr(self.k_up_t), v_up=ptr(self.v_up), q_norm=ptr(self.q_norm),
+            kv_norm=ptr(self.kv_norm), sink=ptr(self.sink_weight), status=ptr(ctx.status), hidden=s.hidden, n_down=self.down.out_features, q_rank=s.q_rank,
+            kv_rank=s.kv_rank, dim=s.dim, rot=s.rot_dim, rot_dims=self.rot_dims, vdim=s.vdim, heads=s.n_heads, kv_col=self.kv_col, gate_col=self.gate_col,
+            gated=int(s.gated), per_feature=int(self.wide_gate), norm_dtype=ops.F32 if self.kv_norm.dtype == torch.float32 else ops.BF16, window=self.window,
+            hc=self.mma[0], stages=self.mma[2], eps=s.eps, scale=self.scale)
+
+    def _one_call(self, h: torch.Tensor, batch, cache) -> Optional[torch.Tensor]:
+        """The gated heads of a step of few rows as one call, or None where it does not take the step (or kernel classes are being timed)."""
+        T = batch.n_rows
+        if self._args is None or T > self.HEADS_ROWS or ops.profiling() or h.dtype != torch.bfloat16 or h.shape[0] != T or h.stride(1) != 1 or h.stride(0) % 8 \
+                or batch.positions.numel() != T \
+                or (self.wide_gate and T >= self.WIDE_ROWS):
+            return None
+        down, q = self.down.few_rows(T, True), self.q_up.few_rows(T, False)
+        if down is None or q is None:
+            return None
+        qblk, n_qblk, bq = self._query_blocks(batch)
+        return ops.latent_step(self._args, h, self.position.table(batch) if self.rot_dims else None, batch.positions, batch.row_req, cache.block_table,
+                               cache.pool, qblk, n_qblk, batch.max_position, bq, self.ctx.kv_split, down, q)
+
+    def _query_blocks(self, batch):
+        """(blocks of query rows, their number, rows a block) of the attention's kernel."""
+        bq = self.bq if self.mma is None else self.mma[1]
+        if getattr(batch, "decode_only", False):
+            bq = 1                                                      # one row per request: a CTA's rows are its heads
+        qblk, n_qblk = batch.query_blocks(bq)
+        if qblk is None:                                                # a decoding graph's batch keeps its list implicit
+            batch.implicit_blocks = False
+            qblk, n_qblk = batch.query_blocks(bq)
+        return qblk, n_qblk, bq
+
+    HEADS_ROWS = 64            # up to this many rows the per-head products run on this package's kernel (64 rows of 32 heads, both products and the
+                               # gates: 8.1 us, by the library and the gates' kernel 7.8; 14 rows 5.8 and 7.5), and a step may be one call
     WIDE_ROWS = 17             # from this many rows on gates per feature are a product of their own
     EXPAND_ROWS = 128          # portions of one request of at least this many rows make per-head keys and values
 
@@ -194,6 +239,9 @@ class LatentAttention:
         output product itself) or left owed to it, and None is returned; without, the addend is returned."""
         if isinstance(h, NormedInput):
             h = h.tensor()
+        heads = self._one_call(h, batch, cache)
+        if heads is not None:
+            return self._result(heads, stream)
         s, ctx = self.spec, self.ctx
         T, H = batch.n_rows, s.n_heads
         if self.wide_gate and T >= self.WIDE_ROWS:
@@ -218,22 +266,25 @@ class LatentAttention:
         if self.expand is not None and batch.n_req == 1 and T >= self.EXPAND_ROWS:
             return self._result(self._per_head_keys(q, gate, gate_col, cos_sin, batch, cache), stream)
         q_plain = q.view(T, H, s.dim + s.rot_dim)[:, :, :s.dim].transpose(0, 1)          # [H, T, dim]
-        q_lat = self._per_head(q_plain, self.k_up_t, torch.float32)    # [H, T, kv_rank] float
-        hc, bq, stages = (self.hc, self.bq, 0) if self.mma is None else self.mma
-        if getattr(batch, "decode_only", False):
-            bq = 1                                                      # one row per request: a CTA's rows are its heads
-        qblk, n_qblk = batch.query_blocks(bq)
-        if qblk is None:                                                # a decoding graph's batch keeps its list implicit
-            batch.implicit_blocks = False
-            qblk, n_qblk = batch.query_blocks(bq)
+        few = self.heads_tc and T <= self.HEADS_ROWS
+        if few:
+            q_lat = torch.empty((H, T, s.kv_rank), dtype=torch.float32, device=h.device)
+            ops.gemm_heads(q_plain, self.k_up_t, q_lat, ctx.status)
+        else:
+            q_lat = self._per_head(q_plain, self.k_up_t, torch.float32)    # [H, T, kv_rank] float
+        hc, stages = (self.hc, 0) if self.mma is None else (self.mma[0], self.mma[2])
+        qblk, n_qblk, bq = self._query_blocks(batch)
         split = ctx.kv_split
         o_lat = torch.empty((H, T, s.kv_rank), dtype=ctx.compute_dtype, device=h.device)
         ops.latent_attention(q_lat, q, s.dim, s.rot_dim, self.rot_dims, cos_sin, cache.pool, cache.block_table,
                              batch.positions, qblk, n_qblk, batch.max_position, bq, hc, self.tile, split,
                              self.scale, o_lat, ctx.status, mma_stages=stages, window=self.window, sink_weight=self.sink_weight)
-        v = self._per_head(o_lat, self.v_up, ctx.compute_dtype)        # [H, T, vdim]
         out = torch.empty((T, H * s.vdim), dtype=ctx.compute_dtype, device=h.device)
-        ops.gate_heads(v, gate if s.gated else None, gate_col, out, per_feature=self.wide_gate)      # (without gates: the heads row by row)
+        if few:
+            ops.gemm_heads(o_lat, self.v_up, out, ctx.status, gate if s.gated else None, gate_col, per_feature=self.wide_gate)
+        else:
+            v = self._per_head(o_lat, self.v_up, ctx.compute_dtype)        # [H, T, vdim]
+            ops.gate_heads(v, gate if s.gated else None, gate_col, out, per_feature=self.wide_gate)      # (without gates: the heads row by row)
         return self._result(out, stream)
 
     def _result(self, heads: torch.Tensor, stream: Optional[ResidualStream]) -> Optional[torch.Tensor]:

@@ -79,6 +79,16 @@ class Linear:
         """Whether a step of T rows runs the fused product (bfloat16, few tokens, sizes it takes)."""
         return self._tc is not None and self._tc.fuses(T)
 
+    def few_rows(self, T: int, full: bool):
+        """(whether the fused product runs, its ranges) for the complete product of T contiguous rows by `full_f32` (`full`) or by `__call__`, or
+        None where the tcgen05 products of few rows do not run."""
+        if self._tc is None or T > tensor_core.FEW_TOKENS or not (self._tc_always or self._tc.wins(T)):
+            return None
+        if full and self.fuses(T):
+            return True, self._tc.fused_splits(T)
+        s = self._tc.complete_splits(T)
+        return s > 1, s
+
     def fused_splits(self, T: int) -> int:
         """The ranges of the inner size in which the fused product of T rows runs (only where `fuses`)."""
         return self._tc.fused_splits(T)
