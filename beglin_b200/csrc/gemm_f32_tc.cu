@@ -469,12 +469,17 @@ static int gt_range(int N, int K) {
     return ((K + ranges - 1) / ranges + GT_BK - 1) / GT_BK * GT_BK;
 }
 
-// Cycles of a call, roughly: a stage takes the tensor cores 12 NT and the warps that cut some 1,000.
+// Cycles of a call, roughly, from those that a stage of each form was seen to take with most SMs at it: up to 96 tokens a stage waits for its bytes
+// (weights as floats and the tokens' parts, some 23 a cycle and SM), above for the tensor cores at the clock that their power leaves.  The sums of
+// ranges pass through memory.  In us, planned by 1,000 cycles a stage or the tensor cores' if that is more, and by these: 550 x 1,536 with k of
+// 1,536 33.4 and 29.3, 550 x 1,536 with 8,960 111 and 102, 424 x 3,136 with 3,072 77.7 and 71.6, 200 x 8,192 with 2,048 56.5 and 52.4,
+// 128 x 4,096 with 4,096 51.2 and 48.0.
+static double gt_stage(int nt) { return nt <= 16 ? 1430.0 : nt <= 32 ? 1900.0 : nt <= 64 ? 2250.0 : nt <= 96 ? 2650.0 : nt <= 128 ? 3000.0 : nt <= 144 ? 2750.0 : 2950.0; }
 static double gt_cost(int M, int N, int K, int batch, int range_len, int ranges, int nt, bool cut) {
     const long long slots = sm_count(), units = (long long)((M + nt - 1) / nt) * ((N + GT_BM - 1) / GT_BM) * batch * (cut ? ranges : 1);
-    const double stages = (double)((cut ? range_len : K) + GT_BK - 1) / GT_BK, stage = 60.0 + (12.0 * nt > 1000.0 ? 12.0 * nt : 1000.0);
+    const double stages = (double)((cut ? range_len : K) + GT_BK - 1) / GT_BK;
     const double rounds = (double)((units + slots - 1) / slots);
-    return 2000.0 + rounds * (stages * stage + 600.0 + (cut ? 0 : 20.0 * nt * (ranges - 1))) + (cut ? 5000.0 + 8.0 * M * N * ranges * batch / 2500.0 : 0.0);
+    return 2000.0 + rounds * (stages * gt_stage(nt) + 600.0 + (cut ? 0 : 20.0 * nt * (ranges - 1))) + (cut ? 5000.0 + 8.0 * M * N * ranges * batch / 2500.0 : 0.0);
 }
 
 static GtPlan gt_plan(int M, int N, int K, int batch) {
