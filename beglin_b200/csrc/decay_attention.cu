@@ -14,6 +14,7 @@
 //                                 starts, then every chunk's outputs in parallel (the earlier chunks through the state,
 //                                 the chunk's own tokens through their decayed scores).
 #include "common.cuh"
+#include "chunk_scan.cuh"
 #include "chunk_tc.cuh"
 
 namespace bg {
@@ -300,6 +301,28 @@ __global__ void __launch_bounds__(256) decay_chunk_scan_kernel(DecayChunkParams 
             }
     }
     *st = S;
+}
+
+// The same, four values a thread (heads of whole 16-byte pieces).
+__global__ void __launch_bounds__(CS_THREADS) decay_chunk_scan4_kernel(DecayChunkParams p) {
+    pdl_launch();
+    const int e = (blockIdx.x * blockDim.x + threadIdx.x) * 4, h = blockIdx.y, l = blockIdx.z, sz = p.n * p.nv;
+    const float d = p.decay[h], dfull = decay_power(d, DC);
+    pdl_wait();
+    if (e >= sz) return;
+    const int req = p.longs[l * 4 + 0], rows = p.longs[l * 4 + 2], c0 = p.longs[l * 4 + 3];
+    const int n_chunks = (rows + DC - 1) / DC;
+    const float dlast = decay_power(d, rows - (n_chunks - 1) * DC);
+    float4* st = reinterpret_cast<float4*>(p.state + (size_t)p.slots[req] * p.slot_stride + (size_t)h * sz + e);
+    *st = chunk_walk4(p.work + ((size_t)c0 * p.H + h) * sz + e, (size_t)p.H * sz, n_chunks, [&](int c) { return c == n_chunks - 1 ? dlast : dfull; }, *st);
+}
+static bool decay_scan4(const DecayChunkParams& p) {
+    return p.nv % 4 == 0 && p.slot_stride % 4 == 0 && (uintptr_t)p.state % 16 == 0 && (uintptr_t)p.work % 16 == 0;
+}
+static void decay_scan(const DecayChunkParams& p, int n_long, cudaStream_t stream) {
+    const int sz = p.n * p.nv;
+    if (decay_scan4(p)) launch(decay_chunk_scan4_kernel, dim3((sz / 4 + CS_THREADS - 1) / CS_THREADS, p.H, n_long), dim3(CS_THREADS), 0, stream, p);
+    else launch(decay_chunk_scan_kernel, dim3((sz + 255) / 256, p.H, n_long), dim3(256), 0, stream, p);
 }
 
 template <typename TS>
@@ -738,7 +761,7 @@ extern "C" int bg_decay_attention_chunked(const void* src, int src_dtype, int sr
         r.p = p; r.n = n; r.nv = r.nv_ld = nv; r.status = status;
         int rc = ct_sum(r, H, n_chunks, stream);
         if (rc != BG_OK) return rc;
-        launch(decay_chunk_scan_kernel, dim3((n * nv + 255) / 256, H, n_long), dim3(256), 0, stream, p);
+        decay_scan(p, n_long, stream);
         BG_LAUNCH_CHECK();
         rc = ct_out(r, H, n_chunks, stream);
         if (rc != BG_OK) return rc;
@@ -761,7 +784,7 @@ extern "C" int bg_decay_attention_chunked(const void* src, int src_dtype, int sr
         }
         launch(ksum, dim3(H, n_chunks), dim3(DC_THREADS), smem_sum, stream, p);
         BG_LAUNCH_CHECK();
-        launch(decay_chunk_scan_kernel, dim3((n * nv + 255) / 256, H, n_long), dim3(256), 0, stream, p);
+        decay_scan(p, n_long, stream);
         BG_LAUNCH_CHECK();
         launch(kout, dim3(H, n_chunks), dim3(DC_THREADS), smem_out, stream, p);
     });

@@ -20,6 +20,7 @@
 // over tokens of several blocks is split at the blocks' borders: (from the key's token to its block's end) x (whole blocks
 // between) x (from the start of the query's block to its token), each a running product of numbers in [0, 1].
 #include "common.cuh"
+#include "chunk_scan.cuh"
 #include "chunk_tc.cuh"
 
 namespace bg {
@@ -515,6 +516,27 @@ __global__ void __launch_bounds__(256) gla_chunk_scan_kernel(GlaParams p) {
     *st = S;
 }
 
+// The same, four values a thread (heads of whole 16-byte pieces).
+__global__ void __launch_bounds__(CS_THREADS) gla_chunk_scan4_kernel(GlaParams p) {
+    pdl_launch();
+    pdl_wait();
+    const int e = (blockIdx.x * blockDim.x + threadIdx.x) * 4, h = blockIdx.y, l = blockIdx.z, sz = p.n * p.nv;
+    if (e >= sz) return;
+    const int req = p.longs[l * 4 + 0], rows = p.longs[l * 4 + 2], c0 = p.longs[l * 4 + 3];
+    const int i = e / p.nv;
+    float4* st = reinterpret_cast<float4*>(p.state + (size_t)p.slots[req] * p.slot_stride + (size_t)h * sz + e);
+    const size_t pad = (size_t)p.np * p.nvp, dstep = (size_t)p.H * p.n;
+    const float* d0 = p.decay + ((size_t)c0 * p.H + h) * p.n + i;
+    *st = chunk_walk4(p.work + ((size_t)c0 * p.H + h) * pad + (size_t)i * p.nvp + (e - i * p.nv), (size_t)p.H * pad, (rows + GC - 1) / GC,
+                      [&](int c) { return d0[(size_t)c * dstep]; }, *st);
+}
+static void gla_scan(const GlaParams& p, int n_long, cudaStream_t stream) {
+    const int sz = p.n * p.nv;
+    if (p.nv % 4 == 0 && p.slot_stride % 4 == 0 && (uintptr_t)p.state % 16 == 0)          // (the scratch lies on 16 bytes)
+        launch(gla_chunk_scan4_kernel, dim3((sz / 4 + CS_THREADS - 1) / CS_THREADS, p.H, n_long), dim3(CS_THREADS), 0, stream, p);
+    else launch(gla_chunk_scan_kernel, dim3((sz + 255) / 256, p.H, n_long), dim3(256), 0, stream, p);
+}
+
 // The token that a thread's row u (of eight) stands for: a warp holds sixteen tokens, a half of it four neighbours and the four
 // eight further on, so that the two halves' reads of a tile of rows fall on different banks.
 __device__ __forceinline__ int gla_token(int u) {
@@ -782,7 +804,7 @@ extern "C" int bg_gla_chunked(const GlaArgs* args, const int* chunks, int n_chun
         r.p = p; r.n = p.n; r.nv = r.nv_ld = p.nv; r.status = status; r.gate16 = p.g_col % 4 == 0;
         launch(gla_chunk_sum_kernel, dim3(p.H, n_chunks, tiles), dim3(256), s_sum, stream, p);
         BG_LAUNCH_CHECK();
-        launch(gla_chunk_scan_kernel, dim3((p.n * p.nv + 255) / 256, p.H, n_long), dim3(256), 0, stream, p);
+        gla_scan(p, n_long, stream);
         BG_LAUNCH_CHECK();
         const int trc = ct_out(r, p.H, n_chunks, stream);
         if (trc != BG_OK) return trc;
@@ -791,7 +813,7 @@ extern "C" int bg_gla_chunked(const GlaArgs* args, const int* chunks, int n_chun
     }
     launch(gla_chunk_sum_kernel, dim3(p.H, n_chunks, tiles), dim3(256), s_sum, stream, p);
     BG_LAUNCH_CHECK();
-    launch(gla_chunk_scan_kernel, dim3((p.n * p.nv + 255) / 256, p.H, n_long), dim3(256), 0, stream, p);
+    gla_scan(p, n_long, stream);
     BG_LAUNCH_CHECK();
     const unsigned cluster = tiles <= 2 ? tiles : tiles <= 4 ? 4 : 8;
     launch_cluster(gla_chunk_out_kernel, dim3(p.H, n_chunks, cluster), dim3(128), s_out, stream, (int)cluster, p);

@@ -11,6 +11,7 @@
 // the chunk), never a quotient or a difference of sums, so that nothing cancels after a token with a large step.
 // Everything is float.  N and P are multiples of 4.  The slot's layout is that of ssm_scan_kernel: [H][P][N].
 #include "common.cuh"
+#include "chunk_scan.cuh"
 #include "chunk_tc.cuh"
 
 namespace bg {
@@ -235,6 +236,33 @@ __global__ void __launch_bounds__(256) ssm_chunk_scan_kernel(SsmChunkParams p) {
     *st = S;
 }
 
+// The same, four values a thread, for N and P that are multiples of 32: a block takes 32 x 32 values, whose slot is read and written in rows of
+// 128 bytes through shared memory (it is stored the other way round: value by value every 4 bytes moved 32).
+__global__ void __launch_bounds__(CS_THREADS) ssm_chunk_scan4_kernel(SsmChunkParams p) {
+    __shared__ float tile[32][33];             // [p][n]
+    pdl_launch();
+    pdl_wait();
+    const int h = blockIdx.y, l = blockIdx.z, sz = p.N * p.P, tiles = p.P / 32;
+    const int n0 = (int)blockIdx.x / tiles * 32, p0 = (int)blockIdx.x % tiles * 32, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int req = p.longs[l * 4 + 0], rows = p.longs[l * 4 + 2], c0 = p.longs[l * 4 + 3];
+    float* st = p.state + (size_t)p.slots[req] * p.slot_stride + (size_t)h * sz + (size_t)p0 * p.N + n0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) tile[warp + 8 * i][lane] = st[(size_t)(warp + 8 * i) * p.N + lane];
+    __syncthreads();
+    const int n = threadIdx.x >> 3, q = (threadIdx.x & 7) * 4;
+    const float* d0 = p.decay + (size_t)c0 * p.H + h;
+    const float4 S = chunk_walk4(p.work + ((size_t)c0 * p.H + h) * sz + (size_t)(n0 + n) * p.P + p0 + q, (size_t)p.H * sz, (rows + MC - 1) / MC,
+                                 [&](int c) { return d0[(size_t)c * p.H]; }, make_float4(tile[q][n], tile[q + 1][n], tile[q + 2][n], tile[q + 3][n]));
+    tile[q][n] = S.x; tile[q + 1][n] = S.y; tile[q + 2][n] = S.z; tile[q + 3][n] = S.w;      // (a thread's own places)
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 4; ++i) st[(size_t)(warp + 8 * i) * p.N + lane] = tile[warp + 8 * i][lane];
+}
+static void ssm_scan(const SsmChunkParams& p, int n_long, cudaStream_t stream) {
+    if (p.N % 32 == 0 && p.P % 32 == 0) launch(ssm_chunk_scan4_kernel, dim3(p.N / 32 * (p.P / 32), p.H, n_long), dim3(CS_THREADS), 0, stream, p);
+    else launch(ssm_chunk_scan_kernel, dim3((p.N * p.P + 255) / 256, p.H, n_long), dim3(256), 0, stream, p);
+}
+
 // The token that a thread's row u (of eight) stands for: a warp holds sixteen tokens, a half of it four neighbours and the four
 // eight further on, so that the two halves' reads of a tile of rows fall on different banks.
 __device__ __forceinline__ int sc_token(int u) {
@@ -456,7 +484,7 @@ extern "C" int bg_ssm_chunked(const float* xbc, int channels, const void* src, i
             r.p = p; r.n = N; r.nv = r.nv_ld = P; r.status = status;
             trc = ct_launch(chunk_sum_tc_kernel<SsmTc<TI, TW>, 5, 5>, r, H, n_chunks, stream);
             if (trc == BG_OK) {
-                launch(ssm_chunk_scan_kernel, dim3((N * P + 255) / 256, H, n_long), dim3(256), 0, stream, p);
+                ssm_scan(p, n_long, stream);
                 trc = ct_launch(chunk_out_tc_kernel<SsmTc<TI, TW>, 5, 5>, r, H, n_chunks, stream);
             }
         }));
@@ -477,7 +505,7 @@ extern "C" int bg_ssm_chunked(const float* xbc, int channels, const void* src, i
         }
         launch(ksum, dim3(H, n_chunks, tiles), dim3(256), s_sum, stream, p);
         BG_LAUNCH_CHECK();
-        launch(ssm_chunk_scan_kernel, dim3((N * P + 255) / 256, H, n_long), dim3(256), 0, stream, p);
+        ssm_scan(p, n_long, stream);
         BG_LAUNCH_CHECK();
         launch(kout, dim3(H, n_chunks, tiles), dim3(128), s_out, stream, p);
     }));
