@@ -15,6 +15,15 @@ namespace bg {
 __device__ __forceinline__ float softplus32(float z) { return fmaxf(z, 0.0f) + log1pf(expf(-fabsf(z))); }
 __device__ __forceinline__ float silu32(float z) { return z / (1.0f + expf(-z)); }
 __device__ __forceinline__ float sigmoid32(float z) { return 1.0f / (1.0f + expf(-z)); }
+// The gates of a result that leaves as TO: with the fast exponential and division (2^-20 of itself) where that is rounded to bfloat16.
+template <typename TO> __device__ __forceinline__ float gate_sigmoid(float z) {
+    if constexpr (sizeof(TO) == 2) return __fdividef(1.0f, 1.0f + __expf(-z));
+    else return sigmoid32(z);
+}
+template <typename TO> __device__ __forceinline__ float gate_silu(float z) {
+    if constexpr (sizeof(TO) == 2) return z * gate_sigmoid<TO>(z);
+    else return silu32(z);
+}
 
 // out[t, c] = silu(b[c] + sum_j w[c, j] * in(t - (taps-1-j), c)), in(.) taken from the step's rows of the same
 // request or, further back, from the slot's conv state.  src row = [.. | channels from col0 | ..].  `src_bias` [channels]
@@ -46,68 +55,71 @@ __global__ void conv_silu_kernel(const TI* __restrict__ src, int src_stride, int
     out[(size_t)t * channels + c] = act ? silu32(acc) : acc;
 }
 
+// Four neighbouring values as floats (on 16 bytes, bfloat16 on 8).
+__device__ __forceinline__ void conv_load4(const float* p, float (&v)[4]) {
+    const float4 x = *reinterpret_cast<const float4*>(p);
+    v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
+}
+__device__ __forceinline__ void conv_load4(const __nv_bfloat16* p, float (&v)[4]) {
+    const uint2 x = *reinterpret_cast<const uint2*>(p);
+    const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&x.x)), b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&x.y));
+    v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
+}
+// Four neighbouring results, and, where asked for, the two bfloat16 numbers of each (the rounding, and that of what it leaves out) as the recurrence's
+// gates want them: x2 [blocks][rows][2 bs].
+struct ConvSplit { __nv_bfloat16* x2; int bs; };
+__device__ __forceinline__ void conv_store4(float* out, int channels, int n_rows, int t, int c, const float (&o)[4], const ConvSplit& s) {
+    *reinterpret_cast<float4*>(out + (size_t)t * channels + c) = make_float4(o[0], o[1], o[2], o[3]);
+    if (!s.x2) return;
+    const __nv_bfloat162 h0 = __floats2bfloat162_rn(o[0], o[1]), h1 = __floats2bfloat162_rn(o[2], o[3]);
+    const float2 f0 = __bfloat1622float2(h0), f1 = __bfloat1622float2(h1);
+    const __nv_bfloat162 l0 = __floats2bfloat162_rn(o[0] - f0.x, o[1] - f0.y), l1 = __floats2bfloat162_rn(o[2] - f1.x, o[3] - f1.y);
+    const int blk = c / s.bs;
+    __nv_bfloat16* dst = s.x2 + ((size_t)blk * n_rows + t) * (2 * s.bs) + (c - blk * s.bs);
+    *reinterpret_cast<uint2*>(dst) = make_uint2(*reinterpret_cast<const unsigned*>(&h0), *reinterpret_cast<const unsigned*>(&h1));
+    *reinterpret_cast<uint2*>(dst + s.bs) = make_uint2(*reinterpret_cast<const unsigned*>(&l0), *reinterpret_cast<const unsigned*>(&l1));
+}
+
 // The same for float rows whose sizes are multiples of 4: a thread takes four channels of CONV_ROWS consecutive rows of the step and
-// keeps the last TAPS - 1 inputs in registers, so that an input is read once and not TAPS times, 16 bytes at a time; where a request
-// begins inside the run the inputs before it come from its state.  Every output is the same chain of multiply-adds.  Bound by bytes
-// (2,048 rows of 3,328 channels, four taps: 57 -> 20 us; 4,096 channels 70 -> 18).
+// keeps the last TAPS - 1 inputs in registers, so that an input is read once and not TAPS times, 16 bytes at a time.  Every output is the same chain
+// of multiply-adds.  The blocks behind those of the runs take a request each: its first TAPS - 1 rows, which reach back into the slot's state, and
+// the state after the step; so nobody else reads the state, and it needs no kernel of its own.  What bounds a run besides its bytes is what every
+// thread fetches for it, one trip to memory after the other: weights, request, the rows ahead (2,048 rows of 3,328 channels, four taps, and the
+// state: 24.8 us -> 17.9; 4,096 channels with float weights, the state and the two bfloat16 numbers of each result 33.7 in three kernels -> 18.6).
 constexpr int CONV_ROWS = 8, CONV_FROM = 96;
 template <typename TW, int TAPS>
 __global__ void __launch_bounds__(128)
 conv_silu_vec4_kernel(const float* __restrict__ src, int src_stride, int col0, int channels, const TW* __restrict__ w,
-                      const TW* __restrict__ b, const float* __restrict__ state, size_t slot_stride, size_t conv_off,
+                      const TW* __restrict__ b, float* __restrict__ state, size_t slot_stride, size_t conv_off,
                       const int* __restrict__ slots, const int* __restrict__ row_req, const int* __restrict__ reqs,
-                      float* __restrict__ out, int n_rows, int act, const float* __restrict__ src_bias) {
+                      float* __restrict__ out, int n_rows, int act, const float* __restrict__ src_bias, ConvSplit split) {
     // (no early start for the kernel behind: where that is the walk over a prompt, its few long-running blocks would be placed while these
     // fill the SMs, several to one SM, and 2,048 rows of 24 heads then took 1,387 us instead of 989)
-    const int c = (blockIdx.y * blockDim.x + threadIdx.x) * 4;
-    const int t0 = blockIdx.x * CONV_ROWS, t1 = min(t0 + CONV_ROWS, n_rows);
+    constexpr int KEEP = TAPS - 1;
+    const int c = (blockIdx.y * blockDim.x + threadIdx.x) * 4, runs = (n_rows + CONV_ROWS - 1) / CONV_ROWS;
     const bool live = c < channels;
     float wt[4][TAPS], bias[4], sb[4] = {0.0f, 0.0f, 0.0f, 0.0f};          // (written by no kernel of the step)
+    {
+        const int at = live ? c : 0;
+        float flat[TAPS][4];                                               // [channel][tap], one behind the other
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-        bias[e] = live ? to_float(b[c + e]) : 0.0f;
-        if (live && src_bias) sb[e] = src_bias[c + e];
+        for (int k = 0; k < TAPS; ++k) conv_load4(w + (size_t)at * TAPS + 4 * k, flat[k]);
+        conv_load4(b + at, bias);
+        if (src_bias) conv_load4(src_bias + at, sb);
 #pragma unroll
-        for (int k = 0; k < TAPS; ++k) wt[e][k] = live ? to_float(w[(size_t)(c + e) * TAPS + k]) : 0.0f;
+        for (int e = 0; e < 4; ++e)
+#pragma unroll
+            for (int k = 0; k < TAPS; ++k) wt[e][k] = flat[(e * TAPS + k) / 4][(e * TAPS + k) % 4];
     }
     pdl_wait();
     if (!live) return;
     const float* in = src + col0 + c;
-    float4 raw[CONV_ROWS];                 // the run's own rows, all on their way at once
-#pragma unroll
-    for (int u = 0; u < CONV_ROWS; ++u)
-        if (t0 + u < t1) raw[u] = *reinterpret_cast<const float4*>(in + (size_t)(t0 + u) * src_stride);
-    float v[TAPS][4];                      // the last inputs, the newest in v[TAPS - 1]
-    int req = -1;
-#pragma unroll
-    for (int u = 0; u < CONV_ROWS; ++u) {
-        const int t = t0 + u;
-        if (t >= t1) break;
-        const int r = row_req[t];
-        if (r != req) {                    // the run's first row, or a request's first: the inputs before it
-            req = r;
-            const int j = t - reqs[r * 3 + 1];                 // rows of this request before this one in the step
-            const float* st = state + (size_t)slots[r] * slot_stride + conv_off + c;
-#pragma unroll
-            for (int k = 1; k < TAPS; ++k) {                   // the input TAPS - k rows back goes to v[k], from where it moves down
-                const int back = TAPS - k;
-                float4 x;
-                if (back <= j) {
-                    x = *reinterpret_cast<const float4*>(in + (size_t)(t - back) * src_stride);
-                    x.x += sb[0]; x.y += sb[1]; x.z += sb[2]; x.w += sb[3];
-                } else {
-                    x = *reinterpret_cast<const float4*>(st + (size_t)(TAPS - 1 - (back - j)) * channels);
-                }
-                v[k][0] = x.x; v[k][1] = x.y; v[k][2] = x.z; v[k][3] = x.w;
-            }
-        }
-#pragma unroll
-        for (int k = 0; k + 1 < TAPS; ++k)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) v[k][e] = v[k + 1][e];
-        v[TAPS - 1][0] = raw[u].x + sb[0]; v[TAPS - 1][1] = raw[u].y + sb[1];
-        v[TAPS - 1][2] = raw[u].z + sb[2]; v[TAPS - 1][3] = raw[u].w + sb[3];
-        float o[4];
+    auto row = [&](int t) {
+        float4 x = *reinterpret_cast<const float4*>(in + (size_t)t * src_stride);
+        x.x += sb[0]; x.y += sb[1]; x.z += sb[2]; x.w += sb[3];
+        return x;
+    };
+    auto result = [&](const float (&v)[TAPS][4], float (&o)[4]) {
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
             float acc = bias[e];
@@ -115,7 +127,68 @@ conv_silu_vec4_kernel(const float* __restrict__ src, int src_stride, int col0, i
             for (int k = 0; k < TAPS; ++k) acc = fmaf(wt[e][k], v[k][e], acc);
             o[e] = act ? silu32(acc) : acc;
         }
-        *reinterpret_cast<float4*>(out + (size_t)t * channels + c) = make_float4(o[0], o[1], o[2], o[3]);
+    };
+    if ((int)blockIdx.x >= runs) {
+        const int r = blockIdx.x - runs, row0 = reqs[r * 3 + 1], n = reqs[r * 3 + 2];
+        if (n <= 0) return;
+        float* st = state + (size_t)slots[r] * slot_stride + conv_off + c;
+        float4 seen[2 * KEEP];                                             // the state, then the first rows
+#pragma unroll
+        for (int k = 0; k < KEEP; ++k) seen[k] = *reinterpret_cast<const float4*>(st + (size_t)k * channels);
+#pragma unroll
+        for (int k = 0; k < KEEP; ++k) seen[KEEP + k] = row(row0 + min(k, n - 1));
+        float4 keep[KEEP];
+#pragma unroll
+        for (int k = 0; k < KEEP; ++k) {
+            if (k + n >= KEEP) keep[k] = row(row0 + k + n - KEEP);
+            else {
+                keep[k] = seen[0];
+#pragma unroll
+                for (int i = 1; i < KEEP; ++i)
+                    if (k + n == i) keep[k] = seen[i];
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < KEEP; ++j) {
+            if (j >= n) break;
+            float v[TAPS][4], o[4];
+#pragma unroll
+            for (int k = 0; k < TAPS; ++k) { v[k][0] = seen[j + k].x; v[k][1] = seen[j + k].y; v[k][2] = seen[j + k].z; v[k][3] = seen[j + k].w; }
+            result(v, o);
+            conv_store4(out, channels, n_rows, row0 + j, c, o, split);
+        }
+#pragma unroll
+        for (int k = 0; k < KEEP; ++k) *reinterpret_cast<float4*>(st + (size_t)k * channels) = keep[k];
+        return;
+    }
+    const int t0 = blockIdx.x * CONV_ROWS, t1 = min(t0 + CONV_ROWS, n_rows);
+    // The run's rows and the KEEP ahead of them, all on their way at once.  Where a request begins inside the run or not far ahead of it, the rows
+    // ahead are another's: they reach its first KEEP rows only, which are left to its own block.
+    float4 raw[CONV_ROWS];
+#pragma unroll
+    for (int u = 0; u < CONV_ROWS; ++u) raw[u] = *reinterpret_cast<const float4*>(in + (size_t)min(t0 + u, t1 - 1) * src_stride);
+    float v[TAPS][4];                      // the last inputs, the newest in v[TAPS - 1]
+#pragma unroll
+    for (int k = 1; k < TAPS; ++k) {       // the input TAPS - k rows back goes to v[k], from where it moves down
+        const float4 x = row(max(t0 - (TAPS - k), 0));
+        v[k][0] = x.x; v[k][1] = x.y; v[k][2] = x.z; v[k][3] = x.w;
+    }
+    const int r0 = row_req[t0], r1 = row_req[t1 - 1], begin0 = reqs[r0 * 3 + 1];
+#pragma unroll
+    for (int u = 0; u < CONV_ROWS; ++u) {
+        const int t = t0 + u;
+        if (t >= t1) break;
+        const int begin = r0 == r1 ? begin0 : reqs[row_req[t] * 3 + 1];
+#pragma unroll
+        for (int k = 0; k + 1 < TAPS; ++k)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) v[k][e] = v[k + 1][e];
+        v[TAPS - 1][0] = raw[u].x + sb[0]; v[TAPS - 1][1] = raw[u].y + sb[1];
+        v[TAPS - 1][2] = raw[u].z + sb[2]; v[TAPS - 1][3] = raw[u].w + sb[3];
+        if (t - begin < KEEP) continue;
+        float o[4];
+        result(v, o);
+        conv_store4(out, channels, n_rows, t, c, o, split);
     }
 }
 
@@ -365,7 +438,7 @@ gated_group_rmsnorm_vec8_kernel(const float* __restrict__ y, const TI* __restric
             load8(src + (size_t)t * src_stride + z_col + i0 + c * 8, zg[it]);
 #pragma unroll
             for (int k = 0; k < 8; ++k) {
-                if (mode) zg[it][k] = sigmoid32(zg[it][k]); else { v[it][k] *= silu32(zg[it][k]); zg[it][k] = 1.0f; }
+                if (mode) zg[it][k] = gate_sigmoid<TO>(zg[it][k]); else { v[it][k] *= gate_silu<TO>(zg[it][k]); zg[it][k] = 1.0f; }
                 ss += v[it][k] * v[it][k];
             }
         }
@@ -395,34 +468,43 @@ using namespace bg;
 // one request 5.1 and 6.3, 96 6.2 and 6.4, 128 7.0 and 6.5, 256 10.2 and 7.1; 256 rows of 32 requests 10.2 and 7.8.
 extern "C" int bg_conv_silu_run(int n_rows, int n_req) { return n_rows >= CONV_FROM && n_rows >= CONV_ROWS * (long long)n_req ? CONV_ROWS : 1; }
 
-extern "C" int bg_conv_silu(const void* src, int src_dtype, int src_stride, int col0, int channels, int taps, const void* w,
-                            const void* b, int w_dtype, float* state, long long slot_stride, long long conv_off,
-                            const int* slots, const int* row_req, const int* reqs, int n_req, float* out, int n_rows,
-                            int act, const float* src_bias, cudaStream_t stream) {
+// out as conv_silu_kernel says; `x2` (with its `blocks`) or null: bfloat16 [blocks][n_rows][2 channels / blocks], rglru_split's of the result, only where
+// runs of rows are taken.  `launched` counts the kernels.
+static int conv_run(const void* src, int src_dtype, int src_stride, int col0, int channels, int taps, const void* w,
+                    const void* b, int w_dtype, float* state, long long slot_stride, long long conv_off, const int* slots, const int* row_req,
+                    const int* reqs, int n_req, float* out, int n_rows, int act, const float* src_bias, void* x2, int blocks, int* launched,
+                    cudaStream_t stream) {
+    if (launched) *launched = 0;
     if (n_rows <= 0 || n_req <= 0) return BG_OK;
-    if (channels <= 0 || taps < 1 || n_req > 65535) return BG_ERR_SHAPE;
+    if (channels <= 0 || taps < 1 || n_req > 65535 || (x2 && (blocks <= 0 || channels % blocks))) return BG_ERR_SHAPE;
     const unsigned bx = (unsigned)((channels + 127) / 128);
     if (bx > 65535) return BG_ERR_SHAPE;
-    // Runs of rows for 2 to 4 taps, where every row of inputs, state and outputs is made of whole 16-byte pieces.
-    if (src_dtype == BG_DTYPE_F32 && bg_conv_silu_run(n_rows, n_req) > 1 && taps >= 2 && taps <= 4 && channels % 4 == 0 && col0 % 4 == 0 && src_stride % 4 == 0 &&
-        slot_stride % 4 == 0 && conv_off % 4 == 0 && (uintptr_t)src % 16 == 0 && (uintptr_t)state % 16 == 0 && (uintptr_t)out % 16 == 0) {
-        const dim3 grid((n_rows + CONV_ROWS - 1) / CONV_ROWS, (channels / 4 + 127) / 128);
+    // Runs of rows for 2 to 4 taps, where every row of inputs, state and outputs and the weights are made of whole 16-byte pieces.
+    const bool runs = src_dtype == BG_DTYPE_F32 && bg_conv_silu_run(n_rows, n_req) > 1 && taps >= 2 && taps <= 4 && channels % 4 == 0 && col0 % 4 == 0 && src_stride % 4 == 0 &&
+        slot_stride % 4 == 0 && conv_off % 4 == 0 && (uintptr_t)src % 16 == 0 && (uintptr_t)state % 16 == 0 && (uintptr_t)out % 16 == 0 &&
+        (uintptr_t)w % 16 == 0 && (uintptr_t)b % 16 == 0 && (uintptr_t)src_bias % 16 == 0;
+    if (x2 && (!runs || channels / blocks % 4 || (uintptr_t)x2 % 8)) return BG_ERR_UNSUPPORTED;
+    if (runs) {
+        const dim3 grid((n_rows + CONV_ROWS - 1) / CONV_ROWS + n_req, (channels / 4 + 127) / 128);
+        const ConvSplit split = {(__nv_bfloat16*)x2, x2 ? channels / blocks : 1};
 #define BG_CONV(TAPS)                                                                                                          \
         launch(conv_silu_vec4_kernel<TW, TAPS>, grid, dim3(128), 0, stream, (const float*)src, src_stride, col0, channels,     \
-               (const TW*)w, (const TW*)b, (const float*)state, (size_t)slot_stride, (size_t)conv_off, slots, row_req, reqs,   \
-               out, n_rows, act, src_bias)
+               (const TW*)w, (const TW*)b, state, (size_t)slot_stride, (size_t)conv_off, slots, row_req, reqs,                 \
+               out, n_rows, act, src_bias, split)
         BG_DISPATCH_DTYPE(w_dtype, TW, {
             if (taps == 2) BG_CONV(2);
             else if (taps == 3) BG_CONV(3);
             else BG_CONV(4);
         });
 #undef BG_CONV
-    } else {
-        BG_DISPATCH_DTYPE(src_dtype, TI, BG_DISPATCH_DTYPE(w_dtype, TW,
-            launch(conv_silu_kernel<TI, TW>, dim3(n_rows, bx), dim3(128), 0, stream, (const TI*)src, src_stride, col0, channels,
-                   taps, (const TW*)w, (const TW*)b, (const float*)state, (size_t)slot_stride, (size_t)conv_off, slots, row_req,
-                   reqs, out, act, src_bias)));
+        BG_LAUNCH_CHECK();
+        if (launched) *launched = 1;
+        return BG_OK;
     }
+    BG_DISPATCH_DTYPE(src_dtype, TI, BG_DISPATCH_DTYPE(w_dtype, TW,
+        launch(conv_silu_kernel<TI, TW>, dim3(n_rows, bx), dim3(128), 0, stream, (const TI*)src, src_stride, col0, channels,
+               taps, (const TW*)w, (const TW*)b, (const float*)state, (size_t)slot_stride, (size_t)conv_off, slots, row_req,
+               reqs, out, act, src_bias)));
     BG_LAUNCH_CHECK();
     if (taps > 1) {
         BG_DISPATCH_DTYPE(src_dtype, TI,
@@ -430,7 +512,27 @@ extern "C" int bg_conv_silu(const void* src, int src_dtype, int src_stride, int 
                    taps, state, (size_t)slot_stride, (size_t)conv_off, slots, reqs, src_bias));
         BG_LAUNCH_CHECK();
     }
+    if (launched) *launched = taps > 1 ? 2 : 1;
     return BG_OK;
+}
+
+extern "C" int bg_conv_silu(const void* src, int src_dtype, int src_stride, int col0, int channels, int taps, const void* w,
+                            const void* b, int w_dtype, float* state, long long slot_stride, long long conv_off,
+                            const int* slots, const int* row_req, const int* reqs, int n_req, float* out, int n_rows,
+                            int act, const float* src_bias, int* launched, cudaStream_t stream) {
+    return conv_run(src, src_dtype, src_stride, col0, channels, taps, w, b, w_dtype, state, slot_stride, conv_off, slots, row_req, reqs, n_req, out, n_rows,
+                    act, src_bias, nullptr, 0, launched, stream);
+}
+
+// The convolution without an activation and bg_rglru_split of its result in one kernel; BG_ERR_UNSUPPORTED, with nothing launched, where its rows are
+// not taken in runs.
+extern "C" int bg_conv_split(const void* src, int src_dtype, int src_stride, int col0, int channels, int taps, const void* w,
+                             const void* b, int w_dtype, float* state, long long slot_stride, long long conv_off,
+                             const int* slots, const int* row_req, const int* reqs, int n_req, float* out, int n_rows,
+                             const float* src_bias, void* x2, int blocks, cudaStream_t stream) {
+    if (!x2) return BG_ERR_SHAPE;
+    return conv_run(src, src_dtype, src_stride, col0, channels, taps, w, b, w_dtype, state, slot_stride, conv_off, slots, row_req, reqs, n_req, out, n_rows,
+                    0, src_bias, x2, blocks, nullptr, stream);
 }
 
 // How the scan lays a head's state over CTAs: tiles of PT columns p, NS lanes per column (a power of two up to 32),

@@ -112,42 +112,46 @@ __device__ __forceinline__ void sc_steps16(const SsmChunkParams& p, int h, int r
     __syncthreads();
 }
 
+// A block takes MQ queries of a chunk, so that one group's chunks of a prompt fill more than a few SMs (32 chunks of one group 8.9 us with a block
+// a chunk -> 6.7).
+constexpr int MQ = 16;
 __global__ void __launch_bounds__(256) ssm_chunk_scores_kernel(SsmChunkParams p) {
     extern __shared__ __align__(16) float sc_s[];
     const int ld = p.N + 4;
-    float* Cs = sc_s;                      // [MC][N + 4]
-    float* Bs = Cs + MC * ld;              // [MC][N + 4]
+    float* Bs = sc_s;                      // [MC][N + 4]
+    float* Cs = Bs + MC * ld;              // [MQ][N + 4]
     pdl_launch();
     pdl_wait();
-    const int g = blockIdx.x, ch = blockIdx.y;
+    const int g = blockIdx.x, ch = blockIdx.y, t0 = blockIdx.z * MQ;
     const int row0 = p.chunks[ch * 4 + 1], rows = p.chunks[ch * 4 + 2];
     const float* base = p.xbc + (size_t)row0 * p.channels + (size_t)p.H * p.P + (size_t)g * p.N;
     sc_rows(Bs, ld, base, p.channels, rows, p.N);
-    sc_rows(Cs, ld, base + (size_t)p.G * p.N, p.channels, rows, p.N);
+    {
+        const int w4 = p.N >> 2;
+        const float* C = base + (size_t)p.G * p.N;
+        for (int idx = threadIdx.x; idx < MQ * w4; idx += blockDim.x) {
+            const int r = idx / w4, c = (idx - r * w4) * 4;
+            if (t0 + r < rows) sc_async16(Cs + r * ld + c, C + (size_t)(t0 + r) * p.channels + c);
+            else *reinterpret_cast<float4*>(Cs + r * ld + c) = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        }
+    }
     sc_async_wait();
     __syncthreads();
-    // a thread takes queries ty, ty + 16, .. and keys tx, tx + 16, ..
+    // a thread takes query t0 + ty and keys tx, tx + 16, ..
     const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    float acc[4][4] = {};
-#pragma unroll 2
+    float acc[4] = {};
+#pragma unroll 4
     for (int n = 0; n < p.N; n += 4) {
-        float4 c[4], b[4];
+        const float4 c = *reinterpret_cast<const float4*>(Cs + ty * ld + n);
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            c[u] = *reinterpret_cast<const float4*>(Cs + (ty + 16 * u) * ld + n);
-            b[u] = *reinterpret_cast<const float4*>(Bs + (tx + 16 * u) * ld + n);
+        for (int v = 0; v < 4; ++v) {
+            const float4 b = *reinterpret_cast<const float4*>(Bs + (tx + 16 * v) * ld + n);
+            acc[v] = fmaf(c.x, b.x, fmaf(c.y, b.y, fmaf(c.z, b.z, fmaf(c.w, b.w, acc[v]))));
         }
-#pragma unroll
-        for (int u = 0; u < 4; ++u)
-#pragma unroll
-            for (int v = 0; v < 4; ++v)
-                acc[u][v] = fmaf(c[u].x, b[v].x, fmaf(c[u].y, b[v].y, fmaf(c[u].z, b[v].z, fmaf(c[u].w, b[v].w, acc[u][v]))));
     }
-    float* out = p.scores + ((size_t)ch * p.G + g) * MC * MC;
+    float* out = p.scores + (((size_t)ch * p.G + g) * MC + t0 + ty) * MC;
 #pragma unroll
-    for (int u = 0; u < 4; ++u)
-#pragma unroll
-        for (int v = 0; v < 4; ++v) out[(ty + 16 * u) * MC + tx + 16 * v] = acc[u][v];
+    for (int v = 0; v < 4; ++v) out[tx + 16 * v] = acc[v];
 }
 
 template <typename TI, typename TW>
@@ -434,7 +438,7 @@ struct SsmTc {
     };
 };
 
-static size_t sc_smem_scores(int N) { return (size_t)2 * MC * (N + 4) * sizeof(float); }
+static size_t sc_smem_scores(int N) { return (size_t)(MC + MQ) * (N + 4) * sizeof(float); }
 static size_t sc_smem_sum(int N) { return ((size_t)MC * N + (size_t)MC * MPT) * sizeof(float); }
 static size_t sc_smem_out(int N) { return ((size_t)MC * (N + 4) + (size_t)N * MPT + (size_t)MC * MPT + (size_t)MC * MCP) * sizeof(float); }
 
@@ -472,7 +476,7 @@ extern "C" int bg_ssm_chunked(const float* xbc, int channels, const void* src, i
         cudaError_t e = cudaFuncSetAttribute(ssm_chunk_scores_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s_scores);
         if (e != cudaSuccess) return (int)e;
     }
-    launch(ssm_chunk_scores_kernel, dim3(G, n_chunks), dim3(256), s_scores, stream, p);
+    launch(ssm_chunk_scores_kernel, dim3(G, n_chunks, MC / MQ), dim3(256), s_scores, stream, p);
     BG_LAUNCH_CHECK();
     // from 80 features on both sides: 24 heads of 128 x 128, 2,048 tokens, 180 -> 121 us; with 64 on one side the conversions cost what the
     // float units need for the products (12 heads of 64 x 128, 2,174 tokens: 70 us there, 78 here)

@@ -69,7 +69,7 @@ _SIGNATURES = {
                       _c_void_p, _c_void_p, _c_int, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_void_p],
     "bg_rglru_scan_chunked": [_c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_ll,
                               _c_void_p, _c_void_p, _c_int, _c_void_p, _c_int, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_int,
-                              _c_int, _c_int, _c_void_p],
+                              _c_int, _c_int, _c_void_p, _c_void_p],
     "bg_rglru_softplus": [_c_void_p, _c_int, _c_float, _c_void_p, _c_int, _c_void_p],
     "bg_rglru_split": [_c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_void_p],
     "bg_route_rows": [_c_void_p, _c_int, _c_int, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void_p, _c_float, _c_void_p,
@@ -170,7 +170,9 @@ _SIGNATURES = {
     "bg_rotate_q": [_c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void_p, _c_int, _c_void_p],
     "bg_conv_silu_run": [_c_int, _c_int],
     "bg_conv_silu": [_c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void_p, _c_void_p, _c_int, _c_void_p, _c_ll, _c_ll,
-                     _c_void_p, _c_void_p, _c_void_p, _c_int, _c_void_p, _c_int, _c_int, _c_void_p, _c_void_p],
+                     _c_void_p, _c_void_p, _c_void_p, _c_int, _c_void_p, _c_int, _c_int, _c_void_p, _c_void_p, _c_void_p],
+    "bg_conv_split": [_c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void_p, _c_void_p, _c_int, _c_void_p, _c_ll, _c_ll,
+                      _c_void_p, _c_void_p, _c_void_p, _c_int, _c_void_p, _c_int, _c_void_p, _c_void_p, _c_int, _c_void_p],
     "bg_ssm_scan": [_c_void_p, _c_int, _c_void_p, _c_int, _c_int, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_void_p,
                     _c_ll, _c_void_p, _c_void_p, _c_int, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_void_p],
     "bg_ssm_chunk_plan": [_c_int, _c_int, _c_int, _c_int, ctypes.POINTER(_c_int)],
@@ -1479,13 +1481,14 @@ def rotate_q(q: torch.Tensor, H: int, head: int, off: int, rot_dims: int, cos_si
 # The Mamba-2 recurrence
 def conv_silu(src: torch.Tensor, col0: int, channels: int, weight: torch.Tensor, bias: torch.Tensor, state: torch.Tensor,
               conv_off: int, slots: torch.Tensor, row_req: torch.Tensor, reqs: torch.Tensor, n_req: int,
-              out: torch.Tensor, activation: str = "silu", src_bias: Optional[torch.Tensor] = None) -> None:
+              out: torch.Tensor, activation: str = "silu", src_bias: Optional[torch.Tensor] = None, split: Optional[torch.Tensor] = None) -> None:
     """The causal convolution per channel with SiLU (`activation` "none": without it) over src[:, col0 : col0 + channels],
     continued from and into the slots' conv state (`src_bias` float32 [channels], when given, is added to the rows' inputs,
     and the state keeps them with it).  weight [channels, taps] (last column the current token's), bias [channels]; state float32
     [slots, slot size] with the conv state, (taps - 1) x channels, at conv_off; reqs int32 [n_req, 3] = (request,
-    first row, rows); out float32 [T, channels]."""
-    _cuda(src, weight, bias, state, slots, row_req, reqs, out)
+    first row, rows); out float32 [T, channels].  `split` bfloat16 [blocks, T, 2 channels / blocks], when given (without an activation),
+    receives `rglru_split` of the result."""
+    _cuda(src, weight, bias, state, slots, row_req, reqs, out, split)
     _i32(slots, "slots"); _i32(row_req, "row_req"); _i32(reqs, "reqs")
     T = row_req.numel()
     taps = weight.shape[1]
@@ -1504,12 +1507,24 @@ def conv_silu(src: torch.Tensor, col0: int, channels: int, weight: torch.Tensor,
         _cuda(src_bias)
         if src_bias.dtype != torch.float32 or src_bias.numel() != channels or not src_bias.is_contiguous():
             raise KernelError("conv_silu: src_bias is contiguous float32 [channels]")
+    args = (_p(src), _dt(src), src.stride(0), col0, channels, taps, _p(weight), _p(bias), _dt(weight), _p(state), state.stride(0), conv_off, _p(slots),
+            _p(row_req), _p(reqs), n_req, _p(out), T)
+    if split is not None:
+        blocks = split.shape[0]
+        if activation != "none" or split.dtype != torch.bfloat16 or not split.is_contiguous() or channels % blocks \
+                or tuple(split.shape) != (blocks, T, 2 * (channels // blocks)):
+            raise KernelError("conv_silu: split is bfloat16 [blocks, T, 2 channels / blocks], without an activation")
+        with phase("conv"):
+            rc = lib().bg_conv_split(*args, _p(src_bias), _p(split), blocks, _stream())
+        if rc != _UNSUPPORTED:
+            _check(rc, "conv_split")
+            return
+    n = _c_int(0)
     with phase("conv"):
-        _check(lib().bg_conv_silu(_p(src), _dt(src), src.stride(0), col0, channels, taps, _p(weight), _p(bias), _dt(weight),
-                                  _p(state), state.stride(0), conv_off, _p(slots), _p(row_req), _p(reqs), n_req, _p(out), T,
-                                  1 if activation == "silu" else 0, _p(src_bias), _stream()), "conv_silu")
-    if taps > 1:
-        count_launches(1)
+        _check(lib().bg_conv_silu(*args, 1 if activation == "silu" else 0, _p(src_bias), ctypes.byref(n), _stream()), "conv_silu")
+    count_launches(n.value - 1)
+    if split is not None:
+        rglru_split(out, split.shape[0], split)
 
 
 def ssm_chunk(H: int, P: int, N: int, G: int) -> int:
@@ -2195,11 +2210,12 @@ def rglru_scan(gates: torch.Tensor, u: torch.Tensor, src: torch.Tensor, y_col: i
                 return
             pq = torch.empty((n_chunks, 2, W), dtype=torch.float32, device=u.device)
             ab = torch.empty((T, W, 2), dtype=torch.float32, device=u.device)
+            n = _c_int(0)
             _check(lib().bg_rglru_scan_chunked(_p(gates), _p(u), _p(src), src.stride(0), y_col, _p(y_bias), _p(gate_bias_r), _p(gate_bias_i),
                                                _p(decay), _p(state), state.stride(0), _p(slots), _p(chunks), n_chunks, _p(longs),
-                                               n_long, chunk_rows, _p(pq), _p(ab), _p(out), _dt(out), T, W, blocks, _stream()),
+                                               n_long, chunk_rows, _p(pq), _p(ab), _p(out), _dt(out), T, W, blocks, ctypes.byref(n), _stream()),
                    "rglru_scan_chunked")
-            count_launches(2)
+            count_launches(n.value - 1)
 
 
 def grouped_pairs(rows: int, experts: int) -> bool:

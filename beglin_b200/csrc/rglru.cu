@@ -46,6 +46,13 @@ __device__ __forceinline__ float gelu_tanh32(float z) {
     return 0.5f * z * (1.0f + tanhf(0.7978845608028654f * (z + 0.044715f * z * z * z)));
 }
 
+// The same for a result that leaves as TO.  Where it is rounded to bfloat16: (1 + tanh x) / 2 = sigmoid(2 x), with the fast exponential and division
+// (2^-20 of itself; the sum 1 + tanh x loses what is left of it for negative x).
+template <typename TO> __device__ __forceinline__ float branch_gelu(float z) {
+    if constexpr (sizeof(TO) == 2) return __fdividef(z, 1.0f + __expf(-1.5957691216057308f * (z + 0.044715f * z * z * z)));
+    else return gelu_tanh32(z);
+}
+
 // (a, b) of S <- a S + b from the gates' arguments and the convolved input
 __device__ __forceinline__ void lru_values(float gr, float gi, float u, float spc, float* a, float* b) {
     const float log_a = -sigmoid32(gr) * spc, e = expm1f(log_a);
@@ -82,7 +89,7 @@ rglru_scan_kernel(LruParams p) {
         float a, b;
         lru_step(p, gbase + (size_t)t * (2 * p.bs), t, c, brc, bic, spc, &a, &b);
         S = fmaf(a, S, b);
-        out[(size_t)t * p.W + c] = from_float<TO>(S * gelu_tanh32(p.src[(size_t)t * p.src_stride + p.y_col + c] + yb));
+        out[(size_t)t * p.W + c] = from_float<TO>(S * branch_gelu<TO>(p.src[(size_t)t * p.src_stride + p.y_col + c] + yb));
     }
     *st = S;
 }
@@ -161,7 +168,7 @@ rglru_chunk_out_kernel(LruParams p, const int* __restrict__ chunks, const float*
         const int t = row0 + j;
         const float2 s = ab[(size_t)t * p.W + c];              // (a, b) of the row, as the first walk formed them
         S = fmaf(s.x, S, s.y);
-        out[(size_t)t * p.W + c] = from_float<TO>(S * gelu_tanh32(p.src[(size_t)t * p.src_stride + p.y_col + c] + yb));
+        out[(size_t)t * p.W + c] = from_float<TO>(S * branch_gelu<TO>(p.src[(size_t)t * p.src_stride + p.y_col + c] + yb));
     }
 }
 
@@ -170,7 +177,7 @@ rglru_chunk_out_kernel(LruParams p, const int* __restrict__ chunks, const float*
 // functions, the second by bytes.  (The whole mixer of 4,096 channels over 2,048 rows: 333 us with a channel a thread, 301 so.)
 constexpr int LRU_BATCH = 4;
 __global__ void __launch_bounds__(LRU_THREADS)
-rglru_chunk_sums_vec2_kernel(LruParams p, const int* __restrict__ chunks, float* __restrict__ pq, float4* __restrict__ ab) {
+rglru_chunk_sums_vec2_kernel(LruParams p, const int* __restrict__ chunks, float* __restrict__ pq, float4* __restrict__ ab, int folded) {
     pdl_launch();
     pdl_wait();
     const int c = (blockIdx.x * LRU_THREADS + threadIdx.x) * 2;
@@ -203,13 +210,23 @@ rglru_chunk_sums_vec2_kernel(LruParams p, const int* __restrict__ chunks, float*
             Q.x = fmaf(v.x, Q.x, v.y); Q.y = fmaf(v.z, Q.y, v.w);
         }
     }
+    if (folded && (ch == 0 || chunks[(ch - 1) * 4] != chunks[ch * 4])) {       // a request's first chunk: its state, and the state behind the chunk
+        const float* st = p.state + (size_t)p.slots[chunks[ch * 4]] * p.slot_stride + c;
+        const float2 S = make_float2(st[0], st[1]);
+        Q = make_float2(fmaf(P.x, S.x, Q.x), fmaf(P.y, S.y, Q.y));
+        P = S;
+    }
     *reinterpret_cast<float2*>(pq + ((size_t)ch * 2 + 0) * p.W + c) = P;
     *reinterpret_cast<float2*>(pq + ((size_t)ch * 2 + 1) * p.W + c) = Q;
 }
 
-template <typename TO>
+// FOLDED: the walk over a request's chunks is made by every chunk for itself, up to its own start, and the last one leaves the state.  For steps of
+// up to LRU_FOLDED chunks and few requests: a kernel less (2,048 rows of 4,096 channels 9.7 us), for reads from the second-level cache.
+constexpr int LRU_FOLDED = 128, LRU_FOLDED_LONGS = 16;
+template <typename TO, bool FOLDED>
 __global__ void __launch_bounds__(LRU_THREADS)
-rglru_chunk_out_vec2_kernel(LruParams p, const int* __restrict__ chunks, const float* __restrict__ pq, const float4* __restrict__ ab) {
+rglru_chunk_out_vec2_kernel(LruParams p, const int* __restrict__ chunks, const int* __restrict__ longs, int n_long, int chunk_rows,
+                            const float* __restrict__ pq, const float4* __restrict__ ab) {
     pdl_launch();
     pdl_wait();
     const int c = (blockIdx.x * LRU_THREADS + threadIdx.x) * 2;
@@ -220,7 +237,37 @@ rglru_chunk_out_vec2_kernel(LruParams p, const int* __restrict__ chunks, const f
     const float* y = p.src + (size_t)row0 * p.src_stride + p.y_col + c;
     const float4* from = ab + ((size_t)row0 * p.W + c) / 2;
     TO* out = (TO*)p.out + (size_t)row0 * p.W + c;
-    float2 S = *reinterpret_cast<const float2*>(pq + ((size_t)ch * 2) * p.W + c);
+    float2 S;
+    if constexpr (FOLDED) {
+        bool last = false;
+        int first = ch;
+        for (int l = 0; l < n_long; ++l) {
+            const int from_ch = longs[l * 4 + 3], count = (longs[l * 4 + 2] + chunk_rows - 1) / chunk_rows;
+            if (ch >= from_ch && ch < from_ch + count) { first = from_ch; last = ch == from_ch + count - 1; }
+        }
+        const float* q = pq + (size_t)first * 2 * p.W + c;
+        S = *reinterpret_cast<const float2*>(q + (ch == first ? 0 : p.W));
+        for (int k0 = first + 1; k0 < ch; k0 += 8) {
+            float2 P[8], Q[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                const float* at = pq + (size_t)min(k0 + k, ch) * 2 * p.W + c;
+                P[k] = *reinterpret_cast<const float2*>(at);
+                Q[k] = *reinterpret_cast<const float2*>(at + p.W);
+            }
+#pragma unroll
+            for (int k = 0; k < 8; ++k)
+                if (k0 + k < ch) S = make_float2(fmaf(P[k].x, S.x, Q[k].x), fmaf(P[k].y, S.y, Q[k].y));
+        }
+        if (last) {                                            // (nobody else looks at the slot any more)
+            const float2 P = *reinterpret_cast<const float2*>(pq + (size_t)ch * 2 * p.W + c), Q = *reinterpret_cast<const float2*>(pq + ((size_t)ch * 2 + 1) * p.W + c);
+            float* st = p.state + (size_t)p.slots[chunks[ch * 4]] * p.slot_stride + c;
+            st[0] = ch == first ? Q.x : fmaf(P.x, S.x, Q.x);
+            st[1] = ch == first ? Q.y : fmaf(P.y, S.y, Q.y);
+        }
+    } else {
+        S = *reinterpret_cast<const float2*>(pq + ((size_t)ch * 2) * p.W + c);
+    }
     for (int j0 = 0; j0 < n; j0 += LRU_BATCH) {
         float4 v[LRU_BATCH];
         float2 z[LRU_BATCH];
@@ -234,7 +281,7 @@ rglru_chunk_out_vec2_kernel(LruParams p, const int* __restrict__ chunks, const f
         for (int k = 0; k < LRU_BATCH; ++k) {
             if (j0 + k >= n) break;
             S.x = fmaf(v[k].x, S.x, v[k].y); S.y = fmaf(v[k].z, S.y, v[k].w);
-            const float o0 = S.x * gelu_tanh32(z[k].x + yb.x), o1 = S.y * gelu_tanh32(z[k].y + yb.y);
+            const float o0 = S.x * branch_gelu<TO>(z[k].x + yb.x), o1 = S.y * branch_gelu<TO>(z[k].y + yb.y);
             TO* d = out + (size_t)(j0 + k) * p.W;
             if constexpr (sizeof(TO) == 4) *reinterpret_cast<float2*>(d) = make_float2(o0, o1);
             else *reinterpret_cast<__nv_bfloat162*>(d) = __floats2bfloat162_rn(o0, o1);
@@ -329,7 +376,8 @@ extern "C" int bg_rglru_scan_chunked(const float* gates, const float* u, const f
                                      const float* by, const float* br, const float* bi, const float* sp, float* state, long long slot_stride,
                                      const int* slots, const int* chunks, int n_chunks, const int* longs, int n_long,
                                      int chunk_rows, float* pq, float* ab, void* out, int out_dtype, int T, int W, int blocks,
-                                     cudaStream_t stream) {
+                                     int* launched, cudaStream_t stream) {
+    if (launched) *launched = 0;
     if (n_chunks <= 0 || n_long <= 0 || T <= 0) return BG_OK;
     if (n_chunks > 65535 || n_long > 65535 || chunk_rows <= 0) return BG_ERR_SHAPE;
     LruParams p;
@@ -339,14 +387,27 @@ extern "C" int bg_rglru_scan_chunked(const float* gates, const float* u, const f
     auto on = [](const void* q, unsigned bytes) { return (uintptr_t)q % bytes == 0; };
     const bool two = p.bs % 2 == 0 && src_stride % 2 == 0 && y_col % 2 == 0 && on(gates, 8) && on(u, 8) && on(src, 8) && on(br, 8) && on(bi, 8) &&
                      on(sp, 8) && on(pq, 8) && on(ab, 16) && on(out, 8) && (!by || on(by, 8));
-    if (two) launch(rglru_chunk_sums_vec2_kernel, dim3(bx2, n_chunks), dim3(LRU_THREADS), 0, stream, p, chunks, pq, (float4*)ab);
-    else launch(rglru_chunk_sums_kernel, dim3(bx, n_chunks), dim3(LRU_THREADS), 0, stream, p, chunks, pq, (float2*)ab);
-    BG_LAUNCH_CHECK();
+    if (launched) *launched = 3;
+    if (two) {
+        const bool folded = n_chunks <= LRU_FOLDED && n_long <= LRU_FOLDED_LONGS;
+        launch(rglru_chunk_sums_vec2_kernel, dim3(bx2, n_chunks), dim3(LRU_THREADS), 0, stream, p, chunks, pq, (float4*)ab, folded ? 1 : 0);
+        BG_LAUNCH_CHECK();
+        if (folded) {
+            if (launched) *launched = 2;
+            BG_DISPATCH_DTYPE(out_dtype, TO, launch(rglru_chunk_out_vec2_kernel<TO, true>, dim3(bx2, n_chunks), dim3(LRU_THREADS), 0, stream, p, chunks, longs,
+                                                    n_long, chunk_rows, (const float*)pq, (const float4*)ab));
+            BG_LAUNCH_CHECK();
+            return BG_OK;
+        }
+    } else {
+        launch(rglru_chunk_sums_kernel, dim3(bx, n_chunks), dim3(LRU_THREADS), 0, stream, p, chunks, pq, (float2*)ab);
+        BG_LAUNCH_CHECK();
+    }
     launch(rglru_chunk_walk_kernel, dim3(bx, n_long), dim3(LRU_THREADS), 0, stream, p, longs, chunk_rows, pq);
     BG_LAUNCH_CHECK();
     if (two)
-        BG_DISPATCH_DTYPE(out_dtype, TO, launch(rglru_chunk_out_vec2_kernel<TO>, dim3(bx2, n_chunks), dim3(LRU_THREADS), 0, stream, p, chunks,
-                                                (const float*)pq, (const float4*)ab));
+        BG_DISPATCH_DTYPE(out_dtype, TO, launch(rglru_chunk_out_vec2_kernel<TO, false>, dim3(bx2, n_chunks), dim3(LRU_THREADS), 0, stream, p, chunks, longs, n_long,
+                                                chunk_rows, (const float*)pq, (const float4*)ab));
     else
         BG_DISPATCH_DTYPE(out_dtype, TO, launch(rglru_chunk_out_kernel<TO>, dim3(bx, n_chunks), dim3(LRU_THREADS), 0, stream, p, chunks,
                                                 (const float*)pq, (const float2*)ab));

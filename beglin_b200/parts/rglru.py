@@ -90,11 +90,10 @@ class RGLRU:
         proj = self.in_proj.full_f32(h)                                 # [T, y | x] without their biases
         reqs, n_req = batch.query_blocks(1 << 30)                       # one (request, first row, rows) per request
         u = torch.empty((T, W), dtype=torch.float32, device=h.device)
+        x2 = None if self.gate_w2 is None else torch.empty((B, T, 2 * (W // B)), dtype=torch.bfloat16, device=h.device)
         ops.conv_silu(proj, W, W, self.conv_w, self.conv_b, cache.state, W, cache.slots, batch.row_req, reqs, n_req, u,
-                      activation="none", src_bias=self.bias_x)
-        if self.gate_w2 is not None:
-            x2 = torch.empty((B, T, 2 * (W // B)), dtype=torch.bfloat16, device=h.device)
-            ops.rglru_split(u, B, x2)
+                      activation="none", src_bias=self.bias_x, split=x2)
+        if x2 is not None:
             with ops.phase("proj_heads"):
                 gates = torch.bmm(x2, self.gate_w2, out_dtype=torch.float32)
         else:
