@@ -56,7 +56,7 @@ struct GtParams {
 
 // The tokens' parts as the images of the stages' right operands, [batch][tile of nt tokens][stage][part][token][64 of k] with the swizzle of
 // shared memory, noughts behind the last token and behind K.  One part of a stage is then one copy of contiguous bytes: boxes of a tensor map, 64 bytes a row, took the copy engine 2.4 cycles a row, 1,750 for 32 of k of 192 tokens.
-// A CTA per row, a warp per 512 of k, 16 values a lane.
+// A CTA (or gridDim.y of them) per row, a warp per 512 of k, 16 values a lane.
 template <bool VEC>
 __global__ void __launch_bounds__(256) gf_parts_kernel(GtParams p, unsigned char* images, int nt) {
     pdl_launch();
@@ -66,7 +66,7 @@ __global__ void __launch_bounds__(256) gf_parts_kernel(GtParams p, unsigned char
     const float* src = p.A + (size_t)b * p.batch_a + (size_t)m * p.lda + k_first;
     unsigned char* tile = images + ((size_t)b * p.tok_tiles + m / nt) * stages * 3 * nt * 128 + in * 128 + (((lane >> 1 & 7) ^ (in & 7)) << 4) + (lane & 1) * 8;
     pdl_wait();
-    for (int k0 = warp * 512; k0 < stages * GT_BK; k0 += blockDim.x / 32 * 512) {
+    for (int k0 = ((int)blockIdx.y * (blockDim.x / 32) + warp) * 512; k0 < stages * GT_BK; k0 += gridDim.y * (blockDim.x / 32) * 512) {
         float4 v[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
@@ -572,9 +572,10 @@ static int gt_piece(const GfParams& f, const GtPlan& g, int r0, int r1, cudaStre
     if (units > 0x3fffffff) return BG_ERR_SHAPE;
     p.units = (int)units;
     const bool vec = f.K % 4 == 0 && f.lda % 4 == 0 && f.batch_a % 4 == 0 && (uintptr_t)f.A % 16 == 0 && p.r0 * (long long)g.range_len % 4 == 0;
-    const int pieces = ((r1 - r0) * g.range_len + 511) / 512, threads = 32 * (pieces < 8 ? pieces : 8);
-    cudaError_t e = vec ? launch(gf_parts_kernel<true>, dim3((unsigned)padded), dim3(threads), 0, stream, p, images, g.nt)
-                        : launch(gf_parts_kernel<false>, dim3((unsigned)padded), dim3(threads), 0, stream, p, images, g.nt);
+    // (a row's pieces of 512 go to more CTAs where the rows leave SMs idle)
+    const int pieces = ((r1 - r0) * g.range_len + 511) / 512, threads = 32 * (pieces < 8 ? pieces : 8), slices = padded <= 64 ? (pieces + 7) / 8 : 1;
+    cudaError_t e = vec ? launch(gf_parts_kernel<true>, dim3((unsigned)padded, slices), dim3(threads), 0, stream, p, images, g.nt)
+                        : launch(gf_parts_kernel<false>, dim3((unsigned)padded, slices), dim3(threads), 0, stream, p, images, g.nt);
     if (e != cudaSuccess) return (int)e;
     if (g.cut) p.part = behind;
     else if (f.accumulate && g.ranges > 1) { p.run = behind; p.ldr = f.N; p.batch_r = (long long)f.M * f.N; }

@@ -121,6 +121,9 @@ _SIGNATURES = {
     "bg_gemm_f32_scratch": [_c_int, _c_int, _c_int, _c_int],
     "bg_gemm_f32_nt": [_c_void_p, _c_int, _c_void_p, _c_int, _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int,
                        _c_int, _c_void_p, _c_void_p, _c_void_p],
+    "bg_mlp_f32_scratch": [_c_int, _c_int, _c_int],
+    "bg_mlp_f32": [_c_void_p, _c_int, _c_int, _c_int, _c_int, _c_void_p, _c_int, _c_void_p, _c_int, _c_float, _c_void_p, _c_ll, _c_void_p, _c_void_p,
+                   _c_void_p],
     "bg_gemm_bf16_tn": [_c_void_p, _c_int, _c_int, _c_int, _c_void_p, _c_int, _c_int, _c_void_p, _c_void_p, _c_int,
                         _c_int, _c_int, _c_void_p, _c_void_p],
     "bg_gemm_pair": [_c_void_p, _c_int, _c_int, _c_int, _c_void_p, _c_int, _c_int, _c_void_p, _c_void_p, _c_int, _c_int,
@@ -188,7 +191,7 @@ _SIGNATURES = {
                        _c_void_p],
 }
 
-_RESULTS = {"bg_gemm_f32_scratch": _c_ll, "bg_experts_scratch": _c_ll, "bg_latent_step_scratch": _c_ll}         # what does not return a code
+_RESULTS = {"bg_gemm_f32_scratch": _c_ll, "bg_experts_scratch": _c_ll, "bg_latent_step_scratch": _c_ll, "bg_mlp_f32_scratch": _c_ll}         # what does not return a code
 
 _lib = None
 
@@ -854,6 +857,26 @@ def gemm_f32_nt(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], 
     scratch = _gemm_f32_scratch(M, N, K, 1, out.device, M * N if accumulate else 0)
     _check(lib().bg_gemm_f32_nt(_p(a), a.stride(0), _p(w), w.stride(0), _p(bias), _p(out), out.stride(0), M, N, K,
                                 1 if accumulate else 0, _p(scratch), _p(status), _stream()), "gemm_f32_nt")
+
+
+def mlp_f32(h: torch.Tensor, up: torch.Tensor, block: int, down: torch.Tensor, activation: str = "silu", limit: float = 0.0,
+            status: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """(act(gate) * up) down^T of h float32 [T, hidden] as one call: `gemm_f32_nt`, `swiglu` (with its block, activation and limit) and `gemm_f32_nt`;
+    up float32 [2 ff, hidden], down float32 [hidden, ff], contiguous, hidden and ff multiples of 4."""
+    _cuda(h, up, down, status)
+    T, hidden = h.shape
+    ff = down.shape[1]
+    if h.dtype != torch.float32 or up.dtype != torch.float32 or down.dtype != torch.float32 or h.stride(1) != 1 or tuple(up.shape) != (2 * ff, hidden) \
+            or down.shape[0] != hidden or not up.is_contiguous() or not down.is_contiguous() or hidden % 4 or ff % 4 or (block and ff % block):
+        raise KernelError("mlp_f32: h [T, hidden], up [2 ff, hidden], down [hidden, ff], float32, sizes that are multiples of 4")
+    L = lib()
+    size = L.bg_mlp_f32_scratch(T, hidden, ff)
+    out = torch.empty((T, hidden), dtype=torch.float32, device=h.device)
+    scratch = torch.empty((size,), dtype=torch.float32, device=h.device)
+    _check(L.bg_mlp_f32(h.data_ptr(), h.stride(0), T, hidden, ff, up.data_ptr(), block, down.data_ptr(), GLU_ACTIVATIONS[activation], float(limit),
+                        scratch.data_ptr(), size, out.data_ptr(), _p(status), _stream()), "mlp_f32")
+    count_launches(2)
+    return out
 
 
 def _gemm_f32_scratch(M: int, N: int, K: int, batch: int, device, more: int = 0) -> Optional[torch.Tensor]:

@@ -45,10 +45,19 @@ class SwiGLU:
             w = torch.cat([gate, up], dim=0)
         self.gate_up = Linear(w, None, ctx, label="proj_gate_up")
         self.down = Linear(tensors["down_proj.weight"], None, ctx, label="proj_down")
+        # float32: the whole as one call (rows of whole 16-byte pieces)
+        self.one_call = ctx.compute_dtype == torch.float32 and spec.hidden % 4 == 0 and im % 4 == 0
 
     def forward(self, h, batch, stream: Optional[ResidualStream] = None) -> Optional[torch.Tensor]:
         """h: the normed rows, or a NormedInput.  With `stream` the result is added to it (or left owed to
         it) and None is returned; without, the addend is returned."""
+        if self.one_call and not ops.profiling():
+            out = ops.mlp_f32(h if isinstance(h, torch.Tensor) else h.tensor(), self.gate_up.weight, self.block, self.down.weight, self.spec.activation,
+                              self.spec.limit, self.ctx.status)
+            if stream is None:
+                return out
+            stream.owe(out)
+            return None
         act = self.gate_up.of(h, swiglu=True, activation=self.spec.activation, limit=self.spec.limit) if self.block else None
         if act is None:
             gu = self.gate_up.of(h)
