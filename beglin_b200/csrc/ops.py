@@ -103,6 +103,8 @@ _SIGNATURES = {
     "bg_gla_chunk_plan": [_c_int, _c_int, ctypes.POINTER(_c_int)],
     "bg_gla_chunked": [_c_void_p, _c_void_p, _c_int, _c_void_p, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p,
                        _c_void_p],
+    "bg_attention_f32_scratch": [_c_void_p, _c_int, _c_int],
+    "bg_attention_f32_step": [_c_void_p, _c_void_p, _c_void_p],
     "bg_attention_mma_plan": [_c_int, _c_int, _c_int, ctypes.POINTER(_c_int)],
     "bg_attention_mma_partial": [_c_void_p, _c_int, _c_void_p, _c_int, _c_int, _c_void_p, _c_int, _c_void_p, _c_void_p,
                                  _c_int, _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int,
@@ -191,7 +193,7 @@ _SIGNATURES = {
                        _c_void_p],
 }
 
-_RESULTS = {"bg_gemm_f32_scratch": _c_ll, "bg_experts_scratch": _c_ll, "bg_latent_step_scratch": _c_ll, "bg_mlp_f32_scratch": _c_ll}         # what does not return a code
+_RESULTS = {"bg_gemm_f32_scratch": _c_ll, "bg_experts_scratch": _c_ll, "bg_latent_step_scratch": _c_ll, "bg_mlp_f32_scratch": _c_ll, "bg_attention_f32_scratch": _c_ll}         # what does not return a code
 
 _lib = None
 
@@ -632,6 +634,44 @@ def decode_splits(n_streams: int, context: int, sms: Optional[int] = None) -> in
     want = max(1, min(sms // max(1, n_streams), -(-context // 256)))
     per = -(-(-(-context // want)) // 256) * 256          # what the kernel makes of it: whole multiples of 256 keys
     return -(-context // per)                             # no CTA without keys
+
+
+class AttnF32Args(ctypes.Structure):
+    """What `attention_f32_step` needs of a layer (csrc/attention_f32_step.cu says what the fields are)."""
+    _fields_ = [(n, _c_void_p) for n in ("qkv", "qkv_bias", "out", "out_bias", "sink_w", "status")] \
+        + [(n, _c_int) for n in ("hidden", "heads", "kv_heads", "hd", "rot", "interleaved", "window", "keep", "split", "bq", "tile", "sink")] \
+        + [("scale", _c_float), ("softcap", _c_float)]
+
+
+class AttnF32Step(ctypes.Structure):
+    """What a step brings to `attention_f32_step`."""
+    _fields_ = [(n, _c_void_p) for n in ("h", "cos_sin", "positions", "row_req", "block_table", "pool", "qblk", "scratch", "out")] \
+        + [("scratch_floats", _c_ll)] + [(n, _c_int) for n in ("T", "ldh", "max_pages", "num_pages", "page_size", "n_qblk", "n_splits", "pad")]
+
+
+def attention_f32_step(args: AttnF32Args, h: torch.Tensor, cos_sin: Optional[torch.Tensor], positions: torch.Tensor, row_req: torch.Tensor,
+                       block_table: torch.Tensor, kv_pool: torch.Tensor, page_size: int, qblk: torch.Tensor, n_qblk: int, max_position: int) -> torch.Tensor:
+    """A step of float attention from the mixer's input h float32 [T, hidden] to its addend [T, hidden] as one call: `gemm_f32_nt`, `rope_kv_append`,
+    `attention` ("generic") and `gemm_f32_nt` with their arguments."""
+    _cuda(h, cos_sin, positions, row_req, block_table, kv_pool, qblk)
+    _i32(positions, "positions"); _i32(row_req, "row_req"); _i32(block_table, "block_table"); _i32(qblk, "qblk")
+    T = h.shape[0]
+    if h.dtype != torch.float32 or h.stride(1) != 1 or h.shape[1] != args.hidden or positions.numel() < T or row_req.numel() < T:
+        raise KernelError("attention_f32_step: h float32 [T, hidden], a position and a request per row")
+    if kv_pool.dtype != torch.float32 or tuple(kv_pool.shape[1:]) != (2, args.kv_heads, page_size, args.hd) or not kv_pool.is_contiguous():
+        raise KernelError(f"attention_f32_step: kv_pool is {tuple(kv_pool.shape)}, expected [pages, 2, {args.kv_heads}, {page_size}, {args.hd}]")
+    if args.rot > 0 and (cos_sin is None or cos_sin.shape[0] < T or cos_sin.shape[1] != args.rot // 2 or cos_sin.dtype != torch.float32):
+        raise KernelError("attention_f32_step: cos_sin must be float32 [T, rot/2, 2]")
+    L, a = lib(), ctypes.byref(args)
+    n_splits = max_position // args.split + 1
+    out = torch.empty((T, args.hidden), dtype=torch.float32, device=h.device)
+    size = L.bg_attention_f32_scratch(a, T, n_splits)
+    scratch = torch.empty((size,), dtype=torch.float32, device=h.device)
+    step = AttnF32Step(h.data_ptr(), _p(cos_sin), positions.data_ptr(), row_req.data_ptr(), block_table.data_ptr(), kv_pool.data_ptr(), qblk.data_ptr(),
+                       scratch.data_ptr(), out.data_ptr(), size, T, h.stride(0), block_table.shape[1], kv_pool.shape[0], page_size, n_qblk, n_splits, 0)
+    _check(L.bg_attention_f32_step(a, ctypes.byref(step), _stream()), "attention_f32_step")
+    count_launches(4)
+    return out
 
 
 def attention(*args, **kwargs) -> None:

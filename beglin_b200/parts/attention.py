@@ -156,12 +156,42 @@ class GQAAttention:
                                 and ctx.compute_dtype == torch.bfloat16 and ctx.cache_dtype == torch.bfloat16
                                 and not self.extended)
 
+        self._args = self._step_args()
+
+    def _step_args(self):
+        """The layer as the one-call float step takes it, for each of its two plans (portions, single tokens), or None: the plain form in float32."""
+        s, ctx = self.spec, self.ctx
+        if ctx.compute_dtype != torch.float32 or ctx.cache_dtype != torch.float32 or self.extended or not s.own_kv or self.stored is not None \
+                or any(plan[0] != "generic" for plan in self.plans.values()):
+            return None
+        ptr = lambda t: None if t is None else t.data_ptr()
+        return {d: ops.AttnF32Args(qkv=ptr(self.qkv.weight), qkv_bias=ptr(self.qkv.bias_f32), out=ptr(self.o_proj.weight), out_bias=ptr(self.o_proj.bias_f32),
+                                   sink_w=ptr(self.sink_weight), status=ptr(ctx.status), hidden=s.hidden, heads=self.nh, kv_heads=self.nkv, hd=self.hd,
+                                   rot=self.position.rotary_dim, interleaved=int(self.position.interleaved), window=self.window, keep=s.keep_first,
+                                   split=ctx.kv_split, bq=bq, tile=tile, sink=int(bool(s.sink)), scale=self.scale, softcap=self.score_cap)
+                for d, (_, bq, tile) in self.plans.items()}
+
     takes_stream = True        # forward takes a NormedInput and may add its result to the stream itself
 
     def forward(self, h, batch, cache: PagedKVView, stream: Optional[ResidualStream] = None) -> Optional[torch.Tensor]:
         """h: the normed rows, or a NormedInput.  With `stream` the result is added to it (or left owed to
         it) and None is returned; without, the addend is returned."""
         T = batch.n_rows
+        if self._args is not None and not ops.profiling():
+            rows = h if isinstance(h, torch.Tensor) else h.tensor()
+            args = self._args[bool(getattr(batch, "decode_only", False))]
+            qblk, n_qblk = batch.query_blocks(args.bq)
+            if qblk is None:
+                batch.implicit_blocks = False          # this kernel wants the list
+                qblk, n_qblk = batch.query_blocks(args.bq)
+            if rows.shape[0] == T and rows.dtype == torch.float32 and rows.stride(1) == 1:
+                out = ops.attention_f32_step(args, rows, self.position.table(batch), batch.positions, batch.row_req, cache.block_table, cache.pool,
+                                             cache.page_size, qblk, n_qblk, batch.max_position)
+                if stream is None:
+                    return out
+                stream.owe(out)
+                return None
+            h = rows
         qkv = None
         khd, kvd_ = (self.hd, self.vd) if self.stored is None else (self.stored, self.stored)
         if self.extended:
