@@ -184,6 +184,8 @@ _SIGNATURES = {
     "bg_ssm_chunked": [_c_void_p, _c_int, _c_void_p, _c_int, _c_int, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_void_p, _c_ll,
                        _c_void_p, _c_void_p, _c_int, _c_void_p, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_int,
                        _c_int, _c_int, _c_int, _c_void_p, _c_void_p],
+    "bg_mamba2_scratch": [_c_void_p, _c_int, _c_int],
+    "bg_mamba2_step": [_c_void_p, _c_void_p, _c_void_p, _c_void_p],
     "bg_gated_group_rmsnorm": [_c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_void_p, _c_int, _c_float, _c_void_p, _c_int,
                                _c_int, _c_int, _c_int, _c_int, _c_void_p],
     "bg_gemm_f32_nt_batched": [_c_void_p, _c_int, _c_ll, _c_void_p, _c_int, _c_ll, _c_void_p, _c_int, _c_ll, _c_int, _c_int,
@@ -193,7 +195,8 @@ _SIGNATURES = {
                        _c_void_p],
 }
 
-_RESULTS = {"bg_gemm_f32_scratch": _c_ll, "bg_experts_scratch": _c_ll, "bg_latent_step_scratch": _c_ll, "bg_mlp_f32_scratch": _c_ll, "bg_attention_f32_scratch": _c_ll}         # what does not return a code
+_RESULTS = {"bg_gemm_f32_scratch": _c_ll, "bg_experts_scratch": _c_ll, "bg_latent_step_scratch": _c_ll, "bg_mlp_f32_scratch": _c_ll, "bg_attention_f32_scratch": _c_ll,
+            "bg_mamba2_scratch": _c_ll}         # what does not return a code
 
 _lib = None
 
@@ -1653,6 +1656,49 @@ def gated_group_rmsnorm(y: torch.Tensor, src: torch.Tensor, z_col: int, weight: 
     with phase("rmsnorm"):
         _check(lib().bg_gated_group_rmsnorm(_p(y), _p(src), _dt(src), src.stride(0), z_col, _p(weight), _dt(weight), float(eps),
                                             _p(out), _dt(out), T, inner, groups, 1 if gate_after else 0, _stream()), "gated_group_rmsnorm")
+
+
+class Mamba2Args(ctypes.Structure):
+    """What `mamba2_step` needs of a layer (csrc/mamba2_step.cu says what the fields are)."""
+    _fields_ = [(n, _c_void_p) for n in ("conv_w", "conv_b", "dt_bias", "A_log", "D", "norm_w", "status")] \
+        + [(n, _c_int) for n in ("w_dtype", "norm_dtype", "out_dtype", "inner", "channels", "taps", "H", "P", "N", "G", "norm_groups", "tensor_cores", "chunk")] \
+        + [("eps", _c_float)]
+
+
+class Mamba2Step(ctypes.Structure):
+    """What a step brings to `mamba2_step`."""
+    _fields_ = [(n, _c_void_p) for n in ("proj", "state", "slots", "row_req", "requests", "reqs", "chunks", "longs", "scratch", "out")] \
+        + [(n, _c_ll) for n in ("slot_stride", "conv_off", "scratch_bytes")] + [(n, _c_int) for n in ("T", "ldp", "n_requests", "n_req", "n_chunks", "n_long")]
+
+
+def mamba2_step(args: Mamba2Args, proj: torch.Tensor, state: torch.Tensor, conv_off: int, slots: torch.Tensor, row_req: torch.Tensor, requests: torch.Tensor,
+                n_requests: int, reqs: torch.Tensor, n_req: int, chunks: Optional[torch.Tensor], n_chunks: int, longs: Optional[torch.Tensor], n_long: int,
+                out: torch.Tensor) -> None:
+    """Mamba-2 from its product's rows proj float32 [T, z | x B C | dt ..] to the rows of its output product, out [T, inner], as one call: `conv_silu`
+    over the step's `requests`, `ssm_scan` (its lists) and `gated_group_rmsnorm`."""
+    _cuda(proj, state, slots, row_req, requests, reqs, chunks, longs, out)
+    _i32(slots, "slots"); _i32(row_req, "row_req"); _i32(requests, "requests")
+    if n_req:
+        _i32(reqs, "reqs")
+    if n_chunks:
+        _i32(chunks, "chunks"); _i32(longs, "longs")
+        if chunks.shape[0] < n_chunks or longs.shape[0] < n_long or n_long < 1:
+            raise KernelError("mamba2_step: the lists of chunks and of long requests are shorter than their counts")
+    T = row_req.numel()
+    if proj.dtype != torch.float32 or proj.dim() != 2 or proj.stride(1) != 1 or proj.shape[0] < T or proj.shape[1] < args.inner + args.channels + args.H:
+        raise KernelError(f"mamba2_step: rows of {tuple(proj.shape)} hold no gates, channels and step sizes")
+    if state.dtype != torch.float32 or state.dim() != 2 or state.stride(1) != 1 or conv_off < args.H * args.N * args.P \
+            or conv_off + (args.taps - 1) * args.channels > state.shape[1]:
+        raise KernelError(f"mamba2_step: the state is {tuple(state.shape)}")
+    if tuple(out.shape) != (T, args.inner) or not out.is_contiguous() or _dt(out) != args.out_dtype:
+        raise KernelError("mamba2_step: out is contiguous [T, inner] of the layer's type")
+    L, a, n = lib(), ctypes.byref(args), _c_int(0)
+    size = L.bg_mamba2_scratch(a, T, n_chunks)
+    scratch = torch.empty((size,), dtype=torch.uint8, device=out.device)
+    step = Mamba2Step(proj.data_ptr(), state.data_ptr(), slots.data_ptr(), row_req.data_ptr(), requests.data_ptr(), _p(reqs), _p(chunks), _p(longs),
+                      scratch.data_ptr(), out.data_ptr(), state.stride(0), conv_off, size, T, proj.stride(0), n_requests, n_req, n_chunks, n_long)
+    _check(L.bg_mamba2_step(a, ctypes.byref(step), ctypes.byref(n), _stream()), "mamba2_step")
+    count_launches(n.value - 1)
 
 
 def rmsnorm_add(x: torch.Tensor, y: torch.Tensor, weight: torch.Tensor, eps: float, lowp: Optional[torch.Tensor] = None) -> None:

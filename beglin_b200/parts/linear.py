@@ -28,6 +28,7 @@ class Linear:
         self.label = label
         self.weight = ctx.matrix(weight)
         self.out_features, self.in_features = self.weight.shape
+        self._weight_t = self.weight.t()
         self.bias_f32 = None if bias is None else bias.to(device=ctx.device, dtype=torch.float32).contiguous()
         self.bias_c = None if bias is None else self.bias_f32.to(ctx.compute_dtype)
         self.f32 = ctx.compute_dtype == torch.float32
@@ -49,13 +50,13 @@ class Linear:
         if self._tc is not None and (self._tc_always or self._tc.wins(T)):
             return self._tc(x, self.bias_f32, out_dtype, partial)
         if out_dtype == torch.float32:
-            y = torch.mm(x, self.weight.t(), out_dtype=torch.float32)
+            y = torch.mm(x, self._weight_t, out_dtype=torch.float32)
             if self.bias_f32 is not None:
                 y += self.bias_f32
             return y
         if self.bias_c is not None:
-            return torch.addmm(self.bias_c, x, self.weight.t())
-        return torch.mm(x, self.weight.t())
+            return torch.addmm(self.bias_c, x, self._weight_t)
+        return torch.mm(x, self._weight_t)
 
     def __call__(self, x: torch.Tensor, out_dtype: Optional[torch.dtype] = None) -> torch.Tensor:
         """x is [T, in] in the compute type; the result is [T, out] in `out_dtype` (default: compute type)."""

@@ -83,6 +83,13 @@ class Mamba2:
         # rows whose chunks' states still fit CHUNK_BYTES; a longer step of a spec that does not ask for chunks is walked
         self.long_from = self.LONG_FROM if spec.chunked else self.LONG_FROM_BF16
         self.most_rows = None if spec.chunked or not self.chunk else self.CHUNK_BYTES // (4 * self.conv_off) * self.chunk
+        ptr = lambda t: None if t is None else t.data_ptr()
+        code = lambda t: ops.F32 if t.dtype == torch.float32 else ops.BF16
+        self._args = ops.Mamba2Args(
+            conv_w=ptr(self.conv_w), conv_b=ptr(self.conv_b), dt_bias=ptr(self.dt_bias), A_log=ptr(self.A_log), D=ptr(self.D), norm_w=ptr(self.norm_w),
+            status=ptr(ctx.status), w_dtype=code(self.conv_w), norm_dtype=code(self.norm_w), out_dtype=ops.F32 if ctx.compute_dtype == torch.float32 else ops.BF16,
+            inner=inner, channels=channels, taps=spec.conv, H=spec.n_heads, P=spec.vdim, N=spec.state, G=spec.groups, norm_groups=spec.norm_groups,
+            tensor_cores=int(ctx.compute_dtype == torch.bfloat16), chunk=self.chunk, eps=spec.eps)
 
     # Rows of a request in a step from which its tokens run in chunks: with the spec's `chunked`, and in bfloat16 without it, where the
     # five kernels of the chunks are a later choice than the walk's one (the whole mixer of 24 heads of 128 x 128, walked and in chunks:
@@ -101,18 +108,23 @@ class Mamba2:
         T = batch.n_rows
         proj = self.in_proj(h, out_dtype=torch.float32)                 # [T, z | x B C | dt]
         reqs, n_req = batch.query_blocks(1 << 30)                       # one (request, first row, rows) per request
-        xbc = torch.empty((T, self.channels), dtype=torch.float32, device=h.device)
-        ops.conv_silu(proj, self.inner, self.channels, self.conv_w, self.conv_b, cache.state, self.conv_off, cache.slots,
-                      batch.row_req, reqs, n_req, xbc)
-        y = torch.empty((T, self.inner), dtype=torch.float32, device=h.device)
+        requests, n_requests = reqs, n_req
         chunks, n_chunks, longs, n_long = None, 0, None, 0
         if self.chunk and not batch.decode_only and hasattr(batch, "long_blocks") and (self.most_rows is None or T <= self.most_rows):
             reqs, n_req, chunks, n_chunks, longs, n_long = batch.long_blocks(self.chunk, self.long_from)
-        ops.ssm_scan(xbc, proj, self.inner + self.channels, self.dt_bias, self.A_log, self.D, cache.state, cache.slots,
-                     reqs, n_req, y, s.n_heads, s.vdim, s.state, s.groups, chunks, n_chunks, longs, n_long,
-                     tensor_cores=ctx.compute_dtype == torch.bfloat16, status=ctx.status)
         out = torch.empty((T, self.inner), dtype=ctx.compute_dtype, device=h.device)
-        ops.gated_group_rmsnorm(y, proj, 0, self.norm_w, s.eps, s.norm_groups, out)
+        if not ops.profiling():
+            ops.mamba2_step(self._args, proj, cache.state, self.conv_off, cache.slots, batch.row_req, requests, n_requests, reqs, n_req, chunks, n_chunks,
+                            longs, n_long, out)
+        else:                                                           # (kernel classes are being timed)
+            xbc = torch.empty((T, self.channels), dtype=torch.float32, device=h.device)
+            ops.conv_silu(proj, self.inner, self.channels, self.conv_w, self.conv_b, cache.state, self.conv_off, cache.slots,
+                          batch.row_req, requests, n_requests, xbc)
+            y = torch.empty((T, self.inner), dtype=torch.float32, device=h.device)
+            ops.ssm_scan(xbc, proj, self.inner + self.channels, self.dt_bias, self.A_log, self.D, cache.state, cache.slots,
+                         reqs, n_req, y, s.n_heads, s.vdim, s.state, s.groups, chunks, n_chunks, longs, n_long,
+                         tensor_cores=ctx.compute_dtype == torch.bfloat16, status=ctx.status)
+            ops.gated_group_rmsnorm(y, proj, 0, self.norm_w, s.eps, s.norm_groups, out)
         if stream is None:
             return self.o_proj.partial(out)
         self.o_proj.into(out, stream)
