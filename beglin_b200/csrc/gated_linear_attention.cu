@@ -19,6 +19,8 @@
 // chunk's start (which underflow) nor from logarithms (a may be 0).  A chunk is cut into blocks of GB tokens, and a product
 // over tokens of several blocks is split at the blocks' borders: (from the key's token to its block's end) x (whole blocks
 // between) x (from the start of the query's block to its token), each a running product of numbers in [0, 1].
+#include <type_traits>
+
 #include "common.cuh"
 #include "chunk_scan.cuh"
 #include "chunk_tc.cuh"
@@ -200,6 +202,7 @@ constexpr int GCP = GC + 4;               // row stride of the score tile
 constexpr int GPT = 64;                   // value columns of a block
 constexpr int GC_BATCH = 8;               // loads (of 16 bytes: half as many) a thread has on their way at a time
 constexpr int GLA_RANK = 16;              // features of the short row taken at a time
+constexpr int GLA_WS = GLA_RANK + 4;      // row stride of the decay's matrix in shared memory
 
 // The (row, column) of element tid + k * blockDim.x of a [rows][w] tile, stepped without a division per element.
 struct GlaWalk {
@@ -235,195 +238,263 @@ __device__ __forceinline__ void gla_rows(float* dst, int ld, const float* src, s
     }
 }
 
-// (M groups of 32 channels cover np; a block of 256 threads)
-template <int M>
+// Scores inside the blocks of a chunk: a warp takes four neighbouring keys of a block and walks the queries from the first of them to the
+// block's end; a lane carries its channels of k_j times the decay from j to t along as t moves on, so that a score is one sum per query.
+// L lanes share a key's channels, four neighbours at a time (M such groups a lane), and carry KEYS keys: the four keys read the same rows of
+// queries and decays, once.
+template <int L, int M>
 __device__ __forceinline__ void gla_block_scores(const float* Qs, const float* Ks, const float* As, float* sc, int np, int ld) {
-    for (int pass = 0; pass < 2; ++pass) {
-        const int slot = (int)threadIdx.x + pass * 256;
-        const int g = slot & 7, jb = (slot >> 3) & (GB - 1), b = slot >> 7;         // 4 blocks x 16 keys x 8 threads
-        const int j = b * GB + jb, steps = GB - (jb & ~3);                          // a warp's four keys are neighbours
-        float4 w[M];
+    constexpr int KEYS = L / 8;                      // of a lane's group; 32 / L groups a warp
+    const int lane = threadIdx.x & 31, l = lane & (L - 1), warp = threadIdx.x >> 5;
+    const int b0 = (warp >> 2) * GB, first = (warp & 3) * 4;                        // the warp's block and its first key in it
+    const int key = (lane / L) * KEYS;                                              // the lane's first key of the four
+    float w[KEYS][4 * M];
+#pragma unroll
+    for (int e = 0; e < KEYS; ++e)
 #pragma unroll
         for (int m = 0; m < M; ++m) {
-            const int i = 4 * g + 32 * m;
-            w[m] = i < np ? *reinterpret_cast<const float4*>(Ks + j * ld + i) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            const int i = 4 * (l + L * m);
+            const float4 x = i < np ? *reinterpret_cast<const float4*>(Ks + (b0 + first + key + e) * ld + i) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            w[e][4 * m] = x.x; w[e][4 * m + 1] = x.y; w[e][4 * m + 2] = x.z; w[e][4 * m + 3] = x.w;
         }
-        for (int s = 0; s < steps; ++s) {
-            const int t = j + s;
-            const bool on = jb + s < GB;
-            float acc = 0.0f;
-            if (on) {
+    float* out = sc + b0 * GC + b0 + first;
+    if (lane < 4)
+        for (int t = 0; t < first; ++t) out[t * GC + lane] = 0.0f;                  // queries in front of the keys
+    auto step = [&](int d, auto head) {                                             // query first + d; `head`: not all four keys are behind it
+        const int row = (b0 + first + d) * ld;
+        float acc[KEYS];
 #pragma unroll
-                for (int m = 0; m < M; ++m) {
-                    const int i = 4 * g + 32 * m;
-                    if (i < np) {
-                        if (s > 0) {
-                            const float4 a = *reinterpret_cast<const float4*>(As + t * ld + i);
-                            w[m].x *= a.x; w[m].y *= a.y; w[m].z *= a.z; w[m].w *= a.w;
-                        }
-                        const float4 q = *reinterpret_cast<const float4*>(Qs + t * ld + i);
-                        acc = fmaf(w[m].x, q.x, fmaf(w[m].y, q.y, fmaf(w[m].z, q.z, fmaf(w[m].w, q.w, acc))));
-                    }
+        for (int e = 0; e < KEYS; ++e) acc[e] = 0.0f;
+#pragma unroll
+        for (int m = 0; m < M; ++m) {
+            const int i = 4 * (l + L * m);                                          // (a lane beyond the channels carries noughts)
+            const float4 none = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            const float4 a4 = i < np ? *reinterpret_cast<const float4*>(As + row + i) : none;
+            const float4 q4 = i < np ? *reinterpret_cast<const float4*>(Qs + row + i) : none;
+            const float a[4] = {a4.x, a4.y, a4.z, a4.w}, q[4] = {q4.x, q4.y, q4.z, q4.w};
+#pragma unroll
+            for (int e = 0; e < KEYS; ++e) {
+                const bool on = !decltype(head)::value || d > key + e;
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    w[e][4 * m + c] *= on ? a[c] : 1.0f;
+                    acc[e] = fmaf(w[e][4 * m + c], q[c], acc[e]);
                 }
             }
-            acc += __shfl_xor_sync(0xffffffffu, acc, 1);
-            acc += __shfl_xor_sync(0xffffffffu, acc, 2);
-            acc += __shfl_xor_sync(0xffffffffu, acc, 4);
-            if (g == 0 && on) sc[t * GC + j] = acc;
         }
-        for (int t = g; t < jb; t += 8) sc[(b * GB + t) * GC + j] = 0.0f;           // queries in front of the key
-    }
+        // KEYS sums over L lanes: the lanes halve the keys between them first, so that each carries one, then add up the rest
+        float v;
+        if constexpr (KEYS == 4) {
+            const bool hi = lane & 16;
+            float x = (hi ? acc[2] : acc[0]) + __shfl_xor_sync(0xffffffffu, hi ? acc[0] : acc[2], 16);
+            float y = (hi ? acc[3] : acc[1]) + __shfl_xor_sync(0xffffffffu, hi ? acc[1] : acc[3], 16);
+            const bool odd = lane & 8;
+            v = (odd ? y : x) + __shfl_xor_sync(0xffffffffu, odd ? x : y, 8);
+        } else if constexpr (KEYS == 2) {
+            const bool odd = lane & 8;
+            v = (odd ? acc[1] : acc[0]) + __shfl_xor_sync(0xffffffffu, odd ? acc[0] : acc[1], 8);
+        } else {
+            v = acc[0];
+        }
+        v += __shfl_xor_sync(0xffffffffu, v, 4);
+        v += __shfl_xor_sync(0xffffffffu, v, 2);
+        v += __shfl_xor_sync(0xffffffffu, v, 1);
+        const int mine = lane >> 3;                                                 // (every eight lanes end with one key's)
+        if ((lane & 7) == 0) out[(first + d) * GC + mine] = !decltype(head)::value || d >= mine ? v : 0.0f;
+    };
+#pragma unroll
+    for (int d = 0; d < 4; ++d) step(d, std::true_type{});
+#pragma unroll 2
+    for (int d = 4; d < GB - first; ++d) step(d, std::false_type{});
 }
 
-__global__ void __launch_bounds__(256) gla_chunk_prep_kernel(GlaParams p) {
+// Gates, decayed queries and keys and scores of a chunk's head.  Bound by instructions (4,200 a warp, issued in 65 % of the cycles), which the
+// scores inside the blocks, those across, the decays' small product and roots, and the loads share about evenly; two blocks an SM by the three
+// tiles of 64 rows.  Sixteen warps each (with eight, 46 %); the raw rows by asynchronous copies, the decay's matrix through shared memory
+// (read by a thread per channel it took 16 x 32 sectors a warp), scores of four keys a warp at once: 135 -> 105 us for 2,048 rows of 32
+// heads of 128 features, rank 16 (32 -> 20 us of that the decays).  Storing the results in front of the last products lost 6 us (64 registers).
+constexpr int GP_THREADS = 512;           // a warp per four keys of the chunk
+
+__global__ void __launch_bounds__(GP_THREADS, 2) gla_chunk_prep_kernel(GlaParams p) {
     extern __shared__ __align__(16) float gc_s[];
     const int n = p.n, np = p.np, ld = np + 8;
     float* Qs = gc_s;                          // [GC][ld]
     float* Ks = Qs + (size_t)GC * ld;          // [GC][ld]
     float* As = Ks + (size_t)GC * ld;          // [GC][ld]
     float* F = As + (size_t)GC * ld;           // [GNB][np] a block's whole decay
+    const int h = blockIdx.x, ch = blockIdx.y, tid = threadIdx.x;
+    float* Rs = F;                             // [GC][GLA_RANK] the short rows, a few features at a time
+    float* Ws = As;                            // [np][GLA_WS] the head's rows of the decay's matrix, its first features
+    if (!p.forget) {
+        const bool vec = p.rank % 4 == 0 && (uintptr_t)p.wa % 16 == 0;
+        for (int idx = tid; idx < np * (GLA_RANK / 4); idx += GP_THREADS) {
+            const int i = idx / (GLA_RANK / 4), r = idx % (GLA_RANK / 4) * 4;
+            const float* w = p.wa + (size_t)(h * n + (i < n ? i : 0)) * p.rank + r;
+            float* dst = Ws + i * GLA_WS + r;
+            if (vec && i < n && r < p.rank) gla_async16(dst, w);
+            else
+#pragma unroll
+                for (int e = 0; e < 4; ++e) dst[e] = i < n && r + e < p.rank ? w[e] : 0.0f;
+        }
+    }
     pdl_launch();
     pdl_wait();
-    const int h = blockIdx.x, ch = blockIdx.y, tid = threadIdx.x;
     const int row0 = p.chunks[ch * 4 + 1], rows = p.chunks[ch * 4 + 2];
     const float* src = p.src + (size_t)row0 * p.src_stride;
-    {
-        // four channels of a token at a time; GC_BATCH / 2 such groups' loads on their way together
-        const int n4 = np >> 2;
-        for (GlaWalk w(n4); w.j < GC;) {
-            float4 x[GC_BATCH / 2], y[GC_BATCH / 2];
-            int jj[GC_BATCH / 2], ii[GC_BATCH / 2];
+    // the raw rows into the tiles, all on their way at once; then a thread makes queries, keys and decays of what it asked for itself
+    const int n4 = np >> 2;
+    for (GlaWalk w(n4); w.j < GC; w.next()) {
+        const int i = 4 * w.i, at = w.j * ld + i;
+        const float* r = src + (size_t)w.j * p.src_stride + h * n + i;
+        if (p.vec_qk && w.j < rows) {
+            gla_async16(Qs + at, r + p.q_col);
+            gla_async16(Ks + at, r + p.k_col);
+        } else {
 #pragma unroll
-            for (int u = 0; u < GC_BATCH / 2; ++u) {
-                jj[u] = w.j; ii[u] = 4 * w.i; w.next();
-                x[u] = y[u] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                if (jj[u] < rows) {
-                    const float* r = src + (size_t)jj[u] * p.src_stride + h * n + ii[u];
-                    if (p.vec_qk) {
-                        x[u] = *reinterpret_cast<const float4*>(r + p.q_col);
-                        y[u] = *reinterpret_cast<const float4*>(r + p.k_col);
-                    } else {
-                        const int m = n - ii[u];
-                        x[u] = make_float4(r[p.q_col], m > 1 ? r[p.q_col + 1] : 0.0f, m > 2 ? r[p.q_col + 2] : 0.0f, m > 3 ? r[p.q_col + 3] : 0.0f);
-                        y[u] = make_float4(r[p.k_col], m > 1 ? r[p.k_col + 1] : 0.0f, m > 2 ? r[p.k_col + 2] : 0.0f, m > 3 ? r[p.k_col + 3] : 0.0f);
-                    }
-                }
-            }
-#pragma unroll
-            for (int u = 0; u < GC_BATCH / 2; ++u) {
-                if (jj[u] >= GC) continue;
-                const float xs[4] = {x[u].x, x[u].y, x[u].z, x[u].w}, ys[4] = {y[u].x, y[u].y, y[u].z, y[u].w};
-                float q[4], k[4], a[4];
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    q[e] = k[e] = 0.0f; a[e] = 1.0f;
-                    if (jj[u] < rows && ii[u] + e < n) {
-                        q[e] = gla_query(p, xs[e]);
-                        if (p.forget) gla_forget(p, h * n + ii[u] + e, ys[e], &a[e], &k[e]); else k[e] = ys[e];
-                    }
-                }
-                const int at = jj[u] * ld + ii[u];
-                *reinterpret_cast<float4*>(Qs + at) = make_float4(q[0], q[1], q[2], q[3]);
-                *reinterpret_cast<float4*>(Ks + at) = make_float4(k[0], k[1], k[2], k[3]);
-                if (p.forget) *reinterpret_cast<float4*>(As + at) = make_float4(a[0], a[1], a[2], a[3]);
+            for (int e = 0; e < 4; ++e) {
+                const bool on = w.j < rows && i + e < n;
+                Qs[at + e] = on ? r[p.q_col + e] : 0.0f;
+                Ks[at + e] = on ? r[p.k_col + e] : 0.0f;
             }
         }
     }
-    if (!p.forget) {
-        // z = W r + b: the short rows in F's place (a few features at a time), a thread per channel and every tokens-th token
-        float* Rs = F;                         // [GC][GLA_RANK]
+    if (!p.forget)
+        for (int idx = tid; idx < GC * GLA_RANK; idx += GP_THREADS) {
+            const int t = idx / GLA_RANK, r = idx % GLA_RANK;
+            Rs[idx] = (t < rows && r < p.rank) ? src[(size_t)t * p.src_stride + p.r_col + r] : 0.0f;
+        }
+    gla_async_wait();
+    if (p.forget || p.q_silu || p.q_scale != 1.0f)
+        for (GlaWalk w(n4); w.j < rows; w.next()) {
+            const int at = w.j * ld + 4 * w.i;
+            float4 q = *reinterpret_cast<const float4*>(Qs + at);
+            q = make_float4(gla_query(p, q.x), gla_query(p, q.y), gla_query(p, q.z), gla_query(p, q.w));
+            *reinterpret_cast<float4*>(Qs + at) = q;
+            if (p.forget) {
+                const float4 y = *reinterpret_cast<const float4*>(Ks + at);
+                const float ys[4] = {y.x, y.y, y.z, y.w};
+                float a[4], k[4];
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    a[e] = 1.0f; k[e] = 0.0f;
+                    if (4 * w.i + e < n) gla_forget(p, h * n + 4 * w.i + e, ys[e], &a[e], &k[e]);
+                }
+                *reinterpret_cast<float4*>(Ks + at) = make_float4(k[0], k[1], k[2], k[3]);
+                *reinterpret_cast<float4*>(As + at) = make_float4(a[0], a[1], a[2], a[3]);
+            }
+        }
+    if (p.forget) {
+        for (int idx = tid; idx < (GC - rows) * n4; idx += GP_THREADS)
+            *reinterpret_cast<float4*>(As + (rows + idx / n4) * ld + idx % n4 * 4) = make_float4(1.0f, 1.0f, 1.0f, 1.0f);
+    } else {
+        // z = W r + b, a thread per channel and every lanes-th token
+        const int lanes = GP_THREADS / np;                                   // threads that share a channel (np is 256 at most)
+        const int i = tid % np, part = tid / np;
+        const int c = h * n + (i < n ? i : 0);
+        const float b = i < n ? p.bias[c] : 0.0f;
         for (int r0 = 0; r0 < p.rank; r0 += GLA_RANK) {
-            __syncthreads();
-            for (int idx = tid; idx < GC * GLA_RANK; idx += blockDim.x) {
-                const int t = idx / GLA_RANK, r = idx % GLA_RANK;
-                Rs[idx] = (t < rows && r0 + r < p.rank) ? src[(size_t)t * p.src_stride + p.r_col + r0 + r] : 0.0f;
+            if (r0 > 0) {
+                __syncthreads();
+                for (int idx = tid; idx < GC * GLA_RANK; idx += GP_THREADS) {
+                    const int t = idx / GLA_RANK, r = idx % GLA_RANK;
+                    Rs[idx] = (t < rows && r0 + r < p.rank) ? src[(size_t)t * p.src_stride + p.r_col + r0 + r] : 0.0f;
+                }
             }
             __syncthreads();
-            const int lanes = np < 256 ? 256 / np : 1;                       // threads that share a channel
-            for (int i = lanes > 1 ? tid % np : tid; i < np; i += 256) {
-                const int part = lanes > 1 ? tid / np : 0;
-                if (part >= lanes) break;
-                const int c = h * n + (i < n ? i : 0);
-                float w[GLA_RANK];
+            float w[GLA_RANK];
+            if (r0 == 0) {
+#pragma unroll
+                for (int r = 0; r < GLA_RANK; r += 4) {
+                    const float4 v = *reinterpret_cast<const float4*>(Ws + i * GLA_WS + r);
+                    w[r] = v.x; w[r + 1] = v.y; w[r + 2] = v.z; w[r + 3] = v.w;
+                }
+                __syncthreads();                                             // (the decays take the matrix's place)
+            } else {
 #pragma unroll
                 for (int r = 0; r < GLA_RANK; ++r) w[r] = (i < n && r0 + r < p.rank) ? p.wa[(size_t)c * p.rank + r0 + r] : 0.0f;
-                const float b = i < n ? p.bias[c] : 0.0f;
-                const bool last = r0 + GLA_RANK >= p.rank;
-                for (int t = part; t < GC; t += lanes) {
-                    float z = r0 == 0 ? b : As[t * ld + i];
+            }
+            const bool last = r0 + GLA_RANK >= p.rank;
+            for (int t = part < lanes ? part : GC; t < GC; t += lanes) {
+                float z = r0 == 0 ? b : As[t * ld + i];
 #pragma unroll
-                    for (int r = 0; r < GLA_RANK; r += 4) {
-                        const float4 v = *reinterpret_cast<const float4*>(Rs + t * GLA_RANK + r);
-                        z = fmaf(w[r], v.x, z); z = fmaf(w[r + 1], v.y, z); z = fmaf(w[r + 2], v.z, z); z = fmaf(w[r + 3], v.w, z);
-                    }
-                    if (last) z = (t < rows && i < n) ? gla_root(z, p.power) : 1.0f;
-                    As[t * ld + i] = z;
+                for (int r = 0; r < GLA_RANK; r += 4) {
+                    const float4 v = *reinterpret_cast<const float4*>(Rs + t * GLA_RANK + r);
+                    z = fmaf(w[r], v.x, z); z = fmaf(w[r + 1], v.y, z); z = fmaf(w[r + 2], v.z, z); z = fmaf(w[r + 3], v.w, z);
                 }
-                if (lanes > 1) break;
+                if (last) z = (t < rows && i < n) ? gla_root(z, p.power) : 1.0f;
+                As[t * ld + i] = z;
             }
         }
     }
     __syncthreads();
     float* sc = p.scores + ((size_t)ch * p.H + h) * GC * GC;
-    // scores inside a block of GB tokens: eight threads per key j share the channels, four neighbours at a time; each carries k_j
-    // times the decay from j to t along as t moves on, so a score is one sum per query
-    if (np <= 32) gla_block_scores<1>(Qs, Ks, As, sc, np, ld);
-    else if (np <= 64) gla_block_scores<2>(Qs, Ks, As, sc, np, ld);
-    else if (np <= 128) gla_block_scores<4>(Qs, Ks, As, sc, np, ld);
-    else gla_block_scores<8>(Qs, Ks, As, sc, np, ld);
+    if (np <= 32) gla_block_scores<8, 1>(Qs, Ks, As, sc, np, ld);
+    else if (np <= 64) gla_block_scores<16, 1>(Qs, Ks, As, sc, np, ld);
+    else if (np <= 128) gla_block_scores<32, 1>(Qs, Ks, As, sc, np, ld);
+    else gla_block_scores<32, 2>(Qs, Ks, As, sc, np, ld);
     __syncthreads();
-    // q_t times the decay from its block's start up to t, k_j times the decay behind j to its block's end, the block's decay
-    for (int e = tid; e < GNB * np; e += blockDim.x) {
+    // q_t times the decay from its block's start up to t, k_j times the decay behind j to its block's end, the block's decay: a thread per
+    // block and channel, whose values are read before any is written
+    for (int e = tid; e < GNB * np; e += GP_THREADS) {
         const int b = e / np, i = e - b * np;
         const int at = b * GB * ld + i;
-        float w = 1.0f;
+        float a[GB], x[GB], w = 1.0f;
 #pragma unroll
-        for (int t = 0; t < GB; ++t) { w *= As[at + t * ld]; Qs[at + t * ld] *= w; }
-        F[b * np + i] = w;
+        for (int t = 0; t < GB; ++t) { a[t] = As[at + t * ld]; x[t] = Qs[at + t * ld]; }
+#pragma unroll
+        for (int t = 0; t < GB; ++t) { w *= a[t]; Qs[at + t * ld] = x[t] * w; }
+        F[e] = w;
+#pragma unroll
+        for (int t = 0; t < GB; ++t) x[t] = Ks[at + t * ld];
         w = 1.0f;
 #pragma unroll
-        for (int t = GB - 1; t >= 0; --t) { Ks[at + t * ld] *= w; w *= As[at + t * ld]; }
+        for (int t = GB - 1; t >= 0; --t) { Ks[at + t * ld] = x[t] * w; w *= a[t]; }
     }
     __syncthreads();
-    // scores across blocks: a tile of 4 x 4 (queries tq + 4 u, keys jq + 4 v of their blocks) per two threads, which share the
+    // scores across blocks: a tile of 4 x 4 (queries tq + 4 u, keys jq + 4 v of their blocks) per four threads, which share the
     // channels; a warp's tiles are those of one pair of blocks
     constexpr int PAIRS = GNB * (GNB - 1) / 2, PER_PAIR = (GB / 4) * (GB / 4);
-    if (tid < PAIRS * PER_PAIR * 2) {
-        const int part = tid & 1, tile = tid >> 1;
+    if (tid < PAIRS * PER_PAIR * 4) {
+        const int part = tid & 3, tile = tid >> 2;
         const int pair = tile / PER_PAIR, in = tile % PER_PAIR;
         int I = 1, J = pair;                                                         // pairs (1,0) (2,0) (2,1) (3,0) ...
         while (J >= I) { J -= I; ++I; }
         const int t0 = I * GB + in / (GB / 4), j0 = J * GB + in % (GB / 4);
         float acc[4][4] = {};
-        for (int i = 4 * part; i < np; i += 8) {
-            float4 k[4];
+        auto products = [&](auto apart) {                                            // `apart`: whole blocks lie between the two
+            for (int i = 4 * part; i < np; i += 16) {
+                float4 k[4], q[4];
 #pragma unroll
-            for (int v = 0; v < 4; ++v) k[v] = *reinterpret_cast<const float4*>(Ks + (j0 + 4 * v) * ld + i);
-            for (int b = J + 1; b < I; ++b) {
-                const float4 f = *reinterpret_cast<const float4*>(F + b * np + i);
+                for (int v = 0; v < 4; ++v) {
+                    k[v] = *reinterpret_cast<const float4*>(Ks + (j0 + 4 * v) * ld + i);
+                    q[v] = *reinterpret_cast<const float4*>(Qs + (t0 + 4 * v) * ld + i);
+                }
+                if constexpr (decltype(apart)::value) {
+                    for (int b = J + 1; b < I; ++b) {
+                        const float4 f = *reinterpret_cast<const float4*>(F + b * np + i);
 #pragma unroll
-                for (int v = 0; v < 4; ++v) { k[v].x *= f.x; k[v].y *= f.y; k[v].z *= f.z; k[v].w *= f.w; }
+                        for (int v = 0; v < 4; ++v) { k[v].x *= f.x; k[v].y *= f.y; k[v].z *= f.z; k[v].w *= f.w; }
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+#pragma unroll
+                    for (int v = 0; v < 4; ++v)
+                        acc[u][v] = fmaf(q[u].x, k[v].x, fmaf(q[u].y, k[v].y, fmaf(q[u].z, k[v].z, fmaf(q[u].w, k[v].w, acc[u][v]))));
             }
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const float4 q = *reinterpret_cast<const float4*>(Qs + (t0 + 4 * u) * ld + i);
-#pragma unroll
-                for (int v = 0; v < 4; ++v)
-                    acc[u][v] = fmaf(q.x, k[v].x, fmaf(q.y, k[v].y, fmaf(q.z, k[v].z, fmaf(q.w, k[v].w, acc[u][v]))));
-            }
-        }
+        };
+        if (I - J > 1) products(std::true_type{}); else products(std::false_type{});
 #pragma unroll
         for (int u = 0; u < 4; ++u)
 #pragma unroll
             for (int v = 0; v < 4; ++v) {
                 acc[u][v] += __shfl_xor_sync(0xffffffffu, acc[u][v], 1);
-                if ((u >> 1) == part) sc[(t0 + 4 * u) * GC + j0 + 4 * v] = acc[u][v];
+                acc[u][v] += __shfl_xor_sync(0xffffffffu, acc[u][v], 2);
+                if (u == part) sc[(t0 + 4 * u) * GC + j0 + 4 * v] = acc[u][v];
             }
     }
-    __syncthreads();
     // the queries with the whole blocks in front of theirs, the keys with those behind
-    const int n4 = np >> 2;
-    for (int idx = tid; idx < rows * n4; idx += blockDim.x) {
+    for (int idx = tid; idx < rows * n4; idx += GP_THREADS) {
         const int t = idx / n4, i = (idx - t * n4) * 4, b = t / GB;
         float4 q = *reinterpret_cast<const float4*>(Qs + t * ld + i), k = *reinterpret_cast<const float4*>(Ks + t * ld + i);
 #pragma unroll
@@ -795,7 +866,7 @@ extern "C" int bg_gla_chunked(const GlaArgs* args, const int* chunks, int n_chun
     if (e == cudaSuccess && s_sum > BG_SMEM_OPT_IN) e = cudaFuncSetAttribute(gla_chunk_sum_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s_sum);
     if (e == cudaSuccess && s_out > BG_SMEM_OPT_IN) e = cudaFuncSetAttribute(gla_chunk_out_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s_out);
     if (e != cudaSuccess) return (int)e;
-    launch(gla_chunk_prep_kernel, dim3(p.H, n_chunks), dim3(256), s_prep, stream, p);
+    launch(gla_chunk_prep_kernel, dim3(p.H, n_chunks), dim3(GP_THREADS), s_prep, stream, p);
     BG_LAUNCH_CHECK();
     // (the float32 path, whose results leave as floats, uses no tensor cores; the sums that become the state stay on the float units, whose
     // error against 64 bits is the smaller: 1.20e-7 against 1.25e-7 for 2,048 rows of 16 heads of 128 x 128)
