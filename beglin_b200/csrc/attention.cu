@@ -485,7 +485,7 @@ __global__ void attention_merge_few_kernel(const float* __restrict__ part_o, con
 // The same, four neighbouring features a lane (heads of whole 16-byte pieces): a quarter of the loads, a split's maximum and sum and its
 // exponential by one lane instead of by all 32, results stored at once, and of the parts only those of the row's own splits (asked for
 // under predicates, still all at once).  The same sums in the same order.  Bound by latency and the parts' bytes: 550 rows of 12 float
-// heads of 64 over up to 3,000 positions 14.3 -> 9.6 us, a decoding step of 28 layers level (1.291 and 1.286 ms; all parts read: 10.3).
+// heads of 128 over up to 3,000 positions 14.3 -> 9.6 us, a decoding step of 28 layers level (1.291 and 1.286 ms; all parts read: 10.3).
 __device__ __forceinline__ void merge_store4(float* o, float a, float b, float c, float d) { *reinterpret_cast<float4*>(o) = make_float4(a, b, c, d); }
 __device__ __forceinline__ void merge_store4(__nv_bfloat16* o, float a, float b, float c, float d) {
     const __nv_bfloat162 x = __floats2bfloat162_rn(a, b), y = __floats2bfloat162_rn(c, d);

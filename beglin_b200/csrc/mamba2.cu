@@ -3,8 +3,8 @@
 //   slot = [ S: heads x P x N | conv: (taps - 1) x channels ]
 // S is the state of the recurrence, conv the last taps-1 inputs of the causal convolution (oldest first).
 // A slot is zero when its request starts, so a convolution that reaches back beyond a sequence's first
-// token finds zeros there.  Four kernels: the convolution with SiLU, the update of its state, the scan, and the gate
-// with the grouped RMS norm.  Everything that enters the recurrence is float: step sizes, decays, B, C, x.
+// token finds zeros there.  Three kernels: the convolution with SiLU and the update of its state (two where its rows are not taken in
+// runs), the scan, and the gate with the grouped RMS norm.  Everything that enters the recurrence is float: step sizes, decays, B, C, x.
 //
 // Requests are given as a list of (request, first row, number of rows), one entry per request of the step (the scan's list
 // may leave out requests whose rows run in chunks: mamba2_chunked.cu).
