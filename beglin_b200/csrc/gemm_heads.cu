@@ -119,15 +119,17 @@ gemm_heads_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
                         r[j] = __float_as_uint(__uint_as_float(r[j]) * g);
                     }
                 }
-                if (n >= p.n_out) continue;
-                if (c + 16 <= rows) {
+                if (n < p.n_out) {
+                    if (c + 16 <= rows) {
 #pragma unroll
-                    for (int j = 0; j < 16; ++j) to[(size_t)j * p.out_row] = from_float<TO>(__uint_as_float(r[j]));
-                } else {
+                        for (int j = 0; j < 16; ++j) to[(size_t)j * p.out_row] = from_float<TO>(__uint_as_float(r[j]));
+                    } else {
 #pragma unroll
-                    for (int j = 0; j < 16; ++j)
-                        if (c + j < rows) to[(size_t)j * p.out_row] = from_float<TO>(__uint_as_float(r[j]));
+                        for (int j = 0; j < 16; ++j)
+                            if (c + j < rows) to[(size_t)j * p.out_row] = from_float<TO>(__uint_as_float(r[j]));
+                    }
                 }
+                __syncwarp();                  // a load of tensor memory is the whole warp's: lanes without a feature wait for the others
             }
         }
     }

@@ -70,3 +70,25 @@ def test_one_call_gives_the_bits_of_the_single_entries(how, lens, held):
         pools.append(reqs.cache.kv_groups[0].device_pool.clone())
     assert torch.equal(outs[0], outs[1]) and torch.equal(pools[0], pools[1]) and launched[0] == launched[1]
     ops.raise_on_status(ctx.status)
+
+
+@pytest.mark.parametrize("H,T,N", [(48, 33, 72), (48, 64, 72), (80, 64, 72), (80, 61, 8), (50, 64, 100), (80, 200, 132)])
+@pytest.mark.parametrize("gate", [None, "head", "feature"])
+def test_per_head_products_whose_features_end_inside_a_warp(H, T, N, gate):
+    """More rows a CTA than one load of tensor memory gives (two loads of 16 columns and more), where lanes of a warp have no feature to store."""
+    from beglin_b200.csrc import ops
+    g = torch.Generator().manual_seed(H + T + N)
+    rnd = lambda *n: torch.randn(*n, generator=g).to(DEV, torch.bfloat16)
+    assert -(-N // 128) * H * -(-T // 16) > ops.sm_count() and N % 32
+    x, w, status = rnd(H, T, 128), rnd(H, N, 128), ops.new_status(DEV)
+    want, off = x.double() @ w.double().transpose(1, 2), 128 * 2.0 ** -24 * (x.double().abs() @ w.double().abs().transpose(1, 2))
+    gates = None if gate is None else torch.randn(T, H * N, generator=g).to(DEV)
+    out = torch.full((T, H * N + 4), 7.0, device=DEV)[:, :H * N]
+    ops.gemm_heads(x, w, out, status, gates, 0, per_feature=gate == "feature")
+    want, off = want.transpose(0, 1), off.transpose(0, 1)
+    if gate is not None:
+        s = torch.sigmoid(gates.double())
+        s = s.view(T, H, N) if gate == "feature" else s[:, :H, None]
+        want, off = want * s, off * s + 2.0 ** -20 * (want * s).abs()          # (the gate's own roundings)
+    assert ((out.view(T, H, N).double() - want).abs() <= off).all()
+    ops.raise_on_status(status)
