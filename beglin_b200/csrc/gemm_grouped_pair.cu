@@ -219,6 +219,7 @@ gemm_grouped_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid
                             if (j < left) to[(size_t)j * p.ldo] = __float2bfloat16_rn(v[j]);
                     }
                 }
+                __syncwarp();                                            // (the next load of tensor memory is the whole warp's)
             }
             tc_fence_before();
             __syncwarp();

@@ -130,6 +130,7 @@ gemm_grouped_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __g
                         else ((__nv_bfloat16*)p.out)[o] = __float2bfloat16_rn(v);
                     }
                 }
+                __syncwarp();                                            // (the next load of tensor memory is the whole warp's)
             }
         }
     }

@@ -148,6 +148,7 @@ gemm_bf16_tn_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __g
                             if (t0 + c + j < p.T) o[(size_t)j * p.ldo] = __float2bfloat16_rn(__uint_as_float(r[j]) + bias);
                     }
                 }
+                __syncwarp();                                              // (the next load of tensor memory is the whole warp's)
             }
         }
     }
