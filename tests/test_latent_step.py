@@ -72,7 +72,7 @@ def test_one_call_gives_the_bits_of_the_single_entries(how, lens, held):
     ops.raise_on_status(ctx.status)
 
 
-@pytest.mark.parametrize("H,T,N", [(48, 33, 72), (48, 64, 72), (80, 64, 72), (80, 61, 8), (50, 64, 100), (80, 200, 132)])
+@pytest.mark.parametrize("H,T,N", [(48, 49, 72), (48, 64, 72), (80, 64, 72), (80, 61, 8), (50, 64, 100), (80, 200, 132)])
 @pytest.mark.parametrize("gate", [None, "head", "feature"])
 def test_per_head_products_whose_features_end_inside_a_warp(H, T, N, gate):
     """More rows a CTA than one load of tensor memory gives (two loads of 16 columns and more), where lanes of a warp have no feature to store."""
