@@ -15,15 +15,6 @@ namespace bg {
 __device__ __forceinline__ float softplus32(float z) { return fmaxf(z, 0.0f) + log1pf(expf(-fabsf(z))); }
 __device__ __forceinline__ float silu32(float z) { return z / (1.0f + expf(-z)); }
 __device__ __forceinline__ float sigmoid32(float z) { return 1.0f / (1.0f + expf(-z)); }
-// The gates of a result that leaves as TO: with the fast exponential and division (2^-20 of itself) where that is rounded to bfloat16.
-template <typename TO> __device__ __forceinline__ float gate_sigmoid(float z) {
-    if constexpr (sizeof(TO) == 2) return __fdividef(1.0f, 1.0f + __expf(-z));
-    else return sigmoid32(z);
-}
-template <typename TO> __device__ __forceinline__ float gate_silu(float z) {
-    if constexpr (sizeof(TO) == 2) return z * gate_sigmoid<TO>(z);
-    else return silu32(z);
-}
 
 // out[t, c] = silu(b[c] + sum_j w[c, j] * in(t - (taps-1-j), c)), in(.) taken from the step's rows of the same
 // request or, further back, from the slot's conv state.  src row = [.. | channels from col0 | ..].  `src_bias` [channels]
@@ -438,7 +429,7 @@ gated_group_rmsnorm_vec8_kernel(const float* __restrict__ y, const TI* __restric
             load8(src + (size_t)t * src_stride + z_col + i0 + c * 8, zg[it]);
 #pragma unroll
             for (int k = 0; k < 8; ++k) {
-                if (mode) zg[it][k] = gate_sigmoid<TO>(zg[it][k]); else { v[it][k] *= gate_silu<TO>(zg[it][k]); zg[it][k] = 1.0f; }
+                if (mode) zg[it][k] = sigmoid32(zg[it][k]); else { v[it][k] *= silu32(zg[it][k]); zg[it][k] = 1.0f; }
                 ss += v[it][k] * v[it][k];
             }
         }
