@@ -9,6 +9,8 @@ int bg_route_rows(const void*, int, int, const float*, int, int, int, int, int, 
                   cudaStream_t);
 int bg_route_layout(const void*, int, int, const float*, int, int, int, int, int, int, const float*, float, const float*, int*, float*, int*, int*, int*, void*, int,
                     int*, int, cudaStream_t);
+int bg_route_layout_counts(int, int, int, int);
+int bg_route_rows_takes(int, int, int, int);
 int bg_gemm_grouped_tc(const void*, int, int, int, int, const void*, int, int, void*, int, int, const int*, int, unsigned*, cudaStream_t);
 int bg_gemm_grouped_pair(const void*, int, int, int, int, const void*, int, int, void*, int, int, const int*, int, unsigned*, cudaStream_t);
 int bg_glu_clamped(const void*, int, int, void*, int, int, int, float, float, cudaStream_t);
@@ -36,8 +38,6 @@ struct ExpertsArgs {
 
 namespace {
 
-constexpr int EX_COUNTS = 8192;                // of bg_route_layout
-
 struct Scratch {
     size_t ids, weights, offsets, row_of, src_of, counts, xp, gu, hp, yp, shared_gu, shared_act, shared_out, bytes;
     int n_counts;
@@ -45,7 +45,7 @@ struct Scratch {
         const size_t A = (size_t)T * a.top;
         size_t at = 0;
         auto take = [&](size_t n) { const size_t p = at; at += (n + 255) & ~(size_t)255; return p; };
-        n_counts = T <= a.few ? 0 : (int)((long long)T * a.outputs < EX_COUNTS ? (long long)T * a.outputs : EX_COUNTS);
+        n_counts = T <= a.few ? 0 : bg_route_layout_counts(T, a.hidden, a.outputs, a.top);
         ids = take(A * 4); weights = take(A * 4); offsets = take((size_t)(a.outputs + 1) * 4); row_of = take(A * 4); src_of = take(A * 4);
         counts = take((size_t)n_counts * 4);
         xp = take(A * a.hidden * 2);
@@ -61,7 +61,13 @@ struct Scratch {
 
 using namespace bg;
 
-extern "C" long long bg_experts_scratch(const ExpertsArgs* a, int T) { return (long long)Scratch(*a, T).bytes; }
+// -1 where bg_experts_step does not take a step of T tokens (on 16 bytes): to be asked before anything is made for it.
+extern "C" long long bg_experts_scratch(const ExpertsArgs* a, int T) {
+    if (T < 0 || a->hidden <= 0 || a->hidden % 8 || a->intermediate <= 0 || a->intermediate % 8 || (uintptr_t)a->router % 16) return -1;
+    if (T == 0) return 0;
+    if (T <= a->few ? !bg_route_rows_takes(T, a->hidden, a->outputs, a->top) : !bg_route_layout_counts(T, a->hidden, a->outputs, a->top)) return -1;
+    return (long long)Scratch(*a, T).bytes;
+}
 
 // out [T][hidden] float = the step's result for h [T][hidden] bfloat16.  With a shared expert its rows come from the two fused products of few tokens
 // (up_splits and down_splits ranges of their inner sizes), or, with up_splits nought, from the caller: shared [T][hidden] float and, behind a gate, sg

@@ -794,19 +794,28 @@ extern "C" int bg_route(const void* h, int h_dtype, int ldh, const float* W, int
     return BG_OK;
 }
 
+// The integers of scratch that bg_route_layout wants for a step of T tokens; nought where it does not take the sizes: rows that are not whole 16-byte
+// pieces, more than RL_MAX counts (every block of the second kernel adds them all up: 2,048 tokens of 8 experts are 1,024), more assignments to a
+// block than fit.  (Besides sizes it wants its rows on 16 bytes.)
+extern "C" int bg_route_layout_counts(int T, int d, int E, int top) {
+    if (T <= 0 || E <= 0 || E > RL_MAX_E || top <= 0 || top > E || top > 32 || d <= 0 || d % 8) return 0;
+    const RouteCut c = route_cut(T, E);
+    const long long counts = (long long)((T + c.tokens - 1) / c.tokens) * E;
+    return c.tokens * top > RL_MAX_A || counts > RL_MAX ? 0 : (int)counts;
+}
+// Whether bg_route_rows takes the sizes (it wants its rows on 16 bytes, too).
+extern "C" int bg_route_rows_takes(int T, int d, int E, int top) { return T > 0 && T <= RR_TOKENS && T * top <= RR_MAX_A && E <= 1024 && d % 8 == 0; }
+
 // bg_route, bg_route_sort and bg_route_gather (xp in h's type) of a step of any number of tokens as two kernels; hist: `n_hist` integers of
-// scratch.  BG_ERR_UNSUPPORTED, with nothing launched, where they do not take the sizes: rows that are not whole 16-byte pieces, more than
-// RL_MAX counts (every block of the second kernel adds them all up: 2,048 tokens of 8 experts are 1,024), more assignments to a block than fit.
+// scratch, bg_route_layout_counts of them at least.  BG_ERR_UNSUPPORTED, with nothing launched, where they do not take the sizes.
 extern "C" int bg_route_layout(const void* h, int h_dtype, int ldh, const float* W, int T, int d, int E, int top, int mode, int renorm,
                                const float* bias, float scale, const float* logit_bias, int* ids, float* weights, int* offsets, int* row_of,
                                int* src_of, void* xp, int scale_input, int* hist, int n_hist, cudaStream_t stream) {
     if (T <= 0) return BG_OK;
     if (E <= 0 || top <= 0 || top > E || top > 32 || d <= 0 || mode < 0 || mode > 3 || (mode == 3 && bias)) return BG_ERR_SHAPE;
     const RouteCut c = route_cut(T, E);
-    const int blocks = (T + c.tokens - 1) / c.tokens;
-    if (!route_vec(h, ldh, W, d) || (uintptr_t)xp % 16 || E > RL_MAX_E || c.tokens * top > RL_MAX_A || (long long)blocks * E > RL_MAX ||
-        (long long)blocks * E > n_hist)
-        return BG_ERR_UNSUPPORTED;
+    const int blocks = (T + c.tokens - 1) / c.tokens, counts = bg_route_layout_counts(T, d, E, top);
+    if (!counts || counts > n_hist || !route_vec(h, ldh, W, d) || (uintptr_t)xp % 16) return BG_ERR_UNSUPPORTED;
     const RouteRule rule = {mode, renorm, bias, scale, logit_bias};
     const int rc = route_launch(h, h_dtype, ldh, W, T, d, E, top, rule, ids, weights, nullptr, hist, stream);
     if (rc != BG_OK) return rc;
@@ -824,8 +833,7 @@ extern "C" int bg_route_rows(const void* h, int h_dtype, int ldh, const float* W
                              int* src_of, void* xp, int scale_input, cudaStream_t stream) {
     if (T <= 0) return BG_OK;
     if (E <= 0 || top <= 0 || top > E || top > 32 || d <= 0 || mode < 0 || mode > 3 || (mode == 3 && bias)) return BG_ERR_SHAPE;
-    if (T > RR_TOKENS || T * top > RR_MAX_A || E > 1024 || d % 8 || ldh % 8 || (uintptr_t)h % 16 || (uintptr_t)W % 16 || (uintptr_t)xp % 16)
-        return BG_ERR_UNSUPPORTED;
+    if (!bg_route_rows_takes(T, d, E, top) || ldh % 8 || (uintptr_t)h % 16 || (uintptr_t)W % 16 || (uintptr_t)xp % 16) return BG_ERR_UNSUPPORTED;
     const RouteRule rule = {mode, renorm, bias, scale, logit_bias};
     const size_t smem = (size_t)E * sizeof(float);
 #define BG_ROUTE_ROWS(G)                                                                                                    \

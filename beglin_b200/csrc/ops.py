@@ -76,6 +76,7 @@ _SIGNATURES = {
                       _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_void_p],
     "bg_route_layout": [_c_void_p, _c_int, _c_int, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void_p, _c_float, _c_void_p,
                         _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_void_p, _c_int, _c_void_p],
+    "bg_route_layout_counts": [_c_int, _c_int, _c_int, _c_int],
     "bg_experts_scratch": [_c_void_p, _c_int],
     "bg_experts_step": [_c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_void_p, _c_void_p, _c_int, _c_int, _c_void_p, _c_ll, _c_void_p,
                         _c_void_p, _c_void_p],
@@ -2096,15 +2097,20 @@ def route_rows(h: torch.Tensor, router: torch.Tensor, top: int, ids: torch.Tenso
                             scale, logit_bias)
 
 
-ROUTE_LAYOUT_COUNTS = 8192    # integers of scratch that `route_layout` can use
+ROUTE_LAYOUT_COUNTS = 8192    # integers of scratch that `route_layout` can use at most
+
+
+def route_layout_counts(T: int, d: int, E: int, top: int) -> int:
+    """The integers of scratch that `route_layout` wants for T tokens of d features and E outputs; 0 where it does not take the sizes."""
+    return lib().bg_route_layout_counts(T, d, E, top)
 
 
 def route_layout(h: torch.Tensor, router: torch.Tensor, top: int, ids: torch.Tensor, weights: torch.Tensor, offsets: torch.Tensor,
                  row_of: torch.Tensor, src_of: torch.Tensor, out: torch.Tensor, scale_input: bool, counts: torch.Tensor, sigmoid=True,
                  renorm: bool = False, bias: Optional[torch.Tensor] = None, scale: float = 1.0,
                  logit_bias: Optional[torch.Tensor] = None) -> bool:
-    """The same for any number of tokens, as two kernels, with `counts` int32 as scratch (T * E integers suffice, and no more than
-    ROUTE_LAYOUT_COUNTS are used); False, with nothing done, where they do not take the sizes."""
+    """The same for any number of tokens, as two kernels, with `counts` int32 as scratch (`route_layout_counts` says how many; T * E suffice, and
+    ROUTE_LAYOUT_COUNTS); False, with nothing done, where they do not take the sizes."""
     _i32(counts, "counts")
     return _route_and_place("route_layout", h, router, top, ids, weights, offsets, row_of, src_of, out, scale_input, counts, sigmoid, renorm, bias,
                             scale, logit_bias)
@@ -2366,7 +2372,7 @@ class ExpertsArgs(ctypes.Structure):
 
 
 def experts_scratch(args: ExpertsArgs, T: int) -> int:
-    """Bytes of scratch that `experts_step` wants for T tokens."""
+    """Bytes of scratch that `experts_step` wants for T tokens; -1 where it does not take that many (on 16 bytes)."""
     return lib().bg_experts_scratch(ctypes.byref(args), T)
 
 

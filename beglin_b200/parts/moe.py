@@ -137,9 +137,16 @@ class RoutedExperts:
 
     def _one_call(self, h: torch.Tensor):
         """The whole step as one call, or None where it does not take the step (or kernel classes are being timed)."""
-        if self._args is None or ops.profiling() or h.dtype != torch.bfloat16 or not h.is_contiguous():
+        if self._args is None or ops.profiling() or h.dtype != torch.bfloat16 or not h.is_contiguous() or h.data_ptr() % 16:
             return None
         T, s = h.shape[0], self.spec
+        size = self._scratch.get(T)
+        if size is None:
+            if len(self._scratch) >= 4096:
+                self._scratch.clear()
+            size = self._scratch[T] = ops.experts_scratch(self._args, T)
+        if size < 0:                   # asked before the shared expert runs: whoever takes the step then runs it
+            return None
         up = down = 0
         shared = gate = None
         if s.shared is not None:
@@ -147,11 +154,6 @@ class RoutedExperts:
                 up, down = self.shared_up.fused_splits(T), self.shared_down.fused_splits(T)
             else:
                 shared, gate = self._shared(h)
-        size = self._scratch.get(T)
-        if size is None:
-            if len(self._scratch) >= 4096:
-                self._scratch.clear()
-            size = self._scratch[T] = ops.experts_scratch(self._args, T)
         out = torch.empty((T, s.hidden), dtype=torch.float32, device=h.device)
         scratch = torch.empty((size,), dtype=torch.uint8, device=h.device)
         return out if ops.experts_step(self._args, h, scratch, out, up, down, shared, gate) else None
@@ -188,14 +190,14 @@ class RoutedExperts:
         T, A = h.shape[0], h.shape[0] * s.top
         outputs = s.experts + s.identity
         few = T <= ops.ROUTE_ROWS_TOKENS
-        counts = 0 if few else min(T * outputs, ops.ROUTE_LAYOUT_COUNTS)
+        counts = 0 if few else ops.route_layout_counts(T, s.hidden, outputs, s.top)
         ints = torch.empty((3 * A + outputs + 1 + counts,), dtype=torch.int32, device=dev)
         ids, row_of, src_of, offsets = ints[:A].view(T, s.top), ints[A:2 * A], ints[2 * A:3 * A], ints[3 * A:3 * A + outputs + 1]
         weights = torch.empty((T, s.top), dtype=torch.float32, device=dev)
         xp = torch.empty((A, s.hidden), dtype=ct, device=dev)
         how = dict(sigmoid=s.router_activation, renorm=s.renormalize, bias=self.choice_bias, scale=s.route_scale, logit_bias=self.logit_bias)
         place = (h, self.router, s.top, ids, weights, offsets, row_of, src_of, xp, s.scale_input)
-        if not (ops.route_rows(*place, **how) if few else ops.route_layout(*place, ints[3 * A + outputs + 1:], **how)):
+        if not (ops.route_rows(*place, **how) if few else counts and ops.route_layout(*place, ints[3 * A + outputs + 1:], **how)):
             ops.route(h, self.router, s.top, ids, weights, **how)
             ops.route_sort(ids.view(-1), outputs, offsets, row_of, src_of)
             ops.route_gather(h, weights.view(-1), src_of, xp, s.top, scale=s.scale_input)

@@ -50,3 +50,55 @@ def test_one_call_leaves_sizes_of_odd_pieces_to_the_single_entries():
     assert part._one_call(h) is None and part.forward(h, None).shape == (40, 192)
     wide = torch.randn(8, 400, generator=gen).to(DEV, torch.bfloat16)
     assert layer("plain", 4, 2, gen)._one_call(wide[:, :192]) is None       # rows that do not lie one behind the other
+
+
+@pytest.mark.parametrize("form,experts,T", [("clamped", 16, 2000), ("clamped", 62, 130), ("clamped", 62, 300), ("clamped", 62, 600), ("silu", 128, 65), ("silu", 64, 2048),
+                                            ("clamped", 32, 250), ("silu_odd", 255, 40), ("silu", 300, 20), ("clamped", 1200, 3)])
+def test_a_shared_expert_runs_once_whatever_the_routing_takes(form, experts, T):
+    """Steps on both sides of what the routing's kernels take (300 outputs and more, and 8,192 counts), with a shared expert: the result and the launches of the
+    single entries, and no result of the shared expert's that nobody uses."""
+    from beglin_b200.csrc import ops
+    gen = torch.Generator().manual_seed(T)
+    part = layer(form, experts, 2, gen, hidden=64, ff=16)
+    h = torch.randn(T, 64, generator=gen).to(DEV, torch.bfloat16)
+    ran, shared = [], part._shared
+    part._shared = lambda x: ran.append(x) or shared(x)
+    before = ops.launch_count()
+    got = part.forward(h, None)
+    counted = ops.launch_count() - before
+    once = len(ran)
+    part._args = None
+    before = ops.launch_count()
+    want = part.forward(h, None)
+    assert torch.equal(got, want) and counted == ops.launch_count() - before and once <= 1
+    ops.raise_on_status(part.ctx.status)
+
+
+def test_rows_off_16_bytes_run_the_shared_expert_once():
+    from beglin_b200.csrc import ops
+    gen = torch.Generator().manual_seed(0)
+    part = layer("clamped", 4, 2, gen)
+    rows = torch.randn(40 * 192, generator=gen).to(DEV, torch.bfloat16)
+    off = torch.cat([rows.new_zeros(1), rows])[1:].view(40, 192)
+    assert off.data_ptr() % 16
+    ran, shared = [], part._shared
+    part._shared = lambda x: ran.append(x) or shared(x.clone())      # (the products want their rows on 16 bytes)
+    got = part.forward(off, None)
+    assert len(ran) == 1
+    want = part.forward(rows.view(40, 192), None)
+    # (the router adds rows off 16 bytes up in another order: 192 x 2^-24 of logits below eight)
+    assert float((got - want).norm() / want.norm()) < 1e-4
+    ops.raise_on_status(part.ctx.status)
+
+
+def test_scratch_of_the_layout_is_what_its_kernels_take():
+    from beglin_b200.csrc import ops
+    gen = torch.Generator().manual_seed(1)
+    for T, E, top in [(9, 10, 2), (256, 32, 4), (257, 33, 1), (1820, 18, 2), (1824, 18, 2), (32, 256, 3), (33, 256, 3), (40, 257, 2), (2048, 8, 8)]:
+        n = ops.route_layout_counts(T, 64, E, top)
+        assert 0 <= n <= min(T * E, ops.ROUTE_LAYOUT_COUNTS)
+        i32 = lambda k: torch.empty(k, dtype=torch.int32, device=DEV)
+        args = (torch.randn(T, 64, generator=gen).to(DEV), torch.randn(E, 64, generator=gen).to(DEV), top, i32((T, top)), torch.zeros((T, top), device=DEV), i32(E + 1),
+                i32(T * top), i32(T * top), torch.empty((T * top, 64), device=DEV), False)
+        assert ops.route_layout(*args, i32(max(n, 1))) == (n > 0) and (n < 2 or not ops.route_layout(*args, i32(n - 1)))
+    assert ops.route_layout_counts(64, 60, 8, 2) == 0
