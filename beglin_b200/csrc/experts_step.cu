@@ -41,7 +41,7 @@ namespace {
 struct Scratch {
     size_t ids, weights, offsets, row_of, src_of, counts, xp, gu, hp, yp, shared_gu, shared_act, shared_out, bytes;
     int n_counts;
-    Scratch(const ExpertsArgs& a, int T) {
+    Scratch(const ExpertsArgs& a, int T, bool inside) {        // inside: the shared expert's products run in the call
         const size_t A = (size_t)T * a.top;
         size_t at = 0;
         auto take = [&](size_t n) { const size_t p = at; at += (n + 255) & ~(size_t)255; return p; };
@@ -52,7 +52,8 @@ struct Scratch {
         gu = take(a.gated ? A * 2 * a.intermediate * 2 : 0);
         hp = take(A * a.intermediate * 2);
         yp = take(A * a.hidden * 4);
-        shared_gu = take((size_t)T * a.shared_rows * 4); shared_act = take((size_t)T * a.shared * 2); shared_out = take(a.shared ? (size_t)T * a.hidden * 4 : 0);
+        const size_t own = inside && a.shared ? T : 0;
+        shared_gu = take(own * a.shared_rows * 4); shared_act = take(own * a.shared * 2); shared_out = take(own * a.hidden * 4);
         bytes = at;
     }
 };
@@ -61,12 +62,13 @@ struct Scratch {
 
 using namespace bg;
 
-// -1 where bg_experts_step does not take a step of T tokens (on 16 bytes): to be asked before anything is made for it.
-extern "C" long long bg_experts_scratch(const ExpertsArgs* a, int T) {
+// -1 where bg_experts_step does not take a step of T tokens (on 16 bytes): to be asked before anything is made for it.  inside: whether the shared
+// expert's products run in the call (with up_splits).
+extern "C" long long bg_experts_scratch(const ExpertsArgs* a, int T, int inside) {
     if (T < 0 || a->hidden <= 0 || a->hidden % 8 || a->intermediate <= 0 || a->intermediate % 8 || (uintptr_t)a->router % 16) return -1;
     if (T == 0) return 0;
     if (T <= a->few ? !bg_route_rows_takes(T, a->hidden, a->outputs, a->top) : !bg_route_layout_counts(T, a->hidden, a->outputs, a->top)) return -1;
-    return (long long)Scratch(*a, T).bytes;
+    return (long long)Scratch(*a, T, inside).bytes;
 }
 
 // out [T][hidden] float = the step's result for h [T][hidden] bfloat16.  With a shared expert its rows come from the two fused products of few tokens
@@ -79,7 +81,7 @@ extern "C" int bg_experts_step(const ExpertsArgs* args, const void* h, int T, in
     const ExpertsArgs& a = *args;
     if (a.hidden <= 0 || a.hidden % 8 || a.intermediate <= 0 || a.intermediate % 8 || (uintptr_t)h % 16 || (uintptr_t)scratch % 16)
         return BG_ERR_UNSUPPORTED;
-    const Scratch s(a, T);
+    const Scratch s(a, T, up_splits != 0);
     if (scratch_bytes < (long long)s.bytes) return BG_ERR_SHAPE;
     char* w = (char*)scratch;
     int* ids = (int*)(w + s.ids); float* weights = (float*)(w + s.weights); int* offsets = (int*)(w + s.offsets);

@@ -77,7 +77,7 @@ _SIGNATURES = {
     "bg_route_layout": [_c_void_p, _c_int, _c_int, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void_p, _c_float, _c_void_p,
                         _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_void_p, _c_int, _c_void_p],
     "bg_route_layout_counts": [_c_int, _c_int, _c_int, _c_int],
-    "bg_experts_scratch": [_c_void_p, _c_int],
+    "bg_experts_scratch": [_c_void_p, _c_int, _c_int],
     "bg_experts_step": [_c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_void_p, _c_void_p, _c_int, _c_int, _c_void_p, _c_ll, _c_void_p,
                         _c_void_p, _c_void_p],
     "bg_route_sort": [_c_void_p, _c_int, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_void_p],
@@ -2371,9 +2371,10 @@ class ExpertsArgs(ctypes.Structure):
                 ("shared_gated", _c_int), ("few", _c_int), ("route_scale", _c_float), ("limit", _c_float), ("shared_limit", _c_float), ("alpha", _c_float)]
 
 
-def experts_scratch(args: ExpertsArgs, T: int) -> int:
-    """Bytes of scratch that `experts_step` wants for T tokens; -1 where it does not take that many (on 16 bytes)."""
-    return lib().bg_experts_scratch(ctypes.byref(args), T)
+def experts_scratch(args: ExpertsArgs, T: int, inside: bool) -> int:
+    """Bytes of scratch that `experts_step` wants for T tokens, with the shared expert's products `inside` it or without; -1 where it does not
+    take that many (on 16 bytes)."""
+    return lib().bg_experts_scratch(ctypes.byref(args), T, inside)
 
 
 def experts_step(args: ExpertsArgs, h: torch.Tensor, scratch: torch.Tensor, out: torch.Tensor, up_splits: int = 0, down_splits: int = 0,

@@ -140,20 +140,20 @@ class RoutedExperts:
         if self._args is None or ops.profiling() or h.dtype != torch.bfloat16 or not h.is_contiguous() or h.data_ptr() % 16:
             return None
         T, s = h.shape[0], self.spec
+        inside = s.shared is not None and s.shared.intermediate % 8 == 0 and self.shared_up.fuses(T) and self.shared_down.fuses(T)
         size = self._scratch.get(T)
         if size is None:
             if len(self._scratch) >= 4096:
                 self._scratch.clear()
-            size = self._scratch[T] = ops.experts_scratch(self._args, T)
+            size = self._scratch[T] = ops.experts_scratch(self._args, T, inside)
         if size < 0:                   # asked before the shared expert runs: whoever takes the step then runs it
             return None
         up = down = 0
         shared = gate = None
-        if s.shared is not None:
-            if s.shared.intermediate % 8 == 0 and self.shared_up.fuses(T) and self.shared_down.fuses(T):
-                up, down = self.shared_up.fused_splits(T), self.shared_down.fused_splits(T)
-            else:
-                shared, gate = self._shared(h)
+        if inside:
+            up, down = self.shared_up.fused_splits(T), self.shared_down.fused_splits(T)
+        elif s.shared is not None:
+            shared, gate = self._shared(h)
         out = torch.empty((T, s.hidden), dtype=torch.float32, device=h.device)
         scratch = torch.empty((size,), dtype=torch.uint8, device=h.device)
         return out if ops.experts_step(self._args, h, scratch, out, up, down, shared, gate) else None

@@ -102,3 +102,15 @@ def test_scratch_of_the_layout_is_what_its_kernels_take():
                 i32(T * top), i32(T * top), torch.empty((T * top, 64), device=DEV), False)
         assert ops.route_layout(*args, i32(max(n, 1))) == (n > 0) and (n < 2 or not ops.route_layout(*args, i32(n - 1)))
     assert ops.route_layout_counts(64, 60, 8, 2) == 0
+
+
+def test_scratch_holds_the_shared_experts_rows_only_where_they_are_made_in_the_call():
+    from beglin_b200.csrc import ops
+    part = layer("clamped", 4, 2, torch.Generator().manual_seed(1))
+    up = lambda n: -(-n // 256) * 256
+    for T in (8, 300):
+        more = up(T * part.shared_up.out_features * 4) + up(T * 128 * 2) + up(T * 192 * 4)
+        assert ops.experts_scratch(part._args, T, True) - ops.experts_scratch(part._args, T, False) == more
+    for T in (8, 17, 300):
+        part.forward(torch.randn(T, 192).to(DEV, torch.bfloat16), None)
+        assert part._scratch[T] == ops.experts_scratch(part._args, T, part.shared_up.fuses(T))
