@@ -103,7 +103,7 @@ __global__ void route_topk_kernel(const float* __restrict__ logits, int T, int E
 // forms the float logits of all the block's tokens against that expert's row (the row is read once per block; a lane
 // walks the features 32 apart and the warp adds up, so a logit's order of summation depends on nothing but the width);
 // then warp w chooses for token w.  `logits_out`, when given, also receives the logits.
-constexpr int ROUTE_TOKENS = 8, ROUTE_UNROLL = 8;
+constexpr int ROUTE_LOG = 3, ROUTE_TOKENS = 1 << ROUTE_LOG, ROUTE_UNROLL = 8;
 template <typename TI>
 __global__ void __launch_bounds__(32 * ROUTE_TOKENS)
 route_kernel(const TI* __restrict__ h, int ldh, const float* __restrict__ W, int T, int d, int E, int top, RouteRule rule,
@@ -152,7 +152,8 @@ route_kernel(const TI* __restrict__ h, int ldh, const float* __restrict__ W, int
 // The logits of TPW tokens' rows (row, row + ldh, ..; those from `live` on are the first one's again and not stored) by `warps` warps of a block
 // (this is the `warp`-th), each a group of G experts at a time: a lane walks the features in chunks of eight, 32 chunks apart (16-byte
 // loads), and the warp adds up.  An expert's row is fetched once for all the tokens; a logit's sum does not depend on TPW, G or `warps`.
-// Experts from E on are the last one again and not stored: a condition on the loads keeps them from being on their way together.
+// Several tokens: experts from E on are the last one again and not stored, since a condition on the loads keeps them from being on their way
+// together.  One token: loads under conditions, which fetch nothing twice (18 outputs of 4,096 features 9.8 us, without conditions 10.4).
 template <typename TI, int TPW, int G>
 __device__ __forceinline__ void route_logits_of(const TI* row, int ldh, int live, const float* __restrict__ W, int d8, int d, int E, float* sc,
                                                 float* logits_out, int warp, int warps, int lane) {
@@ -167,6 +168,15 @@ __device__ __forceinline__ void route_logits_of(const TI* row, int ldh, int live
             float hv[TPW][8], wv[G][8];
 #pragma unroll
             for (int q = 0; q < TPW; ++q) load8(row + (size_t)(q < live ? q : 0) * ldh + 8 * c, hv[q]);
+            if constexpr (TPW == 1) {
+#pragma unroll
+                for (int u = 0; u < G; ++u)
+                    if (e0 + u < E) {
+                        load8(W + (size_t)(e0 + u) * d + 8 * c, wv[u]);
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) acc[0][u] = fmaf(hv[0][i], wv[u][i], acc[0][u]);
+                    }
+            } else {
 #pragma unroll
             for (int u = 0; u < G; ++u) load8(W + (size_t)min(e0 + u, E - 1) * d + 8 * c, wv[u]);
 #pragma unroll
@@ -175,6 +185,7 @@ __device__ __forceinline__ void route_logits_of(const TI* row, int ldh, int live
                 for (int q = 0; q < TPW; ++q)
 #pragma unroll
                     for (int i = 0; i < 8; ++i) acc[q][u] = fmaf(hv[q][i], wv[u][i], acc[q][u]);
+            }
         }
 #pragma unroll
         for (int q = 0; q < TPW; ++q)
@@ -197,20 +208,21 @@ __device__ __forceinline__ void route_logits_of(const TI* row, int ldh, int live
 // `hist`, when given, receives how many of the block's assignments each expert has, [blocks][E].
 template <typename TI, int TPW, int G>
 __global__ void __launch_bounds__(32 * ROUTE_TOKENS)
-route_vec8_kernel(const TI* __restrict__ h, int ldh, const float* __restrict__ W, int T, int d, int E, int top, RouteRule rule, int wpt,
+route_vec8_kernel(const TI* __restrict__ h, int ldh, const float* __restrict__ W, int T, int d, int E, int top, RouteRule rule, int wpt_log,
                   int* __restrict__ ids, float* __restrict__ weights, float* __restrict__ logits_out, int* __restrict__ hist) {
     extern __shared__ float logit_s[];                     // [tokens][E], then the experts' counts
     pdl_launch();
-    pdl_wait();
+    const int wpt = 1 << wpt_log;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int tokens = TPW * (ROUTE_TOKENS / wpt), t0 = blockIdx.x * tokens, n = min(tokens, T - t0);
-    const int first = warp / wpt * TPW;                    // of this warp's tokens, in the block
+    const int tokens = TPW << (ROUTE_LOG - wpt_log), t0 = blockIdx.x * tokens, n = min(tokens, T - t0);
+    const int first = (warp >> wpt_log) * TPW;                // of this warp's tokens, in the block
     const int live = min(TPW, n - first);
     int* count_s = (int*)(logit_s + tokens * E);
     if (hist) for (int e = threadIdx.x; e < E; e += blockDim.x) count_s[e] = 0;
+    pdl_wait();
     if (live > 0)
         route_logits_of<TI, TPW, G>(h + (size_t)(t0 + first) * ldh, ldh, live, W, d >> 3, d, E, logit_s + first * E,
-                                    logits_out ? logits_out + (size_t)(t0 + first) * E : nullptr, warp % wpt, wpt, lane);
+                                    logits_out ? logits_out + (size_t)(t0 + first) * E : nullptr, warp & (wpt - 1), wpt, lane);
     __syncthreads();                                       // every warp comes here, with or without a token
     for (int tl = warp; tl < n; tl += ROUTE_TOKENS) {
         choose_experts(logit_s + tl * E, E, top, rule, ids, weights, (size_t)(t0 + tl), lane);
@@ -748,15 +760,17 @@ extern "C" int bg_route_topk(const float* logits, int T, int E, int top, int mod
     return BG_OK;
 }
 
-// How the router's kernel of 16-byte loads cuts a step: `tpw` tokens and `g` experts a warp at a time, `wpt` warps to the same tokens, `tokens` a
+// How the router's kernel of 16-byte loads cuts a step: `tpw` tokens and `g` experts a warp at a time, 2^`wpt_log` warps to the same tokens, `tokens` a
 // block.  Few tokens: a block each, and as many experts a warp as let them go through in one pass (the loads of a pass are all on their way
-// together; ten router outputs: 9.3 -> 7.8 us).  More than 256: four tokens a warp.
-struct RouteCut { int tpw, g, wpt, tokens; };
+// together; ten router outputs: 9.3 -> 7.8 us).  More than 256: four tokens a warp, where there are more than four experts: for four a block of eight
+// warps would be 32 tokens (300 to 2,048 tokens of four outputs: 1,536 features 5.7 to 10.6 us with a token a warp, 11.6 to 12.4 with four).
+struct RouteCut { int tpw, g, wpt_log, tokens; };
 static RouteCut route_cut(int T, int E) {
-    if (T <= 256) return {1, E <= ROUTE_TOKENS ? 1 : E <= 2 * ROUTE_TOKENS ? 2 : 4, ROUTE_TOKENS, 1};
-    int wpt = 1;
-    while (wpt < ROUTE_TOKENS && wpt * 4 < E) wpt *= 2;
-    return {4, 4, wpt, 4 * (ROUTE_TOKENS / wpt)};
+    if (T <= 256) return {1, E <= ROUTE_TOKENS ? 1 : E <= 2 * ROUTE_TOKENS ? 2 : 4, ROUTE_LOG, 1};
+    if (E <= 4) return {1, 4, 0, ROUTE_TOKENS};
+    int log = 0;
+    while (log < ROUTE_LOG && (4 << log) < E) ++log;
+    return {4, 4, log, 4 << (ROUTE_LOG - log)};
 }
 static bool route_vec(const void* h, int ldh, const float* W, int d) {
     return d % 8 == 0 && ldh % 8 == 0 && (uintptr_t)h % 16 == 0 && (uintptr_t)W % 16 == 0;
@@ -768,7 +782,7 @@ static int route_launch(const void* h, int h_dtype, int ldh, const float* W, int
     if (smem > 40 * 1024) return BG_ERR_UNSUPPORTED;
 #define BG_ROUTE_VEC(TPW, G)                                                                                                     \
     BG_DISPATCH_DTYPE(h_dtype, TI, launch(route_vec8_kernel<TI, TPW, G>, dim3((T + c.tokens - 1) / c.tokens), dim3(32 * ROUTE_TOKENS), smem, \
-                                          stream, (const TI*)h, ldh, W, T, d, E, top, rule, c.wpt, ids, weights, logits_out, hist))
+                                          stream, (const TI*)h, ldh, W, T, d, E, top, rule, c.wpt_log, ids, weights, logits_out, hist))
     if (c.tpw == 4) BG_ROUTE_VEC(4, 4);
     else if (c.g == 1) BG_ROUTE_VEC(1, 1);
     else if (c.g == 2) BG_ROUTE_VEC(1, 2);
