@@ -817,6 +817,13 @@ extern "C" int bg_route_layout_counts(int T, int d, int E, int top) {
     const long long counts = (long long)((T + c.tokens - 1) / c.tokens) * E;
     return c.tokens * top > RL_MAX_A || counts > RL_MAX ? 0 : (int)counts;
 }
+// The same where the two kernels are no slower than three.  Every block of the second one adds up the counts and lays out its own rows, which takes
+// longer than one block's sort and a gather as long as the sort has few experts or the blocks are many
+// (us for three and two kernels: 10 outputs, 768 features, 64 tokens 6.8 and 8.1, 1,536 features, 512 tokens 12.1 and 13.1; 32 outputs, 1,536 features, 64
+// tokens 11.2 and 11.0, 256 15.3 and 16.2, 1,024 17.9 and 16.6; 64 outputs, 4,096 features, 300 tokens 35.9 and 30.7).
+extern "C" int bg_route_layout_wins(int T, int d, int E, int top) {
+    return E >= 32 && d >= 1024 && (T <= 128 || T > 256) ? bg_route_layout_counts(T, d, E, top) : 0;
+}
 // Whether bg_route_rows takes the sizes (it wants its rows on 16 bytes, too).
 extern "C" int bg_route_rows_takes(int T, int d, int E, int top) { return T > 0 && T <= RR_TOKENS && T * top <= RR_MAX_A && E <= 1024 && d % 8 == 0; }
 

@@ -77,6 +77,7 @@ _SIGNATURES = {
     "bg_route_layout": [_c_void_p, _c_int, _c_int, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void_p, _c_float, _c_void_p,
                         _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_void_p, _c_int, _c_void_p],
     "bg_route_layout_counts": [_c_int, _c_int, _c_int, _c_int],
+    "bg_route_layout_wins": [_c_int, _c_int, _c_int, _c_int],
     "bg_experts_scratch": [_c_void_p, _c_int, _c_int],
     "bg_experts_step": [_c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_void_p, _c_void_p, _c_int, _c_int, _c_void_p, _c_ll, _c_void_p,
                         _c_void_p, _c_void_p],
@@ -2103,6 +2104,11 @@ ROUTE_LAYOUT_COUNTS = 8192    # integers of scratch that `route_layout` can use 
 def route_layout_counts(T: int, d: int, E: int, top: int) -> int:
     """The integers of scratch that `route_layout` wants for T tokens of d features and E outputs; 0 where it does not take the sizes."""
     return lib().bg_route_layout_counts(T, d, E, top)
+
+
+def route_layout_wins(T: int, d: int, E: int, top: int) -> int:
+    """The same where `route_layout` is no slower than `route`, `route_sort` and `route_gather`, else 0."""
+    return lib().bg_route_layout_wins(T, d, E, top)
 
 
 def route_layout(h: torch.Tensor, router: torch.Tensor, top: int, ids: torch.Tensor, weights: torch.Tensor, offsets: torch.Tensor,

@@ -190,7 +190,7 @@ class RoutedExperts:
         T, A = h.shape[0], h.shape[0] * s.top
         outputs = s.experts + s.identity
         few = T <= ops.ROUTE_ROWS_TOKENS
-        counts = 0 if few else ops.route_layout_counts(T, s.hidden, outputs, s.top)
+        counts = 0 if few else ops.route_layout_wins(T, s.hidden, outputs, s.top)
         ints = torch.empty((3 * A + outputs + 1 + counts,), dtype=torch.int32, device=dev)
         ids, row_of, src_of, offsets = ints[:A].view(T, s.top), ints[A:2 * A], ints[2 * A:3 * A], ints[3 * A:3 * A + outputs + 1]
         weights = torch.empty((T, s.top), dtype=torch.float32, device=dev)

@@ -114,3 +114,21 @@ def test_scratch_holds_the_shared_experts_rows_only_where_they_are_made_in_the_c
     for T in (8, 17, 300):
         part.forward(torch.randn(T, 192).to(DEV, torch.bfloat16), None)
         assert part._scratch[T] == ops.experts_scratch(part._args, T, part.shared_up.fuses(T))
+
+
+@pytest.mark.parametrize("T,two", [(9, True), (128, True), (129, False), (256, False), (257, True), (1024, True), (1025, None)])
+def test_routing_of_many_outputs_in_two_kernels_or_three(T, two):
+    """32 outputs of 1,024 features, where the layout's kernel wins but for 129 to 256 tokens, up to its 8,192 counts."""
+    from beglin_b200.csrc import ops
+    gen = torch.Generator().manual_seed(T)
+    part = layer("silu", 32, 2, gen, hidden=1024, ff=16)
+    h = torch.randn(T, 1024, generator=gen).to(DEV, torch.bfloat16)
+    assert bool(ops.route_layout_wins(T, 1024, 32, 2)) == bool(two) and (part._one_call(h) is None) == (two is None)
+    before = ops.launch_count()
+    got = part.forward(h, None)
+    counted = ops.launch_count() - before
+    args, part._args = part._args, None
+    before = ops.launch_count()
+    want = part.forward(h, None)
+    assert torch.equal(got, want) and counted == ops.launch_count() - before
+    ops.raise_on_status(part.ctx.status)
