@@ -79,8 +79,8 @@ _SIGNATURES = {
     "bg_route_layout_counts": [_c_int, _c_int, _c_int, _c_int],
     "bg_route_layout_wins": [_c_int, _c_int, _c_int, _c_int],
     "bg_experts_scratch": [_c_void_p, _c_int, _c_int],
-    "bg_experts_step": [_c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_void_p, _c_void_p, _c_int, _c_int, _c_void_p, _c_ll, _c_void_p,
-                        _c_void_p, _c_void_p],
+    "bg_experts_step": [_c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_void_p, _c_ll, _c_void_p, _c_void_p, _c_void_p],
+    "bg_experts_sum": [_c_void_p, _c_void_p, _c_int, _c_void_p, _c_void_p, _c_int, _c_int, _c_void_p, _c_ll, _c_void_p, _c_void_p],
     "bg_route_sort": [_c_void_p, _c_int, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_void_p],
     "bg_route_gather": [_c_void_p, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void_p],
     "bg_route_combine": [_c_void_p, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_void_p],
@@ -2383,25 +2383,28 @@ def experts_scratch(args: ExpertsArgs, T: int, inside: bool) -> int:
     return lib().bg_experts_scratch(ctypes.byref(args), T, inside)
 
 
-def experts_step(args: ExpertsArgs, h: torch.Tensor, scratch: torch.Tensor, out: torch.Tensor, up_splits: int = 0, down_splits: int = 0,
-                 shared: Optional[torch.Tensor] = None, sg: Optional[torch.Tensor] = None) -> bool:
+def experts_step(args: ExpertsArgs, h: torch.Tensor, scratch: torch.Tensor, out: torch.Tensor, up_splits: int = 0, down_splits: int = 0) -> bool:
     """A step's routed experts as one call: h bfloat16 [T, hidden], scratch bytes, out float32 [T, hidden], all contiguous.  A shared expert runs
-    inside (`up_splits`, `down_splits`: the ranges of its two fused products) or comes as its rows `shared` float32 [T, hidden] and the gate's
-    numbers `sg` [T].  False, with nothing launched, where the routing does not take the sizes."""
+    inside (`up_splits`, `down_splits`: the ranges of its two fused products), or, without them, `experts_sum` ends the step with its rows.
+    False, with nothing launched, where the routing does not take the sizes."""
     T = h.shape[0]
     if not h.is_cuda or h.dtype != torch.bfloat16 or not h.is_contiguous() or h.shape[1] != args.hidden or out.dtype != torch.float32 \
             or tuple(out.shape) != (T, args.hidden) or not out.is_contiguous():
         raise KernelError(f"experts_step: h bfloat16 [T, {args.hidden}], out float32 like it, contiguous on the device")
-    if shared is not None and (shared.dtype != torch.float32 or tuple(shared.shape) != (T, args.hidden) or not shared.is_contiguous()):
-        raise KernelError("experts_step: shared float32 [T, d]")
-    if args.shared and not up_splits and (shared is None or (sg is None) != (not args.shared_gated)):
-        raise KernelError("experts_step: the shared expert's rows (and gate) are missing")
     n = _c_int(0)
-    rc = lib().bg_experts_step(ctypes.byref(args), h.data_ptr(), T, grouped_pairs(T * args.top, args.experts), up_splits, down_splits, _p(shared), _p(sg),
-                               F32 if sg is None else _dt(sg), 0 if sg is None else sg.stride(0), scratch.data_ptr(), scratch.numel(), out.data_ptr(),
-                               ctypes.byref(n), _stream())
+    rc = lib().bg_experts_step(ctypes.byref(args), h.data_ptr(), T, grouped_pairs(T * args.top, args.experts), up_splits, down_splits, scratch.data_ptr(),
+                               scratch.numel(), out.data_ptr(), ctypes.byref(n), _stream())
     if rc == _UNSUPPORTED:
         return False
     _check(rc, "experts_step")
     count_launches(n.value - 1)
     return True
+
+
+def experts_sum(args: ExpertsArgs, h: torch.Tensor, scratch: torch.Tensor, out: torch.Tensor, shared: torch.Tensor, sg: Optional[torch.Tensor] = None) -> None:
+    """The end of an `experts_step` without its shared expert's products: the same h, scratch and out, the shared expert's rows `shared` float32
+    [T, hidden] and the gate's numbers `sg` [T]."""
+    if shared.dtype != torch.float32 or shared.shape != out.shape or h.shape != out.shape or not shared.is_contiguous() or (sg is None) != (not args.shared_gated):
+        raise KernelError("experts_sum: shared float32 [T, d], with the gate's numbers where the layer has one")
+    _check(lib().bg_experts_sum(ctypes.byref(args), h.data_ptr(), h.shape[0], shared.data_ptr(), _p(sg), F32 if sg is None else _dt(sg), 0 if sg is None else sg.stride(0),
+                                scratch.data_ptr(), scratch.numel(), out.data_ptr(), _stream()), "experts_sum")

@@ -148,15 +148,14 @@ class RoutedExperts:
             size = self._scratch[T] = ops.experts_scratch(self._args, T, inside)
         if size < 0:                   # asked before the shared expert runs: whoever takes the step then runs it
             return None
-        up = down = 0
-        shared = gate = None
-        if inside:
-            up, down = self.shared_up.fused_splits(T), self.shared_down.fused_splits(T)
-        elif s.shared is not None:
-            shared, gate = self._shared(h)
         out = torch.empty((T, s.hidden), dtype=torch.float32, device=h.device)
         scratch = torch.empty((size,), dtype=torch.uint8, device=h.device)
-        return out if ops.experts_step(self._args, h, scratch, out, up, down, shared, gate) else None
+        up, down = (self.shared_up.fused_splits(T), self.shared_down.fused_splits(T)) if inside else (0, 0)
+        if not ops.experts_step(self._args, h, scratch, out, up, down):
+            return None
+        if s.shared is not None and not inside:
+            ops.experts_sum(self._args, h, scratch, out, *self._shared(h))
+        return out
 
     def _gate(self, gate_up: torch.Tensor, out: torch.Tensor, limit: float, block: int = 0) -> None:
         """The experts' activation: gate_up [rows, >= 2 n] = [gate | up | ...] (or gate and up in turns of `block` columns)
