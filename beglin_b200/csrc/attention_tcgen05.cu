@@ -414,7 +414,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_kv, typename At
 #pragma unroll
                 for (int c0 = 0; c0 < HD; c0 += 32) {
                     float t[32], u[32];
-                    __syncwarp();                        // (lanes without a row wait for the stores of the others: the loads are the whole warp's)
+                    if (n_rows & 31) __syncwarp();       // (lanes without a row wait for the stores of the others: the loads are the whole warp's)
                     tc_ld32(tmem + lane_addr + O_COL + c0, t);
                     tc_ld32(tmem + lane_addr + O_COL + 128u + c0, u);
                     if (!real) continue;
@@ -449,7 +449,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_kv, typename At
 #pragma unroll
             for (int c0 = 0; c0 < HD; c0 += 32) {
                 float t[32], u[32];
-                __syncwarp();
+                if (n_rows & 31) __syncwarp();
                 tc_ld32(tmem + lane_addr + O_COL + c0, t);        // all lanes take part; only real rows store
                 tc_ld32(tmem + lane_addr + O_COL + 128u + c0, u);
                 if (real) {

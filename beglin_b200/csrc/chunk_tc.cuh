@@ -194,7 +194,7 @@ __global__ void __launch_bounds__(CT_THREADS, 2) chunk_sum_tc_kernel(R r) {
 #pragma unroll
                 for (int e = 0; e < 16; ++e) A[(size_t)(i0 + e) * r.nv_ld + v] = __uint_as_float(a[e]) + __uint_as_float(b[e]);
             }
-            __syncwarp();                    // (a load of tensor memory is the whole warp's: lanes without a column wait for the others)
+            if (r.nv & 31) __syncwarp();     // (a load of tensor memory is the whole warp's: lanes without a column wait for the others)
         }
     }
     ct_end(s, r.status);
@@ -315,7 +315,7 @@ __global__ void __launch_bounds__(CT_THREADS, 2) chunk_out_tc_kernel(R r) {
                     out[(t0 + e) * CT_OUT_LD + v] = fmaf(c.factor(t0 + e), __uint_as_float(a[e]) + __uint_as_float(b[e]),
                                                          __uint_as_float(f[e]) + __uint_as_float(g[e]));
             }
-            __syncwarp();                    // (as in the sums)
+            if (r.nv & 31) __syncwarp();     // (as in the sums)
         }
     }
     tc_fence_before();

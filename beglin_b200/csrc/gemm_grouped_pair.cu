@@ -197,6 +197,8 @@ gemm_grouped_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid
             if (!ok) break;
             tc_fence_after();
             const unsigned t_addr = tmem_base + ((unsigned)(quarter * 32) << 16) + (unsigned)(b * GGP_ROWS);
+            // lanes without a feature wait for the others: a load of tensor memory is the whole warp's
+            const bool ragged = p.n_out % 32 != 0 && t.m0 + (int)rank * TC_BM + TC_BM > p.n_out;
             for (int c = 0; c < t.rows; c += 32) {
                 float v[32];
                 tc_ld32(t_addr + (unsigned)c, v);
@@ -219,7 +221,7 @@ gemm_grouped_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid
                             if (j < left) to[(size_t)j * p.ldo] = __float2bfloat16_rn(v[j]);
                     }
                 }
-                __syncwarp();                                            // (the next load of tensor memory is the whole warp's)
+                if (ragged) __syncwarp();
             }
             tc_fence_before();
             __syncwarp();

@@ -114,6 +114,7 @@ gemm_grouped_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __g
         if (!ok) atomicExch(&failed, 1);
         tc_fence_after();
         if (ok) {
+            const bool ragged = p.n_out % 32 != 0 && tile_m * TC_BM + TC_BM > p.n_out;         // lanes without a feature wait for the others: a load of tensor memory is the whole warp's
 #pragma unroll 1
             for (int c = 0; c < BN; c += 16) {
                 if (c >= n_rows) break;                                  // warp-uniform
@@ -130,7 +131,7 @@ gemm_grouped_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __g
                         else ((__nv_bfloat16*)p.out)[o] = __float2bfloat16_rn(v);
                     }
                 }
-                __syncwarp();                                            // (the next load of tensor memory is the whole warp's)
+                if (ragged) __syncwarp();
             }
         }
     }

@@ -106,6 +106,8 @@ gemm_heads_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
         if (__all_sync(0xffffffffu, ok)) {
             TO* to = (TO*)p.out + (size_t)h * p.out_head + (size_t)t0 * p.out_row + n;
             const unsigned t_addr = tmem_base + ((unsigned)(quarter * 32) << 16);
+            // a load of tensor memory is the whole warp's: where features end inside a warp, lanes without one wait for the others
+            const bool ragged = p.n_out % 32 != 0 && m0 + TC_BM > p.n_out;
 #pragma unroll 1
             for (int c = 0; c < rows; c += 16, to += (size_t)16 * p.out_row) {
                 unsigned r[16];
@@ -129,7 +131,7 @@ gemm_heads_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
                             if (c + j < rows) to[(size_t)j * p.out_row] = from_float<TO>(__uint_as_float(r[j]));
                     }
                 }
-                __syncwarp();                  // a load of tensor memory is the whole warp's: lanes without a feature wait for the others
+                if (ragged) __syncwarp();
             }
         }
     }

@@ -125,6 +125,9 @@ gemm_bf16_tn_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __g
         if (ok) {
             const float bias = (p.bias && split == 0 && m < p.n_out) ? p.bias[m] : 0.0f;
             const int t0 = tile_n * BN;
+            // features end inside a warp: its lanes without one wait for the others, since a load of tensor memory is the whole warp's (a wait in every
+            // turn of every warp: 64 rows of 2,048 features 0.6 us more)
+            const bool ragged = p.n_out % 32 != 0 && tile_m * TC_BM + TC_BM > p.n_out;
 #pragma unroll 1
             for (int c = 0; c < BN; c += 16) {
                 if (t0 + c >= p.T) break;                                  // warp-uniform
@@ -148,7 +151,7 @@ gemm_bf16_tn_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __g
                             if (t0 + c + j < p.T) o[(size_t)j * p.ldo] = __float2bfloat16_rn(__uint_as_float(r[j]) + bias);
                     }
                 }
-                __syncwarp();                                              // (the next load of tensor memory is the whole warp's)
+                if (ragged) __syncwarp();
             }
         }
     }
