@@ -515,15 +515,22 @@ extern "C" int bg_conv_silu(const void* src, int src_dtype, int src_stride, int 
                     act, src_bias, nullptr, 0, launched, stream);
 }
 
-// The convolution without an activation and bg_rglru_split of its result in one kernel; BG_ERR_UNSUPPORTED, with nothing launched, where its rows are
-// not taken in runs.
+// The convolution without an activation and bg_rglru_split of its result: in one kernel where its rows are taken in runs, else one behind the other (from one
+// call: a step of few rows that asked for the first and then made two calls more took its host 94 us for 89).
+extern "C" int bg_rglru_split(const float* u, void* x2, int T, int W, int blocks, cudaStream_t stream);
 extern "C" int bg_conv_split(const void* src, int src_dtype, int src_stride, int col0, int channels, int taps, const void* w,
                              const void* b, int w_dtype, float* state, long long slot_stride, long long conv_off,
                              const int* slots, const int* row_req, const int* reqs, int n_req, float* out, int n_rows,
-                             const float* src_bias, void* x2, int blocks, cudaStream_t stream) {
+                             const float* src_bias, void* x2, int blocks, int* launched, cudaStream_t stream) {
     if (!x2) return BG_ERR_SHAPE;
-    return conv_run(src, src_dtype, src_stride, col0, channels, taps, w, b, w_dtype, state, slot_stride, conv_off, slots, row_req, reqs, n_req, out, n_rows,
-                    0, src_bias, x2, blocks, nullptr, stream);
+    int rc = conv_run(src, src_dtype, src_stride, col0, channels, taps, w, b, w_dtype, state, slot_stride, conv_off, slots, row_req, reqs, n_req, out, n_rows,
+                      0, src_bias, x2, blocks, launched, stream);
+    if (rc != BG_ERR_UNSUPPORTED) return rc;
+    rc = conv_run(src, src_dtype, src_stride, col0, channels, taps, w, b, w_dtype, state, slot_stride, conv_off, slots, row_req, reqs, n_req, out, n_rows,
+                  0, src_bias, nullptr, 0, launched, stream);
+    if (rc == BG_OK) rc = bg_rglru_split(out, x2, n_rows, channels, blocks, stream);
+    if (launched) ++*launched;
+    return rc;
 }
 
 // How the scan lays a head's state over CTAs: tiles of PT columns p, NS lanes per column (a power of two up to 32),

@@ -179,7 +179,7 @@ _SIGNATURES = {
     "bg_conv_silu": [_c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void_p, _c_void_p, _c_int, _c_void_p, _c_ll, _c_ll,
                      _c_void_p, _c_void_p, _c_void_p, _c_int, _c_void_p, _c_int, _c_int, _c_void_p, _c_void_p, _c_void_p],
     "bg_conv_split": [_c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void_p, _c_void_p, _c_int, _c_void_p, _c_ll, _c_ll,
-                      _c_void_p, _c_void_p, _c_void_p, _c_int, _c_void_p, _c_int, _c_void_p, _c_void_p, _c_int, _c_void_p],
+                      _c_void_p, _c_void_p, _c_void_p, _c_int, _c_void_p, _c_int, _c_void_p, _c_void_p, _c_int, _c_void_p, _c_void_p],
     "bg_ssm_scan": [_c_void_p, _c_int, _c_void_p, _c_int, _c_int, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_void_p,
                     _c_ll, _c_void_p, _c_void_p, _c_int, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_void_p],
     "bg_ssm_chunk_plan": [_c_int, _c_int, _c_int, _c_int, ctypes.POINTER(_c_int)],
@@ -1582,17 +1582,13 @@ def conv_silu(src: torch.Tensor, col0: int, channels: int, weight: torch.Tensor,
         if activation != "none" or split.dtype != torch.bfloat16 or not split.is_contiguous() or channels % blocks \
                 or tuple(split.shape) != (blocks, T, 2 * (channels // blocks)):
             raise KernelError("conv_silu: split is bfloat16 [blocks, T, 2 channels / blocks], without an activation")
-        with phase("conv"):
-            rc = lib().bg_conv_split(*args, _p(src_bias), _p(split), blocks, _stream())
-        if rc != _UNSUPPORTED:
-            _check(rc, "conv_split")
-            return
     n = _c_int(0)
     with phase("conv"):
-        _check(lib().bg_conv_silu(*args, 1 if activation == "silu" else 0, _p(src_bias), ctypes.byref(n), _stream()), "conv_silu")
+        if split is not None:
+            _check(lib().bg_conv_split(*args, _p(src_bias), _p(split), blocks, ctypes.byref(n), _stream()), "conv_split")
+        else:
+            _check(lib().bg_conv_silu(*args, 1 if activation == "silu" else 0, _p(src_bias), ctypes.byref(n), _stream()), "conv_silu")
     count_launches(n.value - 1)
-    if split is not None:
-        rglru_split(out, split.shape[0], split)
 
 
 def ssm_chunk(H: int, P: int, N: int, G: int) -> int:

@@ -45,3 +45,28 @@ def test_runs(taps, lens, w_dtype, bias):
     ops.conv_silu(to(src), 4, C, to(w), to(b), st2, 8, to(slots), to(row_req), to(reqs), R, silu, src_bias=to(sb))
     z = out.double()
     assert ((silu.double() - z * torch.sigmoid(z)).abs() <= 2.0 ** -21 * (z * torch.sigmoid(z)).abs() + 2.0 ** -126).all() and torch.equal(st, st2)
+
+
+@pytest.mark.parametrize("lens,C,blocks", [([1], 520, 2), ([5, 3], 520, 2), ([95], 520, 2), ([40] * 13, 520, 2), ([100], 516, 3), ([97], 35, 5), ([2] * 60, 64, 1)])
+def test_split_of_steps_that_are_not_taken_in_runs(lens, C, blocks):
+    """Few rows, many short requests, and sizes off 16 bytes: the convolution, its state and the split as kernels of their own, from the same call."""
+    from beglin_b200.csrc import ops
+    T, R, taps = sum(lens), len(lens), 4
+    g = torch.Generator().manual_seed(T)
+    rnd = lambda *n: torch.randn(*n, generator=g).to(DEV)
+    src, w, b, state = rnd(T, C + 12), rnd(C, taps), rnd(C), rnd(R, 3 * C)
+    starts = [sum(lens[:i]) for i in range(R)]
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    reqs, slots, row_req = i32([[i, s, n] for i, (s, n) in enumerate(zip(starts, lens))]), i32(list(range(R))), i32([i for i, n in enumerate(lens) for _ in range(n)])
+    outs = []
+    for split in (torch.full((blocks, T, 2 * C // blocks), float("nan"), dtype=torch.bfloat16, device=DEV), None):
+        st, out = state.clone(), torch.full((T, C), float("nan"), device=DEV)
+        before = ops.launch_count()
+        ops.conv_silu(src, 4, C, w, b, st, 0, slots, row_req, reqs, R, out, activation="none", split=split)
+        counted = ops.launch_count() - before
+        if split is None:
+            split = torch.empty_like(outs[0][2])
+            ops.rglru_split(out, blocks, split)
+            counted += 1
+        outs.append((out, st, split, counted))
+    assert all(torch.equal(x, y) for x, y in zip(outs[0][:3], outs[1][:3])) and outs[0][3] == outs[1][3] - (ops.lib().bg_conv_silu_run(T, R) > 1 and C % 4 == 0 and C // blocks % 4 == 0)
