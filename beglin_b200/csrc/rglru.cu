@@ -179,7 +179,7 @@ rglru_chunk_out_kernel(LruParams p, const int* __restrict__ chunks, const float*
 constexpr int LRU_BATCH = 4;
 __global__ void __launch_bounds__(LRU_THREADS)
 rglru_chunk_sums_vec2_kernel(LruParams p, const int* __restrict__ chunks, float* __restrict__ pq, float4* __restrict__ ab, int folded) {
-    pdl_launch();
+    if (!folded) pdl_launch();
     pdl_wait();
     const int c = (blockIdx.x * LRU_THREADS + threadIdx.x) * 2;
     if (c >= p.W) return;
@@ -211,6 +211,9 @@ rglru_chunk_sums_vec2_kernel(LruParams p, const int* __restrict__ chunks, float*
             Q.x = fmaf(v.x, Q.x, v.y); Q.y = fmaf(v.z, Q.y, v.w);
         }
     }
+    // (the kernel behind is the outputs', as many blocks as these: let in earlier, they crowd on the SMs that are free first.  2,560 channels, 64 chunks 61 us,
+    // so 52)
+    if (folded) pdl_launch();
     if (folded && (ch == 0 || chunks[(ch - 1) * 4] != chunks[ch * 4])) {       // a request's first chunk: its state, and the state behind the chunk
         const float* st = p.state + (size_t)p.slots[chunks[ch * 4]] * p.slot_stride + c;
         const float2 S = make_float2(st[0], st[1]);
@@ -222,7 +225,9 @@ rglru_chunk_sums_vec2_kernel(LruParams p, const int* __restrict__ chunks, float*
 }
 
 // FOLDED: the walk over a request's chunks is made by every chunk for itself, up to its own start, and the last one leaves the state.  For steps of
-// up to LRU_FOLDED chunks and few requests: a kernel less (2,048 rows of 4,096 channels 9.7 us), for reads from the second-level cache.
+// up to LRU_FOLDED chunks and few requests: a kernel less, for reads from the second-level cache that grow with the square of the chunks.  The recurrence's
+// kernels, us, apart and folded: one request of 1,024 channels 64 chunks 36.4 and 31.7, 128 65.7 and 48.7; 2,560 channels 54.3 and 51.6, 96.6 and 98.5; 4,096 75.5
+// and 69.4, 139 and 128; 8,192 131 and 122, 241 and 233; sixteen requests of eight chunks 52.3 and 43.6, 86.4 and 91.6, 125 and 119, 223 and 222.
 constexpr int LRU_FOLDED = 128, LRU_FOLDED_LONGS = 16;
 template <typename TO, bool FOLDED>
 __global__ void __launch_bounds__(LRU_THREADS)

@@ -164,6 +164,33 @@ def test_recurrence_in_chunks_two_channels_a_thread(W, blocks, dtype):
         assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1]) and not got[0][0].isnan().any()
 
 
+@pytest.mark.parametrize("lens", [[128 * 32], [128 * 32 + 1], [127 * 32, 5], [70 * 32, 59 * 32], [64] * 16, [64] * 17, [33] * 40 + [4000]])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_recurrence_on_both_sides_of_the_folded_walk(lens, dtype):
+    """128 and 129 chunks, sixteen requests and seventeen: the walk over the chunks inside the outputs' kernel and as one of its own, two channels a
+    thread, against one channel a thread, which always walks apart: the same bits out and in the state."""
+    from beglin_b200.engine.batch import cut_long_requests
+    o, g, W, blocks = ops(), torch.Generator().manual_seed(len(lens)), 24, 3
+    T, R = sum(lens), len(lens)
+    starts = [sum(lens[:i]) for i in range(R)]
+    rnd = lambda *n: torch.randn(*n, generator=g).to(DEV)
+    gates, u, y, br, bi = rnd(blocks, T, 2 * W // blocks), rnd(T, W), rnd(T, W), rnd(W), rnd(W)
+    decay, state0 = torch.rand(W, generator=g).to(DEV), rnd(R, W)
+    slots = torch.randperm(R, generator=g).to(DEV, torch.int32)
+    _, chunks, longs = cut_long_requests(starts, lens, 32, 1)
+    chunked = (torch.from_numpy(chunks).to(DEV), chunks.shape[0], torch.from_numpy(longs).to(DEV), longs.shape[0], 32)
+    got = []
+    for col in (4, 3):
+        src = torch.full((T, W + col), float("nan"), device=DEV)
+        src[:, col:] = y
+        state, out = state0.clone(), torch.full((T, W), float("nan"), dtype=dtype, device=DEV)
+        before = o.launch_count()
+        o.rglru_scan(gates, u, src, col, br, bi, decay, state, slots, None, 0, out, chunked=chunked)
+        got.append((out, state, o.launch_count() - before))
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1]) and not got[0][0].isnan().any()
+    assert got[1][2] == 3 and got[0][2] == (2 if chunks.shape[0] <= 128 and longs.shape[0] <= 16 else 3)
+
+
 def test_recurrence_keeps_a_far_token():
     """One token 900 rows back whose input gate is open while all others are shut: a decay of e^(-8 r softplus(lam)) per
     row with lam = -12 keeps it, lam = -4 fades it."""
