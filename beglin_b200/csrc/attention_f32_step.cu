@@ -3,16 +3,6 @@
 // cost the host 80 to 90 us for kernels of 55 to 75.
 #include "common.cuh"
 
-extern "C" {
-long long bg_gemm_f32_scratch(int, int, int, int);
-int bg_gemm_f32_nt(const float*, int, const float*, int, const float*, float*, int, int, int, int, int, float*, unsigned*, cudaStream_t);
-int bg_rope_kv_append(const void*, int, int, int, long long, void*, int, int, const float*, const int*, const int*, const int*, int, void*, int, int, int, int, int, int,
-                      int, int, int, unsigned*, cudaStream_t);
-int bg_attention_partial(const void*, int, int, const void*, int, int, int, const int*, int, const int*, const int*, int, float*, float*, int, int, int, int, int, int,
-                         int, int, int, int, float, float, int, const float*, int, unsigned*, cudaStream_t);
-int bg_attention_merge(const float*, const float*, const int*, void*, int, int, int, int, int, int, int, int, int, const float*, int, cudaStream_t);
-}
-
 // A layer's attention, float32, its plain form (heads of one size, no gates, no norms of queries and keys, a cache of its own in float32).  The host
 // side fills the fields by name.
 struct AttnF32Args {
@@ -46,6 +36,9 @@ struct Scratch {
 }  // namespace
 
 using namespace bg;
+
+// Bytes of what the host side mirrors field by field; it compares them when it loads the library.
+extern "C" int bg_attention_f32_bytes(int step) { return (int)(step ? sizeof(AttnF32Step) : sizeof(AttnF32Args)); }
 
 extern "C" long long bg_attention_f32_scratch(const AttnF32Args* a, int T, int n_splits) { return Scratch(*a, T, n_splits).floats; }
 

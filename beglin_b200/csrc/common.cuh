@@ -286,3 +286,5 @@ __device__ __forceinline__ float sum_parts(const T* p, int parts, size_t stride)
         else if ((code) == BG_DTYPE_BF16) { using T = __nv_bfloat16; __VA_ARGS__; } \
         else return BG_ERR_DTYPE;                                         \
     } while (0)
+
+#include "entries.cuh"

@@ -4,28 +4,6 @@
 // arguments and seven tensors in all, for kernels of 42; as one call 47 (host 29).
 #include "common.cuh"
 
-extern "C" {
-int bg_route_rows(const void*, int, int, const float*, int, int, int, int, int, int, const float*, float, const float*, int*, float*, int*, int*, int*, void*, int,
-                  cudaStream_t);
-int bg_route_layout(const void*, int, int, const float*, int, int, int, int, int, int, const float*, float, const float*, int*, float*, int*, int*, int*, void*, int,
-                    int*, int, cudaStream_t);
-int bg_route_layout_counts(int, int, int, int);
-int bg_route_layout_wins(int, int, int, int);
-int bg_route(const void*, int, int, const float*, int, int, int, int, int, int, const float*, float, const float*, int*, float*, float*, cudaStream_t);
-int bg_route_sort(const int*, int, int, int*, int*, int*, cudaStream_t);
-int bg_route_gather(const void*, int, const float*, const int*, void*, int, int, int, int, int, cudaStream_t);
-int bg_route_rows_takes(int, int, int, int);
-int bg_gemm_grouped_tc(const void*, int, int, int, int, const void*, int, int, void*, int, int, const int*, int, unsigned*, cudaStream_t);
-int bg_gemm_grouped_pair(const void*, int, int, int, int, const void*, int, int, void*, int, int, const int*, int, unsigned*, cudaStream_t);
-int bg_glu_clamped(const void*, int, int, void*, int, int, int, float, float, cudaStream_t);
-int bg_swiglu(const void*, int, int, long long, void*, int, int, int, int, int, float, cudaStream_t);
-int bg_gemm_fused(const void*, int, int, int, const void*, int, const float*, int, const float*, int, int, const void*, float, int, const float*, int, void*, int,
-                  int, float*, int, int, float, unsigned*, cudaStream_t);
-int bg_route_combine(const void*, int, const float*, const int*, float*, int, int, int, int, cudaStream_t);
-int bg_route_combine_ext(const void*, int, const float*, const int*, const int*, int, const void*, int, int, const float*, const void*, int, int, float*, int, int,
-                         int, cudaStream_t);
-}
-
 // A layer's experts, bfloat16: what does not change from step to step.  The host side fills the fields by name.
 struct ExpertsArgs {
     const float* router; const float* choice_bias; const float* logit_bias;    // [outputs][hidden], [outputs] or null
@@ -77,6 +55,9 @@ int total(const ExpertsArgs& a, const Scratch& s, char* w, const void* h, int T,
 }  // namespace
 
 using namespace bg;
+
+// Bytes of what the host side mirrors field by field; it compares them when it loads the library.
+extern "C" int bg_experts_bytes() { return (int)sizeof(ExpertsArgs); }
 
 // -1 where bg_experts_step does not take a step of T tokens (on 16 bytes): to be asked before anything is made for it.  inside: whether the shared
 // expert's products run in the call (with up_splits).

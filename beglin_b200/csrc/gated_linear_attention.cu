@@ -784,6 +784,9 @@ struct GlaArgs {
     void* out; int out_dtype, H, n, nv;
 };
 
+// Bytes of what the host side mirrors field by field; it compares them when it loads the library.
+extern "C" int bg_gla_bytes() { return (int)sizeof(GlaArgs); }
+
 static int gla_params(GlaParams& p, const GlaArgs* a) {
     if (a->H <= 0 || a->n <= 0 || a->nv <= 0 || a->H > 65535 || (a->forget ? !a->lower : (!a->wa || a->rank < 1)) || !a->bias || !a->norm_w) return BG_ERR_SHAPE;
     if (a->out_dtype != BG_DTYPE_F32 && a->out_dtype != BG_DTYPE_BF16) return BG_ERR_DTYPE;

@@ -134,7 +134,6 @@ extern "C" int bg_gemm_f32_nt_batched(const float* A, int lda, long long batch_a
 // rows in turns of `block`, or halves), down [hidden, ff], both one row behind the other; act and limit as bg_swiglu's.  (silu made where the down
 // product cuts its tokens, a kernel less, was no gain: 550 x 1,536 by 8,960 246.6 us and 248, 8 rows 60.5 and 53, whose down product has less time
 // to fetch its weights ahead.)
-extern "C" int bg_swiglu(const void*, int, int, long long, void*, int, int, int, int, int, float, cudaStream_t);
 extern "C" long long bg_mlp_f32_scratch(int T, int hidden, int ff) {
     const long long a = bg_gemm_f32_scratch(T, 2 * ff, hidden, 1), b = bg_gemm_f32_scratch(T, hidden, ff, 1);
     return 3LL * T * ff + (a > b ? a : b);

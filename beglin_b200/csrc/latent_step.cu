@@ -3,21 +3,6 @@
 // 150 us a step (thirteen tensors, four views, nine entries with their checks) for kernels of 45 to 140.
 #include "common.cuh"
 
-extern "C" {
-int bg_gemm_fused(const void*, int, int, int, const void*, int, const float*, int, const float*, int, int, const void*, float, int, const float*, int, void*, int,
-                  int, float*, int, int, float, unsigned*, cudaStream_t);
-int bg_gemm_bf16_tn(const void*, int, int, int, const void*, int, int, const float*, void*, int, int, int, unsigned*, cudaStream_t);
-int bg_gemm_heads(const void*, int, int, int, const void*, long long, int, int, int, int, int, void*, int, long long, int, const void*, int, int, int, int, unsigned*,
-                  cudaStream_t);
-int bg_latent_append(const void*, int, int, int, int, int, int, const void*, int, float, const float*, const int*, const int*, const int*, int, void*, int, int, int, int,
-                     unsigned*, int, int, const void*, void*, int, cudaStream_t);
-int bg_latent_attention_tc_partial(const float*, long long, int, const void*, int, int, int, const float*, const void*, int, int, const int*, int, const int*, const int*,
-                                   int, float*, float*, int, int, int, int, int, int, float, unsigned*, cudaStream_t);
-int bg_latent_attention_mma_partial(const float*, long long, int, const void*, int, int, int, const float*, const void*, int, int, const int*, int, const int*, const int*,
-                                    int, float*, float*, int, int, int, int, int, int, int, int, int, int, int, float, unsigned*, cudaStream_t);
-int bg_latent_attention_merge(const float*, const float*, const int*, void*, int, long long, int, int, int, int, int, int, int, const float*, int, cudaStream_t);
-}
-
 // A layer's attention, bfloat16: what does not change from step to step.  The host side fills the fields by name.
 struct LatentArgs {
     const void* down; const void* q_up; const void* k_up_t; const void* v_up;      // [n_down][hidden], [heads (dim + rot)][q_rank], [heads][kv_rank][dim], [heads][vdim][kv_rank]
@@ -58,6 +43,9 @@ int product(const void* W, int n_out, int K, const void* X, int ldx, int T, void
 }  // namespace
 
 using namespace bg;
+
+// Bytes of what the host side mirrors field by field; it compares them when it loads the library.
+extern "C" int bg_latent_bytes(int step) { return (int)(step ? sizeof(LatentStep) : sizeof(LatentArgs)); }
 
 extern "C" long long bg_latent_step_scratch(const LatentArgs* a, int T, int n_splits) { return (long long)Scratch(*a, T, n_splits).bytes; }
 

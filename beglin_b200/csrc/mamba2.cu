@@ -517,7 +517,6 @@ extern "C" int bg_conv_silu(const void* src, int src_dtype, int src_stride, int 
 
 // The convolution without an activation and bg_rglru_split of its result: in one kernel where its rows are taken in runs, else one behind the other (from one
 // call: a step of few rows that asked for the first and then made two calls more took its host 94 us for 89).
-extern "C" int bg_rglru_split(const float* u, void* x2, int T, int W, int blocks, cudaStream_t stream);
 extern "C" int bg_conv_split(const void* src, int src_dtype, int src_stride, int col0, int channels, int taps, const void* w,
                              const void* b, int w_dtype, float* state, long long slot_stride, long long conv_off,
                              const int* slots, const int* row_req, const int* reqs, int n_req, float* out, int n_rows,

@@ -3,16 +3,6 @@
 // step those cost the host some 65 us beside the products' 28, for kernels of 30 to 40 in portions of a few hundred rows.
 #include "common.cuh"
 
-extern "C" {
-int bg_conv_silu(const void*, int, int, int, int, int, const void*, const void*, int, float*, long long, long long, const int*, const int*, const int*, int, float*, int,
-                 int, const float*, int*, cudaStream_t);
-int bg_ssm_scan(const float*, int, const void*, int, int, int, const void*, const void*, const void*, int, float*, long long, const int*, const int*, int, float*, int, int,
-                int, int, cudaStream_t);
-int bg_ssm_chunked(const float*, int, const void*, int, int, int, const void*, const void*, const void*, int, float*, long long, const int*, const int*, int, const int*,
-                   int, float*, float*, float*, float*, int, int, int, int, int, unsigned*, cudaStream_t);
-int bg_gated_group_rmsnorm(const float*, const void*, int, int, int, const void*, int, float, void*, int, int, int, int, int, cudaStream_t);
-}
-
 // What does not change from step to step; the host side fills the fields by name.
 struct Mamba2Args {
     const void* conv_w; const void* conv_b; const void* dt_bias; const void* A_log; const void* D; const void* norm_w; unsigned* status;
@@ -43,6 +33,9 @@ struct Scratch {
 }  // namespace
 
 using namespace bg;
+
+// Bytes of what the host side mirrors field by field; it compares them when it loads the library.
+extern "C" int bg_mamba2_bytes(int step) { return (int)(step ? sizeof(Mamba2Step) : sizeof(Mamba2Args)); }
 
 extern "C" long long bg_mamba2_scratch(const Mamba2Args* a, int T, int n_chunks) { return (long long)Scratch(*a, T, n_chunks).bytes; }
 

@@ -81,6 +81,11 @@ _SIGNATURES = {
     "bg_experts_scratch": [_c_void_p, _c_int, _c_int],
     "bg_experts_step": [_c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_void_p, _c_ll, _c_void_p, _c_void_p, _c_void_p],
     "bg_experts_sum": [_c_void_p, _c_void_p, _c_int, _c_void_p, _c_void_p, _c_int, _c_int, _c_void_p, _c_ll, _c_void_p, _c_void_p],
+    "bg_attention_f32_bytes": [_c_int],
+    "bg_latent_bytes": [_c_int],
+    "bg_mamba2_bytes": [_c_int],
+    "bg_experts_bytes": [],
+    "bg_gla_bytes": [],
     "bg_route_sort": [_c_void_p, _c_int, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_void_p],
     "bg_route_gather": [_c_void_p, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void_p],
     "bg_route_combine": [_c_void_p, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_void_p],
@@ -218,6 +223,11 @@ def lib():
                 raise KernelError(f"the kernel library lacks '{name}'") from e
             fn.argtypes = argtypes
             fn.restype = _RESULTS.get(name, _c_int)
+        for cls, name, which in ((AttnF32Args, "bg_attention_f32_bytes", (0,)), (AttnF32Step, "bg_attention_f32_bytes", (1,)), (LatentArgs, "bg_latent_bytes", (0,)),
+                                 (LatentStep, "bg_latent_bytes", (1,)), (Mamba2Args, "bg_mamba2_bytes", (0,)), (Mamba2Step, "bg_mamba2_bytes", (1,)),
+                                 (ExpertsArgs, "bg_experts_bytes", ()), (_GlaArgs, "bg_gla_bytes", ())):
+            if getattr(handle, name)(*which) != ctypes.sizeof(cls):
+                raise KernelError(f"the kernel library's {cls.__name__} has another size than its mirror here")
         _lib = handle
     return _lib
 

@@ -9,9 +9,6 @@
 #include "common.cuh"
 
 // The two-stage sampler of sampling.cu, which takes its scratch from the caller.
-extern "C" int bg_sample(const float* logits, int n, int V, const float* temperature, const float* uniform, int* out,
-                         void* scratch, cudaStream_t stream);
-extern "C" long long bg_sample_scratch_bytes(int n);
 
 namespace {
 
