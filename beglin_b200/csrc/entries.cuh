@@ -66,19 +66,12 @@ int bg_ssm_chunked(const float* xbc, int channels, const void* src, int src_dtyp
     void* D, int w_dtype, float* state, long long slot_stride, const int* slots, const int* chunks, int n_chunks, const int* longs, int n_long, float* scores,
     float* work, float* decay, float* y, int H, int P, int N, int G, int tensor_cores, unsigned* status, cudaStream_t stream);
 // moe.cu
-int bg_route(const void* h, int h_dtype, int ldh, const float* W, int T, int d, int E, int top, int mode, int renorm, const float* bias, float scale, const
-    float* logit_bias, int* ids, float* weights, float* logits_out, cudaStream_t stream);
 int bg_route_layout_counts(int T, int d, int E, int top);
 int bg_route_layout_wins(int T, int d, int E, int top);
 int bg_route_rows_takes(int T, int d, int E, int top);
-int bg_route_layout(const void* h, int h_dtype, int ldh, const float* W, int T, int d, int E, int top, int mode, int renorm, const float* bias, float scale,
-    const float* logit_bias, int* ids, float* weights, int* offsets, int* row_of, int* src_of, void* xp, int scale_input, int* hist, int n_hist, cudaStream_t
-    stream);
-int bg_route_rows(const void* h, int h_dtype, int ldh, const float* W, int T, int d, int E, int top, int mode, int renorm, const float* bias, float scale,
-    const float* logit_bias, int* ids, float* weights, int* offsets, int* row_of, int* src_of, void* xp, int scale_input, cudaStream_t stream);
-int bg_route_sort(const int* ids, int A, int E, int* offsets, int* row_of, int* src_of, cudaStream_t stream);
-int bg_route_gather(const void* x, int x_dtype, const float* weights, const int* src_of, void* xp, int xp_dtype, int A, int d, int top, int scale,
-    cudaStream_t stream);
+int bg_route_place(const void* h, int h_dtype, int ldh, const float* W, int T, int d, int E, int top, int mode, int renorm, const float* bias, float scale,
+    const float* logit_bias, int* ids, float* weights, int* offsets, int* row_of, int* src_of, void* xp, int scale_input, int* hist, int n_hist, int*
+    launched, cudaStream_t stream);
 int bg_route_combine(const void* yp, int y_dtype, const float* weights, const int* row_of, float* out, int T, int d, int top, int scale, cudaStream_t stream);
 int bg_route_combine_ext(const void* yp, int y_dtype, const float* weights, const int* row_of, const int* ids, int n_real, const void* h, int h_dtype, int
     ldh, const float* shared, const void* sg, int sg_dtype, int sg_stride, float* out, int T, int d, int top, cudaStream_t stream);

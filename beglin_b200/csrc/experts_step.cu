@@ -23,13 +23,11 @@ namespace {
 struct Scratch {
     size_t ids, weights, offsets, row_of, src_of, counts, xp, gu, hp, yp, shared_gu, shared_act, shared_out, bytes;
     int n_counts;
-    bool rows;                 // routing, layout and gather as one kernel, with n_counts as two, else as three
     Scratch(const ExpertsArgs& a, int T, bool inside) {        // inside: the shared expert's products run in the call
         const size_t A = (size_t)T * a.top;
         size_t at = 0;
         auto take = [&](size_t n) { const size_t p = at; at += (n + 255) & ~(size_t)255; return p; };
-        rows = T <= a.few && bg_route_rows_takes(T, a.hidden, a.outputs, a.top);
-        n_counts = rows ? 0 : bg_route_layout_wins(T, a.hidden, a.outputs, a.top);
+        n_counts = bg_route_layout_wins(T, a.hidden, a.outputs, a.top);
         ids = take(A * 4); weights = take(A * 4); offsets = take((size_t)(a.outputs + 1) * 4); row_of = take(A * 4); src_of = take(A * 4);
         counts = take((size_t)n_counts * 4);
         xp = take(A * a.hidden * 2);
@@ -87,20 +85,8 @@ extern "C" int bg_experts_step(const ExpertsArgs* args, const void* h, int T, in
     int* row_of = (int*)(w + s.row_of); int* src_of = (int*)(w + s.src_of);
     const int A = T * a.top, F = BG_DTYPE_F32, B = BG_DTYPE_BF16;
     int rc, n = 0;
-    if (s.rows) {
-        rc = bg_route_rows(h, B, a.hidden, a.router, T, a.hidden, a.outputs, a.top, a.mode, a.renorm, a.choice_bias, a.route_scale, a.logit_bias, ids, weights,
-                           offsets, row_of, src_of, w + s.xp, a.scale_input, stream);
-        n = 1;
-    } else if (s.n_counts) {
-        rc = bg_route_layout(h, B, a.hidden, a.router, T, a.hidden, a.outputs, a.top, a.mode, a.renorm, a.choice_bias, a.route_scale, a.logit_bias, ids, weights,
-                             offsets, row_of, src_of, w + s.xp, a.scale_input, (int*)(w + s.counts), s.n_counts, stream);
-        n = 2;
-    } else {
-        rc = bg_route(h, B, a.hidden, a.router, T, a.hidden, a.outputs, a.top, a.mode, a.renorm, a.choice_bias, a.route_scale, a.logit_bias, ids, weights, nullptr, stream);
-        if (rc == BG_OK) rc = bg_route_sort(ids, A, a.outputs, offsets, row_of, src_of, stream);
-        if (rc == BG_OK) rc = bg_route_gather(h, B, weights, src_of, w + s.xp, B, A, a.hidden, a.top, a.scale_input, stream);
-        n = 3;
-    }
+    rc = bg_route_place(h, B, a.hidden, a.router, T, a.hidden, a.outputs, a.top, a.mode, a.renorm, a.choice_bias, a.route_scale, a.logit_bias, ids, weights, offsets,
+                        row_of, src_of, w + s.xp, a.scale_input, (int*)(w + s.counts), s.n_counts, &n, stream);
     if (rc != BG_OK) return rc;
     auto grouped = pairs ? bg_gemm_grouped_pair : bg_gemm_grouped_tc;
     auto gate = [&](const void* gu, int dtype, int ld, void* to, int rows, int cols, float limit, int block) {

@@ -892,6 +892,32 @@ extern "C" int bg_route_gather(const void* x, int x_dtype, const float* weights,
     return BG_OK;
 }
 
+// Routing, layout and gather of a step from one call: as one kernel (bg_route_rows), as two (bg_route_layout, with `n_hist` integers of scratch that are
+// bg_route_layout_wins of the sizes or more) or as three, whichever takes the step and is no slower.  `launched` counts the kernels.
+extern "C" int bg_route_place(const void* h, int h_dtype, int ldh, const float* W, int T, int d, int E, int top, int mode, int renorm,
+                              const float* bias, float scale, const float* logit_bias, int* ids, float* weights, int* offsets, int* row_of,
+                              int* src_of, void* xp, int scale_input, int* hist, int n_hist, int* launched, cudaStream_t stream) {
+    int n = 0, rc = BG_ERR_UNSUPPORTED;
+    if (launched) *launched = 0;
+    if (T <= 0) return BG_OK;
+    if (bg_route_rows_takes(T, d, E, top)) {
+        rc = bg_route_rows(h, h_dtype, ldh, W, T, d, E, top, mode, renorm, bias, scale, logit_bias, ids, weights, offsets, row_of, src_of, xp, scale_input, stream);
+        n = 1;
+    }
+    if (rc == BG_ERR_UNSUPPORTED && bg_route_layout_wins(T, d, E, top)) {
+        rc = bg_route_layout(h, h_dtype, ldh, W, T, d, E, top, mode, renorm, bias, scale, logit_bias, ids, weights, offsets, row_of, src_of, xp, scale_input, hist, n_hist, stream);
+        n = 2;
+    }
+    if (rc == BG_ERR_UNSUPPORTED) {
+        rc = bg_route(h, h_dtype, ldh, W, T, d, E, top, mode, renorm, bias, scale, logit_bias, ids, weights, nullptr, stream);
+        if (rc == BG_OK) rc = bg_route_sort(ids, T * top, E, offsets, row_of, src_of, stream);
+        if (rc == BG_OK) rc = bg_route_gather(h, h_dtype, weights, src_of, xp, h_dtype, T * top, d, top, scale_input, stream);
+        n = 3;
+    }
+    if (launched) *launched = rc == BG_OK ? n : 0;
+    return rc;
+}
+
 extern "C" int bg_route_combine(const void* yp, int y_dtype, const float* weights, const int* row_of, float* out, int T, int d,
                                 int top, int scale, cudaStream_t stream) {
     if (T <= 0) return BG_OK;

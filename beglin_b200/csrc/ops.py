@@ -76,6 +76,8 @@ _SIGNATURES = {
                       _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_void_p],
     "bg_route_layout": [_c_void_p, _c_int, _c_int, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void_p, _c_float, _c_void_p,
                         _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_void_p, _c_int, _c_void_p],
+    "bg_route_place": [_c_void_p, _c_int, _c_int, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void_p, _c_float, _c_void_p,
+                       _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_void_p, _c_int, _c_void_p, _c_void_p],
     "bg_route_layout_counts": [_c_int, _c_int, _c_int, _c_int],
     "bg_route_layout_wins": [_c_int, _c_int, _c_int, _c_int],
     "bg_experts_scratch": [_c_void_p, _c_int, _c_int],
@@ -2128,6 +2130,18 @@ def route_layout(h: torch.Tensor, router: torch.Tensor, top: int, ids: torch.Ten
                             scale, logit_bias)
 
 
+def route_place(h: torch.Tensor, router: torch.Tensor, top: int, ids: torch.Tensor, weights: torch.Tensor, offsets: torch.Tensor,
+                row_of: torch.Tensor, src_of: torch.Tensor, out: torch.Tensor, scale_input: bool, counts: Optional[torch.Tensor] = None, sigmoid=True,
+                renorm: bool = False, bias: Optional[torch.Tensor] = None, scale: float = 1.0,
+                logit_bias: Optional[torch.Tensor] = None) -> bool:
+    """`route`, `route_sort` and `route_gather` (out of h's type) of any step from one call, as one kernel, two (with `route_layout_wins` integers
+    of `counts` as scratch) or three; False, with nothing done, where h or out is not of their form."""
+    if counts is not None:
+        _i32(counts, "counts")
+    return _route_and_place("route_place", h, router, top, ids, weights, offsets, row_of, src_of, out, scale_input, counts, sigmoid, renorm, bias,
+                            scale, logit_bias)
+
+
 def _route_and_place(what, h, router, top, ids, weights, offsets, row_of, src_of, out, scale_input, counts, sigmoid, renorm, bias, scale,
                      logit_bias) -> bool:
     T, d = h.shape
@@ -2147,15 +2161,18 @@ def _route_and_place(what, h, router, top, ids, weights, offsets, row_of, src_of
     with phase("router"):
         args = (_p(h), _dt(h), h.stride(0), _p(router), T, d, E, top, rule, 1 if renorm else 0, _p(bias), float(scale), _p(logit_bias), _p(ids),
                 _p(weights), _p(offsets), _p(row_of), _p(src_of), _p(out), 1 if scale_input else 0)
-        if counts is None:
+        n = _c_int(1)
+        if what == "route_rows":
             rc = lib().bg_route_rows(*args, _stream())
-        else:
+        elif what == "route_layout":
+            n.value = 2
             rc = lib().bg_route_layout(*args, _p(counts), counts.numel(), _stream())
+        else:
+            rc = lib().bg_route_place(*args, _p(counts), 0 if counts is None else counts.numel(), ctypes.byref(n), _stream())
         if rc == _UNSUPPORTED:
             return False
         _check(rc, what)
-    if counts is not None:
-        count_launches(1)
+    count_launches(n.value - 1)
     return True
 
 

@@ -117,7 +117,7 @@ class RoutedExperts:
                 rows += [w, torch.zeros((7, w.shape[1]), dtype=w.dtype, device=w.device)]
             self.shared_up = Linear(torch.cat(rows, dim=0), None, ctx, label="proj_gate_up")
             self.shared_down = Linear(tensors["shared.down.weight"], None, ctx, label="proj_down")
-        self._args, self._scratch = self._step_args(outputs), {}
+        self._args, self._scratch, self._counts = self._step_args(outputs), {}, {}      # (sizes by the number of tokens)
 
     def _step_args(self, outputs: int):
         """The layer as the one-call step takes it (bfloat16, inner sizes of whole 16-byte pieces), or None."""
@@ -188,15 +188,18 @@ class RoutedExperts:
         s, dev, ct = self.spec, h.device, self.ctx.compute_dtype
         T, A = h.shape[0], h.shape[0] * s.top
         outputs = s.experts + s.identity
-        few = T <= ops.ROUTE_ROWS_TOKENS
-        counts = 0 if few else ops.route_layout_wins(T, s.hidden, outputs, s.top)
+        counts = self._counts.get(T)
+        if counts is None:
+            if len(self._counts) >= 4096:
+                self._counts.clear()
+            counts = self._counts[T] = ops.route_layout_wins(T, s.hidden, outputs, s.top)
         ints = torch.empty((3 * A + outputs + 1 + counts,), dtype=torch.int32, device=dev)
         ids, row_of, src_of, offsets = ints[:A].view(T, s.top), ints[A:2 * A], ints[2 * A:3 * A], ints[3 * A:3 * A + outputs + 1]
         weights = torch.empty((T, s.top), dtype=torch.float32, device=dev)
         xp = torch.empty((A, s.hidden), dtype=ct, device=dev)
         how = dict(sigmoid=s.router_activation, renorm=s.renormalize, bias=self.choice_bias, scale=s.route_scale, logit_bias=self.logit_bias)
         place = (h, self.router, s.top, ids, weights, offsets, row_of, src_of, xp, s.scale_input)
-        if not (ops.route_rows(*place, **how) if few else counts and ops.route_layout(*place, ints[3 * A + outputs + 1:], **how)):
+        if not (ops.route_rows(*place, **how) if T <= ops.ROUTE_ROWS_TOKENS else ops.route_place(*place, ints[3 * A + outputs + 1:] if counts else None, **how)):
             ops.route(h, self.router, s.top, ids, weights, **how)
             ops.route_sort(ids.view(-1), outputs, offsets, row_of, src_of)
             ops.route_gather(h, weights.view(-1), src_of, xp, s.top, scale=s.scale_input)

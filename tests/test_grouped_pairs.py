@@ -120,3 +120,29 @@ def test_routing_of_many_tokens_refuses_what_it_does_not_take(ops):
         assert not ops.route_layout(h, W, 2, ids, torch.zeros((T, 2), device=DEV), i32(E + 1), i32(2 * T), i32(2 * T), torch.empty((2 * T, d), device=DEV),
                                     False, i32(n))
         assert (ids == -7).all()
+
+
+@pytest.mark.parametrize("T,E,top,d,kernels", [(8, 10, 2, 64, 1), (9, 10, 2, 64, 3), (64, 40, 3, 1024, 2), (200, 40, 3, 1024, 3), (300, 40, 3, 1024, 2), (2000, 40, 3, 1024, 3),
+                                               (5, 9, 2, 36, 3), (40, 300, 2, 1024, 3), (3, 1100, 2, 64, 3)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_routing_from_one_call(ops, T, E, top, d, kernels, dtype):
+    """One, two or three kernels, whichever take the step: the same choices and weights, a layout in which every expert holds its rows, those rows."""
+    g = torch.Generator().manual_seed(T + E)
+    h, W = torch.randn(T, d, generator=g).to(DEV, dtype), torch.randn(E, d, generator=g).to(DEV)
+    i32 = lambda *n: torch.full(n, -7, dtype=torch.int32, device=DEV)
+    A = T * top
+    ids, weights, offsets, row_of, src_of = i32(T, top), torch.zeros((T, top), device=DEV), i32(E + 1), i32(A), i32(A)
+    xp = torch.full((A, d), float("nan"), dtype=dtype, device=DEV)
+    before = ops.launch_count()
+    assert ops.route_place(h, W, top, ids, weights, offsets, row_of, src_of, xp, True, i32(ops.route_layout_wins(T, d, E, top)), sigmoid="sigmoid")
+    assert ops.launch_count() - before == kernels
+    ids2, weights2, xp2 = i32(T, top), torch.zeros((T, top), device=DEV), torch.full_like(xp, float("nan"))
+    ops.route(h, W, top, ids2, weights2, sigmoid="sigmoid")
+    assert torch.equal(ids, ids2) and torch.equal(weights, weights2)
+    chosen = ids.view(-1).long()
+    assert torch.equal(offsets.long(), torch.cat([torch.zeros(1, device=DEV), torch.bincount(chosen, minlength=E).cumsum(0)]).long())
+    assert torch.equal(torch.sort(src_of).values.long(), torch.arange(A, device=DEV)) and torch.equal(row_of[src_of.long()].long(), torch.arange(A, device=DEV))
+    starts = offsets.long()
+    assert ((row_of.long() >= starts[chosen]) & (row_of.long() < starts[chosen + 1])).all()
+    ops.route_gather(h, weights.view(-1), src_of, xp2, top, scale=True)
+    assert torch.equal(xp, xp2)
