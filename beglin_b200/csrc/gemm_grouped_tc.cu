@@ -114,25 +114,29 @@ gemm_grouped_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __g
         if (!ok) atomicExch(&failed, 1);
         tc_fence_after();
         if (ok) {
-            const bool ragged = p.n_out % 32 != 0 && tile_m * TC_BM + TC_BM > p.n_out;         // lanes without a feature wait for the others: a load of tensor memory is the whole warp's
+            // where features end inside a warp, lanes without one wait for the others, since a load of tensor memory is the whole warp's
+            auto drain = [&](auto wait) {
 #pragma unroll 1
-            for (int c = 0; c < BN; c += 16) {
-                if (c >= n_rows) break;                                  // warp-uniform
-                unsigned r[16];
-                tc_ld16(tmem_base + ((unsigned)(quarter * 32) << 16) + (unsigned)c, r);
-                if (m < p.n_out) {
+                for (int c = 0; c < BN; c += 16) {
+                    if (c >= n_rows) break;                                  // warp-uniform
+                    unsigned r[16];
+                    tc_ld16(tmem_base + ((unsigned)(quarter * 32) << 16) + (unsigned)c, r);
+                    if (m < p.n_out) {
 #pragma unroll
-                    for (int j = 0; j < 16; ++j) {
-                        if (c + j >= n_rows) break;
-                        float v = __uint_as_float(r[j]);
-                        if (p.act == 1) { v = fmaxf(v, 0.0f); v *= v; }
-                        const size_t o = (size_t)(row0 + c + j) * p.ldo + m;
-                        if (p.out_dtype == BG_DTYPE_F32) ((float*)p.out)[o] = v;
-                        else ((__nv_bfloat16*)p.out)[o] = __float2bfloat16_rn(v);
+                        for (int j = 0; j < 16; ++j) {
+                            if (c + j >= n_rows) break;
+                            float v = __uint_as_float(r[j]);
+                            if (p.act == 1) { v = fmaxf(v, 0.0f); v *= v; }
+                            const size_t o = (size_t)(row0 + c + j) * p.ldo + m;
+                            if (p.out_dtype == BG_DTYPE_F32) ((float*)p.out)[o] = v;
+                            else ((__nv_bfloat16*)p.out)[o] = __float2bfloat16_rn(v);
+                        }
                     }
+                    if constexpr (decltype(wait)::value) __syncwarp();
                 }
-                if (ragged) __syncwarp();
-            }
+            };
+            if (p.n_out % 32 != 0 && tile_m * TC_BM + TC_BM > p.n_out) drain(std::true_type{});
+            else drain(std::false_type{});
         }
     }
     tc_fence_before();
