@@ -9,7 +9,7 @@
 //                  src_of[row] the assignment that row holds.  ONE CTA; the order inside an expert is whatever the
 //                  atomics give, which no result depends on (a row's product is a function of that row alone).
 //   route_rows     the three above and below for a step of few tokens in one kernel, a cluster of CTAs.
-//   route_place    route_sort and route_gather in one kernel, from counts that the router's kernel leaves.
+//   route_place    route_sort and route_gather in one kernel, from counts that the router's kernel leaves: for many outputs.
 //   route_gather   xp[row] = (weight * x[token]) rounded to the compute type (or x[token] as it is).
 //   gemm_grouped   yp[row] = act(xp[row] W[e]^T) on CUDA cores, float accumulation, every output summed over k in index
 //                  order by one thread: the float32 path, and the sizes the tensor-core product does not take.
@@ -239,8 +239,8 @@ route_vec8_kernel(const TI* __restrict__ h, int ldh, const float* __restrict__ W
 // What route_sort and route_gather do, for the same blocks of `tokens` tokens as the router's kernel ahead, from its counts: every block adds up the
 // counts (RL_MAX of them at most) for itself, so an expert's rows begin behind those of smaller experts, a block's behind those of the
 // blocks before it, and inside a block they stand in the order of the assignments.  No atomics: the order is the same every time.
-// gridDim.y blocks share the columns of a block's rows.  Bound by bytes and by the chain of counts, prefix and rows in front of them (2,048
-// tokens, two of 8 experts, 1,536 features: sort and gather 11.4 us -> 9.0; the whole case of perf/cases.py 122 -> 116).
+// gridDim.y blocks share the columns of a block's rows.  Bound by bytes and by the chain of counts, prefix and rows in front of them
+// (bg_route_layout_wins says where that chain is worth the sort that it saves).
 constexpr int RL_MAX = 8192, RL_MAX_E = 256, RL_MAX_A = 512;
 template <typename TI>
 __global__ void __launch_bounds__(256)
